@@ -133,6 +133,83 @@ VESIN_API int vesin_b200_neighbors_batch_f32(
     const char** error_message
 );
 
+/*
+ * No counterpart in the reference, whose lists live in arrays of the library:
+ * builds that write into arrays of the CALLER, so that a caller that wants to
+ * own the result (a framework with its own allocator) does not copy a list out
+ * of the library's arrays before the next call overwrites them.
+ *
+ * `arrays` names the output arrays, device memory that holds `capacity` pairs
+ * each; arrays that are NULL are not written (options.return_* are ignored). The
+ * indices go to `pairs`, or, when that is NULL, to `i` and `j` (one array each).
+ * When the list has more than `capacity` pairs, `allocate(context, n_pairs,
+ * arrays)` is called on the calling thread: it replaces the pointers and sets
+ * `capacity` to at least n_pairs, and returns 0 (anything else is an allocation
+ * failure). Nothing of the old arrays is kept. Start with capacity 0 when the
+ * number of pairs is not known; a good guess is what the last list had. On
+ * return *length is the number of pairs, and `neighbors` holds no pairs: it
+ * keeps the workspace and is passed again next time.
+ *
+ * Everything else (which pairs, argument checks, errors, completeness on
+ * return) as vesin_neighbors, vesin_b200_neighbors_f32
+ * (VESIN_B200_FLOAT32: points and box are float arrays, `distances` and
+ * `vectors` too), vesin_b200_neighbors_canonical (VESIN_B200_CANONICAL) and
+ * vesin_b200_neighbors_batch. Arrays must be aligned to their elements (`pairs`
+ * to 16 bytes); full lists are written fastest when `pairs` is aligned to 32
+ * bytes and the others to 16.
+ */
+struct VesinB200Arrays {
+    size_t capacity;
+    size_t* i;
+    size_t* j;
+    size_t (*pairs)[2];
+    int32_t (*shifts)[3];
+    void* distances;
+    void* vectors;
+};
+
+typedef int (*VesinB200Allocate)(void* context, size_t n_pairs, struct VesinB200Arrays* arrays);
+
+#define VESIN_B200_FLOAT32 1
+#define VESIN_B200_CANONICAL 2
+
+VESIN_API int vesin_b200_neighbors_into(
+    const void* points,
+    size_t n_points,
+    const void* box,
+    const bool periodic[3],
+    struct VesinDevice device,
+    struct VesinOptions options,
+    int flags,
+    struct VesinNeighborList* neighbors,
+    struct VesinB200Arrays* arrays,
+    VesinB200Allocate allocate,
+    void* context,
+    size_t* length,
+    const char** error_message
+);
+
+/* `pair_offsets` is the caller's array too: device memory, n_systems + 1
+ * entries. Only VESIN_B200_FLOAT32 is a valid flag. */
+VESIN_API int vesin_b200_neighbors_batch_into(
+    const void* points,
+    const size_t* system_offsets,
+    size_t n_systems,
+    const void* boxes,
+    const bool (*periodic)[3],
+    struct VesinDevice device,
+    struct VesinOptions options,
+    int flags,
+    bool global_indices,
+    struct VesinNeighborList* neighbors,
+    struct VesinB200Arrays* arrays,
+    VesinB200Allocate allocate,
+    void* context,
+    size_t* pair_offsets,
+    size_t* length,
+    const char** error_message
+);
+
 /* The slab of one rank: the box is cut along direction `axis` (which must be
  * periodic); the rank owns the points whose fractional coordinate along that
  * direction, wrapped into [0, 1), lies in [lower, upper). */

@@ -11,8 +11,9 @@ import ctypes
 import numpy as np
 import torch
 
-from ._c_api import VesinCUDA, VesinDevice, VesinNeighborList, VesinOptions, get_library
+from ._c_api import VESIN_B200_FLOAT32, VesinCUDA, VesinDevice, VesinNeighborList, VesinOptions, get_library
 from ._neighbors import _view
+from ._outputs import OutputTensors, allocate_callback
 
 
 def split_batch(system_offsets, world_size):
@@ -43,6 +44,7 @@ class BatchNeighborList:
         self.cutoff = float(cutoff)
         self.full_list = bool(full_list)
         self._neighbors = VesinNeighborList()
+        self._last_pairs = 0  # length of the last list: what the next one will roughly need
 
     def __del__(self):
         try:
@@ -73,13 +75,17 @@ class BatchNeighborList:
             periodic = torch.as_tensor(periodic, device=device).to(torch.bool).contiguous()
             if tuple(boxes.shape) != (n_systems, 3, 3) or tuple(periodic.shape) != (n_systems, 3):
                 raise ValueError("`boxes` must be (n_systems, 3, 3) and `periodic` (n_systems, 3)")
-        torch.cuda.current_stream(device).synchronize()
+        # the engine works on a stream of its own, which only the legacy default stream is ordered with
+        stream = torch.cuda.current_stream(device)
+        if stream.cuda_stream != 0:
+            stream.synchronize()
+        if copy:
+            return self._build_into(points, system_offsets, boxes, periodic, quantities, global_indices)
         pair_offsets = self.build(points, system_offsets, boxes, periodic, quantities, global_indices)
 
         n_pairs = self._neighbors.length
         owner = self._neighbors
-        finish = (lambda t: t.clone()) if copy else (lambda t: t)
-        offsets_out = finish(_view(pair_offsets, (n_systems + 1,), "<u8", device, owner).view(torch.int64))
+        offsets_out = _view(pair_offsets, (n_systems + 1,), "<u8", device, owner).view(torch.int64)
         if n_pairs == 0:
             pairs = torch.empty((0, 2), dtype=torch.int64, device=device)
             shifts = torch.empty((0, 3), dtype=torch.int32, device=device)
@@ -94,17 +100,17 @@ class BatchNeighborList:
         data = []
         for quantity in quantities:
             if quantity == "P":
-                data.append(finish(pairs))
+                data.append(pairs)
             elif quantity == "i":
-                data.append(finish(pairs[:, 0]))
+                data.append(pairs[:, 0])
             elif quantity == "j":
-                data.append(finish(pairs[:, 1]))
+                data.append(pairs[:, 1])
             elif quantity == "S":
-                data.append(finish(shifts))
+                data.append(shifts)
             elif quantity == "d":
-                data.append(finish(distances))
+                data.append(distances)
             elif quantity == "D":
-                data.append(finish(vectors))
+                data.append(vectors)
         return tuple(data), offsets_out
 
     def build(self, points, system_offsets, boxes=None, periodic=None, quantities="ij", global_indices=False):
@@ -114,12 +120,7 @@ class BatchNeighborList:
         the n_systems + 1 pair offsets."""
         float_io = points.dtype == torch.float32
         offsets = np.ascontiguousarray(system_offsets, dtype=np.uint64)
-        options = VesinOptions()
-        options.cutoff = self.cutoff
-        options.full = self.full_list
-        options.return_shifts = "S" in quantities
-        options.return_distances = "d" in quantities
-        options.return_vectors = "D" in quantities
+        options = self._options(quantities)
         error = ctypes.c_char_p()
         pair_offsets = ctypes.c_void_p()
         entry_point = self._lib.vesin_b200_neighbors_batch_f32 if float_io else self._lib.vesin_b200_neighbors_batch
@@ -138,8 +139,54 @@ class BatchNeighborList:
         )
         if status != 0:
             raise RuntimeError(error.value.decode("utf8"))
+        self._last_pairs = self._neighbors.length
         return pair_offsets.value
+
+    def _options(self, quantities):
+        options = VesinOptions()
+        options.cutoff = self.cutoff
+        options.full = self.full_list
+        options.return_shifts = "S" in quantities
+        options.return_distances = "d" in quantities
+        options.return_vectors = "D" in quantities
+        return options
+
+    def _build_into(self, points, system_offsets, boxes, periodic, quantities, global_indices):
+        """``compute`` with tensors of their own for the outputs, which the
+        engine writes directly (``vesin_b200_neighbors_batch_into``)."""
+        float_io = points.dtype == torch.float32
+        offsets = np.ascontiguousarray(system_offsets, dtype=np.uint64)
+        outputs = OutputTensors(quantities, points.device, torch.int64, points.dtype)
+        if self._last_pairs > 0:
+            outputs.allocate(self._last_pairs + self._last_pairs // 16 + 256)
+        pair_offsets = torch.empty(len(offsets), dtype=torch.int64, device=points.device)
+        n_pairs = ctypes.c_size_t()
+        error = ctypes.c_char_p()
+        with outputs:
+            status = self._lib.vesin_b200_neighbors_batch_into(
+                points.data_ptr(),
+                offsets.ctypes.data,
+                len(offsets) - 1,
+                boxes.data_ptr() if boxes is not None else None,
+                periodic.data_ptr() if periodic is not None else None,
+                VesinDevice(VesinCUDA, points.device.index or 0),
+                self._options(quantities),
+                VESIN_B200_FLOAT32 if float_io else 0,
+                bool(global_indices),
+                ctypes.byref(self._neighbors),
+                ctypes.byref(outputs.arrays),
+                allocate_callback,
+                None,
+                pair_offsets.data_ptr(),
+                ctypes.byref(n_pairs),
+                ctypes.byref(error),
+            )
+        if status != 0:
+            raise outputs.error or RuntimeError(error.value.decode("utf8"))
+        self._last_pairs = n_pairs.value
+        return tuple(outputs.take(n_pairs.value)), pair_offsets
 
     @property
     def n_pairs(self):
-        return self._neighbors.length
+        """Pairs of the last list."""
+        return self._last_pairs

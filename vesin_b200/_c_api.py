@@ -41,6 +41,24 @@ class VesinOptions(ctypes.Structure):
     ]
 
 
+class VesinB200Arrays(ctypes.Structure):
+    _fields_ = [
+        ("capacity", ctypes.c_size_t),
+        ("i", ctypes.c_void_p),
+        ("j", ctypes.c_void_p),
+        ("pairs", ctypes.c_void_p),
+        ("shifts", ctypes.c_void_p),
+        ("distances", ctypes.c_void_p),
+        ("vectors", ctypes.c_void_p),
+    ]
+
+
+VESIN_B200_FLOAT32 = 1
+VESIN_B200_CANONICAL = 2
+# int allocate(void* context, size_t n_pairs, struct VesinB200Arrays* arrays)
+VesinB200Allocate = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_size_t, ctypes.POINTER(VesinB200Arrays))
+
+
 class VesinB200Slab(ctypes.Structure):
     _fields_ = [("axis", ctypes.c_int), ("lower", ctypes.c_double), ("upper", ctypes.c_double)]
 
@@ -67,6 +85,8 @@ EXPORTED_SYMBOLS = (
     "vesin_b200_neighbors_no_alloc",
     "vesin_b200_neighbors_batch",
     "vesin_b200_neighbors_batch_f32",
+    "vesin_b200_neighbors_into",
+    "vesin_b200_neighbors_batch_into",
     "vesin_b200_neighbors_slab",
     "vesin_b200_pack_halo",
     "vesin_b200_neighbors_f32",
@@ -162,6 +182,41 @@ def get_library():
     ]
     lib.vesin_b200_neighbors_batch_f32.restype = ctypes.c_int
     lib.vesin_b200_neighbors_batch_f32.argtypes = lib.vesin_b200_neighbors_batch.argtypes
+    lib.vesin_b200_neighbors_into.restype = ctypes.c_int
+    lib.vesin_b200_neighbors_into.argtypes = [
+        ctypes.c_void_p,  # points (device)
+        ctypes.c_size_t,  # n_points
+        ctypes.c_void_p,  # box (device)
+        ctypes.c_void_p,  # periodic (device)
+        VesinDevice,
+        VesinOptions,
+        ctypes.c_int,  # flags
+        ctypes.POINTER(VesinNeighborList),
+        ctypes.POINTER(VesinB200Arrays),
+        VesinB200Allocate,
+        ctypes.c_void_p,  # context of the allocation callback
+        ctypes.POINTER(ctypes.c_size_t),  # length (out)
+        ctypes.POINTER(ctypes.c_char_p),
+    ]
+    lib.vesin_b200_neighbors_batch_into.restype = ctypes.c_int
+    lib.vesin_b200_neighbors_batch_into.argtypes = [
+        ctypes.c_void_p,  # points (device)
+        ctypes.c_void_p,  # system_offsets (host, size_t)
+        ctypes.c_size_t,  # n_systems
+        ctypes.c_void_p,  # boxes (device or NULL)
+        ctypes.c_void_p,  # periodic (device or NULL)
+        VesinDevice,
+        VesinOptions,
+        ctypes.c_int,  # flags
+        ctypes.c_bool,  # global_indices
+        ctypes.POINTER(VesinNeighborList),
+        ctypes.POINTER(VesinB200Arrays),
+        VesinB200Allocate,
+        ctypes.c_void_p,  # context of the allocation callback
+        ctypes.c_void_p,  # pair_offsets (device, n_systems + 1 words)
+        ctypes.POINTER(ctypes.c_size_t),  # length (out)
+        ctypes.POINTER(ctypes.c_char_p),
+    ]
     lib.vesin_b200_neighbors_slab.restype = ctypes.c_int
     lib.vesin_b200_neighbors_slab.argtypes = [
         ctypes.c_void_p,  # points (device): owned first, then halo

@@ -4,7 +4,8 @@ arguments, ``compute`` signature, quantities string and error behaviour, on
 top of the CUDA engine's C ABI.
 
 Inputs may be torch tensors on a CUDA device (outputs are torch tensors on the
-same device, zero-copy views when ``copy=False``) or anything numpy can convert
+same device: tensors of their own, which the engine writes directly, or with
+``copy=False`` views of the library's arrays that the next call overwrites) or anything numpy can convert
 (the data is copied to the current CUDA device, and the outputs come back as
 numpy arrays). There is no CPU engine behind this class.
 """
@@ -17,6 +18,8 @@ import torch
 from ._c_api import (
     STAGE_NAMES,
     N_STAGES,
+    VESIN_B200_CANONICAL,
+    VESIN_B200_FLOAT32,
     VesinAutoAlgorithm,
     VesinBruteForce,
     VesinCellList,
@@ -27,6 +30,7 @@ from ._c_api import (
     VesinUnknownDevice,
     get_library,
 )
+from ._outputs import OutputTensors, allocate_callback
 
 
 class _DeviceArray:
@@ -48,6 +52,22 @@ def _view(ptr, shape, typestr, device, owner):
     return torch.as_tensor(_DeviceArray(ptr, shape, typestr, owner), device=device)
 
 
+_PERIODIC = {}  # device copies of the (at most eight) constant flag triples, per device
+
+
+def _periodic_flags(periodic, device):
+    """`periodic` as three bools in device memory. Flags that come from the host
+    are uploaded once per device: an upload from pageable memory makes the host
+    wait for it, 15-20 us on every call."""
+    if isinstance(periodic, (list, tuple)) and len(periodic) == 3 and all(isinstance(flag, (bool, np.bool_)) for flag in periodic):
+        key = (device, bool(periodic[0]), bool(periodic[1]), bool(periodic[2]))
+        flags = _PERIODIC.get(key)
+        if flags is None:
+            flags = _PERIODIC[key] = torch.tensor(key[1:], dtype=torch.bool, device=device)
+        return flags
+    return torch.as_tensor(periodic, device=device).to(torch.bool).contiguous()
+
+
 class NeighborList:
     """A neighbor list calculator (CUDA engine)."""
 
@@ -65,6 +85,7 @@ class NeighborList:
         if self.n_threads < 0:
             raise ValueError("n_threads must be zero or a positive integer")
         self._neighbors = VesinNeighborList()
+        self._last_pairs = 0  # length of the last list: what the next one will roughly need
 
     def __del__(self):
         try:
@@ -130,11 +151,12 @@ class NeighborList:
         if from_torch:
             floating = initial_dtype.is_floating_point
             out_dtype = initial_dtype if floating else torch.float64
-            float_io = initial_dtype == torch.float32 and not self.canonical  # the canonical entry point is fp64
+            # (the canonical entry point for arrays of the library is fp64)
+            float_io = initial_dtype == torch.float32 and (copy or not self.canonical)
             work_dtype = torch.float32 if float_io else torch.float64
             d_points = points.to(work_dtype).contiguous()
             d_box = box.to(work_dtype).contiguous()
-            d_periodic = torch.as_tensor(periodic, device=device).to(torch.bool).contiguous()
+            d_periodic = _periodic_flags(periodic, device)
         else:
             floating = np.issubdtype(initial_dtype, np.floating)
             out_dtype = initial_dtype if floating else np.float64
@@ -142,7 +164,9 @@ class NeighborList:
             work_dtype = np.float32 if float_io else np.float64
             d_points = torch.from_numpy(np.ascontiguousarray(points, dtype=work_dtype)).to(device, non_blocking=False)
             d_box = torch.from_numpy(np.ascontiguousarray(box, dtype=work_dtype)).to(device)
-            d_periodic = torch.from_numpy(np.ascontiguousarray(periodic, dtype=np.bool_)).to(device)
+            if not isinstance(periodic, (list, tuple)):
+                periodic = np.ascontiguousarray(periodic, dtype=np.bool_).tolist()
+            d_periodic = _periodic_flags(periodic, device)
         if tuple(d_periodic.shape) != (3,):
             raise ValueError(
                 "`periodic` must be a single boolean or a sequence of three "
@@ -167,10 +191,40 @@ class NeighborList:
             self._lib.vesin_free(ctypes.byref(self._neighbors))
             ctypes.memset(ctypes.byref(self._neighbors), 0, ctypes.sizeof(self._neighbors))
 
-        # inputs produced on another stream of the caller must be complete:
-        # the engine works on its own stream
-        torch.cuda.current_stream(device).synchronize()
+        # inputs produced on another stream of the caller must be complete: the engine works on
+        # a stream of its own, which only the legacy default stream is ordered with
+        stream = torch.cuda.current_stream(device)
+        if stream.cuda_stream != 0:
+            stream.synchronize()
         error_message = ctypes.c_char_p()
+
+        if from_torch and copy:
+            outputs = OutputTensors(quantities, device, torch.uint64, work_dtype)
+            if self._last_pairs > 0:
+                outputs.allocate(self._last_pairs + self._last_pairs // 16 + 256)
+            n_pairs = ctypes.c_size_t()
+            with outputs:
+                status = self._lib.vesin_b200_neighbors_into(
+                    d_points.data_ptr(),
+                    d_points.shape[0],
+                    d_box.data_ptr(),
+                    d_periodic.data_ptr(),
+                    c_device,
+                    options,
+                    (VESIN_B200_FLOAT32 if float_io else 0) | (VESIN_B200_CANONICAL if self.canonical else 0),
+                    ctypes.byref(self._neighbors),
+                    ctypes.byref(outputs.arrays),
+                    allocate_callback,
+                    None,
+                    ctypes.byref(n_pairs),
+                    ctypes.byref(error_message),
+                )
+            if status != 0:
+                raise outputs.error or RuntimeError(error_message.value.decode("utf8"))
+            self._last_pairs = n_pairs.value
+            values = outputs.take(n_pairs.value)
+            return tuple(value.to(out_dtype) if value.dtype == work_dtype else value for value in values)
+
         entry_point = self._lib.vesin_b200_neighbors_f32 if float_io else self._lib.vesin_neighbors
         if self.canonical:
             entry_point = self._lib.vesin_b200_neighbors_canonical
@@ -206,9 +260,7 @@ class NeighborList:
                 vectors = _view(self._neighbors.vectors, (n_pairs, 3), "<f4" if float_io else "<f8", device, owner).to(torch_float)
 
         def finish(tensor):
-            if from_torch:
-                return tensor.clone() if copy else tensor
-            return tensor.cpu().numpy()
+            return tensor if from_torch else tensor.cpu().numpy()
 
         data = []
         for quantity in quantities:

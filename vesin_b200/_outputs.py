@@ -1,0 +1,98 @@
+"""Output tensors of the calculators: lists that the caller owns are written by
+the engine straight into tensors of torch's allocator (``vesin_b200_neighbors_into``),
+instead of being copied out of the library's arrays. A copy moves every byte of
+the list twice more, and an index column picked out of the (i, j) pairs moves
+twice as much again: at 45.6 M pairs that took 0.98 ms beside a build of 0.61 ms."""
+
+import threading
+
+import torch
+
+from ._c_api import VesinB200Allocate, VesinB200Arrays
+
+_active = threading.local()
+
+
+@VesinB200Allocate
+def allocate_callback(_context, n_pairs, arrays):
+    """Called by the engine, on the thread that called it, when a list needs
+    more room than the arrays it was given have."""
+    try:
+        _active.outputs.allocate(n_pairs)
+        return 0
+    except BaseException as error:  # nothing may propagate through the engine: the caller raises it
+        _active.outputs.error = error
+        return 1
+
+
+class OutputTensors:
+    """The tensors of one list: one per quantity asked for. Use as a context
+    manager around the call that fills them."""
+
+    def __init__(self, quantities, device, index_dtype, value_dtype):
+        self.quantities = quantities
+        self.device = device
+        self.index_dtype = index_dtype
+        self.value_dtype = value_dtype
+        self.arrays = VesinB200Arrays()
+        self.i = self.j = self.pairs = self.shifts = self.distances = self.vectors = None
+        self.error = None
+
+    def __enter__(self):
+        self._outer = getattr(_active, "outputs", None)
+        _active.outputs = self
+        return self
+
+    def __exit__(self, *_):
+        _active.outputs = self._outer
+
+    def allocate(self, n_pairs):
+        quantities, device, arrays = self.quantities, self.device, self.arrays
+        # what there is too little of goes back to the allocator first
+        self.i = self.j = self.pairs = self.shifts = self.distances = self.vectors = None
+        arrays.capacity = 0
+        if "P" in quantities:
+            self.pairs = torch.empty((n_pairs, 2), dtype=self.index_dtype, device=device)
+            arrays.pairs = self.pairs.data_ptr()
+        else:
+            if "i" in quantities:
+                self.i = torch.empty(n_pairs, dtype=self.index_dtype, device=device)
+                arrays.i = self.i.data_ptr()
+            if "j" in quantities:
+                self.j = torch.empty(n_pairs, dtype=self.index_dtype, device=device)
+                arrays.j = self.j.data_ptr()
+        if "S" in quantities:
+            self.shifts = torch.empty((n_pairs, 3), dtype=torch.int32, device=device)
+            arrays.shifts = self.shifts.data_ptr()
+        if "d" in quantities:
+            self.distances = torch.empty(n_pairs, dtype=self.value_dtype, device=device)
+            arrays.distances = self.distances.data_ptr()
+        if "D" in quantities:
+            self.vectors = torch.empty((n_pairs, 3), dtype=self.value_dtype, device=device)
+            arrays.vectors = self.vectors.data_ptr()
+        arrays.capacity = n_pairs
+
+    def take(self, n_pairs):
+        """The quantities in the order asked for, `n_pairs` rows each."""
+        if n_pairs == 0 and self.arrays.capacity == 0:
+            self.allocate(0)
+        capacity = self.arrays.capacity
+        # a list that shrank a lot does not hold on to the room that its predecessor needed
+        wasteful = capacity > n_pairs + n_pairs // 8 + 4096
+
+        def rows(tensor):
+            if capacity == n_pairs:
+                return tensor
+            tensor = tensor[:n_pairs]
+            return tensor.clone() if wasteful else tensor
+
+        columns = {"P": self.pairs, "i": self.i, "j": self.j, "S": self.shifts, "d": self.distances, "D": self.vectors}
+        result = []
+        for k, quantity in enumerate(self.quantities):
+            if quantity in "ij" and self.pairs is not None:
+                result.append(self.pairs[:n_pairs, "ij".index(quantity)].clone())
+            elif quantity in columns:
+                tensor = rows(columns[quantity])
+                # a quantity asked for twice comes back as two tensors
+                result.append(tensor.clone() if quantity in self.quantities[:k] else tensor)
+        return result

@@ -60,7 +60,8 @@ static int neighbors_entry(
     VesinNeighborList* neighbors,
     const char** error_message,
     bool float_io,
-    bool canonical = false
+    bool canonical = false,
+    const vb200::CallerArrays* caller = nullptr
 ) {
     // Order and wording of the checks: vesin/src/vesin.cpp:51-105
     if (error_message == nullptr) {
@@ -108,7 +109,7 @@ static int neighbors_entry(
 
     try {
         if (device.type == VesinCUDA) {
-            vb200::neighbors(points, n_points, box, periodic, options, *neighbors, float_io, canonical);
+            vb200::neighbors(points, n_points, box, periodic, options, *neighbors, float_io, canonical, caller);
         } else if (device.type == VesinCPU) {
             throw std::runtime_error(
                 "this build of vesin is the CUDA (sm_100a) engine only: data on VesinCPU is not supported, "
@@ -169,6 +170,50 @@ extern "C" int vesin_b200_neighbors_canonical(
     const char** error_message
 ) {
     return neighbors_entry(points, n_points, box, periodic, device, options, neighbors, error_message, /*float_io=*/false, /*canonical=*/true);
+}
+
+/// Checks of the arguments that only the *_into entry points have.
+static const char* check_arrays(const VesinB200Arrays* arrays, const size_t* length, int flags, int valid_flags) {
+    if (arrays == nullptr) {
+        return "`arrays` can not be a NULL pointer";
+    }
+    if (length == nullptr) {
+        return "`length` can not be a NULL pointer";
+    }
+    if ((flags & ~valid_flags) != 0) {
+        return "unknown bits in `flags`";
+    }
+    return nullptr;
+}
+
+extern "C" int vesin_b200_neighbors_into(
+    const void* points,
+    size_t n_points,
+    const void* box,
+    const bool periodic[3],
+    VesinDevice device,
+    VesinOptions options,
+    int flags,
+    VesinNeighborList* neighbors,
+    VesinB200Arrays* arrays,
+    VesinB200Allocate allocate,
+    void* context,
+    size_t* length,
+    const char** error_message
+) {
+    if (error_message == nullptr) {
+        return EXIT_FAILURE;
+    }
+    *error_message = check_arrays(arrays, length, flags, VESIN_B200_FLOAT32 | VESIN_B200_CANONICAL);
+    if (*error_message != nullptr) {
+        return EXIT_FAILURE;
+    }
+    *length = 0;
+    const vb200::CallerArrays caller{arrays, allocate, context, length};
+    return neighbors_entry(
+        points, n_points, box, periodic, device, options, neighbors, error_message, (flags & VESIN_B200_FLOAT32) != 0,
+        (flags & VESIN_B200_CANONICAL) != 0, &caller
+    );
 }
 
 extern "C" void vesin_free(VesinNeighborList* neighbors) {
@@ -240,7 +285,9 @@ static int batch_entry(
     bool global_indices,
     VesinNeighborList* neighbors,
     const size_t** pair_offsets,
-    const char** error_message
+    const char** error_message,
+    const vb200::CallerArrays* caller = nullptr,
+    size_t* caller_pair_offsets = nullptr
 ) {
     if (error_message == nullptr) {
         return EXIT_FAILURE;
@@ -276,7 +323,7 @@ static int batch_entry(
     }
     neighbors->device = device;
     try {
-        vb200::neighbors_batch(points, float_io, system_offsets, n_systems, boxes, periodic, options, global_indices, *neighbors, pair_offsets);
+        vb200::neighbors_batch(points, float_io, system_offsets, n_systems, boxes, periodic, options, global_indices, *neighbors, pair_offsets, caller, caller_pair_offsets);
     } catch (const std::bad_alloc&) {
         LAST_ERROR = "failed to allocate memory";
         *error_message = LAST_ERROR.c_str();
@@ -319,6 +366,42 @@ extern "C" int vesin_b200_neighbors_batch_f32(
     const char** error_message
 ) {
     return batch_entry(points, true, system_offsets, n_systems, boxes, periodic, device, options, global_indices, neighbors, pair_offsets, error_message);
+}
+
+extern "C" int vesin_b200_neighbors_batch_into(
+    const void* points,
+    const size_t* system_offsets,
+    size_t n_systems,
+    const void* boxes,
+    const bool (*periodic)[3],
+    VesinDevice device,
+    VesinOptions options,
+    int flags,
+    bool global_indices,
+    VesinNeighborList* neighbors,
+    VesinB200Arrays* arrays,
+    VesinB200Allocate allocate,
+    void* context,
+    size_t* pair_offsets,
+    size_t* length,
+    const char** error_message
+) {
+    if (error_message == nullptr) {
+        return EXIT_FAILURE;
+    }
+    *error_message = check_arrays(arrays, length, flags, VESIN_B200_FLOAT32);
+    if (*error_message == nullptr && pair_offsets == nullptr) {
+        *error_message = "`pair_offsets` can not be a NULL pointer";
+    }
+    if (*error_message != nullptr) {
+        return EXIT_FAILURE;
+    }
+    *length = 0;
+    const vb200::CallerArrays caller{arrays, allocate, context, length};
+    return batch_entry(
+        points, (flags & VESIN_B200_FLOAT32) != 0, system_offsets, n_systems, boxes, periodic, device, options, global_indices, neighbors, nullptr,
+        error_message, &caller, pair_offsets
+    );
 }
 
 static int slab_entry(

@@ -15,6 +15,20 @@ namespace vb200 {
 /// Doubles of shared memory a warp needs for the transposes below.
 constexpr int TRANSPOSE_DOUBLES = 192;
 
+/// The two indices of one element of the list.
+__device__ __forceinline__ void store_indices(const PairOutput& out, unsigned long long element, unsigned long long a, unsigned long long b) {
+    if (out.pairs != nullptr) {
+        __stcs(reinterpret_cast<ulonglong2*>(out.pairs) + element, make_ulonglong2(a, b));
+        return;
+    }
+    if (out.column_i != nullptr) {
+        __stcs(out.column_i + element, a);
+    }
+    if (out.column_j != nullptr) {
+        __stcs(out.column_j + element, b);
+    }
+}
+
 /// Write `n_valid` consecutive pairs starting at output element `first`:
 /// lane l holds pair l. 12- and 24-byte elements are transposed through
 /// shared memory so that every store instruction covers one contiguous span.
@@ -23,7 +37,7 @@ __device__ __forceinline__ void store_pairs(
     unsigned long long b, int s0, int s1, int s2, double d, double vx, double vy, double vz
 ) {
     if (lane < n_valid) {
-        __stcs(reinterpret_cast<ulonglong2*>(out.pairs) + first + lane, make_ulonglong2(a, b));
+        store_indices(out, first + lane, a, b);
         if (out.distances != nullptr) {
             if (out.values_float) {
                 __stcs(reinterpret_cast<float*>(out.distances) + first + lane, static_cast<float>(d));
@@ -102,8 +116,17 @@ __device__ __forceinline__ void store_both(
     const unsigned long long mine = first + 2 * lane;
     const bool is_tail = lane == tail_lane;
     if (lane < n_valid && !is_tail) {
-        unsigned long long* dst = out.pairs + 2 * mine;
-        asm volatile("st.global.cs.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(dst), "l"(a), "l"(b), "l"(b), "l"(a) : "memory");
+        if (out.pairs != nullptr) {
+            unsigned long long* dst = out.pairs + 2 * mine;
+            asm volatile("st.global.cs.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(dst), "l"(a), "l"(b), "l"(b), "l"(a) : "memory");
+        } else {
+            if (out.column_i != nullptr) {
+                __stcs(reinterpret_cast<ulonglong2*>(out.column_i + mine), make_ulonglong2(a, b));
+            }
+            if (out.column_j != nullptr) {
+                __stcs(reinterpret_cast<ulonglong2*>(out.column_j + mine), make_ulonglong2(b, a));
+            }
+        }
         if (out.distances != nullptr) {
             if (out.values_float) {
                 const float df = static_cast<float>(d);
@@ -115,8 +138,8 @@ __device__ __forceinline__ void store_both(
     }
     if (is_tail) {
         // forward pair in place, reversed pair at the head of the block, element by element
-        reinterpret_cast<ulonglong2*>(out.pairs)[mine] = make_ulonglong2(a, b);
-        reinterpret_cast<ulonglong2*>(out.pairs)[tail_to] = make_ulonglong2(b, a);
+        store_indices(out, mine, a, b);
+        store_indices(out, tail_to, b, a);
         if (out.distances != nullptr) {
             if (out.values_float) {
                 reinterpret_cast<float*>(out.distances)[mine] = static_cast<float>(d);

@@ -123,7 +123,7 @@ struct Workspace {
 
     // output arrays (capacity in pairs); kept allocated when not requested
     DeviceBuffer out_pairs, out_shifts, out_distances, out_vectors;
-    // second set of output arrays: where a canonical list is sorted into (the sets swap roles)
+    // second set of output arrays: where the rows of a canonical list lie before they are sorted
     DeviceBuffer alt_pairs, alt_shifts, alt_distances, alt_vectors;
 
     // What the last build on this list saw, and the plan made from it: the
@@ -343,40 +343,120 @@ void read_header(Workspace& ws) {
     VB200_CUDA(cudaStreamSynchronize(ws.stream));
 }
 
-/// Pairs that fit every output array this call needs, as allocated now.
-size_t common_capacity(const Workspace& ws, const VesinOptions& options) {
-    size_t capacity = ws.out_pairs.bytes / (2 * sizeof(size_t));
-    if (options.return_shifts) {
-        capacity = std::min(capacity, ws.out_shifts.bytes / (3 * sizeof(int32_t)));
+/// Where the pairs of a build go: the arrays of the list itself (grow-only, as in the reference's
+/// C API), or arrays the caller brings and grows on demand. Which arrays are written follows from
+/// the options in the first case, from the caller's non-null pointers in the second.
+class Target {
+  public:
+    Target(VesinNeighborList& list, Workspace& ws, const VesinOptions& options, bool float_io, const CallerArrays* caller):
+        list_(list), ws_(ws), options_(options), float_io_(float_io), caller_(caller) {
+        list_.length = 0;
+        if (caller_ != nullptr) {
+            // the pairs do not belong to the list
+            list_.pairs = nullptr;
+            list_.shifts = nullptr;
+            list_.distances = nullptr;
+            list_.vectors = nullptr;
+        } else {
+            reserve(std::max<size_t>(capacity(), 256));
+        }
     }
-    if (options.return_distances) {
-        capacity = std::min(capacity, ws.out_distances.bytes / sizeof(double));
-    }
-    if (options.return_vectors) {
-        capacity = std::min(capacity, ws.out_vectors.bytes / (3 * sizeof(double)));
-    }
-    return capacity;
-}
 
-void set_outputs(VesinNeighborList& list, Workspace& ws, const VesinOptions& options, size_t capacity) {
-    ws.out_pairs.reserve(capacity * 2 * sizeof(size_t));
-    list.pairs = reinterpret_cast<size_t(*)[2]>(ws.out_pairs.ptr);
-    list.shifts = nullptr;
-    list.distances = nullptr;
-    list.vectors = nullptr;
-    if (options.return_shifts) {
-        ws.out_shifts.reserve(capacity * 3 * sizeof(int32_t));
-        list.shifts = reinterpret_cast<int32_t(*)[3]>(ws.out_shifts.ptr);
+    /// Pairs that fit every array this call needs, as allocated now.
+    size_t capacity() const {
+        if (caller_ != nullptr) {
+            return caller_->arrays->capacity;
+        }
+        size_t result = ws_.out_pairs.bytes / (2 * sizeof(size_t));
+        if (options_.return_shifts) {
+            result = std::min(result, ws_.out_shifts.bytes / (3 * sizeof(int32_t)));
+        }
+        if (options_.return_distances) {
+            result = std::min(result, ws_.out_distances.bytes / sizeof(double));
+        }
+        if (options_.return_vectors) {
+            result = std::min(result, ws_.out_vectors.bytes / (3 * sizeof(double)));
+        }
+        return result;
     }
-    if (options.return_distances) {
-        ws.out_distances.reserve(capacity * sizeof(double));
-        list.distances = ws.out_distances.as<double>();
+
+    /// Arrays that were never filled, or hold the minimum, cannot hold the pairs of a large
+    /// system: the first pass over it only counts.
+    bool too_small_to_try(size_t n_points) const {
+        return capacity() == 0 || (capacity() <= 256 && n_points >= 4096);
     }
-    if (options.return_vectors) {
-        ws.out_vectors.reserve(capacity * 3 * sizeof(double));
-        list.vectors = reinterpret_cast<double(*)[3]>(ws.out_vectors.ptr);
+
+    /// Arrays for at least `pairs` pairs (contents are lost when they grow).
+    void reserve(size_t pairs) {
+        if (caller_ != nullptr) {
+            if (pairs > caller_->arrays->capacity) {
+                if (caller_->allocate == nullptr || caller_->allocate(caller_->context, pairs, caller_->arrays) != 0 ||
+                    caller_->arrays->capacity < pairs) {
+                    throw std::bad_alloc();
+                }
+            }
+            return;
+        }
+        ws_.out_pairs.reserve(pairs * 2 * sizeof(size_t));
+        list_.pairs = reinterpret_cast<size_t(*)[2]>(ws_.out_pairs.ptr);
+        list_.shifts = nullptr;
+        list_.distances = nullptr;
+        list_.vectors = nullptr;
+        if (options_.return_shifts) {
+            ws_.out_shifts.reserve(pairs * 3 * sizeof(int32_t));
+            list_.shifts = reinterpret_cast<int32_t(*)[3]>(ws_.out_shifts.ptr);
+        }
+        if (options_.return_distances) {
+            ws_.out_distances.reserve(pairs * sizeof(double));
+            list_.distances = ws_.out_distances.as<double>();
+        }
+        if (options_.return_vectors) {
+            ws_.out_vectors.reserve(pairs * 3 * sizeof(double));
+            list_.vectors = reinterpret_cast<double(*)[3]>(ws_.out_vectors.ptr);
+        }
     }
-}
+
+    /// The same for a total that was found by counting: arrays of the list get some headroom, a
+    /// caller is asked for what is needed.
+    void grow(size_t total) {
+        reserve(caller_ != nullptr ? total : total + total / 16 + 256);
+    }
+
+    PairOutput view() const {
+        PairOutput out{};
+        out.values_float = float_io_ ? 1 : 0;
+        if (caller_ != nullptr) {
+            const VesinB200Arrays& arrays = *caller_->arrays;
+            out.pairs = reinterpret_cast<unsigned long long*>(arrays.pairs);
+            out.column_i = reinterpret_cast<unsigned long long*>(arrays.i);
+            out.column_j = reinterpret_cast<unsigned long long*>(arrays.j);
+            out.shifts = reinterpret_cast<int32_t*>(arrays.shifts);
+            out.distances = static_cast<double*>(arrays.distances);
+            out.vectors = static_cast<double*>(arrays.vectors);
+        } else {
+            out.pairs = reinterpret_cast<unsigned long long*>(list_.pairs);
+            out.shifts = reinterpret_cast<int32_t*>(list_.shifts);
+            out.distances = list_.distances;
+            out.vectors = reinterpret_cast<double*>(list_.vectors);
+        }
+        return out;
+    }
+
+    void finish(size_t total) {
+        if (caller_ != nullptr) {
+            *caller_->length = total;
+        } else {
+            list_.length = total;
+        }
+    }
+
+  private:
+    VesinNeighborList& list_;
+    Workspace& ws_;
+    const VesinOptions& options_;
+    bool float_io_;
+    const CallerArrays* caller_;
+};
 
 } // namespace
 
@@ -409,7 +489,7 @@ namespace {
 /// the exact list at the cutoff (vesin/src/verlet_cuda.cpp:307-322).
 void neighbors_with_skin(
     const void* points, size_t n_points, const void* box, const bool periodic[3], VesinOptions options, VesinNeighborList& list,
-    bool float_io
+    bool float_io, const CallerArrays* caller
 ) {
     DeviceGuard guard(list.device.device_id);
     Workspace& ws = workspace_of(list);
@@ -436,7 +516,7 @@ void neighbors_with_skin(
 
     if (cache.disabled) {
         options.skin = 0.0;
-        neighbors(points, n_points, box, periodic, options, list, float_io, false);
+        neighbors(points, n_points, box, periodic, options, list, float_io, false, caller);
         return;
     }
     bool usable = cache.valid && cache.cutoff == options.cutoff && cache.skin == options.skin && cache.full == options.full &&
@@ -446,7 +526,7 @@ void neighbors_with_skin(
         const auto plain_started = std::chrono::steady_clock::now();
         VesinOptions plain = options;
         plain.skin = 0.0;
-        neighbors(points, n_points, box, periodic, plain, list, float_io, false);
+        neighbors(points, n_points, box, periodic, plain, list, float_io, false, caller);
         const double plain_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - plain_started).count();
         if (cache.trial == 2 && plain_seconds < cache.filter_seconds) {
             cache.disabled = true;
@@ -524,17 +604,10 @@ void neighbors_with_skin(
 
         // ---- filter: into the arrays of the previous call first; when the pairs do not fit they
         // have still been counted: grow to the exact total and filter again ----
-        set_outputs(list, ws, options, std::max<size_t>(common_capacity(ws, options), 256));
-        size_t capacity = common_capacity(ws, options);
+        Target target(list, ws, options, float_io, caller);
+        size_t capacity = target.capacity();
         bool stale = false;
         for (int attempt = 0;; attempt++) {
-            PairOutput out{
-                reinterpret_cast<unsigned long long*>(list.pairs),
-                reinterpret_cast<int32_t*>(list.shifts),
-                list.distances,
-                reinterpret_cast<double*>(list.vectors),
-                float_io ? 1 : 0,
-            };
             const auto* built = static_cast<const Workspace*>(cache.candidates.opaque);
             timer.begin(VesinB200StageEmit);
             if (attempt == 0) {
@@ -542,7 +615,7 @@ void neighbors_with_skin(
             }
             launch_verlet_filter(
                 cache.records.as<uint32_t>(), cache.n_records, cache.positions.as<double>(), built->sorted_index.as<int32_t>(), flat_box,
-                options.cutoff * options.cutoff, options.full, out, capacity, d_state, stream
+                options.cutoff * options.cutoff, options.full, target.view(), capacity, d_state, stream
             );
             timer.end(VesinB200StageEmit);
             VB200_CUDA(cudaGetLastError());
@@ -556,7 +629,7 @@ void neighbors_with_skin(
                 cache.disabled = true;
                 cache.valid = false;
                 options.skin = 0.0;
-                neighbors(points, n_points, box, periodic, options, list, float_io, false);
+                neighbors(points, n_points, box, periodic, options, list, float_io, false, caller);
                 return;
             }
             if (cache.h_state->stale) {
@@ -573,7 +646,7 @@ void neighbors_with_skin(
                 );
             }
             if (total <= capacity) {
-                list.length = total;
+                target.finish(total);
                 ws.timed = timer.enabled;
                 if (usable && attempt == 0) {
                     // Re-filtering pays when few candidates lie between cutoff and cutoff + skin per kept
@@ -592,8 +665,8 @@ void neighbors_with_skin(
             if (attempt >= 2) {
                 throw std::runtime_error("internal error: the pair total kept changing between passes");
             }
-            set_outputs(list, ws, options, total + total / 16 + 256);
-            capacity = common_capacity(ws, options);
+            target.grow(total);
+            capacity = target.capacity();
             VB200_CUDA(cudaMemsetAsync(&d_state->pair_cursor, 0, sizeof(unsigned long long), stream));
         }
         if (!stale || round >= 1) {
@@ -613,7 +686,8 @@ void neighbors(
     VesinOptions options,
     VesinNeighborList& list,
     bool float_io,
-    bool canonical
+    bool canonical,
+    const CallerArrays* caller
 ) {
     if (canonical) {
         options.sorted = true; // rows in index order first, then every row is sorted
@@ -630,7 +704,7 @@ void neighbors(
 
     if (options.skin > 0.0 && std::isfinite(options.skin) && !options.sorted && n_points > 0 && options.algorithm != VesinBruteForce) {
         // cached candidates at cutoff + skin, re-filtered (the result is the list at the cutoff all the same)
-        neighbors_with_skin(points, n_points, box, periodic, options, list, float_io);
+        neighbors_with_skin(points, n_points, box, periodic, options, list, float_io, caller);
         return;
     }
 
@@ -752,8 +826,7 @@ void neighbors(
                 header_is_fresh = true;
                 continue;
             }
-            set_outputs(list, ws, options, 256);
-            list.length = 0;
+            Target(list, ws, options, float_io, caller).finish(0);
             ws.timed = timer.enabled;
             return;
         }
@@ -829,24 +902,15 @@ void neighbors(
             // the previous call are tried first; when the pairs do not fit,
             // the pass has still counted them: grow to the exact total and run
             // it again (first build on a list, or a system that grew). ----
-            set_outputs(list, ws, options, std::max<size_t>(common_capacity(ws, options), 256));
-            size_t capacity = common_capacity(ws, options);
+            Target target(list, ws, options, float_io, caller);
+            size_t capacity = target.capacity();
             size_t total = 0;
             bool refused = false;
-            // arrays of the minimum size (a list that was never filled) cannot hold the pairs
-            // of a large system: the first pass then only counts (capacity 0)
-            bool count_only = capacity <= 256 && n_points >= 4096;
+            bool count_only = target.too_small_to_try(n_points); // the first pass then only counts (capacity 0)
             for (int attempt = 0;; attempt++) {
-                PairOutput out{
-                    reinterpret_cast<unsigned long long*>(list.pairs),
-                    reinterpret_cast<int32_t*>(list.shifts),
-                    list.distances,
-                    reinterpret_cast<double*>(list.vectors),
-                    float_io ? 1 : 0,
-                };
                 const size_t pass_capacity = count_only ? 0 : capacity;
                 timer.begin(VesinB200StageEmit);
-                launch_pairs(plan, ws.cell_start.as<int32_t>(), sorted, out, pass_capacity, ws.d_header, stream, n_points);
+                launch_pairs(plan, ws.cell_start.as<int32_t>(), sorted, target.view(), pass_capacity, ws.d_header, stream, n_points);
                 timer.end(VesinB200StageEmit);
                 VB200_CUDA(cudaGetLastError());
                 read_header(ws);
@@ -870,15 +934,15 @@ void neighbors(
                 }
                 count_only = false;
                 if (total > capacity) {
-                    set_outputs(list, ws, options, total + total / 16 + 256);
-                    capacity = common_capacity(ws, options);
+                    target.grow(total);
+                    capacity = target.capacity();
                 }
                 VB200_CUDA(cudaMemsetAsync(&ws.d_header->pair_cursor, 0, 2 * sizeof(unsigned long long), stream)); // and run_cursor
             }
             if (refused) {
                 continue;
             }
-            list.length = total;
+            target.finish(total);
             ws.timed = timer.enabled;
             return;
         }
@@ -946,69 +1010,53 @@ void neighbors(
         if (total > n_points * pair_limit_per_point) {
             throw pair_limit_error();
         }
-        size_t capacity = std::max<size_t>(total, 256);
-        if (capacity > common_capacity(ws, options) && ws.out_pairs.bytes != 0) {
-            capacity += capacity / 16; // a list that keeps growing gets some headroom
+        Target target(list, ws, options, float_io, caller);
+        if (total > target.capacity()) {
+            ws.out_pairs.bytes > 256 * 2 * sizeof(size_t) ? target.grow(total) : target.reserve(total); // (a list that keeps growing gets some headroom)
         }
-        set_outputs(list, ws, options, capacity);
         if (total > 0) {
-            PairOutput out{
-                reinterpret_cast<unsigned long long*>(list.pairs),
-                reinterpret_cast<int32_t*>(list.shifts),
-                list.distances,
-                reinterpret_cast<double*>(list.vectors),
-                float_io ? 1 : 0,
-            };
+            const PairOutput out = target.view();
+            // a canonical list: the rows go to a second set of arrays first, from where they are sorted into the list's
+            PairOutput rows = out;
+            if (canonical) {
+                ws.alt_pairs.reserve(total * 2 * sizeof(size_t));
+                rows = PairOutput{};
+                rows.values_float = out.values_float;
+                rows.pairs = ws.alt_pairs.as<unsigned long long>();
+                if (out.shifts != nullptr) {
+                    ws.alt_shifts.reserve(total * 3 * sizeof(int32_t));
+                    rows.shifts = ws.alt_shifts.as<int32_t>();
+                }
+                if (out.distances != nullptr) {
+                    ws.alt_distances.reserve(total * sizeof(double));
+                    rows.distances = ws.alt_distances.as<double>();
+                }
+                if (out.vectors != nullptr) {
+                    ws.alt_vectors.reserve(total * 3 * sizeof(double));
+                    rows.vectors = ws.alt_vectors.as<double>();
+                }
+            }
             timer.begin(VesinB200StageEmit);
             VB200_CUDA(cudaMemsetAsync(ws.row_fill.ptr, 0, n_points * sizeof(uint32_t), stream));
             launch_emit(
                 plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.unit_mask_base.as<unsigned long long>(),
-                ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), out, stream
+                ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), rows, stream
             );
             if (canonical) {
-                // every row sorted by (second index, shift) into a second set of arrays, which then become the list's
-                ws.alt_pairs.reserve(ws.out_pairs.bytes);
-                PairOutput sorted_out{ws.alt_pairs.as<unsigned long long>(), nullptr, nullptr, nullptr, float_io ? 1 : 0};
-                if (options.return_shifts) {
-                    ws.alt_shifts.reserve(ws.out_shifts.bytes);
-                    sorted_out.shifts = ws.alt_shifts.as<int32_t>();
-                }
-                if (options.return_distances) {
-                    ws.alt_distances.reserve(ws.out_distances.bytes);
-                    sorted_out.distances = ws.alt_distances.as<double>();
-                }
-                if (options.return_vectors) {
-                    ws.alt_vectors.reserve(ws.out_vectors.bytes);
-                    sorted_out.vectors = ws.alt_vectors.as<double>();
-                }
                 // a second index can come twice in a row only with two images of the same point
                 // within the cutoff of the first: a lattice vector shorter than twice the cutoff
                 bool duplicates_possible = false;
                 for (int k = 0; k < 3; k++) {
                     duplicates_possible = duplicates_possible || (plan.periodic[k] && plan.face_dist[k] < 2.0 * options.cutoff * (1.0 + 1e-9));
                 }
-                launch_sort_rows(ws.row_start.as<unsigned long long>(), n_points, out, sorted_out, duplicates_possible, stream);
-                std::swap(ws.out_pairs, ws.alt_pairs);
-                list.pairs = reinterpret_cast<size_t(*)[2]>(ws.out_pairs.ptr);
-                if (options.return_shifts) {
-                    std::swap(ws.out_shifts, ws.alt_shifts);
-                    list.shifts = reinterpret_cast<int32_t(*)[3]>(ws.out_shifts.ptr);
-                }
-                if (options.return_distances) {
-                    std::swap(ws.out_distances, ws.alt_distances);
-                    list.distances = ws.out_distances.as<double>();
-                }
-                if (options.return_vectors) {
-                    std::swap(ws.out_vectors, ws.alt_vectors);
-                    list.vectors = reinterpret_cast<double(*)[3]>(ws.out_vectors.ptr);
-                }
+                launch_sort_rows(ws.row_start.as<unsigned long long>(), n_points, rows, out, duplicates_possible, stream);
             }
             timer.end(VesinB200StageEmit);
             VB200_CUDA(cudaGetLastError());
             VB200_CUDA(cudaStreamSynchronize(stream));
             timer.collect(VesinB200StageEmit);
         }
-        list.length = total;
+        target.finish(total);
         ws.timed = timer.enabled;
         return;
     }
@@ -1024,7 +1072,9 @@ void neighbors_batch(
     VesinOptions options,
     bool global_indices,
     VesinNeighborList& list,
-    const size_t** pair_offsets
+    const size_t** pair_offsets,
+    const CallerArrays* caller,
+    size_t* caller_pair_offsets
 ) {
     if (n_systems >= (1ull << 31)) {
         throw std::runtime_error("too many systems in the batch");
@@ -1055,6 +1105,9 @@ void neighbors_batch(
     if ((boxes != nullptr && !on_device(boxes)) || (periodic != nullptr && !on_device(periodic))) {
         throw std::runtime_error("`boxes` and `periodic` must be NULL or device memory on the CUDA device of `neighbors`");
     }
+    if (caller_pair_offsets != nullptr && !on_device(caller_pair_offsets)) {
+        throw std::runtime_error("`pair_offsets` must be device memory on the CUDA device of `neighbors`");
+    }
     if ((boxes == nullptr) != (periodic == nullptr)) {
         throw std::runtime_error("`boxes` and `periodic` must be given together");
     }
@@ -1075,7 +1128,10 @@ void neighbors_batch(
         }
     }
     ws.unit_count.reserve(std::max<size_t>(n_systems, 1) * sizeof(unsigned long long));
-    ws.unit_start.reserve((n_systems + 1) * sizeof(unsigned long long));
+    if (caller_pair_offsets == nullptr) {
+        ws.unit_start.reserve((n_systems + 1) * sizeof(unsigned long long));
+    }
+    auto* system_start = (caller_pair_offsets != nullptr) ? reinterpret_cast<unsigned long long*>(caller_pair_offsets) : ws.unit_start.as<unsigned long long>();
     ws.scan_tmp.reserve(scan_tmp_bytes(std::max<size_t>(n_systems, 1)));
     static_assert(sizeof(size_t) == sizeof(unsigned long long), "offsets are copied as they are");
     // (a batch with the same layout as the last one, the usual case in a loop over steps, keeps
@@ -1105,31 +1161,22 @@ void neighbors_batch(
 
     // systems with a periodic direction or many points take the CTA-per-system kernel
     const bool any_for_cta_kernel = periodic != nullptr || largest > molecules_max_points();
-    const auto outputs = [&]() {
-        return PairOutput{
-            reinterpret_cast<unsigned long long*>(list.pairs),
-            reinterpret_cast<int32_t*>(list.shifts),
-            list.distances,
-            reinterpret_cast<double*>(list.vectors),
-            float_io ? 1 : 0,
-        };
-    };
+    Target target(list, ws, options, float_io, caller);
     // A list that was filled before writes into the arrays it has, right behind the counting pass
     // and the scan, without waiting for the host to see the total: one read-back per call. A
     // system whose block does not fit writes nothing; the host then grows the arrays and runs the
     // writing pass again.
-    const size_t existing = common_capacity(ws, options);
-    const bool speculative = n_systems > 0 && existing >= 256;
+    const size_t existing = target.capacity();
+    const bool speculative = n_systems > 0 && existing > 256;
     size_t total = 0;
     if (n_systems > 0) {
         launch_small_count(in, largest, any_for_cta_kernel, ws.unit_count.as<unsigned long long>(), ws.d_header, stream);
         launch_scan_units(
-            ws.unit_count.as<unsigned long long>(), ws.unit_start.as<unsigned long long>(), n_systems, ws.scan_tmp.ptr,
+            ws.unit_count.as<unsigned long long>(), system_start, n_systems, ws.scan_tmp.ptr,
             &ws.d_header->total_pairs, stream
         );
         if (speculative) {
-            set_outputs(list, ws, options, existing);
-            launch_small_emit(in, largest, any_for_cta_kernel, ws.unit_start.as<unsigned long long>(), outputs(), ws.d_header, stream, existing);
+            launch_small_emit(in, largest, any_for_cta_kernel, system_start, target.view(), ws.d_header, stream, existing);
         }
         VB200_CUDA(cudaGetLastError());
         read_header(ws);
@@ -1152,24 +1199,20 @@ void neighbors_batch(
             );
         }
     } else {
-        VB200_CUDA(cudaMemsetAsync(ws.unit_start.ptr, 0, sizeof(unsigned long long), stream));
+        VB200_CUDA(cudaMemsetAsync(system_start, 0, sizeof(unsigned long long), stream));
     }
 
-    if (!(speculative && total <= existing)) {
-        size_t capacity = std::max<size_t>(total, 256);
-        if (capacity > common_capacity(ws, options) && ws.out_pairs.bytes != 0) {
-            capacity += capacity / 16;
+    if (!(speculative && total <= existing) && total > 0) {
+        if (total > existing) {
+            speculative ? target.grow(total) : target.reserve(total);
         }
-        set_outputs(list, ws, options, capacity);
-        if (total > 0) {
-            launch_small_emit(in, largest, any_for_cta_kernel, ws.unit_start.as<unsigned long long>(), outputs(), ws.d_header, stream);
-            VB200_CUDA(cudaGetLastError());
-        }
+        launch_small_emit(in, largest, any_for_cta_kernel, system_start, target.view(), ws.d_header, stream);
+        VB200_CUDA(cudaGetLastError());
     }
     VB200_CUDA(cudaStreamSynchronize(stream));
-    list.length = total;
+    target.finish(total);
     if (pair_offsets != nullptr) {
-        *pair_offsets = reinterpret_cast<const size_t*>(ws.unit_start.ptr);
+        *pair_offsets = reinterpret_cast<const size_t*>(system_start);
     }
 }
 
@@ -1294,18 +1337,9 @@ void neighbors_slab_core(
         // everything is sorted together once the messages are there.
         const bool owned_first = with_messages && axis == 2 && n_owned == n_array;
         const size_t owned_cells = owned_first ? n_cells / static_cast<size_t>(plan.n_cells[2]) * static_cast<size_t>(plan.n_cells[2] - 2) : n_cells;
-        set_outputs(list, ws, options, std::max<size_t>(common_capacity(ws, options), 256));
-        size_t capacity = common_capacity(ws, options);
-        bool count_only = capacity <= 256 && n_owned >= 4096;
-        const auto outputs = [&]() {
-            return PairOutput{
-                reinterpret_cast<unsigned long long*>(list.pairs),
-                reinterpret_cast<int32_t*>(list.shifts),
-                list.distances,
-                reinterpret_cast<double*>(list.vectors),
-                float_io ? 1 : 0,
-            };
-        };
+        Target target(list, ws, options, float_io, nullptr);
+        size_t capacity = target.capacity();
+        bool count_only = target.too_small_to_try(n_owned);
         // The units that need nothing from the halo are paired while the halo is received and
         // sorted in on a second stream, which also pairs the units next to the halo; the two
         // streams join before the header is read. (Stage times are taken on one stream: a
@@ -1343,7 +1377,7 @@ void neighbors_slab_core(
                 start_exchange_once(); // before the interior kernel takes every SM
                 VB200_CUDA(cudaEventRecord(ws.owned_sorted, stream));
                 launch_pairs(
-                    plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, outputs(), pass_capacity, ws.d_header, stream, 0, PAIR_PART_INTERIOR
+                    plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, target.view(), pass_capacity, ws.d_header, stream, 0, PAIR_PART_INTERIOR
                 );
                 VB200_CUDA(cudaStreamWaitEvent(halo_stream, ws.owned_sorted, 0));
                 if (halo->received != nullptr) {
@@ -1368,7 +1402,7 @@ void neighbors_slab_core(
             );
             if (overlapped) {
                 launch_pairs(
-                    plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, outputs(), pass_capacity, ws.d_header, halo_stream, 0, PAIR_PART_BOUNDARY
+                    plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, target.view(), pass_capacity, ws.d_header, halo_stream, 0, PAIR_PART_BOUNDARY
                 );
                 // everything queued on `stream` from here on comes after both parts
                 VB200_CUDA(cudaEventRecord(ws.side_done, halo_stream));
@@ -1405,7 +1439,7 @@ void neighbors_slab_core(
             const size_t pass_capacity = count_only ? 0 : capacity;
             if (!(attempt == 0 && pairs_launched)) {
                 timer.begin(VesinB200StageEmit);
-                launch_pairs(plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, outputs(), pass_capacity, ws.d_header, stream);
+                launch_pairs(plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, target.view(), pass_capacity, ws.d_header, stream);
                 timer.end(VesinB200StageEmit);
             }
             VB200_CUDA(cudaGetLastError());
@@ -1456,8 +1490,8 @@ void neighbors_slab_core(
             }
             count_only = false;
             if (total > capacity) {
-                set_outputs(list, ws, options, total + total / 16 + 256);
-                capacity = common_capacity(ws, options);
+                target.grow(total);
+                capacity = target.capacity();
             }
             // mask_cursor (the second run counter of a slab build), pair_cursor and run_cursor
             VB200_CUDA(cudaMemsetAsync(&ws.d_header->mask_cursor, 0, 3 * sizeof(unsigned long long), stream));
@@ -1467,7 +1501,7 @@ void neighbors_slab_core(
         }
         ws.slab.n_local = n_array + static_cast<size_t>(std::min<unsigned long long>(header.halo_count[0], source.capacity)) +
                           static_cast<size_t>(std::min<unsigned long long>(header.halo_count[1], source.capacity));
-        list.length = total;
+        target.finish(total);
         ws.timed = timer.enabled;
         return;
     }

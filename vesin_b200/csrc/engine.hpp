@@ -9,8 +9,17 @@
 #include <cuda_runtime.h>
 
 #include "vesin.h"
+#include "vesin_b200.h"
 
 namespace vb200 {
+
+/// Output arrays a caller brings (see vesin_b200_neighbors_into).
+struct CallerArrays {
+    VesinB200Arrays* arrays;
+    VesinB200Allocate allocate; // may be null: then `arrays` has to hold the list
+    void* context;
+    size_t* length; // out: pairs of the list
+};
 
 /// Compute the list for device-resident inputs. Replaces
 /// vesin::cuda::neighbors (vesin/src/vesin_cuda.cpp:819-923). Throws
@@ -19,6 +28,7 @@ namespace vb200 {
 /// With `float_io`, `points` and `box` are float arrays and the distances /
 /// vectors of the list are float arrays too (the decisions stay fp64).
 /// With `canonical`, the list comes out sorted by (i, j, Sx, Sy, Sz).
+/// With `caller`, the pairs go to the caller's arrays and `list` holds none.
 void neighbors(
     const void* points,
     size_t n_points,
@@ -27,7 +37,8 @@ void neighbors(
     VesinOptions options,
     VesinNeighborList& list,
     bool float_io,
-    bool canonical = false
+    bool canonical = false,
+    const CallerArrays* caller = nullptr
 );
 
 /// Lists of a batch of independent small systems in one call (no counterpart
@@ -42,7 +53,9 @@ void neighbors_batch(
     VesinOptions options,
     bool global_indices,
     VesinNeighborList& list,
-    const size_t** pair_offsets
+    const size_t** pair_offsets,
+    const CallerArrays* caller = nullptr,
+    size_t* caller_pair_offsets = nullptr
 );
 
 /// Halo of a slab that arrives as two messages (see PointSource in

@@ -2358,10 +2358,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_emit_kernel(
                                 plan, sh.home_pos[0][h], sh.home_pos[1][h], sh.home_pos[2][h], sh.x[s], sh.y[s], sh.z[s], s0, s1, s2, vx, vy, vz
                             );
                             const unsigned long long dest = rows.home_row[h] + static_cast<unsigned long long>(round0 + chunk0 + lane - rows.row_offset[h]);
-                            __stcs(
-                                reinterpret_cast<ulonglong2*>(out.pairs) + dest,
-                                make_ulonglong2(static_cast<unsigned long long>(home.w), static_cast<unsigned long long>(cand.w))
-                            );
+                            store_indices(out, dest, static_cast<unsigned long long>(home.w), static_cast<unsigned long long>(cand.w));
                             if (out.shifts != nullptr) {
                                 store_triple_32(out.shifts, dest, s0, s1, s2);
                             }
@@ -2459,7 +2456,7 @@ __device__ __forceinline__ PairInFlight<FLOAT> load_pair(const PairOutput& in, u
 
 template <bool FLOAT>
 __device__ __forceinline__ void store_pair(const PairOutput& out, unsigned long long to, const PairInFlight<FLOAT>& p) {
-    __stcs(reinterpret_cast<ulonglong2*>(out.pairs) + to, p.pair);
+    store_indices(out, to, p.pair.x, p.pair.y);
     if (out.shifts != nullptr) {
         store_triple_32(out.shifts, to, p.s0, p.s1, p.s2);
     }
@@ -2814,11 +2811,7 @@ void launch_pairs(
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         }
     }
-    // paired stores of full lists: 32 bytes of indices, 16 of distances / vectors, 8 of shifts
-    // (half of that for float values); null arrays are not written
-    const auto aligned = [](const void* pointer, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(pointer) % bytes == 0; };
-    const uintptr_t value_bytes = out.values_float ? 8 : 16;
-    out.interleave_ok = aligned(out.pairs, 32) && aligned(out.shifts, 8) && aligned(out.distances, value_bytes) && aligned(out.vectors, value_bytes);
+    out.interleave_ok = paired_stores_fit(out);
 
     const auto launch = [&](auto shape, auto kernel, UnitRanges ranges, unsigned long long* run_cursor, bool follows = false) {
         using Shape = decltype(shape);

@@ -49,15 +49,28 @@ struct SortedPoints {
     int32_t* shift; // [n][3]
 };
 
-/// Output arrays of the C ABI; null pointers are not written.
+/// Output arrays of a build; null pointers are not written. The indices go to `pairs`
+/// (the layout of the C ABI) or, when that is null, to one array each.
 struct PairOutput {
     unsigned long long* pairs; // [total][2]
     int32_t* shifts;           // [total][3]
     double* distances;         // [total]
     double* vectors;           // [total][3]
     int values_float;          // distances / vectors are float arrays (fp32 entry point); decisions stay fp64
-    int interleave_ok;         // set by launch_pairs: the arrays are aligned for the paired stores of full lists
+    int interleave_ok;         // set by the launch wrappers: the arrays are aligned for the paired stores of full lists
+    unsigned long long* column_i; // [total], used when `pairs` is null
+    unsigned long long* column_j;
 };
+
+/// Are the arrays aligned for the paired stores of full lists (store_both)? 32 bytes of indices
+/// (16 per column), 16 of distances / vectors, 8 of shifts; half of that for float values. Null
+/// arrays are not written.
+inline int paired_stores_fit(const PairOutput& out) {
+    const auto aligned = [](const void* pointer, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(pointer) % bytes == 0; };
+    const uintptr_t value_bytes = out.values_float ? 8 : 16;
+    return aligned(out.pairs, 32) && aligned(out.column_i, 16) && aligned(out.column_j, 16) && aligned(out.shifts, 8) &&
+           aligned(out.distances, value_bytes) && aligned(out.vectors, value_bytes);
+}
 
 /// Input coordinates: double (the reference's C API) or float (fp32 entry
 /// point; converted exactly to double when read).

@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_systems_kernel(
                     const unsigned long long gi = index_offset + i, gj = index_offset + j;
                     const double d = __dsqrt_rn(d2);
                     // half lists keep i <= j (i < j, or the image the rule keeps): the forward pair
-                    reinterpret_cast<ulonglong2*>(out.pairs)[dest] = make_ulonglong2(gi, gj);
+                    store_indices(out, dest, gi, gj);
                     if (out.shifts) {
                         out.shifts[3 * dest + 0] = s0;
                         out.shifts[3 * dest + 1] = s1;
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_systems_kernel(
                     }
                     if (in.full) {
                         dest += 1;
-                        reinterpret_cast<ulonglong2*>(out.pairs)[dest] = make_ulonglong2(gj, gi);
+                        store_indices(out, dest, gj, gi);
                         if (out.shifts) {
                             out.shifts[3 * dest + 0] = -s0;
                             out.shifts[3 * dest + 1] = -s1;
@@ -599,7 +599,7 @@ static unsigned molecules_grid(unsigned n_systems) {
 void launch_small_count(
     const BatchInput& in, size_t max_points, bool any_for_cta_kernel, unsigned long long* system_count, DeviceHeader* header, cudaStream_t stream
 ) {
-    const PairOutput nothing{nullptr, nullptr, nullptr, nullptr, 0, 0};
+    const PairOutput nothing{};
     molecules_kernel<false><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, 0, stream>>>(in, system_count, nullptr, nothing, header, 0ull);
     if (any_for_cta_kernel) {
         small_systems_kernel<false><<<small_grid(in.n_systems), SMALL_THREADS, small_shared_bytes(max_points), stream>>>(
@@ -613,9 +613,7 @@ void launch_small_emit(
     DeviceHeader* header, cudaStream_t stream, unsigned long long capacity
 ) {
     // paired stores of full lists need aligned arrays (every system of a full list starts on an even element)
-    const auto aligned = [](const void* pointer, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(pointer) % bytes == 0; };
-    const uintptr_t value_bytes = out.values_float ? 8 : 16;
-    out.interleave_ok = aligned(out.pairs, 32) && aligned(out.shifts, 8) && aligned(out.distances, value_bytes) && aligned(out.vectors, value_bytes);
+    out.interleave_ok = paired_stores_fit(out);
     molecules_kernel<true><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, 0, stream>>>(in, nullptr, system_start, out, header, capacity);
     if (any_for_cta_kernel) {
         small_systems_kernel<true><<<small_grid(in.n_systems), SMALL_THREADS, small_shared_bytes(max_points), stream>>>(

@@ -376,9 +376,7 @@ void launch_verlet_filter(
     if (n == 0) {
         return;
     }
-    const auto aligned = [](const void* pointer, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(pointer) % bytes == 0; };
-    const uintptr_t value_bytes = out.values_float ? 8 : 16;
-    out.interleave_ok = aligned(out.pairs, 32) && aligned(out.shifts, 8) && aligned(out.distances, value_bytes) && aligned(out.vectors, value_bytes);
+    out.interleave_ok = paired_stores_fit(out);
     // a CTA takes 256 records per round; enough CTAs to fill the GPU, few enough that the
     // partly filled chunks at the end of every CTA's walk stay rare
     const size_t rounds = (n + VERLET_THREADS - 1) / VERLET_THREADS;
