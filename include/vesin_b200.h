@@ -482,7 +482,7 @@ VESIN_API int vesin_b200_list_checksum(const struct VesinNeighborList* neighbors
  * system outgrows its workspace; this function never does. The caller passes
  * the inputs AND the output arrays (device memory on `device_id`, `capacity`
  * pairs each; shifts / distances / vectors may be NULL to skip them); the
- * scratch of the kernels is a fixed array of about 2.3 MB that every GPU holds from
+ * scratch of the kernels is a fixed array of about 1.9 MB that every GPU holds from
  * library load to process exit. Hence:
  *   - `pairs` must be aligned to 16 bytes (the other arrays to their element:
  *     4 and 8 bytes); full lists are written fastest when `pairs` is aligned to

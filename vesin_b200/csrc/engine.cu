@@ -103,12 +103,11 @@ struct Workspace {
     DeviceHeader* d_header = nullptr;
     DeviceHeader* h_header = nullptr; // pinned
 
-    DeviceBuffer cell_of, rank, shift, cell_count, cell_start;
-    DeviceBuffer sorted_pos, sorted_index, sorted_shift;
+    DeviceBuffer rank, cell_count, cell_start;
+    DeviceBuffer sorted_records, sorted_wide_shift;
     DeviceBuffer masks, unit_mask_base, unit_words, unit_count, unit_start;
     DeviceBuffer row_count, row_start, row_fill, scan_tmp;
     DeviceBuffer batch_offsets; // batches: where each system starts in the points array
-    DeviceBuffer sorted_global; // slabs: index of every cell-sorted record in the whole system
     DeviceBuffer checksum;      // 4 words of vesin_b200_list_checksum
     bool values_float = false;  // element type of `distances` / `vectors` of the last build
 
@@ -170,8 +169,8 @@ struct Workspace {
 
     ~Workspace() {
         for (DeviceBuffer* buffer :
-             {&cell_of, &rank, &shift, &cell_count, &cell_start, &sorted_pos, &sorted_index, &sorted_shift, &masks, &unit_mask_base,
-              &unit_words, &unit_count, &unit_start, &row_count, &row_start, &row_fill, &scan_tmp, &batch_offsets, &sorted_global, &checksum, &out_pairs,
+             {&rank, &cell_count, &cell_start, &sorted_records, &sorted_wide_shift, &masks, &unit_mask_base,
+              &unit_words, &unit_count, &unit_start, &row_count, &row_start, &row_fill, &scan_tmp, &batch_offsets, &checksum, &out_pairs,
               &out_shifts, &out_distances, &out_vectors, &alt_pairs, &alt_shifts, &alt_distances, &alt_vectors}) {
             buffer->release();
         }
@@ -562,7 +561,7 @@ void neighbors_with_skin(
             cache.positions.reserve(std::max<size_t>(n_points, 1) * 4 * sizeof(double));
             launch_verlet_pack(
                 reinterpret_cast<const unsigned long long*>(cache.candidates.pairs), reinterpret_cast<const int32_t*>(cache.candidates.shifts),
-                cache.n_records, built->sorted_index.as<int32_t>(), n_points, cache.rank_of.as<uint32_t>(), cache.records.as<uint32_t>(), d_state,
+                cache.n_records, built->sorted_records.as<PointRecord>(), n_points, cache.rank_of.as<uint32_t>(), cache.records.as<uint32_t>(), d_state,
                 stream
             );
             if (timer.enabled && built->timed) {
@@ -611,10 +610,10 @@ void neighbors_with_skin(
             const auto* built = static_cast<const Workspace*>(cache.candidates.opaque);
             timer.begin(VesinB200StageEmit);
             if (attempt == 0) {
-                launch_verlet_positions(flat_points, built->sorted_index.as<int32_t>(), n_points, cache.positions.as<double>(), d_state, stream);
+                launch_verlet_positions(flat_points, built->sorted_records.as<PointRecord>(), n_points, cache.positions.as<double>(), d_state, stream);
             }
             launch_verlet_filter(
-                cache.records.as<uint32_t>(), cache.n_records, cache.positions.as<double>(), built->sorted_index.as<int32_t>(), flat_box,
+                cache.records.as<uint32_t>(), cache.n_records, cache.positions.as<double>(), flat_box,
                 options.cutoff * options.cutoff, options.full, target.view(), capacity, d_state, stream
             );
             timer.end(VesinB200StageEmit);
@@ -834,23 +833,19 @@ void neighbors(
         // ---- scratch ----
         const size_t n_cells = static_cast<size_t>(plan.n_cells_total);
         const size_t n_units = static_cast<size_t>(plan.n_units);
-        ws.cell_of.reserve(n_points * sizeof(int32_t));
         ws.rank.reserve(n_points * sizeof(int32_t));
-        ws.shift.reserve(n_points * 3 * sizeof(int32_t));
         ws.cell_count.reserve(n_cells * sizeof(int32_t));
         ws.cell_start.reserve((n_cells + 1) * sizeof(int32_t));
-        ws.sorted_pos.reserve(n_points * 3 * sizeof(double));
-        ws.sorted_index.reserve(n_points * sizeof(int32_t));
-        ws.sorted_shift.reserve(n_points * 3 * sizeof(int32_t));
+        ws.sorted_records.reserve(n_points * sizeof(PointRecord));
+        ws.sorted_wide_shift.reserve(n_points * 3 * sizeof(int32_t));
         ws.scan_tmp.reserve(scan_tmp_bytes(std::max(n_points, n_cells)));
-        SortedPoints sorted{ws.sorted_pos.as<double>(), ws.sorted_index.as<int32_t>(), ws.sorted_shift.as<int32_t>()};
+        SortedPoints sorted{ws.sorted_records.as<PointRecord>(), ws.sorted_wide_shift.as<int32_t>()};
 
         // ---- cell list ----
         if (fused_front || (!speculative && small_front_fits(n_points, plan))) {
             timer.begin(VesinB200StageBin);
             launch_small_front(
-                flat_points, n_points, plan, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(),
-                ws.cell_start.as<int32_t>(), sorted, ws.d_header, flat_box, periodic, speculative, ws.cache.box, ws.cache.periodic, stream
+                flat_points, n_points, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, flat_box, periodic, speculative, ws.cache.box, ws.cache.periodic, stream
             );
             timer.end(VesinB200StageBin);
             timer.begin(VesinB200StageScanCells);
@@ -863,18 +858,14 @@ void neighbors(
                 VB200_CUDA(cudaMemsetAsync(ws.cell_count.ptr, 0, n_cells * sizeof(int32_t), stream));
             }
             launch_bin(
-                source, 0, n_points, plan, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(),
-                ws.cell_count.as<int32_t>(), ws.d_header, speculative, true, stream
+                source, 0, n_points, plan, ws.rank.as<int32_t>(), ws.cell_count.as<int32_t>(), ws.d_header, speculative, true, stream
             );
             timer.end(VesinB200StageBin);
             timer.begin(VesinB200StageScanCells);
             launch_scan_cells(ws.cell_count.as<int32_t>(), ws.cell_start.as<int32_t>(), n_cells, ws.scan_tmp.ptr, stream);
             timer.end(VesinB200StageScanCells);
             timer.begin(VesinB200StageScatter);
-            launch_scatter(
-                source, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(), ws.cell_start.as<int32_t>(), n_cells,
-                sorted, nullptr, ws.d_header, stream
-            );
+            launch_scatter(source, 0, n_points, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, stream);
             timer.end(VesinB200StageScatter);
         }
         const auto collect_front_stages = [&]() {
@@ -1317,19 +1308,13 @@ void neighbors_slab_core(
 
         const size_t n_cells = static_cast<size_t>(plan.n_cells_total);
         const size_t n_slots = std::max<size_t>(n_index, 1);
-        ws.cell_of.reserve(n_slots * sizeof(int32_t));
         ws.rank.reserve(n_slots * sizeof(int32_t));
-        ws.shift.reserve(n_slots * 3 * sizeof(int32_t));
         ws.cell_count.reserve(n_cells * sizeof(int32_t));
         ws.cell_start.reserve((n_cells + 1) * sizeof(int32_t));
-        ws.sorted_pos.reserve(n_slots * 3 * sizeof(double));
-        ws.sorted_index.reserve(n_slots * sizeof(int32_t));
-        ws.sorted_shift.reserve(n_slots * 3 * sizeof(int32_t));
-        ws.sorted_global.reserve(n_slots * sizeof(int32_t));
+        ws.sorted_records.reserve(n_slots * sizeof(PointRecord));
+        ws.sorted_wide_shift.reserve(n_slots * 3 * sizeof(int32_t));
         ws.scan_tmp.reserve(scan_tmp_bytes(std::max(n_slots, n_cells)));
-        SortedPoints sorted{ws.sorted_pos.as<double>(), ws.sorted_index.as<int32_t>(), ws.sorted_shift.as<int32_t>()};
-        // the pair pass writes global indices: it reads them where a plain build keeps local ones
-        SortedPoints sorted_for_pairs{sorted.pos, ws.sorted_global.as<int32_t>(), sorted.shift};
+        SortedPoints sorted{ws.sorted_records.as<PointRecord>(), ws.sorted_wide_shift.as<int32_t>()};
 
         // Cut along the last direction: the cells of the owned layers come first in the cell
         // order (see window_storage_layer), so the owned points are sorted on their own, while
@@ -1351,7 +1336,7 @@ void neighbors_slab_core(
         launch_header_reset(ws.d_header, ws.cell_count.as<int32_t>(), n_cells, stream);
         // points of the caller's array first: their binning runs while the messages are on their way
         launch_bin(
-            source, 0, n_array, plan, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(), ws.cell_count.as<int32_t>(),
+            source, 0, n_array, plan, ws.rank.as<int32_t>(), ws.cell_count.as<int32_t>(),
             ws.d_header, true, true, stream
         );
         timer.end(VesinB200StageBin);
@@ -1360,10 +1345,7 @@ void neighbors_slab_core(
             launch_scan_cells(ws.cell_count.as<int32_t>(), ws.cell_start.as<int32_t>(), owned_cells, ws.scan_tmp.ptr, stream);
             timer.end(VesinB200StageScanCells);
             timer.begin(VesinB200StageScatter);
-            launch_scatter(
-                source, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(), ws.cell_start.as<int32_t>(), n_cells, sorted,
-                ws.sorted_global.as<int32_t>(), ws.d_header, stream, 0, n_array
-            );
+            launch_scatter(source, 0, n_array, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, stream);
             timer.end(VesinB200StageScatter);
             cudaStream_t halo_stream = stream;
             const size_t pass_capacity = count_only ? 0 : capacity;
@@ -1377,7 +1359,7 @@ void neighbors_slab_core(
                 start_exchange_once(); // before the interior kernel takes every SM
                 VB200_CUDA(cudaEventRecord(ws.owned_sorted, stream));
                 launch_pairs(
-                    plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, target.view(), pass_capacity, ws.d_header, stream, 0, PAIR_PART_INTERIOR
+                    plan, ws.cell_start.as<int32_t>(), sorted, target.view(), pass_capacity, ws.d_header, stream, 0, PAIR_PART_INTERIOR
                 );
                 VB200_CUDA(cudaStreamWaitEvent(halo_stream, ws.owned_sorted, 0));
                 if (halo->received != nullptr) {
@@ -1389,20 +1371,17 @@ void neighbors_slab_core(
             }
             // the halo: binned, scanned behind the owned cells, scattered behind the owned records
             launch_bin(
-                source, n_array, n_index, plan, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(),
+                source, n_array, n_index, plan, ws.rank.as<int32_t>(),
                 ws.cell_count.as<int32_t>(), ws.d_header, true, false, halo_stream
             );
             launch_scan_cells(
                 ws.cell_count.as<int32_t>() + owned_cells, ws.cell_start.as<int32_t>() + owned_cells, n_cells - owned_cells, ws.scan_tmp.ptr,
                 halo_stream, ws.cell_start.as<int32_t>() + owned_cells
             );
-            launch_scatter(
-                source, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(), ws.cell_start.as<int32_t>(), n_cells, sorted,
-                ws.sorted_global.as<int32_t>(), ws.d_header, halo_stream, n_array, n_index
-            );
+            launch_scatter(source, n_array, n_index, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, halo_stream);
             if (overlapped) {
                 launch_pairs(
-                    plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, target.view(), pass_capacity, ws.d_header, halo_stream, 0, PAIR_PART_BOUNDARY
+                    plan, ws.cell_start.as<int32_t>(), sorted, target.view(), pass_capacity, ws.d_header, halo_stream, 0, PAIR_PART_BOUNDARY
                 );
                 // everything queued on `stream` from here on comes after both parts
                 VB200_CUDA(cudaEventRecord(ws.side_done, halo_stream));
@@ -1417,7 +1396,7 @@ void neighbors_slab_core(
                 timer.begin(VesinB200StageHalo);
                 await_messages();
                 launch_bin(
-                    source, n_array, n_index, plan, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(),
+                    source, n_array, n_index, plan, ws.rank.as<int32_t>(),
                     ws.cell_count.as<int32_t>(), ws.d_header, true, false, stream
                 );
                 timer.end(VesinB200StageHalo);
@@ -1426,10 +1405,7 @@ void neighbors_slab_core(
             launch_scan_cells(ws.cell_count.as<int32_t>(), ws.cell_start.as<int32_t>(), n_cells, ws.scan_tmp.ptr, stream);
             timer.end(VesinB200StageScanCells);
             timer.begin(VesinB200StageScatter);
-            launch_scatter(
-                source, ws.cell_of.as<int32_t>(), ws.rank.as<int32_t>(), ws.shift.as<int32_t>(), ws.cell_start.as<int32_t>(), n_cells, sorted,
-                ws.sorted_global.as<int32_t>(), ws.d_header, stream
-            );
+            launch_scatter(source, 0, n_index, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, stream);
             timer.end(VesinB200StageScatter);
         }
 
@@ -1439,7 +1415,7 @@ void neighbors_slab_core(
             const size_t pass_capacity = count_only ? 0 : capacity;
             if (!(attempt == 0 && pairs_launched)) {
                 timer.begin(VesinB200StageEmit);
-                launch_pairs(plan, ws.cell_start.as<int32_t>(), sorted_for_pairs, target.view(), pass_capacity, ws.d_header, stream);
+                launch_pairs(plan, ws.cell_start.as<int32_t>(), sorted, target.view(), pass_capacity, ws.d_header, stream);
                 timer.end(VesinB200StageEmit);
             }
             VB200_CUDA(cudaGetLastError());

@@ -41,12 +41,22 @@ constexpr unsigned int STATUS_HALO_OVERFLOW = 16u; // slab decomposition: a halo
 constexpr unsigned int STATUS_INDEX_RANGE = 32u;   // slab decomposition: a global index does not fit 31 bits
 constexpr unsigned long long NO_BAD_POINT = ~0ull;
 
-/// Cell-sorted copy of the points ("records"): original position, original
-/// index and the wrap shift that brings the point into the box.
+/// One cell-sorted point: original position, the index written into the pairs
+/// (the caller's, or the global one of a slab-decomposed system) and the wrap
+/// shift that brings the point into the box, three components in 10 bits each.
+/// 32 bytes, one sector: written with one store by the scatter, read with one
+/// load by the pair passes.
+struct alignas(32) PointRecord {
+    double x, y, z;
+    int32_t index;
+    uint32_t shift; // (s + WRAP_BIAS) per component; WRAP_WIDE: the shift is in SortedPoints::wide_shift
+};
+constexpr int WRAP_BIAS = 512;
+constexpr uint32_t WRAP_WIDE = 0x80000000u;
+
 struct SortedPoints {
-    double* pos;    // [n][3]
-    int32_t* index; // [n]
-    int32_t* shift; // [n][3]
+    PointRecord* records; // [n]
+    int32_t* wide_shift;  // [n][3], written for records whose shift does not fit 10 bits per component
 };
 
 /// Output arrays of a build; null pointers are not written. The indices go to `pairs`
@@ -132,8 +142,8 @@ void launch_bounds(const PointSource& source, DeviceHeader* header, cudaStream_t
 /// Bins the local indices [first, last). `chained`: the launch follows the
 /// previous kernel of the stream as a programmatic dependent launch.
 void launch_bin(
-    const PointSource& source, size_t first, size_t last, const GridPlan& plan, int32_t* cell_of, int32_t* rank, int32_t* shift,
-    int32_t* cell_count, DeviceHeader* header, bool check_points, bool chained, cudaStream_t stream
+    const PointSource& source, size_t first, size_t last, const GridPlan& plan, int32_t* rank, int32_t* cell_count, DeviceHeader* header,
+    bool check_points, bool chained, cudaStream_t stream
 );
 
 /// Exclusive scan of int32 counts into int32 starts (n + 1 entries).
@@ -149,16 +159,13 @@ void launch_scan_rows(
 /// Bytes of temporary storage the scans need for n elements.
 size_t scan_tmp_bytes(size_t n);
 
-/// Counting-sort scatter into the cell-sorted records. `n_cells`: cells of the
-/// plan (cell_start[n_cells] is the number of records). `sorted_global`, when
-/// not null, receives the global index of every record (31 bits; a larger one
-/// sets STATUS_INDEX_RANGE). With [first, last): only these local indices are
-/// scattered and only these records gathered (a slab build sorts its owned
-/// points, whose records come first, before the halo has arrived).
+/// Counting-sort scatter of the local indices [first, last) into the cell-sorted
+/// records (a slab build scatters its owned points, whose records come first,
+/// before the halo has arrived). Where the source has global indices, those go
+/// into the records (31 bits; a larger one sets STATUS_INDEX_RANGE).
 void launch_scatter(
-    const PointSource& source, const int32_t* cell_of, const int32_t* rank, const int32_t* shift, const int32_t* cell_start,
-    size_t n_cells, SortedPoints sorted, int32_t* sorted_global, DeviceHeader* header, cudaStream_t stream, size_t first = 0,
-    size_t last = static_cast<size_t>(-1)
+    const PointSource& source, size_t first, size_t last, const GridPlan& plan, const int32_t* rank, const int32_t* cell_start,
+    SortedPoints sorted, DeviceHeader* header, cudaStream_t stream
 );
 
 /// Small systems: header reset and plan check (when `speculative`), binning,
@@ -168,8 +175,8 @@ void launch_scatter(
 /// between two runs of those). Use when small_front_fits().
 bool small_front_fits(size_t n_points, const GridPlan& plan);
 void launch_small_front(
-    RealView points, size_t n, const GridPlan& plan, int32_t* cell_of, int32_t* rank, int32_t* shift, int32_t* cell_start,
-    SortedPoints sorted, DeviceHeader* header, RealView box, const bool* periodic, bool speculative, const double expected_box[9],
+    RealView points, size_t n, const GridPlan& plan, int32_t* rank, int32_t* cell_start, SortedPoints sorted, DeviceHeader* header,
+    RealView box, const bool* periodic, bool speculative, const double expected_box[9],
     const bool expected_periodic[3], cudaStream_t stream
 );
 
@@ -207,9 +214,7 @@ void launch_sort_rows(
 /// stencil once and writes the pairs into ranges claimed from
 /// header->pair_cursor. Blocks whose range would pass `capacity` (in pairs)
 /// only count.
-/// The indices written into the pairs are sorted.index: for a slab of a
-/// decomposed system (plan.window_axis >= 0) the caller passes the records'
-/// global indices there.
+/// The indices written into the pairs are those of the records.
 /// Slab builds cut along the last direction can launch the pair kernel in two parts: the
 /// units whose candidates are all owned points (they need nothing from the halo), and the
 /// units next to the halo. PAIR_PART_ALL launches both, back to back.
@@ -277,19 +282,18 @@ struct VerletState {
 };
 
 /// Candidates (pairs + shifts of a half list) to 12-byte records: the two
-/// points as positions in the cell-sorted order `sorted_index` (position ->
-/// index) of the build that found them, and the three shift components in 10
+/// points as positions in the cell-sorted order `sorted` of the build that found them, and the three shift components in 10
 /// bits each; a shift outside [-512, 511] sets state->unpackable. `rank_of`:
 /// n_points words of scratch (index -> position).
 void launch_verlet_pack(
-    const unsigned long long* pairs, const int32_t* shifts, size_t n, const int32_t* sorted_index, size_t n_points, uint32_t* rank_of,
+    const unsigned long long* pairs, const int32_t* shifts, size_t n, const PointRecord* sorted, size_t n_points, uint32_t* rank_of,
     uint32_t* records, VerletState* state, cudaStream_t stream
 );
 
-/// Row p of `positions` (4 doubles, 32 bytes) = x, y, z of points[sorted_index[p]]
-/// and sorted_index[p] as raw bits (nothing when state->stale is set).
+/// Row p of `positions` (4 doubles, 32 bytes) = x, y, z of the point of record p as
+/// it is now, and its index as raw bits (nothing when state->stale is set).
 void launch_verlet_positions(
-    RealView points, const int32_t* sorted_index, size_t n_points, double* positions, const VerletState* state, cudaStream_t stream
+    RealView points, const PointRecord* sorted, size_t n_points, double* positions, const VerletState* state, cudaStream_t stream
 );
 
 /// Sets state->stale when some point moved further than (skin - corner
@@ -306,7 +310,7 @@ void launch_verlet_check(
 /// gets both orientations of every kept record. Does nothing when
 /// state->stale is set. Ranges past `capacity` are counted, not written.
 void launch_verlet_filter(
-    const uint32_t* records, size_t n, const double* positions, const int32_t* sorted_index, RealView box, double cutoff2, bool full,
+    const uint32_t* records, size_t n, const double* positions, RealView box, double cutoff2, bool full,
     PairOutput out, unsigned long long capacity, VerletState* state, cudaStream_t stream
 );
 

@@ -58,19 +58,16 @@ constexpr size_t align_up(size_t value) {
 
 // carve-up of the scratch array (byte offsets, each 256-byte aligned)
 constexpr size_t OFF_HEADER = 0;
-constexpr size_t OFF_CELL_OF = OFF_HEADER + align_up(sizeof(DeviceHeader));
-constexpr size_t OFF_RANK = OFF_CELL_OF + align_up(MAX_POINTS * sizeof(int32_t));
-constexpr size_t OFF_SHIFT = OFF_RANK + align_up(MAX_POINTS * sizeof(int32_t));
-constexpr size_t OFF_CELL_COUNT = OFF_SHIFT + align_up(MAX_POINTS * 3 * sizeof(int32_t));
+constexpr size_t OFF_RANK = OFF_HEADER + align_up(sizeof(DeviceHeader));
+constexpr size_t OFF_CELL_COUNT = OFF_RANK + align_up(MAX_POINTS * sizeof(int32_t));
 constexpr size_t OFF_CELL_START = OFF_CELL_COUNT + align_up(MAX_CELLS * sizeof(int32_t));
-constexpr size_t OFF_SORTED_POS = OFF_CELL_START + align_up((MAX_CELLS + 1) * sizeof(int32_t));
-constexpr size_t OFF_SORTED_INDEX = OFF_SORTED_POS + align_up(MAX_POINTS * 3 * sizeof(double));
-constexpr size_t OFF_SORTED_SHIFT = OFF_SORTED_INDEX + align_up(MAX_POINTS * sizeof(int32_t));
-constexpr size_t OFF_SCAN_TMP = OFF_SORTED_SHIFT + align_up(MAX_POINTS * 3 * sizeof(int32_t));
+constexpr size_t OFF_RECORDS = OFF_CELL_START + align_up((MAX_CELLS + 1) * sizeof(int32_t));
+constexpr size_t OFF_WIDE_SHIFT = OFF_RECORDS + align_up(MAX_POINTS * sizeof(PointRecord));
+constexpr size_t OFF_SCAN_TMP = OFF_WIDE_SHIFT + align_up(MAX_POINTS * 3 * sizeof(int32_t));
 constexpr size_t SCAN_TMP_BYTES = 4096;
 constexpr size_t SCRATCH_BYTES = OFF_SCAN_TMP + SCAN_TMP_BYTES;
 
-// The scratch itself: about 2.3 MB per GPU. In host code this name is only a
+// The scratch itself: about 1.9 MB per GPU. In host code this name is only a
 // handle for cudaGetSymbolAddress, never a device address.
 static __device__ __align__(256) unsigned char NO_ALLOC_SCRATCH[SCRATCH_BYTES];
 
@@ -150,16 +147,10 @@ size_t build(
     }
     unsigned char* base = state.scratch;
     auto* d_header = reinterpret_cast<DeviceHeader*>(base + OFF_HEADER);
-    auto* cell_of = reinterpret_cast<int32_t*>(base + OFF_CELL_OF);
     auto* rank = reinterpret_cast<int32_t*>(base + OFF_RANK);
-    auto* shift = reinterpret_cast<int32_t*>(base + OFF_SHIFT);
     auto* cell_count = reinterpret_cast<int32_t*>(base + OFF_CELL_COUNT);
     auto* cell_start = reinterpret_cast<int32_t*>(base + OFF_CELL_START);
-    SortedPoints sorted{
-        reinterpret_cast<double*>(base + OFF_SORTED_POS),
-        reinterpret_cast<int32_t*>(base + OFF_SORTED_INDEX),
-        reinterpret_cast<int32_t*>(base + OFF_SORTED_SHIFT),
-    };
+    SortedPoints sorted{reinterpret_cast<PointRecord*>(base + OFF_RECORDS), reinterpret_cast<int32_t*>(base + OFF_WIDE_SHIFT)};
     void* scan_tmp = base + OFF_SCAN_TMP;
     cudaStream_t stream = nullptr; // legacy default stream
 
@@ -189,12 +180,10 @@ size_t build(
 
     // the histogram is the one array that has to start at zero
     check(cudaMemsetAsync(cell_count, 0, static_cast<size_t>(plan.n_cells_total) * sizeof(int32_t), stream), "cudaMemsetAsync");
-    launch_bin(flat_source(RealView{points, 0}, n_points), 0, n_points, plan, cell_of, rank, shift, cell_count, d_header, false, true, stream);
+    const PointSource source = flat_source(RealView{points, 0}, n_points);
+    launch_bin(source, 0, n_points, plan, rank, cell_count, d_header, false, true, stream);
     launch_scan_cells(cell_count, cell_start, static_cast<size_t>(plan.n_cells_total), scan_tmp, stream);
-    launch_scatter(
-        flat_source(RealView{points, 0}, n_points), cell_of, rank, shift, cell_start, static_cast<size_t>(plan.n_cells_total), sorted, nullptr,
-        d_header, stream
-    );
+    launch_scatter(source, 0, n_points, plan, rank, cell_start, sorted, d_header, stream);
     launch_pairs(plan, cell_start, sorted, out, capacity, d_header, stream);
     check(cudaGetLastError(), "launch");
     check(cudaMemcpy(&header, d_header, sizeof(header), cudaMemcpyDeviceToHost), "cudaMemcpy(header)");

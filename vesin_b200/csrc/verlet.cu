@@ -46,10 +46,10 @@ __device__ __forceinline__ double load_value(const RealView& view, size_t k) {
 // ---------------------------------------------------------------------------
 
 /// rank_of[i] = position of point i in the cell-sorted order.
-__global__ void __launch_bounds__(VERLET_THREADS) verlet_rank_kernel(const int32_t* __restrict__ sorted_index, size_t n, uint32_t* __restrict__ rank_of) {
+__global__ void __launch_bounds__(VERLET_THREADS) verlet_rank_kernel(const PointRecord* __restrict__ sorted, size_t n, uint32_t* __restrict__ rank_of) {
     const size_t p = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (p < n) {
-        rank_of[sorted_index[p]] = static_cast<uint32_t>(p);
+        rank_of[sorted[p].index] = static_cast<uint32_t>(p);
     }
 }
 
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(VERLET_THREADS) verlet_pack_kernel(
 /// gathers touch a different cache line per lane, so the number of load
 /// instructions is what they cost.
 __global__ void __launch_bounds__(VERLET_THREADS) verlet_positions_kernel(
-    const RealView points, const int32_t* __restrict__ sorted_index, size_t n, double* __restrict__ positions, const VerletState* state
+    const RealView points, const PointRecord* __restrict__ sorted, size_t n, double* __restrict__ positions, const VerletState* state
 ) {
     if (*reinterpret_cast<const volatile int*>(&state->stale)) {
         return;
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(VERLET_THREADS) verlet_positions_kernel(
     }
     const size_t p = f >> 2;
     const size_t c = f & 3;
-    const int32_t index = sorted_index[p];
+    const int32_t index = sorted[p].index;
     positions[f] = (c == 3) ? __longlong_as_double(static_cast<long long>(index)) : load_value(points, 3 * static_cast<size_t>(index) + c);
 }
 
@@ -206,7 +206,7 @@ __device__ __forceinline__ double record_pair(
 /// capacity is counted only. Called by every thread; ends with a barrier.
 template <bool FULL>
 __device__ __forceinline__ void write_kept(
-    FilterShared& sh, const double* __restrict__ positions, const int32_t* __restrict__ sorted_index, const PairOutput& out,
+    FilterShared& sh, const double* __restrict__ positions, const PairOutput& out,
     unsigned long long capacity, VerletState* state, int n_write
 ) {
     const int lane = threadIdx.x & 31;
@@ -255,8 +255,7 @@ __device__ __forceinline__ void write_kept(
 
 template <bool FULL>
 __global__ void __launch_bounds__(VERLET_THREADS) verlet_filter_kernel(
-    const uint32_t* __restrict__ records, size_t n, const double* __restrict__ positions, const int32_t* __restrict__ sorted_index,
-    const RealView box, double cutoff2, PairOutput out, unsigned long long capacity, VerletState* state
+    const uint32_t* __restrict__ records, size_t n, const double* __restrict__ positions, const RealView box, double cutoff2, PairOutput out, unsigned long long capacity, VerletState* state
 ) {
     __shared__ FilterShared sh;
     if (*reinterpret_cast<volatile int*>(&state->stale)) {
@@ -305,7 +304,7 @@ __global__ void __launch_bounds__(VERLET_THREADS) verlet_filter_kernel(
         __syncthreads();
         const int n_kept = sh.n_kept; // fewer than 2 * FILTER_CHUNK: below FILTER_CHUNK before this round
         if (n_kept >= FILTER_CHUNK) {
-            write_kept<FULL>(sh, positions, sorted_index, out, capacity, state, FILTER_CHUNK);
+            write_kept<FULL>(sh, positions, out, capacity, state, FILTER_CHUNK);
             // what is left moves to the front of the list
             uint32_t moved[3] = {0, 0, 0};
             const int left = n_kept - FILTER_CHUNK;
@@ -328,19 +327,19 @@ __global__ void __launch_bounds__(VERLET_THREADS) verlet_filter_kernel(
     }
     const int n_kept = sh.n_kept;
     if (n_kept > 0) {
-        write_kept<FULL>(sh, positions, sorted_index, out, capacity, state, n_kept);
+        write_kept<FULL>(sh, positions, out, capacity, state, n_kept);
     }
 }
 
 } // namespace
 
 void launch_verlet_pack(
-    const unsigned long long* pairs, const int32_t* shifts, size_t n, const int32_t* sorted_index, size_t n_points, uint32_t* rank_of,
+    const unsigned long long* pairs, const int32_t* shifts, size_t n, const PointRecord* sorted, size_t n_points, uint32_t* rank_of,
     uint32_t* records, VerletState* state, cudaStream_t stream
 ) {
     if (n_points != 0) {
         const size_t blocks = (n_points + VERLET_THREADS - 1) / VERLET_THREADS;
-        verlet_rank_kernel<<<static_cast<unsigned>(blocks), VERLET_THREADS, 0, stream>>>(sorted_index, n_points, rank_of);
+        verlet_rank_kernel<<<static_cast<unsigned>(blocks), VERLET_THREADS, 0, stream>>>(sorted, n_points, rank_of);
     }
     if (n == 0) {
         return;
@@ -350,13 +349,13 @@ void launch_verlet_pack(
 }
 
 void launch_verlet_positions(
-    RealView points, const int32_t* sorted_index, size_t n_points, double* positions, const VerletState* state, cudaStream_t stream
+    RealView points, const PointRecord* sorted, size_t n_points, double* positions, const VerletState* state, cudaStream_t stream
 ) {
     if (n_points == 0) {
         return;
     }
     const size_t blocks = (4 * n_points + VERLET_THREADS - 1) / VERLET_THREADS;
-    verlet_positions_kernel<<<static_cast<unsigned>(blocks), VERLET_THREADS, 0, stream>>>(points, sorted_index, n_points, positions, state);
+    verlet_positions_kernel<<<static_cast<unsigned>(blocks), VERLET_THREADS, 0, stream>>>(points, sorted, n_points, positions, state);
 }
 
 void launch_verlet_check(
@@ -370,7 +369,7 @@ void launch_verlet_check(
 }
 
 void launch_verlet_filter(
-    const uint32_t* records, size_t n, const double* positions, const int32_t* sorted_index, RealView box, double cutoff2, bool full,
+    const uint32_t* records, size_t n, const double* positions, RealView box, double cutoff2, bool full,
     PairOutput out, unsigned long long capacity, VerletState* state, cudaStream_t stream
 ) {
     if (n == 0) {
@@ -383,11 +382,11 @@ void launch_verlet_filter(
     const size_t blocks = std::max<size_t>(1, std::min<size_t>(rounds, 148 * 8));
     if (full) {
         verlet_filter_kernel<true><<<static_cast<unsigned>(blocks), VERLET_THREADS, 0, stream>>>(
-            records, n, positions, sorted_index, box, cutoff2, out, capacity, state
+            records, n, positions, box, cutoff2, out, capacity, state
         );
     } else {
         verlet_filter_kernel<false><<<static_cast<unsigned>(blocks), VERLET_THREADS, 0, stream>>>(
-            records, n, positions, sorted_index, box, cutoff2, out, capacity, state
+            records, n, positions, box, cutoff2, out, capacity, state
         );
     }
 }
