@@ -108,6 +108,7 @@ struct Workspace {
     DeviceBuffer masks, unit_mask_base, unit_words, unit_count, unit_start;
     DeviceBuffer row_count, row_start, row_fill, scan_tmp;
     DeviceBuffer batch_offsets; // batches: where each system starts in the points array
+    DeviceBuffer batch_shares;  // ... and the pairs each of the CTAs that share a system has
     DeviceBuffer checksum;      // 4 words of vesin_b200_list_checksum
     bool values_float = false;  // element type of `distances` / `vectors` of the last build
 
@@ -170,7 +171,7 @@ struct Workspace {
     ~Workspace() {
         for (DeviceBuffer* buffer :
              {&rank, &cell_count, &cell_start, &sorted_records, &sorted_wide_shift, &masks, &unit_mask_base,
-              &unit_words, &unit_count, &unit_start, &row_count, &row_start, &row_fill, &scan_tmp, &batch_offsets, &checksum, &out_pairs,
+              &unit_words, &unit_count, &unit_start, &row_count, &row_start, &row_fill, &scan_tmp, &batch_offsets, &batch_shares, &checksum, &out_pairs,
               &out_shifts, &out_distances, &out_vectors, &alt_pairs, &alt_shifts, &alt_distances, &alt_vectors}) {
             buffer->release();
         }
@@ -1152,6 +1153,10 @@ void neighbors_batch(
 
     // systems with a periodic direction or many points take the CTA-per-system kernel
     const bool any_for_cta_kernel = periodic != nullptr || largest > molecules_max_points();
+    if (any_for_cta_kernel && n_systems > 0) {
+        ws.batch_shares.reserve(n_systems * small_splits(in.n_systems, largest) * sizeof(unsigned long long));
+    }
+    auto* share_count = ws.batch_shares.as<unsigned long long>();
     Target target(list, ws, options, float_io, caller);
     // A list that was filled before writes into the arrays it has, right behind the counting pass
     // and the scan, without waiting for the host to see the total: one read-back per call. A
@@ -1161,13 +1166,13 @@ void neighbors_batch(
     const bool speculative = n_systems > 0 && existing > 256;
     size_t total = 0;
     if (n_systems > 0) {
-        launch_small_count(in, largest, any_for_cta_kernel, ws.unit_count.as<unsigned long long>(), ws.d_header, stream);
+        launch_small_count(in, largest, any_for_cta_kernel, ws.unit_count.as<unsigned long long>(), share_count, ws.d_header, stream);
         launch_scan_units(
             ws.unit_count.as<unsigned long long>(), system_start, n_systems, ws.scan_tmp.ptr,
             &ws.d_header->total_pairs, stream
         );
         if (speculative) {
-            launch_small_emit(in, largest, any_for_cta_kernel, system_start, target.view(), ws.d_header, stream, existing);
+            launch_small_emit(in, largest, any_for_cta_kernel, system_start, share_count, target.view(), ws.d_header, stream, existing);
         }
         VB200_CUDA(cudaGetLastError());
         read_header(ws);
@@ -1197,7 +1202,7 @@ void neighbors_batch(
         if (total > existing) {
             speculative ? target.grow(total) : target.reserve(total);
         }
-        launch_small_emit(in, largest, any_for_cta_kernel, system_start, target.view(), ws.d_header, stream);
+        launch_small_emit(in, largest, any_for_cta_kernel, system_start, share_count, target.view(), ws.d_header, stream);
         VB200_CUDA(cudaGetLastError());
     }
     VB200_CUDA(cudaStreamSynchronize(stream));

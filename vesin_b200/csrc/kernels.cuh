@@ -250,17 +250,21 @@ void configure_small_systems();
 /// Pass 1: pairs of every system -> system_count; the first non-finite point
 /// and the first singular box are reported through the header.
 /// (`any_for_cta_kernel`: some system is periodic or has more points than
-/// molecules_max_points(), so the CTA-per-system kernel runs as well.)
+/// molecules_max_points(), so the kernel with CTAs per system runs as well: small_splits() CTAs
+/// per system, which leave the pairs of their tiles in `share_count`, n_systems x small_splits()
+/// words that pass 2 wants back.)
+unsigned small_splits(unsigned n_systems, size_t max_points);
 void launch_small_count(
-    const BatchInput& in, size_t max_points, bool any_for_cta_kernel, unsigned long long* system_count, DeviceHeader* header, cudaStream_t stream
+    const BatchInput& in, size_t max_points, bool any_for_cta_kernel, unsigned long long* system_count, unsigned long long* share_count,
+    DeviceHeader* header, cudaStream_t stream
 );
 /// Largest system the warp-per-system kernel takes.
 size_t molecules_max_points();
 /// Pass 2: every system writes its pairs at system_start[system]; a system whose block ends
 /// beyond `capacity` elements writes nothing (the pass may run before the host knows the total).
 void launch_small_emit(
-    const BatchInput& in, size_t max_points, bool any_for_cta_kernel, const unsigned long long* system_start, PairOutput out,
-    DeviceHeader* header, cudaStream_t stream, unsigned long long capacity = ~0ull
+    const BatchInput& in, size_t max_points, bool any_for_cta_kernel, const unsigned long long* system_start,
+    unsigned long long* share_count, PairOutput out, DeviceHeader* header, cudaStream_t stream, unsigned long long capacity = ~0ull
 );
 
 /// Order-independent checksum of a list: result[0], result[1] = two sums

@@ -1,14 +1,21 @@
 // Batches of independent small systems. Two passes (count, emit) so that every
 // system owns one contiguous, exactly sized block of the output. Two kernels:
 //   * molecules (no periodic direction, at most 96 points): a WARP per system,
-//     eight systems per CTA; lanes take the pairs i < j of the flattened upper
-//     triangle, decide them with an fp32 screen (coordinates relative to the
-//     first point) and the exact fp64 predicate inside the error band, gather
-//     the hits in a per-warp list and write them 32 at a time through the
-//     coalesced stores of the large-system kernels;
-//   * everything else (periodic systems, up to 2048 points): a CTA per system,
-//     all pairs times the periodic images that can reach the cutoff, exact fp64
-//     predicate for every candidate.
+//     eight systems per CTA;
+//   * everything else (periodic systems, up to 2048 points): one or more CTAs
+//     per system, which list the periodic images that can reach a tile of home
+//     points and stage them a batch at a time.
+// Both decide like the pair kernel of large systems: a lane per home point,
+// candidates broadcast from shared memory four at a time, an fp32 screen on
+// coordinates relative to a point of the system (two candidates per packed
+// instruction) that leaves one hit bit per candidate, and the exact fp64
+// predicate inside the error band. Hits gather in a per-warp list and leave 32
+// at a time through the coalesced stores of the large-system kernels. Walking
+// the (i, j) of the flattened triangle instead, a square root and a few
+// corrections per candidate, the 16 384 molecules of 16 to 64 atoms (float, 5.3 M
+// pairs) took 64 us to count and 120 us to write; now 23 and 64 (the 230 MB of the
+// list take 35 us at the copy bandwidth: half the time is the chain of a warp,
+// points -> decisions -> list -> stores).
 //
 // Replaces, for this use, the per-system loop of the callers
 // (python/vesin/vesin/metatomic/_neighbors.py:197-199) and the brute-force
@@ -20,7 +27,7 @@
 #include "emit.cuh"
 #include "plan.hpp"
 
-#include <cfloat>
+#include <algorithm>
 
 namespace vb200 {
 
@@ -33,8 +40,8 @@ constexpr unsigned FULL_MASK = 0xffffffffu;
 struct SystemFrame {
     double H[3][3];    // box, rows of non-periodic directions replaced by unit vectors
     double Hinv[3][3];
+    double reach[3];   // fractional distance within which points can be neighbors
     int periodic[3];
-    int reach[3];      // images to try on each side of the nearest one
     int singular;
 };
 
@@ -54,7 +61,7 @@ __device__ __forceinline__ void unit3(double v[3]) {
 /// Same normalisation of the box as the host plan (and as the reference CPU
 /// path, vesin/src/types.hpp:41-97): rows of non-periodic directions become
 /// unit vectors orthogonal to the periodic ones.
-__device__ void make_frame(SystemFrame& frame, const BatchInput& in, unsigned system, const bool* periodic, double cutoff) {
+__device__ void normalise_box(SystemFrame& frame, const BatchInput& in, unsigned system, const bool* periodic) {
     int n_periodic = 0, first = -1, second = -1;
     for (int i = 0; i < 3; i++) {
         for (int j = 0; j < 3; j++) {
@@ -103,38 +110,47 @@ __device__ void make_frame(SystemFrame& frame, const BatchInput& in, unsigned sy
             frame.H[3 - first - second][k] = c[k];
         }
     }
-    const double (*m)[3] = frame.H;
-    double det = m[0][0] * (m[1][1] * m[2][2] - m[2][1] * m[1][2]) - m[0][1] * (m[1][0] * m[2][2] - m[1][2] * m[2][0]) +
-                 m[0][2] * (m[1][0] * m[2][1] - m[1][1] * m[2][0]);
-    frame.singular = !(fabs(det) >= 1e-30);
-    if (frame.singular) {
-        return;
+}
+
+/// The frame of a system by one warp: the box by its first lane, the entries of the inverse by
+/// nine lanes, the reach of the images by three. Ends with a __syncwarp().
+__device__ void make_frame(SystemFrame& frame, const BatchInput& in, unsigned system, int lane) {
+    if (lane == 0) {
+        normalise_box(frame, in, system, in.periodic != nullptr ? in.periodic + 3 * static_cast<size_t>(system) : nullptr);
     }
-    double (*inv)[3] = frame.Hinv;
-    inv[0][0] = (m[1][1] * m[2][2] - m[2][1] * m[1][2]) / det;
-    inv[0][1] = (m[0][2] * m[2][1] - m[0][1] * m[2][2]) / det;
-    inv[0][2] = (m[0][1] * m[1][2] - m[0][2] * m[1][1]) / det;
-    inv[1][0] = (m[1][2] * m[2][0] - m[1][0] * m[2][2]) / det;
-    inv[1][1] = (m[0][0] * m[2][2] - m[0][2] * m[2][0]) / det;
-    inv[1][2] = (m[1][0] * m[0][2] - m[0][0] * m[1][2]) / det;
-    inv[2][0] = (m[1][0] * m[2][1] - m[2][0] * m[1][1]) / det;
-    inv[2][1] = (m[2][0] * m[0][1] - m[0][0] * m[2][1]) / det;
-    inv[2][2] = (m[0][0] * m[1][1] - m[1][0] * m[0][1]) / det;
-    for (int k = 0; k < 3; k++) {
-        frame.reach[k] = 0;
-        if (frame.periodic[k]) {
-            // |fractional distance + image| * face distance <= |v| < cutoff, and the
-            // nearest image leaves at most half a cell: images within cutoff / d + 1/2
-            double inv_face = sqrt(inv[0][k] * inv[0][k] + inv[1][k] * inv[1][k] + inv[2][k] * inv[2][k]);
-            double reach = floor(cutoff * inv_face * (1.0 + 1e-9) + 0.5 + 1e-9);
-            frame.reach[k] = static_cast<int>(fmin(reach, 1.0e6));
+    __syncwarp();
+    const double (*m)[3] = frame.H;
+    const double det = m[0][0] * (m[1][1] * m[2][2] - m[2][1] * m[1][2]) - m[0][1] * (m[1][0] * m[2][2] - m[1][2] * m[2][0]) +
+                       m[0][2] * (m[1][0] * m[2][1] - m[1][1] * m[2][0]);
+    const bool singular = !(fabs(det) >= 1e-30);
+    if (lane < 9 && !singular) {
+        const int r = lane / 3;
+        const int c = lane % 3;
+        const int r1 = (r + 1) % 3, r2 = (r + 2) % 3;
+        const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
+        frame.Hinv[r][c] = (m[c1][r1] * m[c2][r2] - m[c1][r2] * m[c2][r1]) / det;
+    }
+    __syncwarp();
+    double images = 1.0;
+    if (lane < 3 && !singular) {
+        frame.reach[lane] = 0.0;
+        if (frame.periodic[lane]) {
+            // |fractional distance| * face distance <= |v| < cutoff
+            const double (*inv)[3] = frame.Hinv;
+            const double inv_face = sqrt(inv[0][lane] * inv[0][lane] + inv[1][lane] * inv[1][lane] + inv[2][lane] * inv[2][lane]);
+            frame.reach[lane] = in.cutoff * inv_face * (1.0 + 1e-9);
+            // images within cutoff / d + 1/2 of the nearest one, which is at most half a cell away
+            images = 2.0 * fmin(floor(frame.reach[lane] + 0.5 + 1e-9), 1.0e6) + 1.0;
+        } else {
+            frame.reach[lane] = in.cutoff * (1.0 + 1e-9); // the row is a unit vector orthogonal to the others
         }
     }
-    // images per pair: beyond the limit the system is refused (2: "cutoff too large for the box")
-    const double images = (2.0 * frame.reach[0] + 1.0) * (2.0 * frame.reach[1] + 1.0) * (2.0 * frame.reach[2] + 1.0);
-    if (images > static_cast<double>(MAX_STENCIL_CELLS)) {
-        frame.singular = 2;
+    images *= __shfl_sync(FULL_MASK, images, 1) * __shfl_sync(FULL_MASK, images, 2);
+    if (lane == 0) {
+        // beyond the limit of images per pair the system is refused (2: "cutoff too large for the box")
+        frame.singular = singular ? 1 : ((images > static_cast<double>(MAX_STENCIL_CELLS)) ? 2 : 0);
     }
+    __syncwarp();
 }
 
 __device__ __forceinline__ bool half_rule_small(int s0, int s1, int s2) {
@@ -170,51 +186,177 @@ __device__ __forceinline__ bool taken_by_warp_kernel(const BatchInput& in, unsig
     return !(periodic[0] || periodic[1] || periodic[2]);
 }
 
+// ---- the fp32 screen -------------------------------------------------------
+
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long packed;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(packed) : "f"(lo), "f"(hi));
+    return packed;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+/// Squared distances outside [lo, hi] are decided by the screen.
+struct ScreenBand {
+    float lo, hi;
+};
+
+/// The band for home points within `m` of the origin of the local frame. A candidate within the
+/// cutoff of one of them is then within M = m + cutoff of it: the band covers the rounding of the
+/// coordinates (relative error 2^-24 of values up to M), of the differences and of the sum. A
+/// candidate further out is at more than the cutoff by more than its own rounding error, as long
+/// as m is not thousands of times the cutoff; beyond that (or with m not finite) every candidate
+/// goes to the exact predicate.
+__device__ __forceinline__ ScreenBand screen_band(float m, double cutoff_exact, double cutoff2_exact) {
+    const float c = static_cast<float>(cutoff_exact) * 1.01f;
+    const float M = (m + c) * 1.0001f;
+    const float eps = 5.9604644775390625e-08f;
+    float band = 4.0f * eps * (2.0f * 1.7320508f * c * (2.0f * M + c) + 3.0f * c * c) + 40.0f * eps * eps * M * M + 4.0f * eps * c * c;
+    band *= 1.01f; // this expression is itself evaluated in fp32
+    const float cutoff2 = static_cast<float>(cutoff2_exact);
+    ScreenBand result{cutoff2 - band, cutoff2 + band};
+    if (!(m < 5.0e3f * c) || !(result.hi < 3.0e38f) || !(c > 1.0e-12f)) {
+        result = ScreenBand{-__int_as_float(0x7f800000), __int_as_float(0x7f800000)};
+    }
+    return result;
+}
+
+/// Screen of candidates [0, 4 * quads) of a word against the home point whose negated
+/// coordinates are (ax, ay, az): `inside` gets a bit for those surely within the cutoff, `maybe`
+/// for those and the ones only the exact predicate can decide. x, y, z: 16-byte aligned arrays in
+/// shared memory, the same addresses for every lane.
+__device__ __forceinline__ void screen_word(
+    const float* x, const float* y, const float* z, int quads, unsigned long long ax, unsigned long long ay, unsigned long long az,
+    const ScreenBand& band, unsigned& inside, unsigned& maybe
+) {
+    inside = 0;
+    maybe = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        if (k >= quads) {
+            break;
+        }
+        const ulonglong2 x4 = reinterpret_cast<const ulonglong2*>(x)[k];
+        const ulonglong2 y4 = reinterpret_cast<const ulonglong2*>(y)[k];
+        const ulonglong2 z4 = reinterpret_cast<const ulonglong2*>(z)[k];
+        const unsigned long long dx0 = add2(x4.x, ax), dy0 = add2(y4.x, ay), dz0 = add2(z4.x, az);
+        const unsigned long long dx1 = add2(x4.y, ax), dy1 = add2(y4.y, ay), dz1 = add2(z4.y, az);
+        const unsigned long long d0 = fma2(dx0, dx0, fma2(dy0, dy0, mul2(dz0, dz0)));
+        const unsigned long long d1 = fma2(dx1, dx1, fma2(dy1, dy1, mul2(dz1, dz1)));
+        float d2[4];
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(d2[0]), "=f"(d2[1]) : "l"(d0));
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(d2[2]), "=f"(d2[3]) : "l"(d1));
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            if (d2[c] < band.lo) {
+                inside |= 1u << (4 * k + c);
+            }
+            if (!(d2[c] > band.hi)) { // (NaN: the exact predicate decides)
+                maybe |= 1u << (4 * k + c);
+            }
+        }
+    }
+}
+
+/// Bits `first` and above of a word.
+__device__ __forceinline__ unsigned bits_from(int first) {
+    return (first <= 0) ? 0xffffffffu : ((first >= 32) ? 0u : (0xffffffffu << first));
+}
+
+constexpr int HIT_WINDOW = 224;                // hits a warp lists at a time
+constexpr int HIT_LIST = HIT_WINDOW + 32;      // ... behind fewer than 32 that wait for company
+
+/// Lists the hits of a word (bit b of lane l -> entry + b) behind the `listed` entries that are
+/// waiting, and hands them on in multiples of 32: write(n) writes entries [0, n) of the list.
+/// Lanes hold different numbers of hits; their order is that of the lanes.
+template <class Write>
+__device__ __forceinline__ void list_hits(unsigned bits, unsigned entry, unsigned short* list, int& listed, int lane, Write write) {
+    const int mine = __popc(bits);
+    int position = mine;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+        const int up = __shfl_up_sync(FULL_MASK, position, offset);
+        if (lane >= offset) {
+            position += up;
+        }
+    }
+    const int total = __shfl_sync(FULL_MASK, position, 31);
+    position -= mine;
+    for (int window = 0; window < total; window += HIT_WINDOW) {
+        while (bits != 0 && position < window + HIT_WINDOW) {
+            const int b = __ffs(bits) - 1;
+            bits &= bits - 1;
+            list[listed + position - window] = static_cast<unsigned short>(entry + b);
+            position++;
+        }
+        listed += min(HIT_WINDOW, total - window);
+        __syncwarp();
+        const int whole = listed & ~31;
+        if (whole != 0) {
+            write(whole);
+            listed -= whole;
+            // what is left moves to the front of the list
+            unsigned short moved = 0;
+            if (lane < listed) {
+                moved = list[whole + lane];
+            }
+            __syncwarp();
+            if (lane < listed) {
+                list[lane] = moved;
+            }
+            __syncwarp();
+        }
+    }
+}
+
 struct MoleculeShared {
+    alignas(16) float fx[MOLECULE_WARPS][MOLECULE_MAX_POINTS]; // relative to the first point of the system
+    alignas(16) float fy[MOLECULE_WARPS][MOLECULE_MAX_POINTS];
+    alignas(16) float fz[MOLECULE_WARPS][MOLECULE_MAX_POINTS];
     double x[MOLECULE_WARPS][MOLECULE_MAX_POINTS]; // original positions
     double y[MOLECULE_WARPS][MOLECULE_MAX_POINTS];
     double z[MOLECULE_WARPS][MOLECULE_MAX_POINTS];
-    float fx[MOLECULE_WARPS][MOLECULE_MAX_POINTS]; // relative to the first point of the system
-    float fy[MOLECULE_WARPS][MOLECULE_MAX_POINTS];
-    float fz[MOLECULE_WARPS][MOLECULE_MAX_POINTS];
     alignas(16) double transpose[MOLECULE_WARPS][TRANSPOSE_DOUBLES];
-    unsigned short list[MOLECULE_WARPS][64]; // hits waiting to be written: (i << 8) | j
+    unsigned short list[MOLECULE_WARPS][HIT_LIST]; // hits waiting to be written: (i << 8) | j
 };
+static_assert(MOLECULE_MAX_POINTS % 32 == 0 && MOLECULE_MAX_POINTS <= 256, "whole words of candidates, indices of 8 bits");
 
-/// Row i of the strict upper triangle of an n x n matrix starts at this
-/// position of the flattened triangle.
-__device__ __forceinline__ int triangle_row_start(int i, int n) {
-    return (i * (2 * n - i - 1)) >> 1;
+/// The reference's arithmetic for S = 0 (vesin/src/cpu_cell_list.cpp:135-138), operation for
+/// operation: the shift term is an exact zero.
+__device__ __forceinline__ double molecule_pair(const MoleculeShared& sh, int warp, int i, int j, double& vx, double& vy, double& vz) {
+    vx = __dadd_rn(__dsub_rn(sh.x[warp][j], sh.x[warp][i]), 0.0);
+    vy = __dadd_rn(__dsub_rn(sh.y[warp][j], sh.y[warp][i]), 0.0);
+    vz = __dadd_rn(__dsub_rn(sh.z[warp][j], sh.z[warp][i]), 0.0);
+    return __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
 }
 
-/// Writes `n_valid` hits of the warp's list (lane l takes entry l) at element
-/// `first` of the output: both orientations side by side for full lists.
-__device__ __forceinline__ void write_molecule_hits(
-    MoleculeShared& sh, const BatchInput& in, const PairOutput& out, int warp, int lane, unsigned long long first, int n_valid,
-    unsigned long long index_offset
+/// Writes the hits of up to 32 lanes from element `first` of the output on, both orientations
+/// side by side for full lists.
+__device__ __forceinline__ void write_hits(
+    double* transpose, const BatchInput& in, const PairOutput& out, int lane, unsigned long long first, int n_valid, unsigned long long gi,
+    unsigned long long gj, int s0, int s1, int s2, double d, double vx, double vy, double vz
 ) {
-    int i = 0, j = 0;
-    if (lane < n_valid) {
-        const unsigned entry = sh.list[warp][lane];
-        i = entry >> 8;
-        j = entry & 255;
-    }
-    // the reference's arithmetic for S = 0 (vesin/src/cpu_cell_list.cpp:135-138): the shift term is an exact zero
-    const double vx = __dadd_rn(__dsub_rn(sh.x[warp][j], sh.x[warp][i]), 0.0);
-    const double vy = __dadd_rn(__dsub_rn(sh.y[warp][j], sh.y[warp][i]), 0.0);
-    const double vz = __dadd_rn(__dsub_rn(sh.z[warp][j], sh.z[warp][i]), 0.0);
-    const double d = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz)));
-    const unsigned long long gi = index_offset + i;
-    const unsigned long long gj = index_offset + j;
-    if (in.full) {
-        if (out.interleave_ok) {
-            store_both(sh.transpose[warp], out, lane, first, n_valid, gi, gj, 0, 0, 0, d, vx, vy, vz);
-        } else {
-            store_pairs(sh.transpose[warp], out, lane, first, n_valid, gi, gj, 0, 0, 0, d, vx, vy, vz);
-            store_pairs(sh.transpose[warp], out, lane, first + n_valid, n_valid, gj, gi, 0, 0, 0, d, -vx, -vy, -vz);
-        }
+    if (!in.full) {
+        // half lists keep i <= j: the forward pair
+        store_pairs(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz);
+    } else if (out.interleave_ok) {
+        store_both(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz);
     } else {
-        store_pairs(sh.transpose[warp], out, lane, first, n_valid, gi, gj, 0, 0, 0, d, vx, vy, vz);
+        store_pairs(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz);
+        store_pairs(transpose, out, lane, first + n_valid, n_valid, gj, gi, -s0, -s1, -s2, d, -vx, -vy, -vz);
     }
 }
 
@@ -223,7 +365,8 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
     const BatchInput in, unsigned long long* __restrict__ system_count, const unsigned long long* __restrict__ system_start, PairOutput out,
     DeviceHeader* header, const unsigned long long capacity
 ) {
-    __shared__ MoleculeShared sh;
+    extern __shared__ __align__(16) unsigned char molecule_smem[];
+    MoleculeShared& sh = *reinterpret_cast<MoleculeShared*>(molecule_smem);
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const unsigned warps_in_grid = gridDim.x * MOLECULE_WARPS;
@@ -232,6 +375,9 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
         const unsigned long long begin = in.offsets[system];
         const int n = static_cast<int>(in.offsets[system + 1] - begin);
         if (!taken_by_warp_kernel(in, system, n)) {
+            if (!EMIT && lane == 0) {
+                system_count[system] = 0; // the CTAs of the other kernel add to it
+            }
             continue;
         }
         if (EMIT && system_start[system + 1] > capacity) {
@@ -239,15 +385,19 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
         }
         __syncwarp();
         // ---- the system's points: originals for the exact arithmetic, fp32 copies relative to the
-        //      first point for the screen; M bounds the relative coordinates ----
+        //      first point for the screen ----
         const double ox = (n > 0) ? batch_coordinate(in, 3 * begin + 0) : 0.0;
         const double oy = (n > 0) ? batch_coordinate(in, 3 * begin + 1) : 0.0;
         const double oz = (n > 0) ? batch_coordinate(in, 3 * begin + 2) : 0.0;
         float reach = 0.0f;
-        for (int k = lane; k < n; k += 32) {
-            const double x = batch_coordinate(in, 3 * (begin + k) + 0);
-            const double y = batch_coordinate(in, 3 * (begin + k) + 1);
-            const double z = batch_coordinate(in, 3 * (begin + k) + 2);
+        bool finite = true;
+        for (int k = lane; k < ((n + 3) & ~3); k += 32) {
+            double x = ox, y = oy, z = oz;
+            if (k < n) {
+                x = batch_coordinate(in, 3 * (begin + k) + 0);
+                y = batch_coordinate(in, 3 * (begin + k) + 1);
+                z = batch_coordinate(in, 3 * (begin + k) + 2);
+            }
             sh.x[warp][k] = x;
             sh.y[warp][k] = y;
             sh.z[warp][k] = z;
@@ -258,304 +408,480 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
             sh.fy[warp][k] = fy;
             sh.fz[warp][k] = fz;
             reach = fmaxf(reach, fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))));
-            if (!EMIT && !(isfinite(x) && isfinite(y) && isfinite(z))) {
-                atomicOr(&header->status, STATUS_BAD_POINT);
-                atomicMin(&header->first_bad, begin + k);
+            if (!(isfinite(x) && isfinite(y) && isfinite(z))) {
+                finite = false;
+                if (!EMIT) {
+                    atomicOr(&header->status, STATUS_BAD_POINT);
+                    atomicMin(&header->first_bad, begin + k);
+                }
             }
+        }
+        if (__any_sync(FULL_MASK, !finite)) {
+            reach = __int_as_float(0x7f800000);
         }
 #pragma unroll
         for (int offset = 16; offset > 0; offset >>= 1) {
             reach = fmaxf(reach, __shfl_xor_sync(FULL_MASK, reach, offset));
         }
         __syncwarp();
-        // fp32 screen: candidates whose squared distance is outside [lo, hi] are decided, the
-        // others go to the exact predicate. The band covers the rounding of the coordinates
-        // (relative error 2^-24 of values up to M), of the differences and of the sum.
-        const float m = reach * 1.7320508f * 1.0001f + 1.0e-30f; // bound on the length of a relative position
-        const float c = static_cast<float>(in.cutoff) * 1.01f;
-        const float eps = 5.9604644775390625e-08f;
-        float band = 4.0f * eps * (2.0f * 1.7320508f * c * (2.0f * m + c) + 3.0f * c * c) + 40.0f * eps * m * m + 4.0f * eps * c * c;
-        band *= 1.01f; // this expression is itself evaluated in fp32
-        const float cutoff2 = static_cast<float>(in.cutoff2);
-        const float lo = cutoff2 - band;
-        const float hi = cutoff2 + band;
+        const ScreenBand band = screen_band(reach * 1.7320508f, in.cutoff, in.cutoff2);
 
-        const unsigned long long base = EMIT ? system_start[system] : 0ull;
         const unsigned long long index_offset = in.global_indices ? begin : 0ull;
         const unsigned per_hit = in.full ? 2u : 1u;
-        unsigned long long written = 0; // output elements of the system written so far
-        int listed = 0;                 // hits waiting in the list (the same value in every lane)
-        unsigned hits_total = 0;
-
-        const int n_candidates = (n * (n - 1)) >> 1;
-        for (int c0 = 0; c0 < n_candidates; c0 += 32) {
-            const int candidate = c0 + lane;
-            bool hit = false;
-            int i = 0, j = 0;
-            if (candidate < n_candidates) {
-                // (i, j) from the position in the flattened strict upper triangle
-                const float b = static_cast<float>(2 * n - 1);
-                i = static_cast<int>(0.5f * (b - sqrtf(b * b - 8.0f * static_cast<float>(candidate))));
-                i = min(max(i, 0), n - 2);
-                while (triangle_row_start(i + 1, n) <= candidate) {
-                    i++;
+        unsigned long long next = EMIT ? system_start[system] : 0ull; // where the next hits go
+        int listed = 0;                                               // hits waiting in the list (the same value in every lane)
+        int hits = 0;
+        const auto write = [&](int count) {
+            for (int c0 = 0; c0 < count; c0 += 32) {
+                const int n_valid = min(32, count - c0);
+                int i = 0, j = 0;
+                if (lane < n_valid) {
+                    const unsigned entry = sh.list[warp][c0 + lane];
+                    i = entry >> 8;
+                    j = entry & 255;
                 }
-                while (triangle_row_start(i, n) > candidate) {
-                    i--;
-                }
-                j = i + 1 + (candidate - triangle_row_start(i, n));
-                const float dx = sh.fx[warp][j] - sh.fx[warp][i];
-                const float dy = sh.fy[warp][j] - sh.fy[warp][i];
-                const float dz = sh.fz[warp][j] - sh.fz[warp][i];
-                const float d2 = dx * dx + dy * dy + dz * dz;
-                if (d2 < lo) {
-                    hit = true;
-                } else if (d2 <= hi || !(d2 == d2)) {
-                    // the reference's arithmetic, operation for operation (vesin/src/cpu_cell_list.cpp:135-138)
-                    const double vx = __dadd_rn(__dsub_rn(sh.x[warp][j], sh.x[warp][i]), 0.0);
-                    const double vy = __dadd_rn(__dsub_rn(sh.y[warp][j], sh.y[warp][i]), 0.0);
-                    const double vz = __dadd_rn(__dsub_rn(sh.z[warp][j], sh.z[warp][i]), 0.0);
-                    hit = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz)) < in.cutoff2;
-                }
+                double vx, vy, vz;
+                const double d = __dsqrt_rn(molecule_pair(sh, warp, i, j, vx, vy, vz));
+                write_hits(sh.transpose[warp], in, out, lane, next, n_valid, index_offset + i, index_offset + j, 0, 0, 0, d, vx, vy, vz);
+                next += static_cast<unsigned long long>(n_valid) * per_hit;
             }
-            const unsigned ballot = __ballot_sync(FULL_MASK, hit);
-            if (ballot == 0) {
-                continue;
-            }
-            const int hits = __popc(ballot);
-            hits_total += hits;
-            if (!EMIT) {
-                continue;
-            }
-            if (hit) {
-                sh.list[warp][listed + __popc(ballot & ((1u << lane) - 1u))] = static_cast<unsigned short>((i << 8) | j);
-            }
-            listed += hits;
-            __syncwarp();
-            if (listed >= 32) {
-                write_molecule_hits(sh, in, out, warp, lane, base + written, 32, index_offset);
-                written += 32ull * per_hit;
-                listed -= 32;
-                // what is left moves to the front of the list
-                unsigned short moved = 0;
-                if (lane < listed) {
-                    moved = sh.list[warp][32 + lane];
+        };
+        // a lane per home point i, words of 32 candidates j; only j > i
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const int i = i0 + lane;
+            const int own = min(i, n - 1);
+            const float ax = -sh.fx[warp][own];
+            const float ay = -sh.fy[warp][own];
+            const float az = -sh.fz[warp][own];
+            const unsigned long long ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+            for (int j0 = i0; j0 < n; j0 += 32) {
+                unsigned inside, maybe;
+                screen_word(
+                    sh.fx[warp] + j0, sh.fy[warp] + j0, sh.fz[warp] + j0, min(8, (n - j0 + 3) >> 2), ax2, ay2, az2, band, inside, maybe
+                );
+                const unsigned keep = (i < n) ? bits_from(i + 1 - j0) & ~bits_from(n - j0) : 0u;
+                inside &= keep;
+                unsigned undecided = maybe & keep & ~inside;
+                while (undecided != 0) {
+                    const int b = __ffs(undecided) - 1;
+                    undecided &= undecided - 1;
+                    double vx, vy, vz;
+                    if (molecule_pair(sh, warp, i, j0 + b, vx, vy, vz) < in.cutoff2) {
+                        inside |= 1u << b;
+                    }
                 }
-                __syncwarp();
-                if (lane < listed) {
-                    sh.list[warp][lane] = moved;
+                if (EMIT) {
+                    list_hits(inside, static_cast<unsigned>((i << 8) | j0), sh.list[warp], listed, lane, write);
+                } else {
+                    hits += __popc(inside);
                 }
-                __syncwarp();
             }
         }
         if (EMIT) {
             if (listed > 0) {
-                write_molecule_hits(sh, in, out, warp, lane, base + written, listed, index_offset);
+                write(listed);
             }
-        } else if (lane == 0) {
-            system_count[system] = static_cast<unsigned long long>(hits_total) * per_hit;
+        } else {
+            hits = __reduce_add_sync(FULL_MASK, hits);
+            if (lane == 0) {
+                system_count[system] = static_cast<unsigned long long>(hits) * per_hit;
+            }
         }
     }
 }
 
+// ---- periodic systems, and larger ones -------------------------------------
+// Candidates of a tile of 32 home points are the images of the points j >= i0
+// whose fractional coordinates lie within the cutoff of the tile's bounding
+// box: a cell as wide as two cutoffs has eight images per point there, not the
+// 27 around every pair. A chunk of 128 points (one per thread) counts its
+// images, a scan numbers them, and the images are staged 256 at a time; warps
+// take words of 32 of them. What bounds it: the latency of the short chain
+// (box, points, scan, stage) for the few thousand tiles that a batch of
+// hundreds of cells has; the work itself is the emission of the hits.
+// Several CTAs share the tiles of a system when the systems alone would not
+// fill the GPU. 512 cells of 4 to 200 atoms (5 A cutoff, 2.7 M pairs): 56 us to
+// count and 107 us to write; exact arithmetic on every image of every pair, a CTA
+// per system, took 640 and 954.
+
+constexpr int SMALL_CHUNK = SMALL_THREADS; // points whose images are listed at a time
+constexpr int SMALL_BATCH = 256;           // images staged at a time
+constexpr int SMALL_TILE = 32;             // home points per tile
+
 struct SmallShared {
+    alignas(16) float near_x[SMALL_BATCH]; // images relative to the first home point of the tile
+    alignas(16) float near_y[SMALL_BATCH];
+    alignas(16) float near_z[SMALL_BATCH];
+    int4 image[SMALL_BATCH];               // x, y, z: image shift minus wrap shift of the point; w: the point in the chunk
+    alignas(16) double transpose[SMALL_WARPS][TRANSPOSE_DOUBLES];
     SystemFrame frame;
-    unsigned long long counter; // pairs counted (pass 1) / written so far (pass 2)
-    unsigned long long warp_sum[SMALL_WARPS];
+    double x[SMALL_CHUNK];                 // original positions of the chunk
+    double y[SMALL_CHUNK];
+    double z[SMALL_CHUNK];
+    int wrap[3][SMALL_CHUNK];              // wrap shift, seen from the first home point
+    int low[3][SMALL_CHUNK];               // first image in each direction
+    int count[2][SMALL_CHUNK];             // images in the first two directions
+    int first_slot[SMALL_CHUNK + 1];       // exclusive scan of the images per point
+    double home[3][SMALL_TILE];
+    int home_wrap[3][SMALL_TILE];
+    double box_lo[3], box_hi[3];           // fractional coordinates images of this tile can have
+    ScreenBand band;
+    int warp_sum[SMALL_WARPS];
+    unsigned self_word[SMALL_BATCH / 32];  // images a point may pair with itself in
+    unsigned short list[SMALL_WARPS][HIT_LIST]; // (home point << 8) | slot
+    unsigned long long counter;            // output elements counted (pass 1) / handed out (pass 2)
 };
 
-template <bool EMIT>
-__global__ void __launch_bounds__(SMALL_THREADS) small_systems_kernel(
-    const BatchInput in, unsigned long long* __restrict__ system_count, const unsigned long long* __restrict__ system_start, PairOutput out,
-    DeviceHeader* header, const unsigned long long capacity
+/// The reference's arithmetic, operation for operation (vesin/src/cpu_cell_list.cpp:135-138, types.hpp:232-243).
+__device__ __forceinline__ double small_pair(
+    const SystemFrame& frame, double rix, double riy, double riz, double rjx, double rjy, double rjz, int s0, int s1, int s2, double& vx,
+    double& vy, double& vz
 ) {
-    extern __shared__ __align__(16) unsigned char small_smem[];
-    SmallShared& sh = *reinterpret_cast<SmallShared*>(small_smem);
-    double* px = reinterpret_cast<double*>(small_smem + sizeof(SmallShared));
+    const double f0 = static_cast<double>(s0), f1 = static_cast<double>(s1), f2 = static_cast<double>(s2);
+    const double shx = __dadd_rn(__dadd_rn(__dmul_rn(f0, frame.H[0][0]), __dmul_rn(f1, frame.H[1][0])), __dmul_rn(f2, frame.H[2][0]));
+    const double shy = __dadd_rn(__dadd_rn(__dmul_rn(f0, frame.H[0][1]), __dmul_rn(f1, frame.H[1][1])), __dmul_rn(f2, frame.H[2][1]));
+    const double shz = __dadd_rn(__dadd_rn(__dmul_rn(f0, frame.H[0][2]), __dmul_rn(f1, frame.H[1][2])), __dmul_rn(f2, frame.H[2][2]));
+    vx = __dadd_rn(__dsub_rn(rjx, rix), shx);
+    vy = __dadd_rn(__dsub_rn(rjy, riy), shy);
+    vz = __dadd_rn(__dsub_rn(rjz, riz), shz);
+    return __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
+}
 
+template <bool EMIT>
+__global__ void __launch_bounds__(SMALL_THREADS, 5) small_systems_kernel(
+    const BatchInput in, const unsigned splits, unsigned long long* __restrict__ system_count, unsigned long long* __restrict__ share_count,
+    const unsigned long long* __restrict__ system_start, PairOutput out, DeviceHeader* header, const unsigned long long capacity
+) {
+    __shared__ SmallShared sh;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
+    const unsigned per_hit = in.full ? 2u : 1u;
 
-    for (unsigned system = blockIdx.x; system < in.n_systems; system += gridDim.x) {
+    const unsigned long long n_items = static_cast<unsigned long long>(in.n_systems) * splits;
+    for (unsigned long long item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const unsigned system = static_cast<unsigned>(item / splits);
+        const int share = static_cast<int>(item - static_cast<unsigned long long>(system) * splits);
         const unsigned long long begin = in.offsets[system];
         const int n = static_cast<int>(in.offsets[system + 1] - begin);
         if (taken_by_warp_kernel(in, system, n)) {
             continue;
         }
+        const int n_tiles = (n + SMALL_TILE - 1) / SMALL_TILE;
+        if (share >= max(n_tiles, 1)) {
+            continue; // (only shares of earlier tiles are ever added up)
+        }
         if (EMIT && system_start[system + 1] > capacity) {
             continue; // as in the warp kernel
         }
-        double* py = px + n;
-        double* pz = py + n;
-        __syncthreads(); // previous system done with shared memory
-        if (threadIdx.x == 0) {
-            make_frame(sh.frame, in, system, in.periodic ? in.periodic + 3 * static_cast<size_t>(system) : nullptr, in.cutoff);
-            sh.counter = 0;
-            if (sh.frame.singular && !EMIT) {
-                atomicOr(&header->status, sh.frame.singular == 2 ? STATUS_STENCIL_TOO_LARGE : STATUS_SINGULAR_BOX);
-                atomicMin(&header->mask_cursor, static_cast<unsigned long long>(system)); // first offending system
+        __syncthreads(); // previous item done with shared memory
+        if (warp == 0) {
+            make_frame(sh.frame, in, system, lane);
+            unsigned long long before = 0;
+            if (EMIT) {
+                before = system_start[system];
+                for (int s = 0; s < share; s++) {
+                    before += share_count[system * static_cast<unsigned long long>(splits) + s];
+                }
             }
-        }
-        for (int k = threadIdx.x; k < n; k += SMALL_THREADS) {
-            const double x = batch_coordinate(in, 3 * (begin + k) + 0);
-            const double y = batch_coordinate(in, 3 * (begin + k) + 1);
-            const double z = batch_coordinate(in, 3 * (begin + k) + 2);
-            px[k] = x;
-            py[k] = y;
-            pz[k] = z;
-            if (!EMIT && !(isfinite(x) && isfinite(y) && isfinite(z))) {
-                atomicOr(&header->status, STATUS_BAD_POINT);
-                atomicMin(&header->first_bad, begin + k);
+            if (lane == 0) {
+                sh.counter = before;
+                if (sh.frame.singular && !EMIT) {
+                    atomicOr(&header->status, sh.frame.singular == 2 ? STATUS_STENCIL_TOO_LARGE : STATUS_SINGULAR_BOX);
+                    atomicMin(&header->mask_cursor, static_cast<unsigned long long>(system)); // first offending system
+                }
             }
         }
         __syncthreads();
         const SystemFrame& frame = sh.frame;
-        if (frame.singular) {
-            if (!EMIT && threadIdx.x == 0) {
-                system_count[system] = 0;
+        const bool usable = frame.singular == 0;
+        if (!EMIT && share == 0) {
+            for (int k = threadIdx.x; k < n; k += SMALL_THREADS) {
+                const bool finite = isfinite(batch_coordinate(in, 3 * (begin + k) + 0)) && isfinite(batch_coordinate(in, 3 * (begin + k) + 1)) &&
+                                    isfinite(batch_coordinate(in, 3 * (begin + k) + 2));
+                if (!finite) {
+                    atomicOr(&header->status, STATUS_BAD_POINT);
+                    atomicMin(&header->first_bad, begin + k);
+                }
             }
-            continue;
         }
-        const int w0 = 2 * frame.reach[0] + 1;
-        const int w1 = 2 * frame.reach[1] + 1;
-        const int w2 = 2 * frame.reach[2] + 1;
-        const int n_images = w0 * w1 * w2;
-        const unsigned long long base = EMIT ? system_start[system] : 0ull;
         const unsigned long long index_offset = in.global_indices ? begin : 0ull;
         unsigned long long my_count = 0;
 
-        // a warp takes point i; its lanes take (j >= i, image) candidates
-        for (int i = warp; i < n; i += SMALL_WARPS) {
-            const double rix = px[i], riy = py[i], riz = pz[i];
-            const long long n_candidates = static_cast<long long>(n - i) * n_images;
-            for (long long c0 = 0; c0 < n_candidates; c0 += 32) {
-                const long long c = c0 + lane;
-                bool hit = false;
-                int s0 = 0, s1 = 0, s2 = 0, j = i;
-                double vx = 0, vy = 0, vz = 0, d2 = 0;
-                if (c < n_candidates) {
-                    j = i + static_cast<int>(c / n_images);
-                    const int image = static_cast<int>(c % n_images);
-                    const double rjx = px[j], rjy = py[j], rjz = pz[j];
-                    const double dx = rjx - rix, dy = rjy - riy, dz = rjz - riz;
-                    int nearest[3];
+        for (int i0 = share * SMALL_TILE; usable && i0 < n; i0 += static_cast<int>(splits) * SMALL_TILE) {
+            const int n_home = min(SMALL_TILE, n - i0);
+            // everything is seen from the first home point: fractional coordinates, wrap shifts
+            // (what they have in common cancels in the shift of a pair) and fp32 positions
+            const double ox = batch_coordinate(in, 3 * (begin + i0) + 0);
+            const double oy = batch_coordinate(in, 3 * (begin + i0) + 1);
+            const double oz = batch_coordinate(in, 3 * (begin + i0) + 2);
+            float hx = 0, hy = 0, hz = 0; // the lane's home point, negated
+            bool exact_only = false;
+            for (int chunk0 = i0; chunk0 < n; chunk0 += SMALL_CHUNK) {
+                const int j = chunk0 + static_cast<int>(threadIdx.x);
+                bool have = j < n;
+                double rx = ox, ry = oy, rz = oz;
+                if (have) {
+                    rx = batch_coordinate(in, 3 * (begin + j) + 0);
+                    ry = batch_coordinate(in, 3 * (begin + j) + 1);
+                    rz = batch_coordinate(in, 3 * (begin + j) + 2);
+                    have = isfinite(rx) && isfinite(ry) && isfinite(rz); // others are reported by the counting pass
+                }
+                const double dx = rx - ox, dy = ry - oy, dz = rz - oz;
+                double f[3];
+                int wrap[3];
+                double slack = 0.0; // covers the rounding of the fractional coordinates
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const double ax = dx * frame.Hinv[0][k], ay = dy * frame.Hinv[1][k], az = dz * frame.Hinv[2][k];
+                    const double t = fmin(fmax(ax + ay + az, -1.0e9), 1.0e9);
+                    slack = fmax(slack, 1.0e-14 * (fabs(ax) + fabs(ay) + fabs(az)));
+                    const double w = frame.periodic[k] ? floor(t) : 0.0;
+                    wrap[k] = static_cast<int>(w);
+                    f[k] = t - w;
+                }
+                const double image_slack = fmin(slack, 1.0e-3); // bounds the images of a point absurdly far out
+                __syncthreads(); // the previous chunk has been consumed
+                sh.x[threadIdx.x] = rx;
+                sh.y[threadIdx.x] = ry;
+                sh.z[threadIdx.x] = rz;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    sh.wrap[k][threadIdx.x] = wrap[k];
+                }
+                if (chunk0 == i0 && warp == 0) {
+                    // the home points open the first chunk: what images can reach them?
+                    const bool home = lane < n_home;
+                    sh.home[0][lane] = rx;
+                    sh.home[1][lane] = ry;
+                    sh.home[2][lane] = rz;
+                    float reach = 0.0f;
+                    float rel[3];
 #pragma unroll
                     for (int k = 0; k < 3; k++) {
-                        const double fractional = dx * frame.Hinv[0][k] + dy * frame.Hinv[1][k] + dz * frame.Hinv[2][k];
-                        nearest[k] = frame.periodic[k] ? -static_cast<int>(rint(fmin(fmax(fractional, -1.0e9), 1.0e9))) : 0;
+                        sh.home_wrap[k][lane] = wrap[k];
+                        const double r = ((k == 0) ? dx : ((k == 1) ? dy : dz)) -
+                                         (wrap[0] * frame.H[0][k] + wrap[1] * frame.H[1][k] + wrap[2] * frame.H[2][k]);
+                        rel[k] = static_cast<float>(r);
+                        reach += rel[k] * rel[k];
                     }
-                    const int e0 = image % w0 - frame.reach[0];
-                    const int e1 = (image / w0) % w1 - frame.reach[1];
-                    const int e2 = image / (w0 * w1) - frame.reach[2];
-                    s0 = nearest[0] + e0;
-                    s1 = nearest[1] + e1;
-                    s2 = nearest[2] + e2;
-                    // a point with itself: only images, and only one of S / -S
-                    // (the other one is written as the reversed pair)
-                    bool keep = (j != i) || (((s0 | s1 | s2) != 0) && half_rule_small(s0, s1, s2));
-                    if (keep) {
-                        const double f0 = static_cast<double>(s0), f1 = static_cast<double>(s1), f2 = static_cast<double>(s2);
-                        // the reference's arithmetic, operation for operation
-                        // (vesin/src/cpu_cell_list.cpp:135-138, types.hpp:232-243)
-                        const double shx = __dadd_rn(__dadd_rn(__dmul_rn(f0, frame.H[0][0]), __dmul_rn(f1, frame.H[1][0])), __dmul_rn(f2, frame.H[2][0]));
-                        const double shy = __dadd_rn(__dadd_rn(__dmul_rn(f0, frame.H[0][1]), __dmul_rn(f1, frame.H[1][1])), __dmul_rn(f2, frame.H[2][1]));
-                        const double shz = __dadd_rn(__dadd_rn(__dmul_rn(f0, frame.H[0][2]), __dmul_rn(f1, frame.H[1][2])), __dmul_rn(f2, frame.H[2][2]));
-                        vx = __dadd_rn(__dsub_rn(rjx, rix), shx);
-                        vy = __dadd_rn(__dsub_rn(rjy, riy), shy);
-                        vz = __dadd_rn(__dsub_rn(rjz, riz), shz);
-                        d2 = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
-                        hit = d2 < in.cutoff2;
+                    reach = sqrtf(reach);
+                    if (!home) {
+                        reach = 0.0f;
+                    } else if (!(reach < 3.0e38f)) {
+                        reach = __int_as_float(0x7f800000);
                     }
-                }
-                const unsigned ballot = __ballot_sync(FULL_MASK, hit);
-                if (ballot == 0) {
-                    continue;
-                }
-                const unsigned per_hit = in.full ? 2u : 1u;
-                if (!EMIT) {
+                    double most_slack = home ? fmin(slack, 1.0e9) : 0.0;
+#pragma unroll
+                    for (int offset = 16; offset > 0; offset >>= 1) {
+                        reach = fmaxf(reach, __shfl_xor_sync(FULL_MASK, reach, offset));
+                        most_slack = fmax(most_slack, __shfl_xor_sync(FULL_MASK, most_slack, offset));
+                    }
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        double lo = home ? f[k] : 1.0e300;
+                        double hi = home ? f[k] : -1.0e300;
+#pragma unroll
+                        for (int offset = 16; offset > 0; offset >>= 1) {
+                            lo = fmin(lo, __shfl_xor_sync(FULL_MASK, lo, offset));
+                            hi = fmax(hi, __shfl_xor_sync(FULL_MASK, hi, offset));
+                        }
+                        if (lane == 0) {
+                            const double margin = frame.reach[k] + 1.0e-9 + (frame.periodic[k] ? fmin(most_slack, 1.0e-3) : most_slack);
+                            sh.box_lo[k] = lo - margin;
+                            sh.box_hi[k] = hi + margin;
+                        }
+                    }
                     if (lane == 0) {
-                        my_count += static_cast<unsigned long long>(__popc(ballot)) * per_hit;
+                        sh.band = screen_band(reach * 1.0001f, in.cutoff, in.cutoff2);
                     }
-                    continue;
                 }
-                unsigned long long first = 0;
-                if (lane == 0) {
-                    first = atomicAdd(&sh.counter, static_cast<unsigned long long>(__popc(ballot)) * per_hit);
+                if (chunk0 == i0) {
+                    __syncthreads();
+                    const int h = lane;
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        const double r = sh.home[k][h] - ((k == 0) ? ox : ((k == 1) ? oy : oz));
+                        const double rel = r - (sh.home_wrap[0][h] * frame.H[0][k] + sh.home_wrap[1][h] * frame.H[1][k] + sh.home_wrap[2][h] * frame.H[2][k]);
+                        (k == 0 ? hx : (k == 1 ? hy : hz)) = -static_cast<float>(rel);
+                    }
                 }
-                first = __shfl_sync(FULL_MASK, first, 0);
-                if (hit) {
-                    const unsigned long long rank = __popc(ballot & ((1u << lane) - 1u));
-                    unsigned long long dest = base + first + rank * per_hit;
-                    const unsigned long long gi = index_offset + i, gj = index_offset + j;
-                    const double d = __dsqrt_rn(d2);
-                    // half lists keep i <= j (i < j, or the image the rule keeps): the forward pair
-                    store_indices(out, dest, gi, gj);
-                    if (out.shifts) {
-                        out.shifts[3 * dest + 0] = s0;
-                        out.shifts[3 * dest + 1] = s1;
-                        out.shifts[3 * dest + 2] = s2;
+                // ---- images of the thread's point inside the reach of the tile ----
+                int images = have ? 1 : 0;
+                bool far = false; // so far out that fp64 rounding of the shift products shows
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    int low = 0;
+                    int count = 1;
+                    if (frame.periodic[k]) {
+                        low = static_cast<int>(ceil(sh.box_lo[k] - image_slack - f[k]));
+                        count = max(0, static_cast<int>(floor(sh.box_hi[k] + image_slack - f[k])) - low + 1);
+                    } else if (f[k] < sh.box_lo[k] - slack || f[k] > sh.box_hi[k] + slack) {
+                        count = 0;
                     }
-                    if (out.distances) {
-                        if (out.values_float) {
-                            reinterpret_cast<float*>(out.distances)[dest] = static_cast<float>(d);
-                        } else {
-                            out.distances[dest] = d;
+                    far = far || wrap[k] > 100000 || wrap[k] < -100000;
+                    sh.low[k][threadIdx.x] = low;
+                    if (k < 2) {
+                        sh.count[k][threadIdx.x] = count;
+                    }
+                    images *= count;
+                }
+                int inclusive = images;
+#pragma unroll
+                for (int offset = 1; offset < 32; offset <<= 1) {
+                    const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
+                    if (lane >= offset) {
+                        inclusive += up;
+                    }
+                }
+                if (lane == 31) {
+                    sh.warp_sum[warp] = inclusive;
+                }
+                exact_only = __syncthreads_or(far) != 0 || exact_only;
+                int before = 0;
+                int total = 0;
+#pragma unroll
+                for (int w = 0; w < SMALL_WARPS; w++) {
+                    before += (w < warp) ? sh.warp_sum[w] : 0;
+                    total += sh.warp_sum[w];
+                }
+                sh.first_slot[threadIdx.x] = before + inclusive - images;
+                if (threadIdx.x == 0) {
+                    sh.first_slot[SMALL_CHUNK] = total;
+                }
+                ScreenBand band = sh.band;
+                if (exact_only) {
+                    band = ScreenBand{-__int_as_float(0x7f800000), __int_as_float(0x7f800000)};
+                }
+                const unsigned long long hx2 = pack2(hx, hx), hy2 = pack2(hy, hy), hz2 = pack2(hz, hz);
+
+                for (int batch0 = 0; batch0 < total; batch0 += SMALL_BATCH) {
+                    const int slots = min(SMALL_BATCH, total - batch0);
+                    const int words = (slots + 31) >> 5;
+                    __syncthreads(); // the scan is visible; the previous batch has been consumed
+                    for (int s = threadIdx.x; s < 32 * words; s += SMALL_THREADS) {
+                        bool self = false;
+                        float nx = 0.0f, ny = 0.0f, nz = 0.0f;
+                        int4 image = make_int4(0, 0, 0, 0);
+                        if (s < slots) {
+                            const int slot = batch0 + s;
+                            int t = 0; // last point whose images start at or before the slot
+#pragma unroll
+                            for (int step = SMALL_CHUNK / 2; step > 0; step >>= 1) {
+                                if (sh.first_slot[t + step] <= slot) {
+                                    t += step;
+                                }
+                            }
+                            const int number = slot - sh.first_slot[t];
+                            const int c0 = sh.count[0][t];
+                            const int c1 = sh.count[1][t];
+                            const int row = number / c0;
+                            const int t0 = sh.low[0][t] + (number - row * c0);
+                            const int plane = row / c1;
+                            const int t1 = sh.low[1][t] + (row - plane * c1);
+                            const int t2 = sh.low[2][t] + plane;
+                            image = make_int4(t0 - sh.wrap[0][t], t1 - sh.wrap[1][t], t2 - sh.wrap[2][t], t);
+                            nx = static_cast<float>((sh.x[t] - ox) + (image.x * frame.H[0][0] + image.y * frame.H[1][0] + image.z * frame.H[2][0]));
+                            ny = static_cast<float>((sh.y[t] - oy) + (image.x * frame.H[0][1] + image.y * frame.H[1][1] + image.z * frame.H[2][1]));
+                            nz = static_cast<float>((sh.z[t] - oz) + (image.x * frame.H[0][2] + image.y * frame.H[1][2] + image.z * frame.H[2][2]));
+                            // a point with itself: only images, and only one of S / -S (the other
+                            // one is written as the reversed pair)
+                            self = (t0 | t1 | t2) != 0 && half_rule_small(t0, t1, t2);
+                        }
+                        sh.near_x[s] = nx;
+                        sh.near_y[s] = ny;
+                        sh.near_z[s] = nz;
+                        sh.image[s] = image;
+                        const unsigned word = __ballot_sync(FULL_MASK, self);
+                        if (lane == 0) {
+                            sh.self_word[s >> 5] = word;
                         }
                     }
-                    if (out.vectors) {
-                        if (out.values_float) {
-                            float* vectors = reinterpret_cast<float*>(out.vectors);
-                            vectors[3 * dest + 0] = static_cast<float>(vx);
-                            vectors[3 * dest + 1] = static_cast<float>(vy);
-                            vectors[3 * dest + 2] = static_cast<float>(vz);
-                        } else {
-                            out.vectors[3 * dest + 0] = vx;
-                            out.vectors[3 * dest + 1] = vy;
-                            out.vectors[3 * dest + 2] = vz;
+                    __syncthreads();
+
+                    int listed = 0;
+                    const auto write = [&](int count) {
+                        unsigned long long first = 0;
+                        if (lane == 0) {
+                            first = atomicAdd(&sh.counter, static_cast<unsigned long long>(count) * per_hit);
                         }
-                    }
-                    if (in.full) {
-                        dest += 1;
-                        store_indices(out, dest, gj, gi);
-                        if (out.shifts) {
-                            out.shifts[3 * dest + 0] = -s0;
-                            out.shifts[3 * dest + 1] = -s1;
-                            out.shifts[3 * dest + 2] = -s2;
+                        first = __shfl_sync(FULL_MASK, first, 0);
+                        for (int c0 = 0; c0 < count; c0 += 32) {
+                            const int n_valid = min(32, count - c0);
+                            int h = 0, s = 0;
+                            if (lane < n_valid) {
+                                const unsigned entry = sh.list[warp][c0 + lane];
+                                h = entry >> 8;
+                                s = entry & 255;
+                            }
+                            const int4 image = sh.image[s];
+                            const int s0 = image.x + sh.home_wrap[0][h];
+                            const int s1 = image.y + sh.home_wrap[1][h];
+                            const int s2 = image.z + sh.home_wrap[2][h];
+                            double vx, vy, vz;
+                            const double d = __dsqrt_rn(small_pair(
+                                frame, sh.home[0][h], sh.home[1][h], sh.home[2][h], sh.x[image.w], sh.y[image.w], sh.z[image.w], s0, s1, s2, vx, vy, vz
+                            ));
+                            write_hits(
+                                sh.transpose[warp], in, out, lane, first + static_cast<unsigned long long>(c0) * per_hit, n_valid, index_offset + i0 + h,
+                                index_offset + chunk0 + image.w, s0, s1, s2, d, vx, vy, vz
+                            );
                         }
-                        if (out.distances) {
-                            if (out.values_float) {
-                                reinterpret_cast<float*>(out.distances)[dest] = static_cast<float>(d);
-                            } else {
-                                out.distances[dest] = d;
+                    };
+                    for (int w = warp; w < words; w += SMALL_WARPS) {
+                        unsigned inside, maybe;
+                        const int in_word = min(32, slots - 32 * w);
+                        screen_word(
+                            sh.near_x + 32 * w, sh.near_y + 32 * w, sh.near_z + 32 * w, (in_word + 3) >> 2, hx2, hy2, hz2, band, inside, maybe
+                        );
+                        unsigned keep = (lane < n_home) ? ~bits_from(in_word) : 0u;
+                        if (chunk0 == i0) {
+                            // of the points of the tile only those after the home point, and its own images
+                            const int own_first = sh.first_slot[lane] - batch0 - 32 * w;
+                            const int own_end = sh.first_slot[lane + 1] - batch0 - 32 * w;
+                            keep &= bits_from(own_end) | (sh.self_word[w] & bits_from(own_first));
+                        }
+                        inside &= keep;
+                        unsigned undecided = maybe & keep & ~inside;
+                        while (undecided != 0) {
+                            const int b = __ffs(undecided) - 1;
+                            undecided &= undecided - 1;
+                            const int4 image = sh.image[32 * w + b];
+                            double vx, vy, vz;
+                            const double d2 = small_pair(
+                                frame, sh.home[0][lane], sh.home[1][lane], sh.home[2][lane], sh.x[image.w], sh.y[image.w], sh.z[image.w],
+                                image.x + sh.home_wrap[0][lane], image.y + sh.home_wrap[1][lane], image.z + sh.home_wrap[2][lane], vx, vy, vz
+                            );
+                            if (d2 < in.cutoff2) {
+                                inside |= 1u << b;
                             }
                         }
-                        if (out.vectors) {
-                            if (out.values_float) {
-                                float* vectors = reinterpret_cast<float*>(out.vectors);
-                                vectors[3 * dest + 0] = -static_cast<float>(vx);
-                                vectors[3 * dest + 1] = -static_cast<float>(vy);
-                                vectors[3 * dest + 2] = -static_cast<float>(vz);
-                            } else {
-                                out.vectors[3 * dest + 0] = -vx;
-                                out.vectors[3 * dest + 1] = -vy;
-                                out.vectors[3 * dest + 2] = -vz;
-                            }
+                        if (EMIT) {
+                            list_hits(inside, static_cast<unsigned>((lane << 8) | (32 * w)), sh.list[warp], listed, lane, write);
+                        } else {
+                            my_count += static_cast<unsigned>(__popc(inside));
                         }
+                    }
+                    if (EMIT && listed > 0) {
+                        write(listed);
                     }
                 }
             }
         }
         if (!EMIT) {
-            if (lane == 0) {
-                sh.warp_sum[warp] = my_count;
+#pragma unroll
+            for (int offset = 16; offset > 0; offset >>= 1) {
+                my_count += __shfl_xor_sync(FULL_MASK, my_count, offset);
+            }
+            if (lane == 0 && my_count != 0) {
+                atomicAdd(&sh.counter, my_count * per_hit);
             }
             __syncthreads();
             if (threadIdx.x == 0) {
-                unsigned long long total = 0;
-                for (int w = 0; w < SMALL_WARPS; w++) {
-                    total += sh.warp_sum[w];
+                const unsigned long long counted = sh.counter;
+                share_count[item] = counted;
+                if (counted != 0) {
+                    atomicAdd(&system_count[system], counted);
                 }
-                system_count[system] = total;
             }
         }
     }
@@ -567,57 +893,66 @@ size_t small_systems_max_points() {
     return 2048;
 }
 
-static size_t small_shared_bytes(size_t max_points) {
-    return sizeof(SmallShared) + 3 * max_points * sizeof(double);
-}
-
 void configure_small_systems() {
-    int bytes = static_cast<int>(small_shared_bytes(small_systems_max_points()));
-    cudaFuncSetAttribute(small_systems_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(small_systems_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const int bytes = static_cast<int>(sizeof(MoleculeShared));
+    cudaFuncSetAttribute(molecules_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(molecules_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-static unsigned small_grid(unsigned n_systems) {
+static unsigned multiprocessors() {
     int device = 0, sms = 148;
     if (cudaGetDevice(&device) == cudaSuccess) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     }
-    unsigned cap = static_cast<unsigned>(sms) * 8;
-    return n_systems < cap ? (n_systems ? n_systems : 1) : cap;
+    return static_cast<unsigned>(sms);
+}
+
+unsigned small_splits(unsigned n_systems, size_t max_points) {
+    // about four waves of CTAs, so that systems of different sizes even out; never more than tiles
+    const unsigned tiles = static_cast<unsigned>((max_points + SMALL_TILE - 1) / SMALL_TILE);
+    const unsigned wanted = 4 * 5 * multiprocessors() / std::max(n_systems, 1u);
+    return std::max(1u, std::min(wanted, tiles));
+}
+
+static unsigned small_grid(unsigned n_systems, unsigned splits) {
+    return static_cast<unsigned>(std::min<unsigned long long>(static_cast<unsigned long long>(n_systems) * splits, 1ull << 20));
 }
 
 static unsigned molecules_grid(unsigned n_systems) {
-    int device = 0, sms = 148;
-    if (cudaGetDevice(&device) == cudaSuccess) {
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    }
     const unsigned wanted = (n_systems + MOLECULE_WARPS - 1) / MOLECULE_WARPS;
-    const unsigned cap = static_cast<unsigned>(sms) * 8;
+    const unsigned cap = multiprocessors() * 8;
     return wanted < cap ? (wanted ? wanted : 1) : cap;
 }
 
 void launch_small_count(
-    const BatchInput& in, size_t max_points, bool any_for_cta_kernel, unsigned long long* system_count, DeviceHeader* header, cudaStream_t stream
+    const BatchInput& in, size_t max_points, bool any_for_cta_kernel, unsigned long long* system_count, unsigned long long* share_count,
+    DeviceHeader* header, cudaStream_t stream
 ) {
     const PairOutput nothing{};
-    molecules_kernel<false><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, 0, stream>>>(in, system_count, nullptr, nothing, header, 0ull);
+    molecules_kernel<false><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
+        in, system_count, nullptr, nothing, header, 0ull
+    );
     if (any_for_cta_kernel) {
-        small_systems_kernel<false><<<small_grid(in.n_systems), SMALL_THREADS, small_shared_bytes(max_points), stream>>>(
-            in, system_count, nullptr, nothing, header, 0ull
+        const unsigned splits = small_splits(in.n_systems, max_points);
+        small_systems_kernel<false><<<small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream>>>(
+            in, splits, system_count, share_count, nullptr, nothing, header, 0ull
         );
     }
 }
 
 void launch_small_emit(
-    const BatchInput& in, size_t max_points, bool any_for_cta_kernel, const unsigned long long* system_start, PairOutput out,
-    DeviceHeader* header, cudaStream_t stream, unsigned long long capacity
+    const BatchInput& in, size_t max_points, bool any_for_cta_kernel, const unsigned long long* system_start,
+    unsigned long long* share_count, PairOutput out, DeviceHeader* header, cudaStream_t stream, unsigned long long capacity
 ) {
     // paired stores of full lists need aligned arrays (every system of a full list starts on an even element)
     out.interleave_ok = paired_stores_fit(out);
-    molecules_kernel<true><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, 0, stream>>>(in, nullptr, system_start, out, header, capacity);
+    molecules_kernel<true><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
+        in, nullptr, system_start, out, header, capacity
+    );
     if (any_for_cta_kernel) {
-        small_systems_kernel<true><<<small_grid(in.n_systems), SMALL_THREADS, small_shared_bytes(max_points), stream>>>(
-            in, nullptr, system_start, out, header, capacity
+        const unsigned splits = small_splits(in.n_systems, max_points);
+        small_systems_kernel<true><<<small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream>>>(
+            in, splits, nullptr, share_count, system_start, out, header, capacity
         );
     }
 }
