@@ -84,7 +84,7 @@ class BatchNeighborList:
         pair_offsets = self.build(points, system_offsets, boxes, periodic, quantities, global_indices)
 
         n_pairs = self._neighbors.length
-        owner = self._neighbors
+        owner = self  # a view keeps the calculator, and with it the arrays, alive
         offsets_out = _view(pair_offsets, (n_systems + 1,), "<u8", device, owner).view(torch.int64)
         if n_pairs == 0:
             pairs = torch.empty((0, 2), dtype=torch.int64, device=device)

@@ -249,7 +249,7 @@ class NeighborList:
             distances = torch.empty((0,), dtype=torch_float, device=device)
             vectors = torch.empty((0, 3), dtype=torch_float, device=device)
         else:
-            owner = self._neighbors
+            owner = self  # a view keeps the calculator, and with it the arrays, alive
             pairs = _view(self._neighbors.pairs, (n_pairs, 2), "<u8", device, owner)
             shifts = distances = vectors = None
             if "S" in quantities:

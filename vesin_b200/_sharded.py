@@ -259,7 +259,7 @@ class ShardedNeighborList:
 
     def _outputs(self, device, quantities, copy, value_dtype=torch.float64):
         n_pairs = self._neighbors.length
-        owner = self._neighbors
+        owner = self  # a view keeps the calculator, and with it the arrays, alive
         finish = (lambda t: t.clone()) if copy else (lambda t: t)
         typestr = "<f4" if value_dtype == torch.float32 else "<f8"
         if n_pairs == 0:
