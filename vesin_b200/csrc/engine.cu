@@ -1008,9 +1008,18 @@ void neighbors(
         }
         if (total > 0) {
             const PairOutput out = target.view();
-            // a canonical list: the rows go to a second set of arrays first, from where they are sorted into the list's
+            // a second index can come twice in a row only with two images of the same point
+            // within the cutoff of the first: a lattice vector shorter than twice the cutoff
+            bool duplicates_possible = false;
+            for (int k = 0; k < 3; k++) {
+                duplicates_possible = duplicates_possible || (plan.periodic[k] && plan.face_dist[k] < 2.0 * options.cutoff * (1.0 + 1e-9));
+            }
+            const int canonical_batch = canonical ? canonical_emit_batch(header.max_candidates, duplicates_possible) : 0;
+            // a canonical list whose rows can not be written in their final order: they go to a second set
+            // of arrays first, from where they are sorted into the list's
+            const bool sort_behind = canonical && canonical_batch == 0;
             PairOutput rows = out;
-            if (canonical) {
+            if (sort_behind) {
                 ws.alt_pairs.reserve(total * 2 * sizeof(size_t));
                 rows = PairOutput{};
                 rows.values_float = out.values_float;
@@ -1032,15 +1041,9 @@ void neighbors(
             VB200_CUDA(cudaMemsetAsync(ws.row_fill.ptr, 0, n_points * sizeof(uint32_t), stream));
             launch_emit(
                 plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.unit_mask_base.as<unsigned long long>(),
-                ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), rows, stream
+                ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), rows, canonical_batch, stream
             );
-            if (canonical) {
-                // a second index can come twice in a row only with two images of the same point
-                // within the cutoff of the first: a lattice vector shorter than twice the cutoff
-                bool duplicates_possible = false;
-                for (int k = 0; k < 3; k++) {
-                    duplicates_possible = duplicates_possible || (plan.periodic[k] && plan.face_dist[k] < 2.0 * options.cutoff * (1.0 + 1e-9));
-                }
+            if (sort_behind) {
                 launch_sort_rows(ws.row_start.as<unsigned long long>(), n_points, rows, out, duplicates_possible, stream);
             }
             timer.end(VesinB200StageEmit);

@@ -303,6 +303,7 @@ __device__ __forceinline__ void reset_header(DeviceHeader* header, const RealVie
         header->pair_cursor = 0;
         header->run_cursor = 0;
         header->status = 0;
+        header->max_candidates = 0;
     }
 }
 
@@ -1904,8 +1905,6 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
 
 struct RowShared {
     FusedShared staged;
-    unsigned long long home_row[TILE_POINTS]; // where the row of a home point continues
-    int row_offset[TILE_POINTS + 1];          // list position where the hits of each home point start
     int tile_hits[TILE_POINTS];               // pass 1: hits of the home points of the tile in the current batch
     unsigned long long mask_base;
 };
@@ -1942,9 +1941,7 @@ __device__ __forceinline__ int row_words_of_unit(
 
 /// Stage `batch_slots` candidates starting at slot `batch0` of the current
 /// segment group: original positions and (shift part, index) for the exact
-/// arithmetic and the output, and, with NEAR, fp32 coordinates relative to the
-/// unit centre for the screen.
-template <bool NEAR>
+/// arithmetic, and fp32 coordinates relative to the unit centre for the screen.
 __device__ __forceinline__ void stage_row_batch(
     FusedShared& sh, const GridPlan& plan, const SortedPoints& sorted, int n_stencil, int batch0, int batch_slots
 ) {
@@ -1962,7 +1959,7 @@ __device__ __forceinline__ void stage_row_batch(
         sh.y[s] = record.y;
         sh.z[s] = record.z;
         sh.sj[s] = make_int4(r0, r1, r2, record.index);
-        if (NEAR) {
+        {
             double ix = record.x;
             double iy = record.y;
             double iz = record.z;
@@ -1980,7 +1977,7 @@ __device__ __forceinline__ void stage_row_batch(
             sh.near_n[s] = fx * fx + fy * fy + fz * fz;
         }
     }
-    if (NEAR) {
+    {
         const int batch_words = (batch_slots + 31) >> 5;
         for (int s = batch_slots + threadIdx.x; s < batch_words * 32; s += CTA_THREADS) {
             sh.near_x[s] = 0.0f;
@@ -2011,6 +2008,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
     if (threadIdx.x < TILE_POINTS) {
         rows.tile_hits[threadIdx.x] = 0;
     }
+    unsigned most_candidates = 0; // of the units of this CTA
 
     for (int u = blockIdx.x; u < plan.n_units; u += gridDim.x) {
         const Unit unit = unit_of(plan, cell_start, u);
@@ -2027,6 +2025,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
 
         int group_total = 0;
         const int words = row_words_of_unit(plan, cell_start, unit, n_groups, sh.table, group_total);
+        most_candidates = max(most_candidates, (n_groups == 1) ? static_cast<unsigned>(group_total) : 0xffffffffu);
         // claim the storage of the hit words: n_tiles blocks of `words` x 32 lanes
         if (threadIdx.x == 0) {
             const unsigned long long need = static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS;
@@ -2061,7 +2060,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
             for (int batch0 = 0; batch0 < group_total; batch0 += FUSED_BATCH) {
                 const int batch_slots = min(FUSED_BATCH, group_total - batch0);
                 const int batch_words = (batch_slots + 31) >> 5;
-                stage_row_batch<true>(sh, plan, sorted, unit.n_stencil, batch0, batch_slots);
+                stage_row_batch(sh, plan, sorted, unit.n_stencil, batch0, batch_slots);
 
                 for (int tile = 0; tile < n_tiles; tile++) {
                     __syncthreads(); // staging done; previous tile done with the hit words and the home points
@@ -2154,6 +2153,411 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
             word_base += (group_total + 31) >> 5;
         }
     }
+    if (threadIdx.x == 0 && most_candidates != 0) {
+        atomicMax(&header->max_candidates, most_candidates);
+    }
+}
+
+// (the rows of a tile are spread over the warps of the CTA: a row is listed and written by one
+// warp, so that every store covers one contiguous span of it)
+
+constexpr int ROW_WINDOW = 128;    // hits of a row a warp lists at a time
+constexpr int RANK_BUCKETS = 1024; // see rank_candidates
+
+/// Shape of the CTAs of the row-writing kernel: BATCH candidates are staged at a time.
+/// CANONICAL: all candidates of a unit fit one batch and are staged in the order of their indices.
+template <bool CANONICAL_, int BATCH_, int CTAS_PER_SM_>
+struct RowShape {
+    static constexpr bool CANONICAL = CANONICAL_;
+    static constexpr int BATCH = BATCH_;
+    static constexpr int WORDS = BATCH_ / 32;
+    static constexpr int LANE_WORDS = (WORDS + 31) / 32; // consecutive words of a row that a lane looks after
+    static constexpr int CTAS_PER_SM = CTAS_PER_SM_;
+    static_assert(BATCH_ % 32 == 0 && BATCH_ <= 65536, "whole words, slots of 16 bits");
+
+    struct Staged {
+        double x[BATCH_]; // original positions of the candidates
+        double y[BATCH_];
+        double z[BATCH_];
+        int4 sj[BATCH_];  // x, y, z: q - wrap shift of the candidate; w: its index
+    };
+    struct Ordering { // what ranking the candidates needs, before they are staged
+        unsigned key[BATCH_];                 // index of the candidate in a slot
+        unsigned gathered[BATCH_];            // the same, bucket by bucket
+        int first[RANK_BUCKETS + 1];          // candidates in a bucket, then where the bucket starts
+        unsigned least, most;
+    };
+    struct Shared {
+        union {
+            Staged staged;
+            Ordering ordering;
+        };
+        union {
+            unsigned mask[TILE_POINTS * (WORDS + 1)]; // [home point][word], padded against bank conflicts
+            unsigned short order[BATCH_];             // place -> slot, until the candidates are staged
+        };
+        alignas(16) double transpose[CTA_WARPS][TRANSPOSE_DOUBLES / 2]; // per warp: on the way to coalesced stores
+        SegmentTable table;
+        double home_pos[3][TILE_POINTS];
+        int4 home_sj[TILE_POINTS];                // x, y, z: wrap shift of the home point; w: its index
+        unsigned long long home_row[TILE_POINTS]; // where the row of a home point continues
+        unsigned short list[CTA_WARPS][ROW_WINDOW];
+        unsigned short rank[CANONICAL_ ? BATCH_ : 1];                              // slot -> place in the order of the indices
+        unsigned bitmap[CANONICAL_ ? CTA_WARPS : 1][CANONICAL_ ? 32 * LANE_WORDS : 1]; // hits of a row in that order
+    };
+    static_assert((sizeof(Shared) + 1024) * CTAS_PER_SM_ <= 228 * 1024, "CTAS_PER_SM CTAs fit on an SM");
+};
+using SortedRows = RowShape<false, 1024, 4>;
+using CanonicalRows = RowShape<true, 896, 4>;
+using CanonicalRowsWide = RowShape<true, 2048, 2>;
+
+/// Ranks the candidates of a unit by their indices (images of one point, which a row never has
+/// two of, in any order): sh.ordering.key[0 ... n) -> sh.rank and sh.order. Buckets of equal width between the smallest and the largest index, counted
+/// and scanned; a candidate's rank is the start of its bucket plus the smaller ones inside it. The
+/// indices around a unit are either scattered (a bucket holds one or two) or come in runs (crystals
+/// in lattice order: about twenty), so this takes a third of the instructions of a bitonic sort of
+/// the same keys, and no more when all fall into one bucket. Starts behind a barrier that follows
+/// the writes of the keys, least and most, and ends with one.
+template <class Shape>
+__device__ __forceinline__ void rank_candidates(typename Shape::Shared& sh, int n) {
+    auto& o = sh.ordering;
+    constexpr int PER_THREAD = (Shape::BATCH + CTA_THREADS - 1) / CTA_THREADS;
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    // (rounding is monotonic: a larger index never falls into an earlier bucket)
+    const float scale = static_cast<float>(RANK_BUCKETS) / (static_cast<float>(o.most - o.least) + 1.0f);
+    int bucket[PER_THREAD], arrival[PER_THREAD];
+#pragma unroll
+    for (int e = 0; e < PER_THREAD; e++) {
+        const int s = threadIdx.x + e * CTA_THREADS;
+        if (s < n) {
+            bucket[e] = min(static_cast<int>(static_cast<float>(o.key[s] - o.least) * scale), RANK_BUCKETS - 1);
+            arrival[e] = atomicAdd(&o.first[bucket[e]], 1);
+        }
+    }
+    __syncthreads();
+    constexpr int SCAN = RANK_BUCKETS / CTA_THREADS;
+    int counts[SCAN];
+    int mine = 0;
+#pragma unroll
+    for (int e = 0; e < SCAN; e++) {
+        counts[e] = o.first[threadIdx.x * SCAN + e];
+        mine += counts[e];
+    }
+    int inclusive = mine;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+        const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
+        if (lane >= offset) {
+            inclusive += up;
+        }
+    }
+    if (lane == 31) {
+        sh.table.scan_tmp[warp] = inclusive;
+    }
+    __syncthreads();
+    int start = inclusive - mine;
+#pragma unroll
+    for (int w = 0; w < CTA_WARPS; w++) {
+        start += (w < warp) ? sh.table.scan_tmp[w] : 0;
+    }
+#pragma unroll
+    for (int e = 0; e < SCAN; e++) {
+        o.first[threadIdx.x * SCAN + e] = start;
+        start += counts[e];
+    }
+    if (threadIdx.x == 0) {
+        o.first[RANK_BUCKETS] = n;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < PER_THREAD; e++) {
+        const int s = threadIdx.x + e * CTA_THREADS;
+        if (s < n) {
+            o.gathered[o.first[bucket[e]] + arrival[e]] = o.key[s];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < PER_THREAD; e++) {
+        const int s = threadIdx.x + e * CTA_THREADS;
+        if (s < n) {
+            const unsigned key = o.key[s];
+            const int first = o.first[bucket[e]];
+            const int last = o.first[bucket[e] + 1];
+            const int mine = first + arrival[e];
+            int place = first;
+            for (int k = first; k < last; k++) {
+                const unsigned other = o.gathered[k];
+                place += (other < key || (other == key && k < mine)) ? 1 : 0;
+            }
+            sh.rank[s] = static_cast<unsigned short>(place);
+            sh.order[place] = static_cast<unsigned short>(s);
+        }
+    }
+    __syncthreads();
+}
+
+/// Hits [from, to) of a row whose words lie in shared memory, lane l being the one that counted the
+/// LANE_WORDS words from l * LANE_WORDS on (`begin`: hits before them): use(number, slot) for each,
+/// the same number of consecutive hits per lane. The bits of a word come in clusters (32 candidates
+/// lie in one or two cells), so a lane per word would wait for the fullest one.
+template <int LANE_WORDS, class Use>
+__device__ __forceinline__ void for_row_hits(const unsigned* words, int begin, int from, int to, int lane, Use use) {
+    const int quota = (to - from + 31) >> 5;
+    int position = from + lane * quota;
+    const int stop = min(position + quota, to);
+    const int target = min(position, to - 1);
+    int owner = 0; // last lane whose words begin at or before the target
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+        if (__shfl_sync(FULL_MASK, begin, owner + step) <= target) {
+            owner += step;
+        }
+    }
+    int skip = target - __shfl_sync(FULL_MASK, begin, owner);
+    if (position < stop) {
+        int w = owner * LANE_WORDS;
+        unsigned word = words[w];
+#pragma unroll
+        for (int k = 1; k < LANE_WORDS; k++) {
+            const int count = __popc(word);
+            if (skip >= count) {
+                skip -= count;
+                word = words[++w];
+            }
+        }
+        word &= 0xffffffffu << select_bit(word, skip);
+        for (; position < stop; position++) {
+            while (word == 0) {
+                word = words[++w];
+            }
+            const int b = __ffs(word) - 1;
+            word &= word - 1;
+            use(position, w * 32 + b);
+        }
+    }
+}
+
+/// Counts the words of a row (lane l: LANE_WORDS from l * LANE_WORDS on, `n_words` in all): returns
+/// the hits before the lane's words and leaves the number of hits in `total`.
+template <int LANE_WORDS>
+__device__ __forceinline__ int count_row_hits(const unsigned* words, int n_words, int lane, int& total) {
+    int mine = 0;
+#pragma unroll
+    for (int k = 0; k < LANE_WORDS; k++) {
+        const int w = lane * LANE_WORDS + k;
+        mine += (w < n_words) ? __popc(words[w]) : 0;
+    }
+    int inclusive = mine;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+        const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
+        if (lane >= offset) {
+            inclusive += up;
+        }
+    }
+    total = __shfl_sync(FULL_MASK, inclusive, 31);
+    return inclusive - mine;
+}
+
+template <class Shape>
+__global__ void __launch_bounds__(CTA_THREADS, Shape::CTAS_PER_SM) row_emit_kernel(
+    const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, const uint32_t* __restrict__ masks,
+    const unsigned long long* __restrict__ unit_mask_base, const uint32_t* __restrict__ unit_words,
+    const unsigned long long* __restrict__ row_start, uint32_t* __restrict__ row_fill, PairOutput out
+) {
+    using Shared = typename Shape::Shared;
+    constexpr int BATCH = Shape::BATCH;
+    constexpr int WORDS = Shape::WORDS;
+    constexpr int LANE_WORDS = Shape::LANE_WORDS;
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    Shared& sh = *reinterpret_cast<Shared*>(row_smem);
+
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+
+    for (int u = blockIdx.x; u < plan.n_units; u += gridDim.x) {
+        const Unit unit = unit_of(plan, cell_start, u);
+        if (unit.n_home == 0) {
+            continue;
+        }
+        const int n_groups = (unit.n_stencil + SEG_MAX - 1) / SEG_MAX;
+        const int n_tiles = (unit.n_home + TILE_POINTS - 1) / TILE_POINTS;
+        const unsigned long long base = unit_mask_base[u];
+        const int words = static_cast<int>(unit_words[u]);
+
+        int word_base = 0;
+        for (int g = 0; g < n_groups; g++) {
+            const int group_total = setup_segments(plan, cell_start, unit, g, sh.table);
+            // (a row whose candidates come in several batches is continued from batch to batch)
+            const bool continued = n_groups > 1 || group_total > BATCH;
+            const auto record_of = [&](int slot, int& t) {
+                t = (unit.n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
+                return static_cast<size_t>(sh.table.start[t]) + (slot - sh.table.slot0[t]);
+            };
+            for (int batch0 = 0; batch0 < group_total; batch0 += BATCH) {
+                const int batch_slots = min(BATCH, group_total - batch0);
+                const int batch_words = (batch_slots + 31) >> 5;
+                if (Shape::CANONICAL) {
+                    // (the only batch of the unit; the caller made sure of that)
+                    for (int k = threadIdx.x; k < RANK_BUCKETS; k += CTA_THREADS) {
+                        sh.ordering.first[k] = 0;
+                    }
+                    if (threadIdx.x == 0) {
+                        sh.ordering.least = 0xffffffffu;
+                        sh.ordering.most = 0u;
+                    }
+                    __syncthreads();
+                    unsigned least = 0xffffffffu;
+                    unsigned most = 0u;
+#pragma unroll 4
+                    for (int s = threadIdx.x; s < batch_slots; s += CTA_THREADS) {
+                        int t;
+                        const unsigned key = static_cast<unsigned>(sorted.records[record_of(s, t)].index);
+                        sh.ordering.key[s] = key;
+                        least = min(least, key);
+                        most = max(most, key);
+                    }
+                    least = __reduce_min_sync(FULL_MASK, least);
+                    most = __reduce_max_sync(FULL_MASK, most);
+                    if (lane == 0 && least <= most) {
+                        atomicMin(&sh.ordering.least, least);
+                        atomicMax(&sh.ordering.most, most);
+                    }
+                    __syncthreads();
+                    rank_candidates<Shape>(sh, batch_slots);
+                }
+                // ---- stage the candidates: in the order of their slots, or of their indices ----
+#pragma unroll 2
+                for (int s = threadIdx.x; s < batch_slots; s += CTA_THREADS) {
+                    const int slot = Shape::CANONICAL ? static_cast<int>(sh.order[s]) : batch0 + s;
+                    int t;
+                    const LoadedRecord record = load_record(sorted, record_of(slot, t));
+                    int r0, r1, r2;
+                    unpack_segment_image(sh.table.image[t], r0, r1, r2);
+                    sh.staged.x[s] = record.x;
+                    sh.staged.y[s] = record.y;
+                    sh.staged.z[s] = record.z;
+                    sh.staged.sj[s] = make_int4(r0 - record.s0, r1 - record.s1, r2 - record.s2, record.index);
+                }
+
+                for (int tile = 0; tile < n_tiles; tile++) {
+                    __syncthreads(); // staging done (and the keys read); previous tile done with the shared arrays
+                    const int n_in_tile = min(TILE_POINTS, unit.n_home - tile * TILE_POINTS);
+                    if (threadIdx.x < n_in_tile) {
+                        const size_t pi = static_cast<size_t>(unit.begin) + tile * TILE_POINTS + threadIdx.x;
+                        const LoadedRecord record = load_record(sorted, pi);
+                        sh.home_pos[0][threadIdx.x] = record.x;
+                        sh.home_pos[1][threadIdx.x] = record.y;
+                        sh.home_pos[2][threadIdx.x] = record.z;
+                        sh.home_sj[threadIdx.x] = make_int4(record.s0, record.s1, record.s2, record.index);
+                        sh.home_row[threadIdx.x] = row_start[record.index] + (continued ? row_fill[record.index] : 0u);
+                    }
+                    // hit words of the tile, from [word][home point] to [home point][word]
+                    const uint32_t* mask_tile = masks + base + (static_cast<unsigned long long>(tile) * words + word_base + (batch0 >> 5)) * TILE_POINTS;
+                    for (int k = threadIdx.x; k < batch_words * TILE_POINTS; k += CTA_THREADS) {
+                        sh.mask[(k & 31) * (WORDS + 1) + (k >> 5)] = mask_tile[k];
+                    }
+                    __syncthreads();
+
+                    for (int h = warp; h < n_in_tile; h += CTA_WARPS) {
+                        const unsigned* row_words = sh.mask + h * (WORDS + 1);
+                        int total;
+                        int begin = count_row_hits<LANE_WORDS>(row_words, batch_words, lane, total);
+                        if (total == 0) {
+                            continue;
+                        }
+                        if (Shape::CANONICAL) {
+                            // hits by slot -> hits by place in the order of the indices
+                            unsigned* bitmap = sh.bitmap[warp];
+                            __syncwarp();
+#pragma unroll
+                            for (int k = 0; k < LANE_WORDS; k++) {
+                                bitmap[lane + 32 * k] = 0;
+                            }
+                            __syncwarp();
+                            for_row_hits<LANE_WORDS>(row_words, begin, 0, total, lane, [&](int, int slot) {
+                                const unsigned place = sh.rank[slot];
+                                atomicOr(&bitmap[place >> 5], 1u << (place & 31));
+                            });
+                            __syncwarp();
+                            row_words = bitmap;
+                            begin = count_row_hits<LANE_WORDS>(row_words, 32 * LANE_WORDS, lane, total);
+                        }
+
+                        const int4 home = sh.home_sj[h];
+                        const double hx = sh.home_pos[0][h];
+                        const double hy = sh.home_pos[1][h];
+                        const double hz = sh.home_pos[2][h];
+                        const unsigned long long row = sh.home_row[h];
+                        for (int window = 0; window < total; window += ROW_WINDOW) {
+                            __syncwarp();
+                            for_row_hits<LANE_WORDS>(row_words, begin, window, min(window + ROW_WINDOW, total), lane, [&](int number, int slot) {
+                                sh.list[warp][number - window] = static_cast<unsigned short>(slot);
+                            });
+                            __syncwarp();
+                            const int in_window = min(ROW_WINDOW, total - window);
+                            for (int c0 = 0; c0 < in_window; c0 += 32) {
+                                const int n_valid = min(32, in_window - c0);
+                                const int s = (lane < n_valid) ? sh.list[warp][c0 + lane] : sh.list[warp][c0];
+                                const int4 cand = sh.staged.sj[s];
+                                const int s0 = cand.x + home.x;
+                                const int s1 = cand.y + home.y;
+                                const int s2 = cand.z + home.z;
+                                double vx, vy, vz, d2;
+                                if (__any_sync(FULL_MASK, (s0 | s1 | s2) != 0)) {
+                                    d2 = exact_pair(plan, hx, hy, hz, sh.staged.x[s], sh.staged.y[s], sh.staged.z[s], s0, s1, s2, vx, vy, vz);
+                                } else {
+                                    // (the signed zeros that the products with S = 0 give)
+                                    vx = __dadd_rn(__dsub_rn(sh.staged.x[s], hx), plan.zero_shift[0]);
+                                    vy = __dadd_rn(__dsub_rn(sh.staged.y[s], hy), plan.zero_shift[1]);
+                                    vz = __dadd_rn(__dsub_rn(sh.staged.z[s], hz), plan.zero_shift[2]);
+                                    d2 = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
+                                }
+                                store_pairs(
+                                    sh.transpose[warp], out, lane, row + static_cast<unsigned long long>(window + c0), n_valid,
+                                    static_cast<unsigned long long>(home.w), static_cast<unsigned long long>(cand.w), s0, s1, s2, __dsqrt_rn(d2), vx, vy,
+                                    vz
+                                );
+                            }
+                        }
+                        if (continued && lane == 0) {
+                            row_fill[home.w] += static_cast<uint32_t>(total); // (read again behind the barriers of the next batch)
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+            word_base += (group_total + 31) >> 5;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// canonical order inside the rows
+// A list sorted by the first index becomes THE canonical list (rows ordered by
+// second index, then by shift) when every row is sorted. Rows are short (tens
+// to hundreds of pairs), so a warp ranks the pairs of a row against each other
+// (the rank of a pair is the number of pairs of the row that come before it)
+// and copies every pair to its place in a second set of arrays. No counterpart
+// in the reference, whose device sort stops at the first index
+// (vesin/src/cuda/sort_pairs.cu:3-12).
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ bool shift_before(const int32_t* __restrict__ shifts, unsigned long long a, unsigned long long b) {
+    if (shifts == nullptr) {
+        return false;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const int sa = shifts[3 * a + c];
+        const int sb = shifts[3 * b + c];
+        if (sa != sb) {
+            return sa < sb;
+        }
+    }
+    return false;
 }
 
 /// 12-byte element at a 4-byte aligned address: one 8-byte and one 4-byte store.
@@ -2190,240 +2594,6 @@ __device__ __forceinline__ void store_triple_64(double* base, unsigned long long
         __stcs(dst, a);
         __stcs(reinterpret_cast<double2*>(dst + 1), make_double2(b, c));
     }
-}
-
-__global__ void __launch_bounds__(CTA_THREADS, 4) row_emit_kernel(
-    const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, const uint32_t* __restrict__ masks,
-    const unsigned long long* __restrict__ unit_mask_base, const uint32_t* __restrict__ unit_words,
-    const unsigned long long* __restrict__ row_start, uint32_t* __restrict__ row_fill, PairOutput out
-) {
-    extern __shared__ __align__(16) unsigned char row_smem[];
-    RowShared& rows = *reinterpret_cast<RowShared*>(row_smem);
-    FusedShared& sh = rows.staged;
-    static_assert(FUSED_WORDS == 16 && FUSED_TASKS == 2, "tasks are (home point, word) pairs: home = task >> 4");
-
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-
-    for (int u = blockIdx.x; u < plan.n_units; u += gridDim.x) {
-        const Unit unit = unit_of(plan, cell_start, u);
-        if (unit.n_home == 0) {
-            continue;
-        }
-        const int n_groups = (unit.n_stencil + SEG_MAX - 1) / SEG_MAX;
-        const int n_tiles = (unit.n_home + TILE_POINTS - 1) / TILE_POINTS;
-        const unsigned long long base = unit_mask_base[u];
-        const int words = static_cast<int>(unit_words[u]);
-
-        int word_base = 0;
-        for (int g = 0; g < n_groups; g++) {
-            const int group_total = setup_segments(plan, cell_start, unit, g, sh.table);
-            for (int batch0 = 0; batch0 < group_total; batch0 += FUSED_BATCH) {
-                const int batch_slots = min(FUSED_BATCH, group_total - batch0);
-                const int batch_words = (batch_slots + 31) >> 5;
-                stage_row_batch<false>(sh, plan, sorted, unit.n_stencil, batch0, batch_slots);
-
-                for (int tile = 0; tile < n_tiles; tile++) {
-                    __syncthreads(); // staging done; previous tile done with the shared arrays
-                    if (threadIdx.x < TILE_POINTS) {
-                        const int il = tile * TILE_POINTS + threadIdx.x;
-                        if (il < unit.n_home) {
-                            const size_t pi = static_cast<size_t>(unit.begin) + il;
-                            const LoadedRecord record = load_record(sorted, pi);
-                            sh.home_pos[0][threadIdx.x] = record.x;
-                            sh.home_pos[1][threadIdx.x] = record.y;
-                            sh.home_pos[2][threadIdx.x] = record.z;
-                            sh.home_sj[threadIdx.x] = make_int4(record.s0, record.s1, record.s2, record.index);
-                            rows.home_row[threadIdx.x] = row_start[record.index] + row_fill[record.index];
-                        }
-                    }
-                    // hit words of the tile, transposed to [home point][word] so that the hits of a
-                    // point are consecutive tasks; words past the batch hold nothing
-                    const uint32_t* mask_tile = masks + base + (static_cast<unsigned long long>(tile) * words + word_base + (batch0 >> 5)) * TILE_POINTS;
-                    for (int k = threadIdx.x; k < FUSED_WORDS * TILE_POINTS; k += CTA_THREADS) {
-                        const int w = k >> 5;
-                        sh.mask[(k & 31) * FUSED_WORDS + w] = (w < batch_words) ? mask_tile[k] : 0u;
-                    }
-                    __syncthreads();
-
-                    // ---- scan of the hit counts of the tasks (two consecutive tasks per thread) ----
-                    const unsigned word_a = sh.mask[2 * threadIdx.x];
-                    const unsigned word_b = sh.mask[2 * threadIdx.x + 1];
-                    const int my_hits = __popc(word_a) + __popc(word_b);
-                    int inclusive = my_hits;
-#pragma unroll
-                    for (int offset = 1; offset < 32; offset <<= 1) {
-                        const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
-                        if (lane >= offset) {
-                            inclusive += up;
-                        }
-                    }
-                    sh.prefix[threadIdx.x] = static_cast<unsigned short>(inclusive - my_hits);
-                    if (lane == 31) {
-                        sh.table.scan_tmp[warp] = inclusive;
-                    }
-                    __syncthreads();
-                    int total_hits = 0;
-                    int before_warp = 0;
-#pragma unroll
-                    for (int w = 0; w < CTA_WARPS; w++) {
-                        const int sum = sh.table.scan_tmp[w];
-                        if (w < warp) {
-                            before_warp += sum;
-                        }
-                        total_hits += sum;
-                    }
-                    // the thread that owns the first task of a home point knows where its hits start
-                    if ((threadIdx.x & 7) == 0) {
-                        rows.row_offset[threadIdx.x >> 3] = before_warp + inclusive - my_hits;
-                    }
-                    if (threadIdx.x == 0) {
-                        rows.row_offset[TILE_POINTS] = total_hits;
-                    }
-
-                    for (int round0 = 0; round0 < total_hits; round0 += FUSED_LIST) {
-                        if (round0 != 0) {
-                            __syncthreads(); // previous round consumed
-                        }
-                        const int in_round = min(FUSED_LIST, total_hits - round0);
-                        {
-                            // every thread writes the same number of consecutive list entries (see the fused pass)
-                            const int quota = (in_round + CTA_THREADS - 1) / CTA_THREADS;
-                            int position = round0 + threadIdx.x * quota;
-                            const int stop = min(position + quota, round0 + in_round);
-                            if (position < stop) {
-                                int owner_warp = 0;
-                                int before = 0;
-                                {
-                                    int running = 0;
-#pragma unroll
-                                    for (int w = 0; w < CTA_WARPS - 1; w++) {
-                                        running += sh.table.scan_tmp[w];
-                                        if (running <= position) {
-                                            owner_warp = w + 1;
-                                            before = running;
-                                        }
-                                    }
-                                }
-                                const int target = position - before;
-                                const unsigned short* local = sh.prefix + owner_warp * 32;
-                                int lo = 0;
-                                int hi = 32;
-#pragma unroll
-                                for (int step = 0; step < 5; step++) {
-                                    const int mid = (lo + hi) >> 1;
-                                    if (static_cast<int>(local[mid]) <= target) {
-                                        lo = mid;
-                                    } else {
-                                        hi = mid;
-                                    }
-                                }
-                                int skip = target - static_cast<int>(local[lo]);
-                                lo += owner_warp * 32;
-                                int task = lo * 2;
-                                unsigned word = sh.mask[task];
-                                {
-                                    const int count = __popc(word);
-                                    if (skip >= count) {
-                                        skip -= count;
-                                        task++;
-                                        word = sh.mask[task];
-                                    }
-                                }
-                                word &= 0xffffffffu << select_bit(word, skip);
-                                for (; position < stop; position++) {
-                                    while (word == 0 && task + 1 < FUSED_WORDS * TILE_POINTS) {
-                                        task++;
-                                        word = sh.mask[task];
-                                    }
-                                    const int bit = __ffs(word) - 1;
-                                    word &= word - 1;
-                                    // (home point << 9) | slot in the batch
-                                    sh.list[position - round0] = static_cast<unsigned short>(((task >> 4) << 9) | ((task & 15) << 5) | (bit & 31));
-                                }
-                            }
-                        }
-                        __syncthreads();
-
-                        for (int chunk0 = warp * 32; chunk0 < in_round; chunk0 += CTA_WARPS * 32) {
-                            if (chunk0 + lane >= in_round) {
-                                continue;
-                            }
-                            const unsigned entry = sh.list[chunk0 + lane];
-                            const int h = entry >> 9;
-                            const int s = entry & 511;
-                            const int4 cand = sh.sj[s];
-                            const int4 home = sh.home_sj[h];
-                            const int s0 = cand.x + home.x;
-                            const int s1 = cand.y + home.y;
-                            const int s2 = cand.z + home.z;
-                            double vx, vy, vz;
-                            const double d2 = exact_pair(
-                                plan, sh.home_pos[0][h], sh.home_pos[1][h], sh.home_pos[2][h], sh.x[s], sh.y[s], sh.z[s], s0, s1, s2, vx, vy, vz
-                            );
-                            const unsigned long long dest = rows.home_row[h] + static_cast<unsigned long long>(round0 + chunk0 + lane - rows.row_offset[h]);
-                            store_indices(out, dest, static_cast<unsigned long long>(home.w), static_cast<unsigned long long>(cand.w));
-                            if (out.shifts != nullptr) {
-                                store_triple_32(out.shifts, dest, s0, s1, s2);
-                            }
-                            if (out.values_float) {
-                                if (out.distances != nullptr) {
-                                    __stcs(reinterpret_cast<float*>(out.distances) + dest, static_cast<float>(__dsqrt_rn(d2)));
-                                }
-                                if (out.vectors != nullptr) {
-                                    store_triple_32(
-                                        reinterpret_cast<float*>(out.vectors), dest, static_cast<float>(vx), static_cast<float>(vy), static_cast<float>(vz)
-                                    );
-                                }
-                            } else {
-                                if (out.distances != nullptr) {
-                                    __stcs(out.distances + dest, __dsqrt_rn(d2));
-                                }
-                                if (out.vectors != nullptr) {
-                                    store_triple_64(out.vectors, dest, vx, vy, vz);
-                                }
-                            }
-                        }
-                    }
-                    __syncthreads();
-                    if (threadIdx.x < TILE_POINTS && tile * TILE_POINTS + threadIdx.x < unit.n_home) {
-                        const int hits = rows.row_offset[threadIdx.x + 1] - rows.row_offset[threadIdx.x];
-                        if (hits != 0) {
-                            row_fill[sh.home_sj[threadIdx.x].w] += static_cast<uint32_t>(hits);
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-            word_base += (group_total + 31) >> 5;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// canonical order inside the rows
-// A list sorted by the first index becomes THE canonical list (rows ordered by
-// second index, then by shift) when every row is sorted. Rows are short (tens
-// to hundreds of pairs), so a warp ranks the pairs of a row against each other
-// (the rank of a pair is the number of pairs of the row that come before it)
-// and copies every pair to its place in a second set of arrays. No counterpart
-// in the reference, whose device sort stops at the first index
-// (vesin/src/cuda/sort_pairs.cu:3-12).
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ bool shift_before(const int32_t* __restrict__ shifts, unsigned long long a, unsigned long long b) {
-    if (shifts == nullptr) {
-        return false;
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const int sa = shifts[3 * a + c];
-        const int sb = shifts[3 * b + c];
-        if (sa != sb) {
-            return sa < sb;
-        }
-    }
-    return false;
 }
 
 constexpr int ROW_SORT_STAGED = 512; // second indices of a row a warp keeps in shared memory
@@ -2620,7 +2790,9 @@ int pair_grid(int n_units, int per_sm) {
 void configure_kernels() {
     cudaFuncSetAttribute(row_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(RowShared)));
     cudaFuncSetAttribute(row_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(RowShared)));
-    cudaFuncSetAttribute(row_emit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(RowShared)));
+    cudaFuncSetAttribute(row_emit_kernel<SortedRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SortedRows::Shared)));
+    cudaFuncSetAttribute(row_emit_kernel<CanonicalRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(CanonicalRows::Shared)));
+    cudaFuncSetAttribute(row_emit_kernel<CanonicalRowsWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(CanonicalRowsWide::Shared)));
     cudaFuncSetAttribute(pairs_kernel<false, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<true, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<false, true, LargeCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(LargeCta::Shared)));
@@ -2761,14 +2933,33 @@ void launch_count(
     }
 }
 
+int canonical_emit_batch(unsigned max_candidates, bool duplicates_possible) {
+    if (duplicates_possible) {
+        return 0;
+    }
+    if (max_candidates <= CanonicalRows::BATCH) {
+        return CanonicalRows::BATCH;
+    }
+    return (max_candidates <= CanonicalRowsWide::BATCH) ? CanonicalRowsWide::BATCH : 0;
+}
+
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
-    const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, cudaStream_t stream
+    const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, int canonical_batch, cudaStream_t stream
 ) {
-    const int grid = pair_grid(plan.n_units, 4);
-    row_emit_kernel<<<grid, CTA_THREADS, sizeof(RowShared), stream>>>(
-        plan, cell_start, sorted, masks, unit_mask_base, unit_words, row_start, row_fill, out
-    );
+    const auto launch = [&](auto shape, auto kernel) {
+        using Shape = decltype(shape);
+        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), CTA_THREADS, sizeof(typename Shape::Shared), stream>>>(
+            plan, cell_start, sorted, masks, unit_mask_base, unit_words, row_start, row_fill, out
+        );
+    };
+    if (canonical_batch == CanonicalRows::BATCH) {
+        launch(CanonicalRows{}, row_emit_kernel<CanonicalRows>);
+    } else if (canonical_batch == CanonicalRowsWide::BATCH) {
+        launch(CanonicalRowsWide{}, row_emit_kernel<CanonicalRowsWide>);
+    } else {
+        launch(SortedRows{}, row_emit_kernel<SortedRows>);
+    }
 }
 
 void launch_sort_rows(

@@ -25,7 +25,7 @@ struct DeviceHeader {
     unsigned long long pair_cursor;  // output elements claimed by the fused pass (= its pair total)
     unsigned long long run_cursor;   // runs of work units handed out by the fused pass (dynamic scheduling)
     unsigned int status;             // sticky error bits, see STATUS_*
-    unsigned int pad;
+    unsigned int max_candidates;     // sorted lists: most candidates a unit has (~0: some unit has several groups of segments)
     double box[9];                   // copy of the caller's box
     unsigned char periodic[8];       // copy of the caller's periodic flags
     unsigned long long halo_count[2]; // slab decomposition: records in the two halo messages of this build
@@ -196,11 +196,16 @@ void launch_count(
 
 /// Sorted lists, pass 2: walks the hit bits and writes i, j, S, d, D, one row
 /// per point in index order (row_start from the scan of row_count; row_fill
-/// must start at zero).
+/// must start at zero). `canonical_batch`: 0, or what canonical_emit_batch()
+/// said: the rows then come out sorted by the second index.
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
-    const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, cudaStream_t stream
+    const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, int canonical_batch, cudaStream_t stream
 );
+/// Can pass 2 write the rows of a canonical list in their final order? It can when a CTA holds all
+/// candidates of a unit at once and no second index comes twice in a row. 0: it can not, the rows
+/// have to be sorted behind it (launch_sort_rows).
+int canonical_emit_batch(unsigned max_candidates, bool duplicates_possible);
 
 /// Sorts the pairs inside every row by (second index, shift): `in` holds rows
 /// [row_start[r], row_start[r + 1]), `out` receives the sorted rows.
