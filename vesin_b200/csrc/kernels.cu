@@ -1085,9 +1085,7 @@ __device__ unsigned long long g_phase_clocks[16];
 constexpr int FUSED_BATCH = 512;
 constexpr int DEFAULT_UNIT_RUN = 2; // neighbouring units handled back to back by one CTA (measured: 2 beats 1, 3, 4 and 8)
 constexpr int MAX_UNIT_SPLITS = 32; // CTAs that share the candidate batches of one unit (launches of few units)
-constexpr int FUSED_WORDS = FUSED_BATCH / 32;
 constexpr int FUSED_LIST = 2048;
-constexpr int FUSED_TASKS = (TILE_POINTS * FUSED_WORDS + CTA_THREADS - 1) / CTA_THREADS;
 
 /// Shared memory of a CTA of THREADS_ threads that stages BATCH_ candidates at a time and
 /// lists up to LIST_ hits per round.
@@ -1129,8 +1127,6 @@ struct FusedSharedT {
     int next_run[2];  // run of units this CTA takes next (two slots: one is read while the other is written)
     int slab_mode;    // slab decomposition: bit 0 = the unit's points are owned, bit 1 = so are all candidates of the group
 };
-/// The row kernels of sorted lists: 256 threads, 512 candidates per batch.
-using FusedShared = FusedSharedT<CTA_THREADS, FUSED_BATCH, FUSED_LIST>;
 
 /// Shape of the CTAs of the pair kernel of unsorted lists.
 template <int THREADS_, int BATCH_, int LIST_, int CTAS_PER_SM_>
@@ -1160,13 +1156,6 @@ using SmallCta = PairShape<128, 256, 1024, 8>;
 /// Units next to the halo of a slab (they sort their hits into owned and halo candidates and go
 /// over every batch twice): CTAs of 8 warps with 512 candidates per batch, 4 per SM.
 using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4>;
-static_assert(
-    offsetof(FusedShared, near_x) % 16 == 0 && offsetof(FusedShared, near_y) % 16 == 0 && offsetof(FusedShared, near_z) % 16 == 0 &&
-        offsetof(FusedShared, near_n) % 16 == 0 && offsetof(FusedShared, transpose) % 16 == 0 && offsetof(FusedShared, sj) % 16 == 0 &&
-        offsetof(FusedShared, home_sj) % 16 == 0,
-    "members read or written as 16-byte vectors"
-);
-
 /// Offset (in cells, relative to the first cell of the unit) of entry `index`
 /// of the half-shell stencil of a unit of `cells` cells.
 __device__ __forceinline__ void half_stencil_offset(const GridPlan& plan, int cells, int index, int& ox, int& oy, int& oz) {
@@ -1275,13 +1264,13 @@ __device__ __forceinline__ int setup_half_segments(
 
 /// Decisions of one lane's home point on BITS consecutive candidates of word `w`
 /// of the staged batch, starting at bit `first_bit`: fp32 screen of every
-/// candidate, the exact fp64 predicate for those too close to the cutoff for
-/// fp32. Returns one bit per candidate that is a pair.
-template <int BITS, class Shared>
+/// candidate, the exact fp64 predicate (`exact`: is the candidate in this slot of
+/// the batch a pair?) for those too close to the cutoff for fp32. Returns one bit
+/// per candidate that is a pair.
+template <int BITS, class Shared, class Exact>
 __device__ __forceinline__ unsigned decide_piece(
-    const Shared& sh, const GridPlan& plan, int w, int first_bit, int batch0, int home_row_slots, int il, unsigned long long ax2,
-    unsigned long long ay2, unsigned long long az2, unsigned long long an2, float cutoff2_lo, float cutoff2_hi, double rix, double riy,
-    double riz, int si0, int si1, int si2
+    const Shared& sh, int w, int first_bit, int batch0, int home_row_slots, int il, unsigned long long ax2, unsigned long long ay2,
+    unsigned long long az2, unsigned long long an2, float cutoff2_lo, float cutoff2_hi, Exact exact
 ) {
     constexpr unsigned ALL = (BITS == 32) ? 0xffffffffu : ((1u << (BITS & 31)) - 1u);
     unsigned inside = 0; // surely inside the cutoff
@@ -1328,11 +1317,7 @@ __device__ __forceinline__ unsigned decide_piece(
         // the exact fp64 predicate of the reference decides
         const int b = __ffs(band) - 1;
         band &= band - 1;
-        const int s = first_slot + b;
-        double vx, vy, vz;
-        const int4 cand = sh.sj[s];
-        const double d2_exact = exact_pair(plan, rix, riy, riz, sh.x[s], sh.y[s], sh.z[s], cand.x + si0, cand.y + si1, cand.z + si2, vx, vy, vz);
-        if (d2_exact < plan.cutoff2) {
+        if (exact(first_slot + b)) {
             inside |= 1u << b;
         }
     }
@@ -1609,14 +1594,18 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                     const unsigned long long az2 = pack_f32x2(az, az);
                     const unsigned long long an2 = pack_f32x2(an, an);
 
+                    const auto exact = [&](int s) {
+                        double vx, vy, vz;
+                        const int4 cand = sh.sj[s];
+                        return exact_pair(plan, rix, riy, riz, sh.x[s], sh.y[s], sh.z[s], cand.x + si0, cand.y + si1, cand.z + si2, vx, vy, vz) <
+                               plan.cutoff2;
+                    };
                     if (narrow) {
                         for (int w = warp; w < batch_words; w += Shape::WARPS) {
                             const int quarter = lane & 3;
-                            unsigned word = decide_piece<8>(
-                                            sh, plan, w, 8 * quarter, batch0, home_row_slots, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, rix, riy, riz,
-                                            si0, si1, si2
-                                        )
-                                        << (8 * quarter);
+                            unsigned word =
+                                decide_piece<8>(sh, w, 8 * quarter, batch0, home_row_slots, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, exact)
+                                << (8 * quarter);
                             // the four lanes of a home point put their quarters together
                             word |= __shfl_xor_sync(FULL_MASK, word, 1);
                             word |= __shfl_xor_sync(FULL_MASK, word, 2);
@@ -1626,9 +1615,8 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                     } else if (batch_words <= Shape::WARPS) {
                         // a word of 32 candidates per warp
                         if (warp < batch_words) {
-                            sh.mask[warp * TILE_POINTS + lane] = decide_piece<32>(
-                                sh, plan, warp, 0, batch0, home_row_slots, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, rix, riy, riz, si0, si1, si2
-                            );
+                            sh.mask[warp * TILE_POINTS + lane] =
+                                decide_piece<32>(sh, warp, 0, batch0, home_row_slots, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, exact);
                         }
                     } else {
                         // more words than warps: halves of words, so that no warp does two words while others do one
@@ -1637,8 +1625,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                             const int half = (piece >= batch_words) ? 1 : 0;
                             const int w = piece - half * batch_words;
                             halves[2 * (w * TILE_POINTS + lane) + half] = static_cast<unsigned short>(decide_piece<16>(
-                                sh, plan, w, 16 * half, batch0, home_row_slots, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, rix, riy, riz, si0, si1,
-                                si2
+                                sh, w, 16 * half, batch0, home_row_slots, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, exact
                             ));
                         }
                     }
@@ -1903,9 +1890,23 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
 // in the order the candidates were staged.
 // ---------------------------------------------------------------------------
 
-struct RowShared {
-    FusedShared staged;
-    int tile_hits[TILE_POINTS];               // pass 1: hits of the home points of the tile in the current batch
+/// Shared memory of the deciding pass. It writes no pairs, so it holds what the screen reads and
+/// little else; the few candidates that the screen can not decide are fetched again from the
+/// cell-sorted records. 1024 candidates at a time: the 600 or so of a unit of a dense crystal are
+/// one batch.
+struct RowCountShared {
+    static constexpr int BATCH = 1024;
+    static constexpr int WORDS = BATCH / 32;
+    SegmentTable table;
+    alignas(16) float near_x[BATCH]; // relative to the unit centre, read as 16-byte vectors
+    alignas(16) float near_y[BATCH];
+    alignas(16) float near_z[BATCH];
+    alignas(16) float near_n[BATCH];
+    int index[BATCH];                   // half lists: indices of the candidates
+    int4 home_sj[TILE_POINTS];          // x, y, z: wrap shift of the home point; w: its index
+    unsigned mask[WORDS * TILE_POINTS]; // [word][lane]
+    double centre[3];                   // centre of the unit: origin of the fp32 local frame
+    int tile_hits[TILE_POINTS];         // hits of the home points of the tile in the current batch
     unsigned long long mask_base;
 };
 
@@ -1939,64 +1940,14 @@ __device__ __forceinline__ int row_words_of_unit(
     return words;
 }
 
-/// Stage `batch_slots` candidates starting at slot `batch0` of the current
-/// segment group: original positions and (shift part, index) for the exact
-/// arithmetic, and fp32 coordinates relative to the unit centre for the screen.
-__device__ __forceinline__ void stage_row_batch(
-    FusedShared& sh, const GridPlan& plan, const SortedPoints& sorted, int n_stencil, int batch0, int batch_slots
-) {
-    for (int s = threadIdx.x; s < batch_slots; s += CTA_THREADS) {
-        const int slot = batch0 + s;
-        const int t = (n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
-        const size_t p = static_cast<size_t>(sh.table.start[t]) + (slot - sh.table.slot0[t]);
-        const LoadedRecord record = load_record(sorted, p);
-        int r0, r1, r2;
-        unpack_segment_image(sh.table.image[t], r0, r1, r2);
-        r0 -= record.s0;
-        r1 -= record.s1;
-        r2 -= record.s2;
-        sh.x[s] = record.x;
-        sh.y[s] = record.y;
-        sh.z[s] = record.z;
-        sh.sj[s] = make_int4(r0, r1, r2, record.index);
-        {
-            double ix = record.x;
-            double iy = record.y;
-            double iz = record.z;
-            if ((r0 | r1 | r2) != 0) {
-                ix += r0 * plan.H[0][0] + r1 * plan.H[1][0] + r2 * plan.H[2][0];
-                iy += r0 * plan.H[0][1] + r1 * plan.H[1][1] + r2 * plan.H[2][1];
-                iz += r0 * plan.H[0][2] + r1 * plan.H[1][2] + r2 * plan.H[2][2];
-            }
-            const float fx = static_cast<float>(ix - sh.centre[0]);
-            const float fy = static_cast<float>(iy - sh.centre[1]);
-            const float fz = static_cast<float>(iz - sh.centre[2]);
-            sh.near_x[s] = fx;
-            sh.near_y[s] = fy;
-            sh.near_z[s] = fz;
-            sh.near_n[s] = fx * fx + fy * fy + fz * fz;
-        }
-    }
-    {
-        const int batch_words = (batch_slots + 31) >> 5;
-        for (int s = batch_slots + threadIdx.x; s < batch_words * 32; s += CTA_THREADS) {
-            sh.near_x[s] = 0.0f;
-            sh.near_y[s] = 0.0f;
-            sh.near_z[s] = 0.0f;
-            sh.near_n[s] = __int_as_float(0x7f800000); // never a hit
-        }
-    }
-}
-
 template <bool FULL>
 __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, uint32_t* __restrict__ masks,
     unsigned long long mask_capacity, unsigned long long* __restrict__ unit_mask_base, uint32_t* __restrict__ unit_words,
     uint32_t* __restrict__ row_count, DeviceHeader* header
 ) {
-    extern __shared__ __align__(16) unsigned char row_smem[];
-    RowShared& rows = *reinterpret_cast<RowShared*>(row_smem);
-    FusedShared& sh = rows.staged;
+    __shared__ RowCountShared sh;
+    constexpr int BATCH = RowCountShared::BATCH;
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -2006,7 +1957,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
         return;
     }
     if (threadIdx.x < TILE_POINTS) {
-        rows.tile_hits[threadIdx.x] = 0;
+        sh.tile_hits[threadIdx.x] = 0;
     }
     unsigned most_candidates = 0; // of the units of this CTA
 
@@ -2037,10 +1988,10 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                 unit_mask_base[u] = base;
                 unit_words[u] = static_cast<uint32_t>(words);
             }
-            rows.mask_base = base;
+            sh.mask_base = base;
         }
         __syncthreads();
-        const unsigned long long base = rows.mask_base;
+        const unsigned long long base = sh.mask_base;
         if (base == ~0ull) {
             __syncthreads();
             continue; // the host grows the storage and runs the pass again
@@ -2057,10 +2008,46 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                 group_total = setup_segments(plan, cell_start, unit, g, sh.table);
             }
             const int own_slot0 = (g == own_group) ? sh.table.slot0[own_entry % SEG_MAX] : 0;
-            for (int batch0 = 0; batch0 < group_total; batch0 += FUSED_BATCH) {
-                const int batch_slots = min(FUSED_BATCH, group_total - batch0);
+            for (int batch0 = 0; batch0 < group_total; batch0 += BATCH) {
+                const int batch_slots = min(BATCH, group_total - batch0);
                 const int batch_words = (batch_slots + 31) >> 5;
-                stage_row_batch(sh, plan, sorted, unit.n_stencil, batch0, batch_slots);
+                // candidate in a slot of the batch, as it lies in the cell-sorted records: image
+                // minus wrap shift and index
+                const auto fetch = [&](int s, LoadedRecord& record) {
+                    const int slot = batch0 + s;
+                    const int t = (unit.n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
+                    record = load_record(sorted, static_cast<size_t>(sh.table.start[t]) + (slot - sh.table.slot0[t]));
+                    int r0, r1, r2;
+                    unpack_segment_image(sh.table.image[t], r0, r1, r2);
+                    return make_int4(r0 - record.s0, r1 - record.s1, r2 - record.s2, record.index);
+                };
+                for (int s = threadIdx.x; s < 32 * batch_words; s += CTA_THREADS) {
+                    float fx = 0.0f, fy = 0.0f, fz = 0.0f;
+                    float norm = __int_as_float(0x7f800000); // past the end: never a hit
+                    if (s < batch_slots) {
+                        LoadedRecord record;
+                        const int4 cand = fetch(s, record);
+                        double ix = record.x;
+                        double iy = record.y;
+                        double iz = record.z;
+                        if ((cand.x | cand.y | cand.z) != 0) {
+                            ix += cand.x * plan.H[0][0] + cand.y * plan.H[1][0] + cand.z * plan.H[2][0];
+                            iy += cand.x * plan.H[0][1] + cand.y * plan.H[1][1] + cand.z * plan.H[2][1];
+                            iz += cand.x * plan.H[0][2] + cand.y * plan.H[1][2] + cand.z * plan.H[2][2];
+                        }
+                        fx = static_cast<float>(ix - sh.centre[0]);
+                        fy = static_cast<float>(iy - sh.centre[1]);
+                        fz = static_cast<float>(iz - sh.centre[2]);
+                        norm = fx * fx + fy * fy + fz * fz;
+                        if (!FULL) {
+                            sh.index[s] = cand.w;
+                        }
+                    }
+                    sh.near_x[s] = fx;
+                    sh.near_y[s] = fy;
+                    sh.near_z[s] = fz;
+                    sh.near_n[s] = norm;
+                }
 
                 for (int tile = 0; tile < n_tiles; tile++) {
                     __syncthreads(); // staging done; previous tile done with the hit words and the home points
@@ -2090,20 +2077,27 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                     const unsigned long long ay2 = pack_f32x2(ay, ay);
                     const unsigned long long az2 = pack_f32x2(az, az);
                     const unsigned long long an2 = pack_f32x2(an, an);
+                    const auto exact = [&](int s) {
+                        LoadedRecord other;
+                        const int4 cand = fetch(s, other);
+                        double vx, vy, vz;
+                        return exact_pair(plan, rix, riy, riz, other.x, other.y, other.z, cand.x + si0, cand.y + si1, cand.z + si2, vx, vy, vz) <
+                               plan.cutoff2;
+                    };
                     // (no half shell here: home_row_slots = 0 keeps every candidate)
                     if (batch_words <= CTA_WARPS) {
                         if (warp < batch_words) {
                             sh.mask[warp * TILE_POINTS + lane] =
-                                decide_piece<32>(sh, plan, warp, 0, batch0, 0, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, rix, riy, riz, si0, si1, si2);
+                                decide_piece<32>(sh, warp, 0, batch0, 0, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, exact);
                         }
                     } else {
                         unsigned short* halves = reinterpret_cast<unsigned short*>(sh.mask);
                         for (int piece = warp; piece < 2 * batch_words; piece += CTA_WARPS) {
                             const int half = (piece >= batch_words) ? 1 : 0;
                             const int w = piece - half * batch_words;
-                            halves[2 * (w * TILE_POINTS + lane) + half] = static_cast<unsigned short>(decide_piece<16>(
-                                sh, plan, w, 16 * half, batch0, 0, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, rix, riy, riz, si0, si1, si2
-                            ));
+                            halves[2 * (w * TILE_POINTS + lane) + half] = static_cast<unsigned short>(
+                                decide_piece<16>(sh, w, 16 * half, batch0, 0, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, exact)
+                            );
                         }
                     }
                     __syncthreads();
@@ -2128,7 +2122,14 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                             while (word != 0) {
                                 const int b = __ffs(word) - 1;
                                 word &= word - 1;
-                                if (row_keeps<FULL>(home, sh.sj[slot0 + b])) {
+                                bool keeps;
+                                if (!FULL && sh.index[slot0 + b] != home.w) {
+                                    keeps = sh.index[slot0 + b] > home.w;
+                                } else {
+                                    LoadedRecord other;
+                                    keeps = row_keeps<FULL>(home, fetch(slot0 + b, other));
+                                }
+                                if (keeps) {
                                     kept |= 1u << b;
                                 }
                             }
@@ -2137,14 +2138,14 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                         my_hits += __popc(kept);
                     }
                     if (my_hits != 0) {
-                        atomicAdd(&rows.tile_hits[lane], my_hits);
+                        atomicAdd(&sh.tile_hits[lane], my_hits);
                     }
                     __syncthreads();
                     if (threadIdx.x < TILE_POINTS) {
-                        const int hits = rows.tile_hits[threadIdx.x];
+                        const int hits = sh.tile_hits[threadIdx.x];
                         if (hits != 0) {
                             atomicAdd(&row_count[sh.home_sj[threadIdx.x].w], static_cast<uint32_t>(hits));
-                            rows.tile_hits[threadIdx.x] = 0;
+                            sh.tile_hits[threadIdx.x] = 0;
                         }
                     }
                 }
@@ -2788,8 +2789,6 @@ int pair_grid(int n_units, int per_sm) {
 // ---------------------------------------------------------------------------
 
 void configure_kernels() {
-    cudaFuncSetAttribute(row_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(RowShared)));
-    cudaFuncSetAttribute(row_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(RowShared)));
     cudaFuncSetAttribute(row_emit_kernel<SortedRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SortedRows::Shared)));
     cudaFuncSetAttribute(row_emit_kernel<CanonicalRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(CanonicalRows::Shared)));
     cudaFuncSetAttribute(row_emit_kernel<CanonicalRowsWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(CanonicalRowsWide::Shared)));
@@ -2923,11 +2922,11 @@ void launch_count(
 ) {
     const int grid = pair_grid(plan.n_units, 4);
     if (plan.full) {
-        row_count_kernel<true><<<grid, CTA_THREADS, sizeof(RowShared), stream>>>(
+        row_count_kernel<true><<<grid, CTA_THREADS, 0, stream>>>(
             plan, cell_start, sorted, masks, mask_capacity, unit_mask_base, unit_words, row_count, header
         );
     } else {
-        row_count_kernel<false><<<grid, CTA_THREADS, sizeof(RowShared), stream>>>(
+        row_count_kernel<false><<<grid, CTA_THREADS, 0, stream>>>(
             plan, cell_start, sorted, masks, mask_capacity, unit_mask_base, unit_words, row_count, header
         );
     }
