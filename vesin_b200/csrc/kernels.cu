@@ -1084,7 +1084,7 @@ __device__ unsigned long long g_phase_clocks[16];
 
 constexpr int FUSED_BATCH = 512;
 constexpr int DEFAULT_UNIT_RUN = 2; // neighbouring units handled back to back by one CTA (measured: 2 beats 1, 3, 4 and 8)
-constexpr int MAX_UNIT_SPLITS = 32; // CTAs that share the candidate batches of one unit (launches of few units)
+constexpr int MAX_UNIT_SPLITS = 64; // CTAs that share the candidate batches of one unit (launches of few units)
 constexpr int FUSED_LIST = 2048;
 
 /// Shared memory of a CTA of THREADS_ threads that stages BATCH_ candidates at a time and
@@ -1153,6 +1153,10 @@ struct PairShape {
 /// holds up 4 warps instead of 8 and twice as many CTAs are there to issue meanwhile: sparse
 /// systems (a unit of 30 points with 400 hits) gain 17 %, dense ones 4 %.
 using SmallCta = PairShape<128, 256, 1024, 8>;
+/// Launches that do not fill the GPU (one small system): 64 candidates per batch, so that the
+/// batches of a unit go to four times as many CTAs (see launch_pairs). What bounds such a launch
+/// is the chain of one CTA, and most of that is writing its hits.
+using TinyCta = PairShape<128, 64, 1024, 8>;
 /// Units next to the halo of a slab (they sort their hits into owned and halo candidates and go
 /// over every batch twice): CTAs of 8 warps with 512 candidates per batch, 4 per SM.
 using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4>;
@@ -1612,14 +1616,15 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                             const unsigned of_home = __shfl_sync(FULL_MASK, word, (lane & 7) * 4);
                             sh.mask[w * TILE_POINTS + lane] = (lane < TILE_POINTS / 4) ? of_home : 0u;
                         }
-                    } else if (batch_words <= Shape::WARPS) {
+                    } else if (batch_words <= Shape::WARPS && 2 * batch_words > Shape::WARPS) {
                         // a word of 32 candidates per warp
                         if (warp < batch_words) {
                             sh.mask[warp * TILE_POINTS + lane] =
                                 decide_piece<32>(sh, warp, 0, batch0, home_row_slots, il, ax2, ay2, az2, an2, cutoff2_lo, cutoff2_hi, exact);
                         }
                     } else {
-                        // more words than warps: halves of words, so that no warp does two words while others do one
+                        // more words than warps: halves of words, so that no warp does two words while others
+                        // do one; or so few that every warp gets half a word
                         unsigned short* halves = reinterpret_cast<unsigned short*>(sh.mask);
                         for (int piece = warp; piece < 2 * batch_words; piece += Shape::WARPS) {
                             const int half = (piece >= batch_words) ? 1 : 0;
@@ -2794,6 +2799,8 @@ void configure_kernels() {
     cudaFuncSetAttribute(row_emit_kernel<CanonicalRowsWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(CanonicalRowsWide::Shared)));
     cudaFuncSetAttribute(pairs_kernel<false, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<true, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
+    cudaFuncSetAttribute(pairs_kernel<false, false, TinyCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(TinyCta::Shared)));
+    cudaFuncSetAttribute(pairs_kernel<true, false, TinyCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(TinyCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<false, true, LargeCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(LargeCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<true, true, LargeCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(LargeCta::Shared)));
 }
@@ -2992,6 +2999,14 @@ void launch_pairs(
         }
     }
     out.interleave_ok = paired_stores_fit(out);
+    // candidates of a unit, about (0: the caller does not know how many points there are)
+    double unit_candidates = 0.0;
+    if (plan.n_cells_total > 0 && n_records > 0) {
+        const int row_width = plan.pencil + 2 * plan.n_search[0];
+        const int rows_above = plan.n_search[1] + plan.n_search[2] * (2 * plan.n_search[1] + 1);
+        const double stencil_cells = static_cast<double>(plan.pencil + plan.n_search[0]) + static_cast<double>(row_width) * rows_above;
+        unit_candidates = stencil_cells * static_cast<double>(n_records) / static_cast<double>(plan.n_cells_total);
+    }
 
     const auto launch = [&](auto shape, auto kernel, UnitRanges ranges, unsigned long long* run_cursor, bool follows = false) {
         using Shape = decltype(shape);
@@ -3006,14 +3021,9 @@ void launch_pairs(
         int runs = (ranges.end0 - ranges.begin0 + unit_run - 1) / unit_run + (ranges.end1 - ranges.begin1 + unit_run - 1) / unit_run;
         // A handful of units whose stencils hold many batches of candidates (a small box with
         // many images): several CTAs share the batches of a unit.
-        if (unit_run == 1 && runs * 2 <= sms * per_sm && plan.n_cells_total > 0 && n_records > 0) {
-            const int row_width = plan.pencil + 2 * plan.n_search[0];
-            const int rows_above = plan.n_search[1] + plan.n_search[2] * (2 * plan.n_search[1] + 1);
-            const double stencil_cells = static_cast<double>(plan.pencil + plan.n_search[0]) + static_cast<double>(row_width) * rows_above;
-            const double per_cell = static_cast<double>(n_records) / static_cast<double>(plan.n_cells_total);
-            const double batches = std::ceil(stencil_cells * per_cell / Shape::BATCH);
+        if (unit_run == 1 && runs * 2 <= sms * per_sm) {
             const int wanted = std::min(MAX_UNIT_SPLITS, (sms * per_sm) / runs);
-            ranges.splits = std::max(1, static_cast<int>(std::min<double>(wanted, batches)));
+            ranges.splits = std::max(1, static_cast<int>(std::min<double>(wanted, std::ceil(unit_candidates / Shape::BATCH))));
             runs *= ranges.splits;
         }
         const int grid = pair_grid(runs, per_sm);
@@ -3022,7 +3032,16 @@ void launch_pairs(
         );
     };
     const UnitRanges all{0, plan.n_units, 0, 0};
-    if (plan.window_axis < 0) {
+    if (plan.window_axis < 0 && unit_candidates > 0.0 && plan.n_units * std::ceil(unit_candidates / SmallCta::BATCH) <= sms) {
+        // Less than a CTA per SM even when every batch of 256 candidates gets its own: batches of
+        // 64 (1000 atoms: 20.6 -> 13.7 us, 64 atoms with 4000 images: 29.5 -> 25.7 us; from two CTAs per
+        // SM on the smaller batches cost more than they spread).
+        if (plan.full) {
+            launch(TinyCta{}, pairs_kernel<true, false, TinyCta>, all, &header->run_cursor);
+        } else {
+            launch(TinyCta{}, pairs_kernel<false, false, TinyCta>, all, &header->run_cursor);
+        }
+    } else if (plan.window_axis < 0) {
         if (plan.full) {
             launch(SmallCta{}, pairs_kernel<true, false, SmallCta>, all, &header->run_cursor);
         } else {
