@@ -5,6 +5,7 @@
 #include <atomic>
 #include <chrono>
 #include <cerrno>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -158,6 +159,7 @@ struct Workspace {
         bool float_io = false;
         size_t n_points = 0;
         size_t n_records = 0;
+        int call = 0; // number of the call, 1 ... INT_MAX: what its check writes into the state when it refuses
         VesinNeighborList candidates{};
         DeviceBuffer records, reference_points, reference_box, state, rank_of, positions;
         VerletState* h_state = nullptr; // pinned
@@ -537,6 +539,7 @@ void neighbors_with_skin(
     }
     std::chrono::steady_clock::time_point filter_started{};
     for (int round = 0;; round++) {
+        cache.call = (cache.call == INT_MAX) ? 1 : cache.call + 1;
         if (!usable) {
             // ---- candidates: the half list at cutoff + skin, built like any list ----
             cache.valid = false;
@@ -593,13 +596,6 @@ void neighbors_with_skin(
             cache.valid = true;
         } else {
             filter_started = std::chrono::steady_clock::now();
-            timer.begin(VesinB200StageBounds);
-            VB200_CUDA(cudaMemsetAsync(d_state, 0, sizeof(VerletState), stream));
-            launch_verlet_check(
-                flat_points, RealView{cache.reference_points.ptr, float_io ? 1 : 0}, n_points, flat_box, periodic, cache.reference_box.as<double>(),
-                reinterpret_cast<const unsigned char*>(cache.reference_box.as<double>() + 9), options.skin, d_state, stream
-            );
-            timer.end(VesinB200StageBounds);
         }
 
         // ---- filter: into the arrays of the previous call first; when the pairs do not fit they
@@ -607,20 +603,24 @@ void neighbors_with_skin(
         Target target(list, ws, options, float_io, caller);
         size_t capacity = target.capacity();
         bool stale = false;
+        timer.begin(VesinB200StageBounds);
+        launch_verlet_front(
+            flat_points, RealView{cache.reference_points.ptr, float_io ? 1 : 0},
+            static_cast<const Workspace*>(cache.candidates.opaque)->sorted_records.as<PointRecord>(), n_points, flat_box, periodic,
+            cache.reference_box.as<double>(), reinterpret_cast<const unsigned char*>(cache.reference_box.as<double>() + 9), options.skin,
+            cache.positions.as<double>(), d_state, cache.call, stream
+        );
+        timer.end(VesinB200StageBounds);
         for (int attempt = 0;; attempt++) {
-            const auto* built = static_cast<const Workspace*>(cache.candidates.opaque);
             timer.begin(VesinB200StageEmit);
-            if (attempt == 0) {
-                launch_verlet_positions(flat_points, built->sorted_records.as<PointRecord>(), n_points, cache.positions.as<double>(), d_state, stream);
-            }
             launch_verlet_filter(
                 cache.records.as<uint32_t>(), cache.n_records, cache.positions.as<double>(), flat_box,
-                options.cutoff * options.cutoff, options.full, target.view(), capacity, d_state, stream
+                options.cutoff * options.cutoff, options.full, target.view(), capacity, d_state, cache.call, stream
             );
             timer.end(VesinB200StageEmit);
             VB200_CUDA(cudaGetLastError());
             read_state();
-            if (attempt == 0 && usable) {
+            if (attempt == 0) {
                 timer.collect(VesinB200StageBounds);
             }
             timer.collect(VesinB200StageEmit);
@@ -632,7 +632,7 @@ void neighbors_with_skin(
                 neighbors(points, n_points, box, periodic, options, list, float_io, false, caller);
                 return;
             }
-            if (cache.h_state->stale) {
+            if (cache.h_state->stale == cache.call) {
                 stale = true;
                 break;
             }

@@ -286,7 +286,7 @@ void launch_checksum(
 /// Device words of the cache of one list: what the check and the filter report.
 struct VerletState {
     unsigned long long pair_cursor; // output elements claimed by the filter (= its pair total)
-    int stale;                      // the candidates do not fit the inputs of this call
+    int stale;                      // number of the last call whose inputs the candidates did not fit
     int unpackable;                 // a candidate's shift does not fit its 10 bits
 };
 
@@ -299,28 +299,25 @@ void launch_verlet_pack(
     uint32_t* records, VerletState* state, cudaStream_t stream
 );
 
-/// Row p of `positions` (4 doubles, 32 bytes) = x, y, z of the point of record p as
-/// it is now, and its index as raw bits (nothing when state->stale is set).
-void launch_verlet_positions(
-    RealView points, const PointRecord* sorted, size_t n_points, double* positions, const VerletState* state, cudaStream_t stream
-);
-
-/// Sets state->stale when some point moved further than (skin - corner
-/// displacement of the box) / 2 from `reference_points`, when the box corners
-/// moved by `skin` or more, or when the periodicity changed. `reference_box`
-/// (9 doubles) and `reference_periodic` (3 bytes) live in device memory.
-void launch_verlet_check(
-    RealView points, RealView reference_points, size_t n, RealView box, const bool* periodic, const double* reference_box,
-    const unsigned char* reference_periodic, double skin, VerletState* state, cudaStream_t stream
+/// One pass over the points. Row p of `positions` (4 doubles, 32 bytes) = x, y, z of the point of
+/// record p as it is now, and its index as raw bits. Sets state->stale to `call` (a number other
+/// than those of earlier calls) when some point moved further than (skin - corner displacement of
+/// the box) / 2 from `reference_points`, when the box corners moved by `skin` or more, or when the
+/// periodicity changed; clears state->pair_cursor. `reference_box` (9 doubles) and
+/// `reference_periodic` (3 bytes) live in device memory.
+void launch_verlet_front(
+    RealView points, RealView reference_points, const PointRecord* sorted, size_t n, RealView box, const bool* periodic,
+    const double* reference_box, const unsigned char* reference_periodic, double skin, double* positions, VerletState* state, int call,
+    cudaStream_t stream
 );
 
 /// Writes the records within the cutoff (exact fp64 predicate on `positions`,
 /// the current points in cell-sorted order, and the box) into ranges claimed from state->pair_cursor; a full list
 /// gets both orientations of every kept record. Does nothing when
-/// state->stale is set. Ranges past `capacity` are counted, not written.
+/// state->stale is `call`. Ranges past `capacity` are counted, not written.
 void launch_verlet_filter(
     const uint32_t* records, size_t n, const double* positions, RealView box, double cutoff2, bool full,
-    PairOutput out, unsigned long long capacity, VerletState* state, cudaStream_t stream
+    PairOutput out, unsigned long long capacity, VerletState* state, int call, cudaStream_t stream
 );
 
 /// One-time per-device kernel attribute setup (shared-memory opt-in).
