@@ -505,24 +505,32 @@ __global__ void __launch_bounds__(CTA_THREADS) bin_kernel(
             atomicOr(&header->status, STATUS_HALO_OVERFLOW);
         }
     }
-    unsigned active_mask = __ballot_sync(FULL_MASK, active);
-    if (!active) {
+    int wrap[3];
+    const int linear = active ? locate_point(rx, ry, rz, i, plan, header, check, wrap) : -1;
+
+    // warp-aggregated histogram: one atomic per distinct cell in the warp. Finding the lanes of a
+    // cell costs a step per distinct cell, which points in random order (no two neighbours in the
+    // same cell) do not gain anything by: they take an atomic each. 2.1 M points of a liquid in
+    // random order: 53 -> 28 us; 512k atoms in lattice order pay for the look at their neighbours, 8.7 -> 9.7.
+    const int lane = threadIdx.x & 31;
+    const int before = __shfl_up_sync(FULL_MASK, linear, 1);
+    const bool scattered = __all_sync(FULL_MASK, lane == 0 || before != linear) != 0;
+    if (scattered) {
+        if (active) {
+            rank[i] = atomicAdd(&cell_count[linear], 1);
+        }
         return;
     }
-    int wrap[3];
-    const int linear = locate_point(rx, ry, rz, i, plan, header, check, wrap);
-
-    // warp-aggregated histogram: one atomic per distinct cell in the warp
-    unsigned peers = __match_any_sync(active_mask, linear);
-    int leader = __ffs(peers) - 1;
-    int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(FULL_MASK, linear);
+    const int leader = __ffs(peers) - 1;
     int base = 0;
-    if (lane == leader) {
+    if (lane == leader && active) {
         base = atomicAdd(&cell_count[linear], __popc(peers));
     }
-    base = __shfl_sync(peers, base, leader);
-
-    rank[i] = base + __popc(peers & lanemask_lt());
+    base = __shfl_sync(FULL_MASK, base, leader);
+    if (active) {
+        rank[i] = base + __popc(peers & lanemask_lt());
+    }
 }
 
 // ---------------------------------------------------------------------------
