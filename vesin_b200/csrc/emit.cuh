@@ -32,9 +32,11 @@ __device__ __forceinline__ void store_indices(const PairOutput& out, unsigned lo
 /// Write `n_valid` consecutive pairs starting at output element `first`:
 /// lane l holds pair l. 12- and 24-byte elements are transposed through
 /// shared memory so that every store instruction covers one contiguous span.
+/// `shifted` (the same in every lane): does any of the pairs have a shift? Most
+/// groups of 32 pairs of a large box have none, and zeros need no transposing.
 __device__ __forceinline__ void store_pairs(
     double* transpose, const PairOutput& out, int lane, unsigned long long first, int n_valid, unsigned long long a,
-    unsigned long long b, int s0, int s1, int s2, double d, double vx, double vy, double vz
+    unsigned long long b, int s0, int s1, int s2, double d, double vx, double vy, double vz, bool shifted
 ) {
     if (lane < n_valid) {
         store_indices(out, first + lane, a, b);
@@ -46,7 +48,16 @@ __device__ __forceinline__ void store_pairs(
             }
         }
     }
-    if (out.shifts != nullptr) {
+    if (out.shifts != nullptr && !shifted) {
+        int32_t* dst = out.shifts + 3 * first;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const int w = k * 32 + lane;
+            if (w < 3 * n_valid) {
+                __stcs(&dst[w], 0);
+            }
+        }
+    } else if (out.shifts != nullptr) {
         int* buffer = reinterpret_cast<int*>(transpose);
         buffer[3 * lane + 0] = s0;
         buffer[3 * lane + 1] = s1;
@@ -110,7 +121,7 @@ __device__ __forceinline__ void store_pairs(
 /// lane that holds that hit in this chunk (-1: none), `tail_to` the element.
 __device__ __forceinline__ void store_both(
     double* transpose, const PairOutput& out, int lane, unsigned long long first, int n_valid, unsigned long long a,
-    unsigned long long b, int s0, int s1, int s2, double d, double vx, double vy, double vz, int tail_lane = -1,
+    unsigned long long b, int s0, int s1, int s2, double d, double vx, double vy, double vz, bool shifted, int tail_lane = -1,
     unsigned long long tail_to = 0
 ) {
     const unsigned long long mine = first + 2 * lane;
@@ -171,7 +182,13 @@ __device__ __forceinline__ void store_both(
     // pieces of the transposed buffers: 3 per lane; of the tail lane's, the second is half
     // forward pair (its first word is written alone) and the third is not written at all
     const int tail_half = (tail_lane >= 0) ? 3 * tail_lane + 1 : -1;
-    if (out.shifts != nullptr) {
+    if (out.shifts != nullptr && !shifted && whole) {
+        // nothing to transpose: 12 of the 90 or so shared and global wavefronts of a group less
+        int2* dst = reinterpret_cast<int2*>(out.shifts + 3 * first) + lane;
+        __stcs(&dst[0], make_int2(0, 0));
+        __stcs(&dst[32], make_int2(0, 0));
+        __stcs(&dst[64], make_int2(0, 0));
+    } else if (out.shifts != nullptr) {
         int2* buffer = reinterpret_cast<int2*>(transpose);
         buffer[3 * lane + 0] = make_int2(s0, s1);
         buffer[3 * lane + 1] = make_int2(s2, -s0);

@@ -1817,7 +1817,8 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                                 int s1 = cand.y + home.y;
                                 int s2 = cand.z + home.z;
                                 double d2;
-                                if (__any_sync(0xffffffffu, (s0 | s1 | s2) != 0)) {
+                                const bool shifted = __any_sync(0xffffffffu, (s0 | s1 | s2) != 0) != 0;
+                                if (shifted) {
                                     d2 = exact_pair(
                                         plan, sh.home_pos[0][h], sh.home_pos[1][h], sh.home_pos[2][h], sh.x[s], sh.y[s], sh.z[s], s0, s1, s2,
                                         vx, vy, vz
@@ -1840,19 +1841,19 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                                     }
                                     store_both(
                                         sh.transpose[warp], out, lane, claim + moved_on + 2ull * (round0 + chunk0), n_valid, index_i, index_j, s0, s1, s2, d,
-                                        vx, vy, vz, tail_lane, claim
+                                        vx, vy, vz, shifted, tail_lane, claim
                                     );
                                     continue;
                                 }
                                 const unsigned long long first = claim + round0 + chunk0;
                                 if (FULL) {
                                     if (write_forward) {
-                                        store_pairs(sh.transpose[warp], out, lane, first, n_valid, index_i, index_j, s0, s1, s2, d, vx, vy, vz);
+                                        store_pairs(sh.transpose[warp], out, lane, first, n_valid, index_i, index_j, s0, s1, s2, d, vx, vy, vz, shifted);
                                     }
                                     if (write_reverse) {
                                         store_pairs(
                                             sh.transpose[warp], out, lane, first + (write_forward ? total_hits : 0), n_valid, index_j, index_i, -s0, -s1, -s2,
-                                            d, -vx, -vy, -vz
+                                            d, -vx, -vy, -vz, shifted
                                         );
                                     }
                                 } else {
@@ -1869,7 +1870,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                                         vy = -vy;
                                         vz = -vz;
                                     }
-                                    store_pairs(sh.transpose[warp], out, lane, first, n_valid, index_i, index_j, s0, s1, s2, d, vx, vy, vz);
+                                    store_pairs(sh.transpose[warp], out, lane, first, n_valid, index_i, index_j, s0, s1, s2, d, vx, vy, vz, shifted);
                                 }
                             }
                             PHASE_MARK(8); // emission
@@ -2520,7 +2521,8 @@ __global__ void __launch_bounds__(CTA_THREADS, Shape::CTAS_PER_SM) row_emit_kern
                                 const int s1 = cand.y + home.y;
                                 const int s2 = cand.z + home.z;
                                 double vx, vy, vz, d2;
-                                if (__any_sync(FULL_MASK, (s0 | s1 | s2) != 0)) {
+                                const bool shifted = __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0;
+                                if (shifted) {
                                     d2 = exact_pair(plan, hx, hy, hz, sh.staged.x[s], sh.staged.y[s], sh.staged.z[s], s0, s1, s2, vx, vy, vz);
                                 } else {
                                     // (the signed zeros that the products with S = 0 give)
@@ -2532,7 +2534,7 @@ __global__ void __launch_bounds__(CTA_THREADS, Shape::CTAS_PER_SM) row_emit_kern
                                 store_pairs(
                                     sh.transpose[warp], out, lane, row + static_cast<unsigned long long>(window + c0), n_valid,
                                     static_cast<unsigned long long>(home.w), static_cast<unsigned long long>(cand.w), s0, s1, s2, __dsqrt_rn(d2), vx, vy,
-                                    vz
+                                    vz, shifted
                                 );
                             }
                         }

@@ -347,16 +347,16 @@ __device__ __forceinline__ double molecule_pair(const MoleculeShared& sh, int wa
 /// side by side for full lists.
 __device__ __forceinline__ void write_hits(
     double* transpose, const BatchInput& in, const PairOutput& out, int lane, unsigned long long first, int n_valid, unsigned long long gi,
-    unsigned long long gj, int s0, int s1, int s2, double d, double vx, double vy, double vz
+    unsigned long long gj, int s0, int s1, int s2, double d, double vx, double vy, double vz, bool shifted
 ) {
     if (!in.full) {
         // half lists keep i <= j: the forward pair
-        store_pairs(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz);
+        store_pairs(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
     } else if (out.interleave_ok) {
-        store_both(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz);
+        store_both(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
     } else {
-        store_pairs(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz);
-        store_pairs(transpose, out, lane, first + n_valid, n_valid, gj, gi, -s0, -s1, -s2, d, -vx, -vy, -vz);
+        store_pairs(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
+        store_pairs(transpose, out, lane, first + n_valid, n_valid, gj, gi, -s0, -s1, -s2, d, -vx, -vy, -vz, shifted);
     }
 }
 
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
                 }
                 double vx, vy, vz;
                 const double d = __dsqrt_rn(molecule_pair(sh, warp, i, j, vx, vy, vz));
-                write_hits(sh.transpose[warp], in, out, lane, next, n_valid, index_offset + i, index_offset + j, 0, 0, 0, d, vx, vy, vz);
+                write_hits(sh.transpose[warp], in, out, lane, next, n_valid, index_offset + i, index_offset + j, 0, 0, 0, d, vx, vy, vz, false);
                 next += static_cast<unsigned long long>(n_valid) * per_hit;
             }
         };
@@ -823,7 +823,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 5) small_systems_kernel(
                             ));
                             write_hits(
                                 sh.transpose[warp], in, out, lane, first + static_cast<unsigned long long>(c0) * per_hit, n_valid, index_offset + i0 + h,
-                                index_offset + chunk0 + image.w, s0, s1, s2, d, vx, vy, vz
+                                index_offset + chunk0 + image.w, s0, s1, s2, d, vx, vy, vz,
+                                __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0
                             );
                         }
                     };

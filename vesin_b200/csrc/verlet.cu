@@ -236,15 +236,16 @@ __device__ __forceinline__ void write_kept(
             j = static_cast<uint32_t>(index_j);
         }
         const unsigned long long first = claim + 32ull * warp * per_hit;
+        const bool shifted = __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0;
         if (FULL) {
             if (out.interleave_ok) {
-                store_both(sh.transpose[warp], out, lane, first, n_valid, i, j, s0, s1, s2, d, vx, vy, vz);
+                store_both(sh.transpose[warp], out, lane, first, n_valid, i, j, s0, s1, s2, d, vx, vy, vz, shifted);
             } else {
-                store_pairs(sh.transpose[warp], out, lane, first, n_valid, i, j, s0, s1, s2, d, vx, vy, vz);
-                store_pairs(sh.transpose[warp], out, lane, first + n_valid, n_valid, j, i, -s0, -s1, -s2, d, -vx, -vy, -vz);
+                store_pairs(sh.transpose[warp], out, lane, first, n_valid, i, j, s0, s1, s2, d, vx, vy, vz, shifted);
+                store_pairs(sh.transpose[warp], out, lane, first + n_valid, n_valid, j, i, -s0, -s1, -s2, d, -vx, -vy, -vz, shifted);
             }
         } else {
-            store_pairs(sh.transpose[warp], out, lane, first, n_valid, i, j, s0, s1, s2, d, vx, vy, vz);
+            store_pairs(sh.transpose[warp], out, lane, first, n_valid, i, j, s0, s1, s2, d, vx, vy, vz, shifted);
         }
     }
     __syncthreads();
