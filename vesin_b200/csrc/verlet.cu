@@ -271,6 +271,7 @@ __global__ void __launch_bounds__(VERLET_THREADS) verlet_filter_kernel(
 
     // a CTA takes 256 consecutive records per round; the kept ones gather in a list of the CTA
     const size_t n_rounds = (n + VERLET_THREADS - 1) / VERLET_THREADS;
+    int n_kept = 0; // records in the list, the same in every thread
     for (size_t round = blockIdx.x; round < n_rounds; round += gridDim.x) {
         const size_t r = round * VERLET_THREADS + threadIdx.x;
         bool hit = false;
@@ -300,8 +301,8 @@ __global__ void __launch_bounds__(VERLET_THREADS) verlet_filter_kernel(
                 sh.kept[slot][2] = packed;
             }
         }
-        __syncthreads();
-        const int n_kept = sh.n_kept; // fewer than 2 * FILTER_CHUNK: below FILTER_CHUNK before this round
+        // (counted by the barrier: a warp that is ahead already adds to sh.n_kept while others are here)
+        n_kept += __syncthreads_count(hit ? 1 : 0); // fewer than 2 * FILTER_CHUNK: below FILTER_CHUNK before this round
         if (n_kept >= FILTER_CHUNK) {
             write_kept<FULL>(sh, positions, out, capacity, state, FILTER_CHUNK);
             // what is left moves to the front of the list
@@ -321,10 +322,10 @@ __global__ void __launch_bounds__(VERLET_THREADS) verlet_filter_kernel(
             if (threadIdx.x == 0) {
                 sh.n_kept = left;
             }
+            n_kept = left;
             __syncthreads();
         }
     }
-    const int n_kept = sh.n_kept;
     if (n_kept > 0) {
         write_kept<FULL>(sh, positions, out, capacity, state, n_kept);
     }
