@@ -345,6 +345,15 @@ void read_header(Workspace& ws) {
     VB200_CUDA(cudaStreamSynchronize(ws.stream));
 }
 
+/// The same behind a kernel that writes the header into the pinned mirror itself (`exported` was
+/// cleared before its launch): nothing to copy unless it did not.
+void read_exported_header(Workspace& ws) {
+    VB200_CUDA(cudaStreamSynchronize(ws.stream));
+    if (*static_cast<volatile unsigned int*>(&ws.h_header->exported) == 0) {
+        read_header(ws);
+    }
+}
+
 /// Where the pairs of a build go: the arrays of the list itself (grow-only, as in the reference's
 /// C API), or arrays the caller brings and grows on demand. Which arrays are written follows from
 /// the options in the first case, from the caller's non-null pointers in the second.
@@ -902,10 +911,13 @@ void neighbors(
             for (int attempt = 0;; attempt++) {
                 const size_t pass_capacity = count_only ? 0 : capacity;
                 timer.begin(VesinB200StageEmit);
-                launch_pairs(plan, ws.cell_start.as<int32_t>(), sorted, target.view(), pass_capacity, ws.d_header, stream, n_points);
+                ws.h_header->exported = 0;
+                launch_pairs(
+                    plan, ws.cell_start.as<int32_t>(), sorted, target.view(), pass_capacity, ws.d_header, stream, n_points, PAIR_PART_ALL, ws.h_header
+                );
                 timer.end(VesinB200StageEmit);
                 VB200_CUDA(cudaGetLastError());
-                read_header(ws);
+                read_exported_header(ws);
                 if (attempt == 0) {
                     collect_front_stages();
                     if (plan_was_refused()) {
@@ -966,13 +978,13 @@ void neighbors(
             );
             timer.end(VesinB200StageCount);
             timer.begin(VesinB200StageScanRows);
+            ws.h_header->exported = 0;
             launch_scan_rows(
-                ws.row_count.as<uint32_t>(), ws.row_start.as<unsigned long long>(), n_points, ws.scan_tmp.ptr,
-                &ws.d_header->total_pairs, stream
+                ws.row_count.as<uint32_t>(), ws.row_start.as<unsigned long long>(), n_points, ws.scan_tmp.ptr, ws.d_header, stream, ws.h_header
             );
             timer.end(VesinB200StageScanRows);
             VB200_CUDA(cudaGetLastError());
-            read_header(ws);
+            read_exported_header(ws);
             if (attempt == 0) {
                 collect_front_stages();
                 if (plan_was_refused()) {

@@ -304,6 +304,8 @@ __device__ __forceinline__ void reset_header(DeviceHeader* header, const RealVie
         header->run_cursor = 0;
         header->status = 0;
         header->max_candidates = 0;
+        header->finished = 0;
+        header->exported = 0;
     }
 }
 
@@ -627,7 +629,7 @@ __global__ void __launch_bounds__(CTA_THREADS) scan_spine_kernel(unsigned long l
 template <typename TIn, typename TOut, bool SPINE>
 __global__ void __launch_bounds__(CTA_THREADS) scan_apply_kernel(
     const TIn* __restrict__ in, TOut* __restrict__ out, size_t n, const unsigned long long* __restrict__ tile_offsets,
-    unsigned long long* __restrict__ total_out, const TOut* __restrict__ first_value
+    unsigned long long* __restrict__ total_out, const TOut* __restrict__ first_value, DeviceHeader* header, DeviceHeader* mirror
 ) {
     let_next_kernel_start();
     wait_for_previous_kernel();
@@ -699,6 +701,14 @@ __global__ void __launch_bounds__(CTA_THREADS) scan_apply_kernel(
             if (SPINE && total_out != nullptr) {
                 *total_out = prefix;
             }
+        }
+    }
+    if (SPINE && mirror != nullptr && blockIdx.x == gridDim.x - 1) {
+        // this block has written the total; everything else in the header is older than the kernel
+        __threadfence();
+        __syncthreads();
+        if (warp == 0) {
+            export_header(header, mirror, lane);
         }
     }
 }
@@ -1347,7 +1357,8 @@ struct UnitRanges {
 template <bool FULL, bool SLAB, class Shape>
 __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, PairOutput out, unsigned long long capacity,
-    DeviceHeader* header, const int UNIT_RUN, const UnitRanges ranges, unsigned long long* run_cursor, const int follows_pair_kernel
+    DeviceHeader* header, const int UNIT_RUN, const UnitRanges ranges, unsigned long long* run_cursor, const int follows_pair_kernel,
+    DeviceHeader* mirror
 ) {
     extern __shared__ __align__(16) unsigned char fused_smem[];
     using Shared = typename Shape::Shared;
@@ -1368,7 +1379,11 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
         let_next_kernel_start();
     }
     if (header->status & STATUS_ABORT_MASK) {
-        return; // the plan was refused: the host will redo the build
+        // the plan was refused: the host will redo the build
+        if (mirror != nullptr && blockIdx.x == 0 && warp == 0) {
+            export_header(header, mirror, lane);
+        }
+        return;
     }
     PHASE_CLOCK_START();
     if (threadIdx.x == 0) {
@@ -1885,6 +1900,23 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
     __syncthreads(); // next_run is visible; nobody reads the other slot any more
     claimed = sh.next_run[run_parity];
     run_parity ^= 1;
+    }
+    if (mirror != nullptr && warp == 0) {
+        // The last CTA reports. The claims of a CTA are atomics of its thread 0 whose results it has
+        // used, so they have taken place; only a counting pass does not look at them.
+        int last = 0;
+        if (lane == 0) {
+            if (capacity == 0) {
+                __threadfence();
+            }
+            last = atomicAdd(&header->finished, 1u) == gridDim.x - 1;
+            if (last) {
+                header->finished = 0;
+            }
+        }
+        if (__shfl_sync(FULL_MASK, last, 0)) {
+            export_header(header, mirror, lane);
+        }
     }
 }
 
@@ -2892,7 +2924,8 @@ size_t scan_tmp_bytes(size_t n) {
 
 template <typename TIn, typename TOut>
 static void launch_scan(
-    const TIn* counts, TOut* starts, size_t n, void* tmp, unsigned long long* total, cudaStream_t stream, const TOut* first_value = nullptr
+    const TIn* counts, TOut* starts, size_t n, void* tmp, unsigned long long* total, cudaStream_t stream, const TOut* first_value = nullptr,
+    DeviceHeader* header = nullptr, DeviceHeader* mirror = nullptr
 ) {
     auto* tile_sums = static_cast<unsigned long long*>(tmp);
     size_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
@@ -2900,11 +2933,12 @@ static void launch_scan(
     if (tiles <= 2048) {
         // short spine: every block of the second kernel adds up the tile sums before it
         launch_chained(
-            scan_apply_kernel<TIn, TOut, true>, static_cast<unsigned>(tiles), CTA_THREADS, 0, stream, counts, starts, n, tile_sums, total, first_value
+            scan_apply_kernel<TIn, TOut, true>, static_cast<unsigned>(tiles), CTA_THREADS, 0, stream, counts, starts, n, tile_sums, total, first_value,
+            header, mirror
         );
     } else {
         scan_spine_kernel<<<1, CTA_THREADS, 0, stream>>>(tile_sums, tiles, total);
-        scan_apply_kernel<TIn, TOut, false><<<static_cast<unsigned>(tiles), CTA_THREADS, 0, stream>>>(counts, starts, n, tile_sums, nullptr, first_value);
+        scan_apply_kernel<TIn, TOut, false><<<static_cast<unsigned>(tiles), CTA_THREADS, 0, stream>>>(counts, starts, n, tile_sums, nullptr, first_value, nullptr, nullptr);
     }
 }
 
@@ -2913,9 +2947,9 @@ void launch_scan_cells(const int32_t* counts, int32_t* starts, size_t n, void* t
 }
 
 void launch_scan_rows(
-    const uint32_t* counts, unsigned long long* starts, size_t n, void* tmp, unsigned long long* total, cudaStream_t stream
+    const uint32_t* counts, unsigned long long* starts, size_t n, void* tmp, DeviceHeader* header, cudaStream_t stream, DeviceHeader* mirror
 ) {
-    launch_scan<uint32_t, unsigned long long>(counts, starts, n, tmp, total, stream);
+    launch_scan<uint32_t, unsigned long long>(counts, starts, n, tmp, &header->total_pairs, stream, nullptr, header, mirror);
 }
 
 void launch_scatter(
@@ -2996,7 +3030,7 @@ void launch_sort_rows(
 
 void launch_pairs(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, PairOutput out, unsigned long long capacity,
-    DeviceHeader* header, cudaStream_t stream, size_t n_records, int part
+    DeviceHeader* header, cudaStream_t stream, size_t n_records, int part, DeviceHeader* mirror
 ) {
     // as many CTAs as are resident (by registers and shared memory), which take
     // runs of units from a shared counter; small systems give every unit its own CTA
@@ -3038,7 +3072,8 @@ void launch_pairs(
         }
         const int grid = pair_grid(runs, per_sm);
         launch_chained(
-            kernel, grid, Shape::THREADS, smem, stream, plan, cell_start, sorted, out, capacity, header, unit_run, ranges, run_cursor, follows ? 1 : 0
+            kernel, grid, Shape::THREADS, smem, stream, plan, cell_start, sorted, out, capacity, header, unit_run, ranges, run_cursor, follows ? 1 : 0,
+            (plan.window_axis < 0) ? mirror : nullptr
         );
     };
     const UnitRanges all{0, plan.n_units, 0, 0};

@@ -29,6 +29,8 @@ struct DeviceHeader {
     double box[9];                   // copy of the caller's box
     unsigned char periodic[8];       // copy of the caller's periodic flags
     unsigned long long halo_count[2]; // slab decomposition: records in the two halo messages of this build
+    unsigned int finished;            // CTAs of the pair kernel that are done (the last one clears it)
+    unsigned int exported;            // pinned mirror: written by a kernel (see export_header)
 };
 
 constexpr unsigned int STATUS_MASK_OVERFLOW = 1u;
@@ -81,6 +83,22 @@ inline int paired_stores_fit(const PairOutput& out) {
     return aligned(out.pairs, 32) && aligned(out.column_i, 16) && aligned(out.column_j, 16) && aligned(out.shifts, 8) &&
            aligned(out.distances, value_bytes) && aligned(out.vectors, value_bytes);
 }
+
+#ifdef __CUDACC__
+/// What the host wants to know of a pass, written into pinned memory by the pass itself, one warp:
+/// a copy behind the kernel costs its own launch and 3 us on the device, a few per cent of a small
+/// build. The host looks after it has waited for the stream, so the stores need no order.
+__device__ __forceinline__ void export_header(const DeviceHeader* header, DeviceHeader* mirror, int lane) {
+    static_assert(sizeof(DeviceHeader) % 8 == 0 && sizeof(DeviceHeader) <= 8 * 32, "a 64-bit word per lane");
+    if (lane < static_cast<int>(sizeof(DeviceHeader) / 8)) {
+        reinterpret_cast<volatile unsigned long long*>(mirror)[lane] = __ldcg(reinterpret_cast<const unsigned long long*>(header) + lane);
+    }
+    __syncwarp();
+    if (lane == 0) {
+        *reinterpret_cast<volatile unsigned int*>(&mirror->exported) = 1u;
+    }
+}
+#endif
 
 /// Input coordinates: double (the reference's C API) or float (fp32 entry
 /// point; converted exactly to double when read).
@@ -152,9 +170,11 @@ void launch_scan_cells(
     const int32_t* counts, int32_t* starts, size_t n, void* tmp, cudaStream_t stream, const int32_t* first_value = nullptr
 );
 /// Exclusive scan of uint32 counts into uint64 starts (n + 1 entries); the
-/// grand total also goes to *total.
+/// grand total also goes to header->total_pairs. `mirror` (pinned host memory, may be
+/// null): the header is written there when the total is known and mirror->exported set
+/// to 1; not for more than 4 M counts.
 void launch_scan_rows(
-    const uint32_t* counts, unsigned long long* starts, size_t n, void* tmp, unsigned long long* total, cudaStream_t stream
+    const uint32_t* counts, unsigned long long* starts, size_t n, void* tmp, DeviceHeader* header, cudaStream_t stream, DeviceHeader* mirror
 );
 /// Bytes of temporary storage the scans need for n elements.
 size_t scan_tmp_bytes(size_t n);
@@ -228,8 +248,10 @@ enum PairPart { PAIR_PART_ALL = 0, PAIR_PART_INTERIOR = 1, PAIR_PART_BOUNDARY = 
 bool pairs_have_interior(const GridPlan& plan);
 void launch_pairs(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, PairOutput out, unsigned long long capacity,
-    DeviceHeader* header, cudaStream_t stream, size_t n_records = 0, int part = PAIR_PART_ALL
+    DeviceHeader* header, cudaStream_t stream, size_t n_records = 0, int part = PAIR_PART_ALL, DeviceHeader* mirror = nullptr
 );
+// (mirror: pinned host memory; the last CTA of a launch that is not part of a slab build writes the
+//  header there and sets mirror->exported to 1)
 // (n_records: how many sorted records there are, if the caller knows; with it a launch of few
 //  units can tell how many batches of candidates a unit holds and share them among CTAs)
 
