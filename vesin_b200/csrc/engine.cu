@@ -1150,9 +1150,7 @@ void neighbors_batch(
             ws.batch_offsets.ptr, ws.batch_offsets_host.data(), (n_systems + 1) * sizeof(size_t), cudaMemcpyHostToDevice, stream
         ));
     }
-    VB200_CUDA(cudaMemsetAsync(ws.d_header, 0, sizeof(DeviceHeader), stream));
-    VB200_CUDA(cudaMemsetAsync(&ws.d_header->first_bad, 0xff, sizeof(unsigned long long), stream));
-    VB200_CUDA(cudaMemsetAsync(&ws.d_header->mask_cursor, 0xff, sizeof(unsigned long long), stream)); // first singular system
+    launch_batch_reset(ws.d_header, stream);
 
     BatchInput in{};
     in.points = points;
@@ -1186,11 +1184,12 @@ void neighbors_batch(
             ws.unit_count.as<unsigned long long>(), system_start, n_systems, ws.scan_tmp.ptr,
             &ws.d_header->total_pairs, stream
         );
+        ws.h_header->exported = 0;
         if (speculative) {
-            launch_small_emit(in, largest, any_for_cta_kernel, system_start, share_count, target.view(), ws.d_header, stream, existing);
+            launch_small_emit(in, largest, any_for_cta_kernel, system_start, share_count, target.view(), ws.d_header, stream, existing, ws.h_header);
         }
         VB200_CUDA(cudaGetLastError());
-        read_header(ws);
+        read_exported_header(ws);
         if (header.status & STATUS_STENCIL_TOO_LARGE) {
             throw std::runtime_error("the cutoff is too large for the box of system " + std::to_string(header.mask_cursor) + " of the batch");
         }

@@ -274,6 +274,8 @@ struct BatchInput {
 /// Largest system the batch kernels accept (its points live in shared memory).
 size_t small_systems_max_points();
 void configure_small_systems();
+/// Header of a batch: nothing found yet (first_bad, mask_cursor: the largest values).
+void launch_batch_reset(DeviceHeader* header, cudaStream_t stream);
 /// Pass 1: pairs of every system -> system_count; the first non-finite point
 /// and the first singular box are reported through the header.
 /// (`any_for_cta_kernel`: some system is periodic or has more points than
@@ -289,9 +291,11 @@ void launch_small_count(
 size_t molecules_max_points();
 /// Pass 2: every system writes its pairs at system_start[system]; a system whose block ends
 /// beyond `capacity` elements writes nothing (the pass may run before the host knows the total).
+/// `mirror` (pinned host memory, may be null) receives the header that pass 1 and the scan left.
 void launch_small_emit(
     const BatchInput& in, size_t max_points, bool any_for_cta_kernel, const unsigned long long* system_start,
-    unsigned long long* share_count, PairOutput out, DeviceHeader* header, cudaStream_t stream, unsigned long long capacity = ~0ull
+    unsigned long long* share_count, PairOutput out, DeviceHeader* header, cudaStream_t stream, unsigned long long capacity = ~0ull,
+    DeviceHeader* mirror = nullptr
 );
 
 /// Order-independent checksum of a list: result[0], result[1] = two sums

@@ -360,16 +360,31 @@ __device__ __forceinline__ void write_hits(
     }
 }
 
+/// Header of a batch: nothing found yet.
+__global__ void batch_header_kernel(DeviceHeader* header) {
+    if (threadIdx.x < sizeof(DeviceHeader) / 4) {
+        reinterpret_cast<unsigned*>(header)[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        header->first_bad = NO_BAD_POINT;
+        header->mask_cursor = ~0ull; // first singular system
+    }
+}
+
 template <bool EMIT>
 __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
     const BatchInput in, unsigned long long* __restrict__ system_count, const unsigned long long* __restrict__ system_start, PairOutput out,
-    DeviceHeader* header, const unsigned long long capacity
+    DeviceHeader* header, const unsigned long long capacity, DeviceHeader* mirror
 ) {
     extern __shared__ __align__(16) unsigned char molecule_smem[];
     MoleculeShared& sh = *reinterpret_cast<MoleculeShared*>(molecule_smem);
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const unsigned warps_in_grid = gridDim.x * MOLECULE_WARPS;
+    if (EMIT && mirror != nullptr && blockIdx.x == 0 && warp == 0) {
+        export_header(header, mirror, lane); // (the writing pass adds nothing to the header)
+    }
 
     for (unsigned system = blockIdx.x * MOLECULE_WARPS + warp; system < in.n_systems; system += warps_in_grid) {
         const unsigned long long begin = in.offsets[system];
@@ -925,13 +940,18 @@ static unsigned molecules_grid(unsigned n_systems) {
     return wanted < cap ? (wanted ? wanted : 1) : cap;
 }
 
+void launch_batch_reset(DeviceHeader* header, cudaStream_t stream) {
+    static_assert(sizeof(DeviceHeader) % 4 == 0 && sizeof(DeviceHeader) <= 4 * 256, "a thread per word");
+    batch_header_kernel<<<1, 256, 0, stream>>>(header);
+}
+
 void launch_small_count(
     const BatchInput& in, size_t max_points, bool any_for_cta_kernel, unsigned long long* system_count, unsigned long long* share_count,
     DeviceHeader* header, cudaStream_t stream
 ) {
     const PairOutput nothing{};
     molecules_kernel<false><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
-        in, system_count, nullptr, nothing, header, 0ull
+        in, system_count, nullptr, nothing, header, 0ull, nullptr
     );
     if (any_for_cta_kernel) {
         const unsigned splits = small_splits(in.n_systems, max_points);
@@ -943,12 +963,13 @@ void launch_small_count(
 
 void launch_small_emit(
     const BatchInput& in, size_t max_points, bool any_for_cta_kernel, const unsigned long long* system_start,
-    unsigned long long* share_count, PairOutput out, DeviceHeader* header, cudaStream_t stream, unsigned long long capacity
+    unsigned long long* share_count, PairOutput out, DeviceHeader* header, cudaStream_t stream, unsigned long long capacity,
+    DeviceHeader* mirror
 ) {
     // paired stores of full lists need aligned arrays (every system of a full list starts on an even element)
     out.interleave_ok = paired_stores_fit(out);
     molecules_kernel<true><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
-        in, nullptr, system_start, out, header, capacity
+        in, nullptr, system_start, out, header, capacity, mirror
     );
     if (any_for_cta_kernel) {
         const unsigned splits = small_splits(in.n_systems, max_points);
