@@ -198,20 +198,15 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
 
-/// Squared distances outside [lo, hi] are decided by the screen.
+/// Squared distances further than `half` from `mid` are decided by the screen.
 struct ScreenBand {
-    float lo, hi;
+    float mid, half;
 };
 
 /// The band for home points within `m` of the origin of the local frame. A candidate within the
@@ -220,55 +215,69 @@ struct ScreenBand {
 /// candidate further out is at more than the cutoff by more than its own rounding error, as long
 /// as m is not thousands of times the cutoff; beyond that (or with m not finite) every candidate
 /// goes to the exact predicate.
+__device__ __forceinline__ ScreenBand everything_exact() {
+    return ScreenBand{0.0f, __int_as_float(0x7f800000)};
+}
 __device__ __forceinline__ ScreenBand screen_band(float m, double cutoff_exact, double cutoff2_exact) {
     const float c = static_cast<float>(cutoff_exact) * 1.01f;
     const float M = (m + c) * 1.0001f;
     const float eps = 5.9604644775390625e-08f;
     float band = 4.0f * eps * (2.0f * 1.7320508f * c * (2.0f * M + c) + 3.0f * c * c) + 40.0f * eps * eps * M * M + 4.0f * eps * c * c;
-    band *= 1.01f; // this expression is itself evaluated in fp32
+    band *= 1.05f; // this expression is itself evaluated in fp32, and the sum starts from -mid
     const float cutoff2 = static_cast<float>(cutoff2_exact);
-    ScreenBand result{cutoff2 - band, cutoff2 + band};
-    if (!(m < 5.0e3f * c) || !(result.hi < 3.0e38f) || !(c > 1.0e-12f)) {
-        result = ScreenBand{-__int_as_float(0x7f800000), __int_as_float(0x7f800000)};
+    if (!(m < 5.0e3f * c) || !(cutoff2 + band < 3.0e38f) || !(c > 1.0e-12f)) {
+        return everything_exact();
     }
-    return result;
+    return ScreenBand{cutoff2, band};
 }
 
-/// Screen of candidates [0, 4 * quads) of a word against the home point whose negated
-/// coordinates are (ax, ay, az): `inside` gets a bit for those surely within the cutoff, `maybe`
-/// for those and the ones only the exact predicate can decide. x, y, z: 16-byte aligned arrays in
-/// shared memory, the same addresses for every lane.
-__device__ __forceinline__ void screen_word(
-    const float* x, const float* y, const float* z, int quads, unsigned long long ax, unsigned long long ay, unsigned long long az,
-    const ScreenBand& band, unsigned& inside, unsigned& maybe
+/// Decisions on candidates [0, 4 * quads) of a word for the home point whose negated coordinates are
+/// (ax, ay, az), as far as `keep` has bits: the sign of d2 - mid, or exact(bit) for a candidate too
+/// close to the cutoff for fp32 (the minimum over the word tells whether there is one). x, y, z:
+/// 16-byte aligned arrays in shared memory, the same addresses for every lane.
+template <class Exact>
+__device__ __forceinline__ unsigned screen_word(
+    const float* x, const float* y, const float* z, int quads, float ax, float ay, float az, const ScreenBand& band, unsigned keep, Exact exact
 ) {
-    inside = 0;
-    maybe = 0;
+    const unsigned long long ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az), mid2 = pack2(-band.mid, -band.mid);
+    unsigned inside = 0;
+    float closest = __int_as_float(0x7f800000);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 7; k >= 0; k--) {
         if (k >= quads) {
-            break;
+            continue;
         }
         const ulonglong2 x4 = reinterpret_cast<const ulonglong2*>(x)[k];
         const ulonglong2 y4 = reinterpret_cast<const ulonglong2*>(y)[k];
         const ulonglong2 z4 = reinterpret_cast<const ulonglong2*>(z)[k];
-        const unsigned long long dx0 = add2(x4.x, ax), dy0 = add2(y4.x, ay), dz0 = add2(z4.x, az);
-        const unsigned long long dx1 = add2(x4.y, ax), dy1 = add2(y4.y, ay), dz1 = add2(z4.y, az);
-        const unsigned long long d0 = fma2(dx0, dx0, fma2(dy0, dy0, mul2(dz0, dz0)));
-        const unsigned long long d1 = fma2(dx1, dx1, fma2(dy1, dy1, mul2(dz1, dz1)));
+        const unsigned long long dx0 = add2(x4.x, ax2), dy0 = add2(y4.x, ay2), dz0 = add2(z4.x, az2);
+        const unsigned long long dx1 = add2(x4.y, ax2), dy1 = add2(y4.y, ay2), dz1 = add2(z4.y, az2);
+        const unsigned long long d0 = fma2(dx0, dx0, fma2(dy0, dy0, fma2(dz0, dz0, mid2)));
+        const unsigned long long d1 = fma2(dx1, dx1, fma2(dy1, dy1, fma2(dz1, dz1, mid2)));
         float d2[4];
         asm("mov.b64 {%0, %1}, %2;" : "=f"(d2[0]), "=f"(d2[1]) : "l"(d0));
         asm("mov.b64 {%0, %1}, %2;" : "=f"(d2[2]), "=f"(d2[3]) : "l"(d1));
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            if (d2[c] < band.lo) {
-                inside |= 1u << (4 * k + c);
-            }
-            if (!(d2[c] > band.hi)) { // (NaN: the exact predicate decides)
-                maybe |= 1u << (4 * k + c);
+        for (int c = 3; c >= 0; c--) {
+            inside = __funnelshift_l(__float_as_uint(d2[c]), inside, 1);
+        }
+        closest = fminf(closest, fminf(fabsf(d2[0]), fabsf(d2[1])));
+        closest = fminf(closest, fminf(fabsf(d2[2]), fabsf(d2[3])));
+    }
+    if (!(closest > band.half)) {
+#pragma unroll 1
+        for (unsigned left = keep; left != 0; left &= left - 1) {
+            const int b = __ffs(left) - 1;
+            const float dx = x[b] + ax, dy = y[b] + ay, dz = z[b] + az;
+            if (!(fabsf(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, -band.mid)))) > band.half)) { // (NaN: the exact predicate decides)
+                inside &= ~(1u << b);
+                if (exact(b)) {
+                    inside |= 1u << b;
+                }
             }
         }
     }
+    return inside & keep;
 }
 
 /// Bits `first` and above of a word.
@@ -468,23 +477,15 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
             const float ax = -sh.fx[warp][own];
             const float ay = -sh.fy[warp][own];
             const float az = -sh.fz[warp][own];
-            const unsigned long long ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
             for (int j0 = i0; j0 < n; j0 += 32) {
-                unsigned inside, maybe;
-                screen_word(
-                    sh.fx[warp] + j0, sh.fy[warp] + j0, sh.fz[warp] + j0, min(8, (n - j0 + 3) >> 2), ax2, ay2, az2, band, inside, maybe
-                );
                 const unsigned keep = (i < n) ? bits_from(i + 1 - j0) & ~bits_from(n - j0) : 0u;
-                inside &= keep;
-                unsigned undecided = maybe & keep & ~inside;
-                while (undecided != 0) {
-                    const int b = __ffs(undecided) - 1;
-                    undecided &= undecided - 1;
-                    double vx, vy, vz;
-                    if (molecule_pair(sh, warp, i, j0 + b, vx, vy, vz) < in.cutoff2) {
-                        inside |= 1u << b;
+                const unsigned inside = screen_word(
+                    sh.fx[warp] + j0, sh.fy[warp] + j0, sh.fz[warp] + j0, min(8, (n - j0 + 3) >> 2), ax, ay, az, band, keep,
+                    [&](int b) {
+                        double vx, vy, vz;
+                        return molecule_pair(sh, warp, i, j0 + b, vx, vy, vz) < in.cutoff2;
                     }
-                }
+                );
                 if (EMIT) {
                     list_hits(inside, static_cast<unsigned>((i << 8) | j0), sh.list[warp], listed, lane, write);
                 } else {
@@ -765,9 +766,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 5) small_systems_kernel(
                 }
                 ScreenBand band = sh.band;
                 if (exact_only) {
-                    band = ScreenBand{-__int_as_float(0x7f800000), __int_as_float(0x7f800000)};
+                    band = everything_exact();
                 }
-                const unsigned long long hx2 = pack2(hx, hx), hy2 = pack2(hy, hy), hz2 = pack2(hz, hz);
 
                 for (int batch0 = 0; batch0 < total; batch0 += SMALL_BATCH) {
                     const int slots = min(SMALL_BATCH, total - batch0);
@@ -844,11 +844,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 5) small_systems_kernel(
                         }
                     };
                     for (int w = warp; w < words; w += SMALL_WARPS) {
-                        unsigned inside, maybe;
                         const int in_word = min(32, slots - 32 * w);
-                        screen_word(
-                            sh.near_x + 32 * w, sh.near_y + 32 * w, sh.near_z + 32 * w, (in_word + 3) >> 2, hx2, hy2, hz2, band, inside, maybe
-                        );
                         unsigned keep = (lane < n_home) ? ~bits_from(in_word) : 0u;
                         if (chunk0 == i0) {
                             // of the points of the tile only those after the home point, and its own images
@@ -856,21 +852,17 @@ __global__ void __launch_bounds__(SMALL_THREADS, 5) small_systems_kernel(
                             const int own_end = sh.first_slot[lane + 1] - batch0 - 32 * w;
                             keep &= bits_from(own_end) | (sh.self_word[w] & bits_from(own_first));
                         }
-                        inside &= keep;
-                        unsigned undecided = maybe & keep & ~inside;
-                        while (undecided != 0) {
-                            const int b = __ffs(undecided) - 1;
-                            undecided &= undecided - 1;
-                            const int4 image = sh.image[32 * w + b];
-                            double vx, vy, vz;
-                            const double d2 = small_pair(
-                                frame, sh.home[0][lane], sh.home[1][lane], sh.home[2][lane], sh.x[image.w], sh.y[image.w], sh.z[image.w],
-                                image.x + sh.home_wrap[0][lane], image.y + sh.home_wrap[1][lane], image.z + sh.home_wrap[2][lane], vx, vy, vz
-                            );
-                            if (d2 < in.cutoff2) {
-                                inside |= 1u << b;
+                        const unsigned inside = screen_word(
+                            sh.near_x + 32 * w, sh.near_y + 32 * w, sh.near_z + 32 * w, (in_word + 3) >> 2, hx, hy, hz, band, keep,
+                            [&](int b) {
+                                const int4 image = sh.image[32 * w + b];
+                                double vx, vy, vz;
+                                return small_pair(
+                                           frame, sh.home[0][lane], sh.home[1][lane], sh.home[2][lane], sh.x[image.w], sh.y[image.w], sh.z[image.w],
+                                           image.x + sh.home_wrap[0][lane], image.y + sh.home_wrap[1][lane], image.z + sh.home_wrap[2][lane], vx, vy, vz
+                                       ) < in.cutoff2;
                             }
-                        }
+                        );
                         if (EMIT) {
                             list_hits(inside, static_cast<unsigned>((lane << 8) | (32 * w)), sh.list[warp], listed, lane, write);
                         } else {
