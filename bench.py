@@ -229,6 +229,9 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    if not reference_cpu_at_hand():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference CPU library is not built and its sources are not here"}))
+        return
     if args.workload in BATCH_WORKLOADS:
         run_reference_batch(args)
         return
@@ -601,6 +604,15 @@ def measure_extra_batch(harness, name):
     }
 
 
+def reference_cpu_at_hand():
+    """Is the reference CPU library built, or can it be built here? Checks and
+    baselines that need it are left out where it is not."""
+    from oracle import oracle
+
+    oracle.build()
+    return oracle.reference_available()
+
+
 def reference_checksum(system, cutoff, full, float_io):
     """Checksum of the list the reference CPU library builds (all host cores)."""
     from oracle import oracle
@@ -758,7 +770,7 @@ def run_sharded_leg(harness, name, steps, reference_parity):
     algorithmic = n_atoms * bytes_per_point(float_io) + total_pairs * bytes_per_pair(float_io)
     entry["bytes"] = algorithmic
     entry["frac"] = algorithmic / (entry["ms_per_step"] * 1e-3) / 1e9 / (peak * harness.world)
-    if reference_parity and harness.rank == 0:
+    if reference_parity and harness.rank == 0 and reference_cpu_at_hand():
         entry["parity_reference_cpu"] = bool(tuple(reference_checksum(system, cutoff, full, float_io)) == tuple(checksum))
     harness.barrier()
     return entry
@@ -812,7 +824,7 @@ def run_ours(args):
         single = single_gpu_reference_build(harness, system, cutoff, full, float_io)
         if rank == 0:
             parity = {"single_gpu": bool(tuple(single["checksum"]) == tuple(checksum)), "rows": checksum[3], "single_gpu_rows": single["n_pairs"]}
-            if world <= 2:
+            if world <= 2 and reference_cpu_at_hand():
                 parity["reference_cpu"] = bool(tuple(reference_checksum(system, cutoff, full, float_io)) == tuple(checksum))
         harness.barrier()
 
@@ -910,11 +922,13 @@ def run_ours(args):
             leg["liquid2m_check"] = {key: check[key] for key in check if key.startswith("parity") or key in ("n_pairs", "ms_per_step", "workload")}
             line["sharded"] = leg
             if world > 1:
-                flags = [leg.get("parity_single_gpu"), check.get("parity_single_gpu"), check.get("parity_reference_cpu")]
+                flags = [leg.get("parity_single_gpu"), check.get("parity_single_gpu")]
+                if "parity_reference_cpu" in check:
+                    flags.append(check["parity_reference_cpu"])
                 line["parity"] = bool(line.get("parity", True) and all(flag is not False for flag in flags) and None not in flags)
 
     if rank == 0:
-        if world == 1 and not args.no_cpu_baseline:
+        if world == 1 and not args.no_cpu_baseline and reference_cpu_at_hand():
             points, box, periodic = system
             used = points.astype(np.float32).astype(np.float64) if float_io else points
             used_box = box.astype(np.float32).astype(np.float64) if float_io else box
@@ -1014,10 +1028,9 @@ def run_batch(args):
             "gpu_launches": 5 * args.steps,
             "clocks": clocks.summary(),
         }
-        if world == 1 and not args.no_cpu_baseline:
+        if world == 1 and not args.no_cpu_baseline and reference_cpu_at_hand():
             from oracle import oracle
 
-            oracle.build()
             cpu = oracle.ReferenceCPU()
             sample = min(n_systems, 4096)
             box = np.zeros((3, 3))
