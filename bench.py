@@ -797,7 +797,7 @@ def run_ours(args):
         build = PlainBuild(harness, system, cutoff, full, float_io, sorted_list, skin=2.0 if name.endswith("_skin") else 0.0)
         n_points_rank = build.n_points
         per_gpu = "one independent copy of the system per GPU, no communication" if world > 1 else "the whole system on one GPU"
-        launches_per_step = 7  # header (reset, zero, box check), bin (+ point checks), 2 x scan, 2 x scatter, pairs
+        launches_per_step = 6  # header (reset, zero, box check), bin (+ point checks), 2 x scan, scatter, pairs
 
     # ---- warm-up (also sizes the workspace and the output arrays) ----
     for _ in range(max(args.warmup, 3)):
@@ -1075,7 +1075,7 @@ def run_sharded(args):
                          "peak": harness.peak * harness.world, "unit": "GB/s", "frac": entry["frac"], "traffic": None},
             "sharded": entry,
             "e2e": None,
-            "gpu_launches": (9 if harness.world > 1 else 7) * args.steps * harness.world,
+            "gpu_launches": (9 if harness.world > 1 else 6) * args.steps * harness.world,
         }
         flags = [value for key, value in entry.items() if key.startswith("parity")]
         if flags:
