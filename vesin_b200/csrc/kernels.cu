@@ -2296,7 +2296,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
 // warp, so that every store covers one contiguous span of it)
 
 constexpr int ROW_WINDOW = 128;    // hits of a row a warp lists at a time
-constexpr int RANK_BUCKETS = 1024; // see rank_candidates
+constexpr int RANK_BUCKETS = 2048; // see rank_candidates (216k crystal, row kernel: 1024 527 us, 2048 513, 4096 534)
 
 /// Shape of the CTAs of the row-writing kernel: BATCH candidates are staged at a time.
 /// CANONICAL: all candidates of a unit fit one batch and are staged in the order of their indices.
@@ -2349,7 +2349,7 @@ using CanonicalRowsWide = RowShape<true, 2048, 2>;
 /// two of, in any order): sh.ordering.key[0 ... n) -> sh.rank and sh.order. Buckets of equal width between the smallest and the largest index, counted
 /// and scanned; a candidate's rank is the start of its bucket plus the smaller ones inside it. The
 /// indices around a unit are either scattered (a bucket holds one or two) or come in runs (crystals
-/// in lattice order: about twenty), so this takes a third of the instructions of a bitonic sort of
+/// in lattice order: about a dozen), so this takes a third of the instructions of a bitonic sort of
 /// the same keys, and no more when all fall into one bucket. Starts behind a barrier that follows
 /// the writes of the keys, least and most, and ends with one.
 template <class Shape>

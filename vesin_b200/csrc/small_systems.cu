@@ -564,7 +564,7 @@ __device__ __forceinline__ double small_pair(
 }
 
 template <bool EMIT>
-__global__ void __launch_bounds__(SMALL_THREADS, 5) small_systems_kernel(
+__global__ void __launch_bounds__(SMALL_THREADS, 6) small_systems_kernel(
     const BatchInput in, const unsigned splits, unsigned long long* __restrict__ system_count, unsigned long long* __restrict__ share_count,
     const unsigned long long* __restrict__ system_start, PairOutput out, DeviceHeader* header, const unsigned long long capacity
 ) {
@@ -918,7 +918,7 @@ static unsigned multiprocessors() {
 unsigned small_splits(unsigned n_systems, size_t max_points) {
     // about four waves of CTAs, so that systems of different sizes even out; never more than tiles
     const unsigned tiles = static_cast<unsigned>((max_points + SMALL_TILE - 1) / SMALL_TILE);
-    const unsigned wanted = 4 * 5 * multiprocessors() / std::max(n_systems, 1u);
+    const unsigned wanted = 4 * 6 * multiprocessors() / std::max(n_systems, 1u);
     return std::max(1u, std::min(wanted, tiles));
 }
 
