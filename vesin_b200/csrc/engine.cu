@@ -852,10 +852,16 @@ void neighbors(
         SortedPoints sorted{ws.sorted_records.as<PointRecord>(), ws.sorted_wide_shift.as<int32_t>()};
 
         // ---- cell list ----
+        uint32_t* row_count = nullptr; // sorted lists: cleared by the kernel that scatters the points
+        if (plan.by_index) {
+            ws.row_count.reserve(n_points * sizeof(uint32_t));
+            row_count = ws.row_count.as<uint32_t>();
+        }
         if (fused_front || (!speculative && small_front_fits(n_points, plan))) {
             timer.begin(VesinB200StageBin);
             launch_small_front(
-                flat_points, n_points, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, flat_box, periodic, speculative, ws.cache.box, ws.cache.periodic, stream
+                flat_points, n_points, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, flat_box, periodic, speculative, ws.cache.box, ws.cache.periodic, stream,
+                row_count
             );
             timer.end(VesinB200StageBin);
             timer.begin(VesinB200StageScanCells);
@@ -875,7 +881,7 @@ void neighbors(
             launch_scan_cells(ws.cell_count.as<int32_t>(), ws.cell_start.as<int32_t>(), n_cells, ws.scan_tmp.ptr, stream);
             timer.end(VesinB200StageScanCells);
             timer.begin(VesinB200StageScatter);
-            launch_scatter(source, 0, n_points, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, stream);
+            launch_scatter(source, 0, n_points, plan, ws.rank.as<int32_t>(), ws.cell_start.as<int32_t>(), sorted, ws.d_header, stream, row_count);
             timer.end(VesinB200StageScatter);
         }
         const auto collect_front_stages = [&]() {
@@ -954,7 +960,6 @@ void neighbors(
         // ---- sorted list: rows in index order need a scan between two passes ----
         ws.unit_mask_base.reserve(n_units * sizeof(unsigned long long));
         ws.unit_words.reserve(n_units * sizeof(uint32_t));
-        ws.row_count.reserve(n_points * sizeof(uint32_t));
         ws.row_start.reserve((n_points + 1) * sizeof(unsigned long long));
         ws.row_fill.reserve(n_points * sizeof(uint32_t));
         if (ws.masks.bytes == 0) {
@@ -971,7 +976,9 @@ void neighbors(
         bool refused = false;
         for (int attempt = 0;; attempt++) {
             timer.begin(VesinB200StageCount);
-            VB200_CUDA(cudaMemsetAsync(ws.row_count.ptr, 0, n_points * sizeof(uint32_t), stream));
+            if (attempt != 0) {
+                VB200_CUDA(cudaMemsetAsync(ws.row_count.ptr, 0, n_points * sizeof(uint32_t), stream));
+            }
             launch_count(
                 plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.masks.bytes / sizeof(uint32_t),
                 ws.unit_mask_base.as<unsigned long long>(), ws.unit_words.as<uint32_t>(), ws.row_count.as<uint32_t>(), ws.d_header, stream
@@ -1050,7 +1057,9 @@ void neighbors(
                 }
             }
             timer.begin(VesinB200StageEmit);
-            VB200_CUDA(cudaMemsetAsync(ws.row_fill.ptr, 0, n_points * sizeof(uint32_t), stream));
+            if (header.max_candidates > static_cast<unsigned>(row_batch(canonical_batch))) {
+                VB200_CUDA(cudaMemsetAsync(ws.row_fill.ptr, 0, n_points * sizeof(uint32_t), stream));
+            }
             launch_emit(
                 plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.unit_mask_base.as<unsigned long long>(),
                 ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), rows, canonical_batch, stream

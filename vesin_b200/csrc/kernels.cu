@@ -540,9 +540,11 @@ __global__ void __launch_bounds__(CTA_THREADS) bin_kernel(
 // block whose 8192-cell limit caps the reference's grid) and the pre-sized
 // output + global append counter (vesin/src/vesin_cuda.cpp:866-886,
 // cell_list.cu:643-668): per-point counts are scanned into private rows.
-// Two launches (tile sums; apply, every block adding up the sums of the tiles
-// before its own) up to 2048 tiles, three beyond (tile sums, spine, apply); no
-// inter-CTA waiting.
+// One launch up to 4 tiles of 2048 elements (every block adds up the elements
+// before its own tile, at most 24 per thread, which takes less than a launch),
+// two up to 2048 tiles (tile sums; apply, every block adding up the sums of the
+// tiles before its own), three beyond (tile sums, spine, apply); no inter-CTA
+// waiting.
 // ---------------------------------------------------------------------------
 
 constexpr int SCAN_ITEMS = 8;
@@ -624,7 +626,8 @@ __global__ void __launch_bounds__(CTA_THREADS) scan_spine_kernel(unsigned long l
 }
 
 /// SPINE: `tile_offsets` still holds the sums of the tiles (the spine kernel
-/// did not run): every block adds up the sums of the tiles before its own.
+/// did not run): every block adds up the sums of the tiles before its own, or
+/// the elements before its tile when there are no sums (null).
 template <typename TIn, typename TOut, bool SPINE>
 __global__ void __launch_bounds__(CTA_THREADS) scan_apply_kernel(
     const TIn* __restrict__ in, TOut* __restrict__ out, size_t n, const unsigned long long* __restrict__ tile_offsets,
@@ -661,8 +664,15 @@ __global__ void __launch_bounds__(CTA_THREADS) scan_apply_kernel(
     unsigned long long tile_offset = 0;
     if (SPINE) {
         unsigned long long before = 0;
-        for (unsigned t = threadIdx.x; t < blockIdx.x; t += CTA_THREADS) {
-            before += tile_offsets[t];
+        if (tile_offsets == nullptr) {
+            const unsigned end = blockIdx.x * SCAN_TILE;
+            for (unsigned k = threadIdx.x; k < end; k += CTA_THREADS) {
+                before += static_cast<unsigned long long>(in[k]);
+            }
+        } else {
+            for (unsigned t = threadIdx.x; t < blockIdx.x; t += CTA_THREADS) {
+                before += tile_offsets[t];
+            }
         }
 #pragma unroll
         for (int offset = 16; offset > 0; offset >>= 1) {
@@ -728,13 +738,16 @@ __global__ void __launch_bounds__(CTA_THREADS) scan_apply_kernel(
 template <bool HALO>
 __global__ void __launch_bounds__(CTA_THREADS) scatter_records_kernel(
     const PointSource source, size_t first, size_t last, const GridPlan plan, const int32_t* __restrict__ rank,
-    const int32_t* __restrict__ cell_start, SortedPoints sorted, DeviceHeader* __restrict__ header
+    const int32_t* __restrict__ cell_start, SortedPoints sorted, DeviceHeader* __restrict__ header, uint32_t* __restrict__ zero
 ) {
     let_next_kernel_start();
     wait_for_previous_kernel();
     const size_t i = first + static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= last || (header->status & STATUS_ABORT_MASK)) {
         return;
+    }
+    if (zero != nullptr) {
+        zero[i] = 0;
     }
     double x, y, z;
     if (!load_point<HALO>(source, i, x, y, z)) {
@@ -771,7 +784,7 @@ constexpr size_t SMALL_FRONT_MAX_POINTS = 16384;
 __global__ void __launch_bounds__(SMALL_FRONT_THREADS) small_front_kernel(
     const RealView points, size_t n, const GridPlan plan, int32_t* __restrict__ rank, int32_t* __restrict__ cell_start, SortedPoints sorted,
     DeviceHeader* header, const RealView box,
-    const bool* periodic, const int speculative, const ExpectedInputs expected
+    const bool* periodic, const int speculative, const ExpectedInputs expected, uint32_t* __restrict__ zero
 ) {
     __shared__ int hist[SMALL_FRONT_MAX_CELLS];
     __shared__ int warp_sums[SMALL_FRONT_THREADS / 32];
@@ -796,6 +809,9 @@ __global__ void __launch_bounds__(SMALL_FRONT_THREADS) small_front_kernel(
     }
     for (int c = t; c < n_cells; c += SMALL_FRONT_THREADS) {
         hist[c] = 0;
+    }
+    for (size_t i = t; zero != nullptr && i < n; i += SMALL_FRONT_THREADS) {
+        zero[i] = 0;
     }
     // (the binning below may set status bits: behind this barrier nobody looks at them any more)
     if (__syncthreads_or(refused ? 1 : 0)) {
@@ -3016,7 +3032,11 @@ static void launch_scan(
 ) {
     auto* tile_sums = static_cast<unsigned long long*>(tmp);
     size_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    launch_chained(scan_tile_sums_kernel<TIn>, static_cast<unsigned>(tiles), CTA_THREADS, 0, stream, counts, n, tile_sums);
+    if (tiles <= 4) {
+        tile_sums = nullptr;
+    } else {
+        launch_chained(scan_tile_sums_kernel<TIn>, static_cast<unsigned>(tiles), CTA_THREADS, 0, stream, counts, n, tile_sums);
+    }
     if (tiles <= 2048) {
         // short spine: every block of the second kernel adds up the tile sums before it
         launch_chained(
@@ -3041,16 +3061,16 @@ void launch_scan_rows(
 
 void launch_scatter(
     const PointSource& source, size_t first, size_t last, const GridPlan& plan, const int32_t* rank, const int32_t* cell_start,
-    SortedPoints sorted, DeviceHeader* header, cudaStream_t stream
+    SortedPoints sorted, DeviceHeader* header, cudaStream_t stream, uint32_t* zero
 ) {
     if (last <= first) {
         return;
     }
     const unsigned blocks = static_cast<unsigned>((last - first + CTA_THREADS - 1) / CTA_THREADS);
     if (source.message[0] != nullptr && source.capacity > 0) {
-        launch_chained(scatter_records_kernel<true>, blocks, CTA_THREADS, 0, stream, source, first, last, plan, rank, cell_start, sorted, header);
+        launch_chained(scatter_records_kernel<true>, blocks, CTA_THREADS, 0, stream, source, first, last, plan, rank, cell_start, sorted, header, zero);
     } else {
-        launch_chained(scatter_records_kernel<false>, blocks, CTA_THREADS, 0, stream, source, first, last, plan, rank, cell_start, sorted, header);
+        launch_chained(scatter_records_kernel<false>, blocks, CTA_THREADS, 0, stream, source, first, last, plan, rank, cell_start, sorted, header, zero);
     }
 }
 
@@ -3078,6 +3098,10 @@ int canonical_emit_batch(unsigned max_candidates, bool duplicates_possible) {
         return CanonicalRows::BATCH;
     }
     return (max_candidates <= CanonicalRowsWide::BATCH) ? CanonicalRowsWide::BATCH : 0;
+}
+
+int row_batch(int canonical_batch) {
+    return (canonical_batch != 0) ? canonical_batch : SortedRows::BATCH;
 }
 
 void launch_emit(
@@ -3301,11 +3325,11 @@ bool small_front_fits(size_t n_points, const GridPlan& plan) {
 void launch_small_front(
     RealView points, size_t n, const GridPlan& plan, int32_t* rank, int32_t* cell_start, SortedPoints sorted, DeviceHeader* header,
     RealView box, const bool* periodic, bool speculative, const double expected_box[9],
-    const bool expected_periodic[3], cudaStream_t stream
+    const bool expected_periodic[3], cudaStream_t stream, uint32_t* zero
 ) {
     small_front_kernel<<<1, SMALL_FRONT_THREADS, 0, stream>>>(
         points, n, plan, rank, cell_start, sorted, header, box, periodic, speculative ? 1 : 0,
-        expected_inputs(expected_box, expected_periodic)
+        expected_inputs(expected_box, expected_periodic), zero
     );
 }
 

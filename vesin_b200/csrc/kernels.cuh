@@ -182,10 +182,11 @@ size_t scan_tmp_bytes(size_t n);
 /// Counting-sort scatter of the local indices [first, last) into the cell-sorted
 /// records (a slab build scatters its owned points, whose records come first,
 /// before the halo has arrived). Where the source has global indices, those go
-/// into the records (31 bits; a larger one sets STATUS_INDEX_RANGE).
+/// into the records (31 bits; a larger one sets STATUS_INDEX_RANGE). `zero` (may be null): a
+/// word per local index that is cleared on the way (what sorted lists count their rows in).
 void launch_scatter(
     const PointSource& source, size_t first, size_t last, const GridPlan& plan, const int32_t* rank, const int32_t* cell_start,
-    SortedPoints sorted, DeviceHeader* header, cudaStream_t stream
+    SortedPoints sorted, DeviceHeader* header, cudaStream_t stream, uint32_t* zero = nullptr
 );
 
 /// Small systems: header reset and plan check (when `speculative`), binning,
@@ -197,7 +198,7 @@ bool small_front_fits(size_t n_points, const GridPlan& plan);
 void launch_small_front(
     RealView points, size_t n, const GridPlan& plan, int32_t* rank, int32_t* cell_start, SortedPoints sorted, DeviceHeader* header,
     RealView box, const bool* periodic, bool speculative, const double expected_box[9],
-    const bool expected_periodic[3], cudaStream_t stream
+    const bool expected_periodic[3], cudaStream_t stream, uint32_t* zero = nullptr
 );
 
 /// Exclusive scan of uint64 counts into uint64 starts (n + 1 entries); the
@@ -216,12 +217,14 @@ void launch_count(
 
 /// Sorted lists, pass 2: walks the hit bits and writes i, j, S, d, D, one row
 /// per point in index order (row_start from the scan of row_count; row_fill
-/// must start at zero). `canonical_batch`: 0, or what canonical_emit_batch()
+/// must start at zero when a unit has more than row_batch() candidates, and is not looked at
+/// otherwise). `canonical_batch`: 0, or what canonical_emit_batch()
 /// said: the rows then come out sorted by the second index.
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
     const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, int canonical_batch, cudaStream_t stream
 );
+int row_batch(int canonical_batch);
 /// Can pass 2 write the rows of a canonical list in their final order? It can when a CTA holds all
 /// candidates of a unit at once and no second index comes twice in a row. 0: it can not, the rows
 /// have to be sorted behind it (launch_sort_rows).
