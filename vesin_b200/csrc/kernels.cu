@@ -2711,11 +2711,18 @@ __device__ __forceinline__ bool shift_before(const int32_t* __restrict__ shifts,
     return false;
 }
 
-/// 12-byte element at a 4-byte aligned address: one 8-byte and one 4-byte store.
+/// 12-byte element: one 8-byte and one 4-byte store where the array starts on 8 bytes (`wide`),
+/// else a store per component.
 template <typename T>
-__device__ __forceinline__ void store_triple_32(T* base, unsigned long long element, T a, T b, T c) {
+__device__ __forceinline__ void store_triple_32(T* base, unsigned long long element, T a, T b, T c, bool wide) {
     static_assert(sizeof(T) == 4, "int32 shifts or float vectors");
     T* dst = base + 3 * element;
+    if (!wide) {
+        __stcs(dst, a);
+        __stcs(dst + 1, b);
+        __stcs(dst + 2, c);
+        return;
+    }
     struct alignas(8) Two {
         T x, y;
     };
@@ -2735,9 +2742,16 @@ __device__ __forceinline__ void store_triple_32(T* base, unsigned long long elem
     }
 }
 
-/// 24-byte element at an 8-byte aligned address: one 16-byte and one 8-byte store.
-__device__ __forceinline__ void store_triple_64(double* base, unsigned long long element, double a, double b, double c) {
+/// 24-byte element: one 16-byte and one 8-byte store where the array starts on 16 bytes (`wide`),
+/// else a store per component.
+__device__ __forceinline__ void store_triple_64(double* base, unsigned long long element, double a, double b, double c, bool wide) {
     double* dst = base + 3 * element;
+    if (!wide) {
+        __stcs(dst, a);
+        __stcs(dst + 1, b);
+        __stcs(dst + 2, c);
+        return;
+    }
     if ((element & 1ull) == 0) {
         __stcs(reinterpret_cast<double2*>(dst), make_double2(a, b));
         __stcs(dst + 2, c);
@@ -2780,24 +2794,24 @@ __device__ __forceinline__ PairInFlight<FLOAT> load_pair(const PairOutput& in, u
 }
 
 template <bool FLOAT>
-__device__ __forceinline__ void store_pair(const PairOutput& out, unsigned long long to, const PairInFlight<FLOAT>& p) {
+__device__ __forceinline__ void store_pair(const PairOutput& out, unsigned long long to, const PairInFlight<FLOAT>& p, bool wide) {
     store_indices(out, to, p.pair.x, p.pair.y);
     if (out.shifts != nullptr) {
-        store_triple_32(out.shifts, to, p.s0, p.s1, p.s2);
+        store_triple_32(out.shifts, to, p.s0, p.s1, p.s2, wide);
     }
     if (FLOAT) {
         if (out.distances != nullptr) {
             __stcs(reinterpret_cast<float*>(out.distances) + to, static_cast<float>(p.d));
         }
         if (out.vectors != nullptr) {
-            store_triple_32(reinterpret_cast<float*>(out.vectors), to, static_cast<float>(p.vx), static_cast<float>(p.vy), static_cast<float>(p.vz));
+            store_triple_32(reinterpret_cast<float*>(out.vectors), to, static_cast<float>(p.vx), static_cast<float>(p.vy), static_cast<float>(p.vz), wide);
         }
     } else {
         if (out.distances != nullptr) {
             __stcs(out.distances + to, static_cast<double>(p.d));
         }
         if (out.vectors != nullptr) {
-            store_triple_64(out.vectors, to, static_cast<double>(p.vx), static_cast<double>(p.vy), static_cast<double>(p.vz));
+            store_triple_64(out.vectors, to, static_cast<double>(p.vx), static_cast<double>(p.vy), static_cast<double>(p.vz), wide);
         }
     }
 }
@@ -2808,10 +2822,10 @@ __device__ __forceinline__ void store_pair(const PairOutput& out, unsigned long 
 /// everything it will copy, ranks both pairs against the row while the loads are in flight
 /// (four comparisons per 16-byte load and pair), then stores. DUPLICATES = false: the caller
 /// knows that no second index comes twice in a row (no lattice vector shorter than twice the
-/// cutoff), so the comparisons of shifts are left out altogether.
+/// cutoff), so the comparisons of shifts are left out altogether. `wide`: see store_triple_32.
 template <bool DUPLICATES, bool FLOAT>
 __global__ void __launch_bounds__(CTA_THREADS, 3) row_sort_kernel(
-    const unsigned long long* __restrict__ row_start, size_t n_rows, PairOutput in, PairOutput out
+    const unsigned long long* __restrict__ row_start, size_t n_rows, PairOutput in, PairOutput out, const bool wide
 ) {
     __shared__ __align__(16) unsigned row_keys[CTA_WARPS][ROW_SORT_STAGED];
     constexpr int PER_LANE = 3; // a row of up to 96 pairs is one pass
@@ -2875,7 +2889,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 3) row_sort_kernel(
                             }
                         }
                     }
-                    store_pair<FLOAT>(out, begin + rank, moving[m]);
+                    store_pair<FLOAT>(out, begin + rank, moving[m], wide);
                 }
             }
         } else {
@@ -2889,7 +2903,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 3) row_sort_kernel(
                         rank++;
                     }
                 }
-                store_pair<FLOAT>(out, begin + rank, load_pair<FLOAT>(in, mine));
+                store_pair<FLOAT>(out, begin + rank, load_pair<FLOAT>(in, mine), wide);
             }
         }
     }
@@ -3131,7 +3145,9 @@ void launch_sort_rows(
     }
     // a warp per row, eight rows per CTA
     const size_t blocks = std::min<size_t>((n_rows + CTA_WARPS - 1) / CTA_WARPS, 148 * 64);
-    const auto launch = [&](auto kernel) { kernel<<<static_cast<unsigned>(blocks), CTA_THREADS, 0, stream>>>(row_start, n_rows, in, out); };
+    // (arrays of a caller need no more than the alignment of their elements)
+    const bool wide = triple_stores_fit(out);
+    const auto launch = [&](auto kernel) { kernel<<<static_cast<unsigned>(blocks), CTA_THREADS, 0, stream>>>(row_start, n_rows, in, out, wide); };
     if (in.values_float) {
         duplicates_possible ? launch(row_sort_kernel<true, true>) : launch(row_sort_kernel<false, true>);
     } else {

@@ -74,14 +74,22 @@ struct PairOutput {
     unsigned long long* column_j;
 };
 
+inline bool aligned_to(const void* pointer, uintptr_t bytes) {
+    return reinterpret_cast<uintptr_t>(pointer) % bytes == 0;
+}
+
+/// Are the arrays of three-component elements aligned for stores of two components at a time
+/// (row_sort_kernel, and store_both of full lists)? Null arrays are not written.
+inline bool triple_stores_fit(const PairOutput& out) {
+    return aligned_to(out.shifts, 8) && aligned_to(out.vectors, out.values_float ? 8 : 16);
+}
+
 /// Are the arrays aligned for the paired stores of full lists (store_both)? 32 bytes of indices
 /// (16 per column), 16 of distances / vectors, 8 of shifts; half of that for float values. Null
 /// arrays are not written.
 inline int paired_stores_fit(const PairOutput& out) {
-    const auto aligned = [](const void* pointer, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(pointer) % bytes == 0; };
-    const uintptr_t value_bytes = out.values_float ? 8 : 16;
-    return aligned(out.pairs, 32) && aligned(out.column_i, 16) && aligned(out.column_j, 16) && aligned(out.shifts, 8) &&
-           aligned(out.distances, value_bytes) && aligned(out.vectors, value_bytes);
+    return aligned_to(out.pairs, 32) && aligned_to(out.column_i, 16) && aligned_to(out.column_j, 16) &&
+           aligned_to(out.distances, out.values_float ? 8 : 16) && triple_stores_fit(out);
 }
 
 #ifdef __CUDACC__
