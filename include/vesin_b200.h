@@ -154,9 +154,10 @@ VESIN_API int vesin_b200_neighbors_batch_f32(
  * return) as vesin_neighbors, vesin_b200_neighbors_f32
  * (VESIN_B200_FLOAT32: points and box are float arrays, `distances` and
  * `vectors` too), vesin_b200_neighbors_canonical (VESIN_B200_CANONICAL) and
- * vesin_b200_neighbors_batch. Arrays must be aligned to their elements (`pairs`
- * to 16 bytes); full lists are written fastest when `pairs` is aligned to 32
- * bytes and the others to 16.
+ * vesin_b200_neighbors_batch. Arrays must be memory of the device of
+ * `neighbors`, aligned to their elements (`pairs` to 16 bytes): others are an
+ * error. Full lists are written fastest when `pairs` is aligned to 32 bytes and
+ * the others to 16.
  */
 struct VesinB200Arrays {
     size_t capacity;

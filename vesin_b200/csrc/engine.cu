@@ -368,6 +368,7 @@ class Target {
             list_.shifts = nullptr;
             list_.distances = nullptr;
             list_.vectors = nullptr;
+            check_arrays();
         } else {
             reserve(std::max<size_t>(capacity(), 256));
         }
@@ -405,6 +406,7 @@ class Target {
                     caller_->arrays->capacity < pairs) {
                     throw std::bad_alloc();
                 }
+                check_arrays();
             }
             return;
         }
@@ -462,6 +464,36 @@ class Target {
     }
 
   private:
+    /// What the kernels would fault on: arrays of the caller that are not memory of this device, or
+    /// not aligned to their elements (`pairs`: to the two indices, which leave in one store).
+    void check_arrays() const {
+        const VesinB200Arrays& arrays = *caller_->arrays;
+        if (arrays.capacity == 0) {
+            return; // nothing is written
+        }
+        const auto check_array = [&](const void* array, const char* name, size_t alignment) {
+            if (array == nullptr) {
+                return;
+            }
+            if (reinterpret_cast<uintptr_t>(array) % alignment != 0) {
+                throw std::runtime_error(std::string("array `") + name + "` is not aligned to " + std::to_string(alignment) + " bytes");
+            }
+            const PointerInfo info = inspect(array);
+            if (!info.on_device || info.device != list_.device.device_id) {
+                throw std::runtime_error(std::string("array `") + name + "` is not device memory on the CUDA device of `neighbors`");
+            }
+        };
+        const size_t value_bytes = float_io_ ? sizeof(float) : sizeof(double);
+        check_array(arrays.pairs, "pairs", 2 * sizeof(size_t));
+        if (arrays.pairs == nullptr) {
+            check_array(arrays.i, "i", sizeof(size_t));
+            check_array(arrays.j, "j", sizeof(size_t));
+        }
+        check_array(arrays.shifts, "shifts", sizeof(int32_t));
+        check_array(arrays.distances, "distances", value_bytes);
+        check_array(arrays.vectors, "vectors", value_bytes);
+    }
+
     VesinNeighborList& list_;
     Workspace& ws_;
     const VesinOptions& options_;
