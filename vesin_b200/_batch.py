@@ -13,7 +13,7 @@ import torch
 
 from ._c_api import VESIN_B200_FLOAT32, VesinCUDA, VesinDevice, VesinNeighborList, VesinOptions, get_library
 from ._neighbors import _view
-from ._outputs import OutputTensors, allocate_callback
+from ._outputs import OutputTensors, allocate_callback, wait_for_caller
 
 
 def split_batch(system_offsets, world_size):
@@ -75,12 +75,9 @@ class BatchNeighborList:
             periodic = torch.as_tensor(periodic, device=device).to(torch.bool).contiguous()
             if tuple(boxes.shape) != (n_systems, 3, 3) or tuple(periodic.shape) != (n_systems, 3):
                 raise ValueError("`boxes` must be (n_systems, 3, 3) and `periodic` (n_systems, 3)")
-        # the engine works on a stream of its own, which only the legacy default stream is ordered with
-        stream = torch.cuda.current_stream(device)
-        if stream.cuda_stream != 0:
-            stream.synchronize()
         if copy:
             return self._build_into(points, system_offsets, boxes, periodic, quantities, global_indices)
+        wait_for_caller(device)
         pair_offsets = self.build(points, system_offsets, boxes, periodic, quantities, global_indices)
 
         n_pairs = self._neighbors.length
@@ -160,6 +157,7 @@ class BatchNeighborList:
         if self._last_pairs > 0:
             outputs.allocate(self._last_pairs + self._last_pairs // 16 + 256)
         pair_offsets = torch.empty(len(offsets), dtype=torch.int64, device=points.device)
+        wait_for_caller(points.device)
         n_pairs = ctypes.c_size_t()
         error = ctypes.c_char_p()
         with outputs:

@@ -30,7 +30,7 @@ from ._c_api import (
     VesinUnknownDevice,
     get_library,
 )
-from ._outputs import OutputTensors, allocate_callback
+from ._outputs import OutputTensors, allocate_callback, wait_for_caller
 
 
 class _DeviceArray:
@@ -191,17 +191,13 @@ class NeighborList:
             self._lib.vesin_free(ctypes.byref(self._neighbors))
             ctypes.memset(ctypes.byref(self._neighbors), 0, ctypes.sizeof(self._neighbors))
 
-        # inputs produced on another stream of the caller must be complete: the engine works on
-        # a stream of its own, which only the legacy default stream is ordered with
-        stream = torch.cuda.current_stream(device)
-        if stream.cuda_stream != 0:
-            stream.synchronize()
         error_message = ctypes.c_char_p()
 
         if from_torch and copy:
             outputs = OutputTensors(quantities, device, torch.uint64, work_dtype)
             if self._last_pairs > 0:
                 outputs.allocate(self._last_pairs + self._last_pairs // 16 + 256)
+            wait_for_caller(device)
             n_pairs = ctypes.c_size_t()
             with outputs:
                 status = self._lib.vesin_b200_neighbors_into(
@@ -225,6 +221,7 @@ class NeighborList:
             values = outputs.take(n_pairs.value)
             return tuple(value.to(out_dtype) if value.dtype == work_dtype else value for value in values)
 
+        wait_for_caller(device)
         entry_point = self._lib.vesin_b200_neighbors_f32 if float_io else self._lib.vesin_neighbors
         if self.canonical:
             entry_point = self._lib.vesin_b200_neighbors_canonical

@@ -13,12 +13,23 @@ from ._c_api import VesinB200Allocate, VesinB200Arrays
 _active = threading.local()
 
 
+def wait_for_caller(device):
+    """The engine works on a stream of its own, which only the legacy default
+    stream is ordered with: on any other stream, what the caller has queued
+    (inputs being made, memory that a stream-ordered allocator has handed out)
+    must be done before the engine touches it."""
+    stream = torch.cuda.current_stream(device)
+    if stream.cuda_stream != 0:
+        stream.synchronize()
+
+
 @VesinB200Allocate
 def allocate_callback(_context, n_pairs, arrays):
     """Called by the engine, on the thread that called it, when a list needs
     more room than the arrays it was given have."""
     try:
         _active.outputs.allocate(n_pairs)
+        wait_for_caller(_active.outputs.device)
         return 0
     except BaseException as error:  # nothing may propagate through the engine: the caller raises it
         _active.outputs.error = error
