@@ -2006,19 +2006,20 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
     run_parity ^= 1;
     }
     if (mirror != nullptr && warp == 0) {
-        // The last CTA reports. The claims of a CTA are atomics of its thread 0 whose results it has
-        // used, so they have taken place; only a counting pass does not look at them.
+        // The last CTA reports. The claims of a CTA are atomics of its thread 0: the first fence
+        // orders them before the CTA's mark, the second one the marks of all CTAs before the look
+        // at what they claimed.
         int last = 0;
         if (lane == 0) {
-            if (capacity == 0) {
-                __threadfence();
-            }
+            __threadfence();
             last = atomicAdd(&header->finished, 1u) == gridDim.x - 1;
             if (last) {
+                __threadfence();
                 header->finished = 0;
             }
         }
         if (__shfl_sync(FULL_MASK, last, 0)) {
+            __syncwarp();
             export_header(header, mirror, lane);
         }
     }
