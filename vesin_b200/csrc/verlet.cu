@@ -73,10 +73,11 @@ __global__ void __launch_bounds__(VERLET_THREADS) verlet_pack_kernel(
     }
 }
 
-/// One row of `positions` (32-byte aligned): a single 256-bit load.
+/// One row of `positions` (32-byte aligned): a single 256-bit load. (volatile: not moved above the wait
+/// for the kernel that wrote the rows)
 __device__ __forceinline__ void load_row(const double* __restrict__ positions, uint32_t p, double& x, double& y, double& z, long long& index) {
     long long a, b, c;
-    asm("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(index) : "l"(positions + 4 * static_cast<size_t>(p)));
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(index) : "l"(positions + 4 * static_cast<size_t>(p)));
     x = __longlong_as_double(a);
     y = __longlong_as_double(b);
     z = __longlong_as_double(c);
