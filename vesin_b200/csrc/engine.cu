@@ -1075,7 +1075,8 @@ void neighbors(
                 rows = PairOutput{};
                 rows.values_float = out.values_float;
                 rows.pairs = ws.alt_pairs.as<unsigned long long>();
-                if (out.shifts != nullptr) {
+                // (a second index that comes twice in a row is ordered by its shifts, asked for or not)
+                if (out.shifts != nullptr || duplicates_possible) {
                     ws.alt_shifts.reserve(total * 3 * sizeof(int32_t));
                     rows.shifts = ws.alt_shifts.as<int32_t>();
                 }
