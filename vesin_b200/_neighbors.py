@@ -164,9 +164,8 @@ class NeighborList:
             work_dtype = np.float32 if float_io else np.float64
             d_points = torch.from_numpy(np.ascontiguousarray(points, dtype=work_dtype)).to(device, non_blocking=False)
             d_box = torch.from_numpy(np.ascontiguousarray(box, dtype=work_dtype)).to(device)
-            if not isinstance(periodic, (list, tuple)):
-                periodic = np.ascontiguousarray(periodic, dtype=np.bool_).tolist()
-            d_periodic = _periodic_flags(periodic, device)
+            # (numpy makes flags of anything with a truth value)
+            d_periodic = _periodic_flags(np.ascontiguousarray(periodic, dtype=np.bool_).tolist(), device)
         if tuple(d_periodic.shape) != (3,):
             raise ValueError(
                 "`periodic` must be a single boolean or a sequence of three "
