@@ -1362,12 +1362,14 @@ struct Screen {
 };
 __device__ __forceinline__ Screen screen_of(const GridPlan& plan) {
     Screen screen;
-    if (plan.cutoff2_lo > 0.0f) {
-        // (5 % more than half the band of the plan: the rounding of both numbers)
+    if (plan.cutoff2_lo > 0.0f && plan.cutoff2_hi < 1.0e30f) {
+        // (5 % more than half the band of the plan: the rounding of both numbers. A candidate is
+        // within 700 cutoffs of the centre of its unit, or the band would be wider than the cutoff:
+        // no square overflows)
         screen.mid = 0.5f * (plan.cutoff2_lo + plan.cutoff2_hi);
         screen.half = 0.525f * (plan.cutoff2_hi - plan.cutoff2_lo);
     } else {
-        // the band is wider than the cutoff: nothing is decided in fp32
+        // the band is wider than the cutoff, or squares leave the range of fp32: nothing is decided in fp32
         screen.mid = 0.0f;
         screen.half = __int_as_float(0x7f800000);
     }
@@ -1408,7 +1410,8 @@ __device__ __forceinline__ unsigned decide_piece(
         float d2[4];
         unpack_f32x2(fma_f32x2(x4.x, ax2, fma_f32x2(y4.x, ay2, fma_f32x2(z4.x, az2, add_f32x2(n4.x, an2)))), d2[0], d2[1]);
         unpack_f32x2(fma_f32x2(x4.y, ax2, fma_f32x2(y4.y, ay2, fma_f32x2(z4.y, az2, add_f32x2(n4.y, an2)))), d2[2], d2[3]);
-        // (NaN, in lanes without a point, is ignored by the minimum and masked below)
+        // (NaN, in lanes without a point, is ignored by the minimum and masked below; a NaN of
+        // squares out of the range of fp32 leaves the minimum at infinity, and `half` is infinite then)
 #pragma unroll
         for (int c = 3; c >= 0; c--) {
             inside = __funnelshift_l(__float_as_uint(d2[c]), inside, 1);
@@ -1437,9 +1440,11 @@ __device__ __forceinline__ unsigned decide_piece(
 #pragma unroll 1
         for (int b = 0; b < BITS; b++) {
             const int s = first_slot + b;
-            const float d2 = fmaf(sh.near_x[s], ax, fmaf(sh.near_y[s], ay, fmaf(sh.near_z[s], az, sh.near_n[s] + an)));
-            // (infinite: past the end of the batch, or out of the range of fp32)
-            if (fabsf(d2) <= half && fabsf(d2) < __int_as_float(0x7f800000) && ((keep >> b) & 1u) != 0) {
+            const float x = sh.near_x[s], y = sh.near_y[s], z = sh.near_z[s], n = sh.near_n[s];
+            const float d2 = fmaf(x, ax, fmaf(y, ay, fmaf(z, az, n + an)));
+            // (past the end of the batch: at the origin, and infinitely far from it)
+            const bool empty = x == 0.0f && y == 0.0f && z == 0.0f && n != 0.0f;
+            if (!(fabsf(d2) > half) && !empty && ((keep >> b) & 1u) != 0) { // (NaN: out of the range of fp32)
                 // the exact fp64 predicate of the reference decides
                 inside &= ~(1u << b);
                 if (exact(s)) {
@@ -1694,7 +1699,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                         xi = valid ? sh.near_x[slot] : nan;
                         yi = valid ? sh.near_y[slot] : nan;
                         zi = valid ? sh.near_z[slot] : nan;
-                        an = sh.near_n[slot];
+                        an = valid ? sh.near_n[slot] : nan;
                     } else {
                         const size_t pi = static_cast<size_t>(unit.begin) + (valid ? il : 0);
                         const LoadedRecord record = load_record(sorted, pi);
