@@ -1,5 +1,6 @@
 """The output tensors of the calculators, without a GPU: what happens around
-the allocation that the engine asks for in the middle of a build."""
+the allocation that the engine asks for in the middle of a build, and the room
+that is guessed before it."""
 
 import ctypes
 
@@ -31,3 +32,40 @@ def test_engine_waits_for_memory_it_was_handed(handle, waits, monkeypatch):
         assert _outputs.allocate_callback(None, 5, ctypes.byref(outputs.arrays)) == 0
     assert events == ["allocate"] + waits
     assert outputs.arrays.capacity == 5 and [len(t) for t in outputs.take(5)] == [5] * 5
+
+
+def _outputs_of(quantities="ijSdD"):
+    return _outputs.OutputTensors(quantities, torch.device("cpu"), torch.int64, torch.float64)
+
+
+def test_room_follows_the_number_of_points():
+    outputs = _outputs_of()
+    outputs.allocate_guess((0, 0), 1000)
+    assert outputs.arrays.capacity == 0
+    for n_points, pairs in ((1000, 80000), (10, 800), (3000, 240000)):
+        outputs.allocate_guess((80000, 1000), n_points)
+        assert pairs <= outputs.arrays.capacity <= pairs + pairs // 8 + 256
+
+
+def test_room_that_is_not_there(monkeypatch):
+    """A guess that does not fit is no error: the engine asks for what it needs."""
+    empty = torch.empty
+    outputs = _outputs_of()
+
+    def no_room_for_vectors(shape, **options):
+        if shape == (1063, 3) and options["dtype"] == torch.float64:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(shape, **options)
+
+    monkeypatch.setattr(torch, "empty", no_room_for_vectors)
+    outputs.allocate_guess((760, 10), 10)
+    arrays = outputs.arrays
+    assert arrays.capacity == 0 and not any((arrays.i, arrays.j, arrays.pairs, arrays.shifts, arrays.distances, arrays.vectors))
+    assert outputs.i is None and outputs.shifts is None
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device: _Stream(0, []))
+    with outputs:
+        assert _outputs.allocate_callback(None, 700, ctypes.byref(outputs.arrays)) == 0
+        assert outputs.arrays.capacity == 700
+        # one that the engine asks for is the caller's error
+        assert _outputs.allocate_callback(None, 1063, ctypes.byref(outputs.arrays)) == 1
+    assert isinstance(outputs.error, torch.cuda.OutOfMemoryError)

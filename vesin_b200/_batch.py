@@ -44,7 +44,7 @@ class BatchNeighborList:
         self.cutoff = float(cutoff)
         self.full_list = bool(full_list)
         self._neighbors = VesinNeighborList()
-        self._last_pairs = 0  # length of the last list: what the next one will roughly need
+        self._last = (0, 0)  # pairs and points of the last list: what the next one will roughly need
 
     def __del__(self):
         try:
@@ -136,7 +136,7 @@ class BatchNeighborList:
         )
         if status != 0:
             raise RuntimeError(error.value.decode("utf8"))
-        self._last_pairs = self._neighbors.length
+        self._last = (self._neighbors.length, points.shape[0])
         return pair_offsets.value
 
     def _options(self, quantities):
@@ -154,8 +154,7 @@ class BatchNeighborList:
         float_io = points.dtype == torch.float32
         offsets = np.ascontiguousarray(system_offsets, dtype=np.uint64)
         outputs = OutputTensors(quantities, points.device, torch.int64, points.dtype)
-        if self._last_pairs > 0:
-            outputs.allocate(self._last_pairs + self._last_pairs // 16 + 256)
+        outputs.allocate_guess(self._last, points.shape[0])
         pair_offsets = torch.empty(len(offsets), dtype=torch.int64, device=points.device)
         wait_for_caller(points.device)
         n_pairs = ctypes.c_size_t()
@@ -181,10 +180,10 @@ class BatchNeighborList:
             )
         if status != 0:
             raise outputs.error or RuntimeError(error.value.decode("utf8"))
-        self._last_pairs = n_pairs.value
+        self._last = (n_pairs.value, points.shape[0])
         return tuple(outputs.take(n_pairs.value)), pair_offsets
 
     @property
     def n_pairs(self):
         """Pairs of the last list."""
-        return self._last_pairs
+        return self._last[0]

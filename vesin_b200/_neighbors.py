@@ -85,7 +85,7 @@ class NeighborList:
         if self.n_threads < 0:
             raise ValueError("n_threads must be zero or a positive integer")
         self._neighbors = VesinNeighborList()
-        self._last_pairs = 0  # length of the last list: what the next one will roughly need
+        self._last = (0, 0)  # pairs and points of the last list: what the next one will roughly need
 
     def __del__(self):
         try:
@@ -194,8 +194,7 @@ class NeighborList:
 
         if from_torch and copy:
             outputs = OutputTensors(quantities, device, torch.uint64, work_dtype)
-            if self._last_pairs > 0:
-                outputs.allocate(self._last_pairs + self._last_pairs // 16 + 256)
+            outputs.allocate_guess(self._last, d_points.shape[0])
             wait_for_caller(device)
             n_pairs = ctypes.c_size_t()
             with outputs:
@@ -216,7 +215,7 @@ class NeighborList:
                 )
             if status != 0:
                 raise outputs.error or RuntimeError(error_message.value.decode("utf8"))
-            self._last_pairs = n_pairs.value
+            self._last = (n_pairs.value, d_points.shape[0])
             values = outputs.take(n_pairs.value)
             return tuple(value.to(out_dtype) if value.dtype == work_dtype else value for value in values)
 

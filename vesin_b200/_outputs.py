@@ -57,11 +57,28 @@ class OutputTensors:
     def __exit__(self, *_):
         _active.outputs = self._outer
 
+    def allocate_guess(self, last, n_points):
+        """Room for as many pairs per point as the last list had (`last`: its
+        pairs and points), so that the engine can write at once. Where there is
+        no such room the engine counts first and asks for what the list needs."""
+        last_pairs, last_points = last
+        if last_pairs == 0:
+            return
+        expected = last_pairs if n_points == last_points else last_pairs * n_points // last_points
+        try:
+            self.allocate(expected + expected // 16 + 256)
+        except torch.cuda.OutOfMemoryError:
+            self.release()
+
+    def release(self):
+        self.i = self.j = self.pairs = self.shifts = self.distances = self.vectors = None
+        arrays = self.arrays
+        arrays.capacity = 0
+        arrays.i = arrays.j = arrays.pairs = arrays.shifts = arrays.distances = arrays.vectors = None
+
     def allocate(self, n_pairs):
         quantities, device, arrays = self.quantities, self.device, self.arrays
-        # what there is too little of goes back to the allocator first
-        self.i = self.j = self.pairs = self.shifts = self.distances = self.vectors = None
-        arrays.capacity = 0
+        self.release()  # what there is too little of goes back to the allocator first
         if "P" in quantities:
             self.pairs = torch.empty((n_pairs, 2), dtype=self.index_dtype, device=device)
             arrays.pairs = self.pairs.data_ptr()
