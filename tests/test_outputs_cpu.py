@@ -51,9 +51,10 @@ def test_room_that_is_not_there(monkeypatch):
     """A guess that does not fit is no error: the engine asks for what it needs."""
     empty = torch.empty
     outputs = _outputs_of()
+    full = [True]
 
     def no_room_for_vectors(shape, **options):
-        if shape == (1063, 3) and options["dtype"] == torch.float64:
+        if full and isinstance(shape, tuple) and options["dtype"] == torch.float64:
             raise torch.cuda.OutOfMemoryError("no room")
         return empty(shape, **options)
 
@@ -63,9 +64,23 @@ def test_room_that_is_not_there(monkeypatch):
     assert arrays.capacity == 0 and not any((arrays.i, arrays.j, arrays.pairs, arrays.shifts, arrays.distances, arrays.vectors))
     assert outputs.i is None and outputs.shifts is None
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device: _Stream(0, []))
+    full.clear()
     with outputs:
         assert _outputs.allocate_callback(None, 700, ctypes.byref(outputs.arrays)) == 0
         assert outputs.arrays.capacity == 700
         # one that the engine asks for is the caller's error
-        assert _outputs.allocate_callback(None, 1063, ctypes.byref(outputs.arrays)) == 1
+        full.append(True)
+        assert _outputs.allocate_callback(None, 1000, ctypes.byref(outputs.arrays)) == 1
     assert isinstance(outputs.error, torch.cuda.OutOfMemoryError)
+
+
+@pytest.mark.parametrize("n_pairs", [0, 1, 60, 128, 700, 100000])
+@pytest.mark.parametrize("capacity", [1.0, 1.06, 1.12, 1.2, 4.0])
+def test_storage_of_a_list(n_pairs, capacity):
+    """A list that is kept or saved takes little more than its own rows with it."""
+    outputs = _outputs_of()
+    outputs.allocate(int(n_pairs * capacity) + 64)
+    for tensor in outputs.take(n_pairs):
+        assert len(tensor) == n_pairs
+        row = tensor.element_size() * (3 if tensor.dim() == 2 else 1)
+        assert tensor.untyped_storage().nbytes() <= row * (n_pairs + n_pairs // 8 + 128)

@@ -66,7 +66,7 @@ class OutputTensors:
             return
         expected = last_pairs if n_points == last_points else last_pairs * n_points // last_points
         try:
-            self.allocate(expected + expected // 16 + 256)
+            self.allocate(expected + expected // 16 + 64)
         except torch.cuda.OutOfMemoryError:
             self.release()
 
@@ -105,8 +105,9 @@ class OutputTensors:
         if n_pairs == 0 and self.arrays.capacity == 0:
             self.allocate(0)
         capacity = self.arrays.capacity
-        # a list that shrank a lot does not hold on to the room that its predecessor needed
-        wasteful = capacity > n_pairs + n_pairs // 8 + 4096
+        # What a tensor holds on to, and what is written when it is saved, is its whole storage: an
+        # eighth and 128 rows more than its own at most, or it is copied
+        wasteful = capacity > n_pairs + n_pairs // 8 + 128
 
         def rows(tensor):
             if capacity == n_pairs:
