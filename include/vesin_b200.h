@@ -460,7 +460,8 @@ VESIN_API int vesin_b200_list_value_bytes(const struct VesinNeighborList* neighb
  * its device: checksum[0] and checksum[1] are sums (mod 2^64) of two 64-bit
  * hashes of every row (i, j, S), checksum[2] the same with the bits of the
  * distance mixed in, checksum[3] the number of rows. Arrays that were not
- * requested count as zeros. Lists of one system built in different orders or
+ * requested count as zeros. A list whose last build wrote into arrays of the
+ * caller holds no rows: an error. Lists of one system built in different orders or
  * split over ranks (add the ranks' sums) have equal checksums exactly when
  * they hold the same rows, up to hash collisions; the row hash is
  *   key = i*0x9e3779b97f4a7c15 + j*0xc2b2ae3d27d4eb4f + u32(Sx)*0x165667b19e3779f9

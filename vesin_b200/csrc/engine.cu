@@ -112,6 +112,7 @@ struct Workspace {
     DeviceBuffer batch_shares;  // ... and the pairs each of the CTAs that share a system has
     DeviceBuffer checksum;      // 4 words of vesin_b200_list_checksum
     bool values_float = false;  // element type of `distances` / `vectors` of the last build
+    bool pairs_elsewhere = false; // the last build wrote into arrays of the caller: the list holds no pairs
 
     // Slab builds: extent of the local points along non-periodic directions as the last build
     // that looked found it (the binning kernel checks every point against it), and the number
@@ -362,6 +363,7 @@ class Target {
     Target(VesinNeighborList& list, Workspace& ws, const VesinOptions& options, bool float_io, const CallerArrays* caller):
         list_(list), ws_(ws), options_(options), float_io_(float_io), caller_(caller) {
         list_.length = 0;
+        ws_.pairs_elsewhere = caller_ != nullptr;
         if (caller_ != nullptr) {
             // the pairs do not belong to the list
             list_.pairs = nullptr;
@@ -1599,6 +1601,9 @@ void list_checksum(const VesinNeighborList& list, unsigned long long result[4]) 
     }
     DeviceGuard guard(list.device.device_id);
     Workspace& ws = *static_cast<Workspace*>(list.opaque);
+    if (ws.pairs_elsewhere) {
+        throw std::runtime_error("the pairs of the last build are in arrays of the caller: the list holds none");
+    }
     ws.checksum.reserve(4 * sizeof(unsigned long long));
     launch_checksum(
         reinterpret_cast<const unsigned long long*>(list.pairs), reinterpret_cast<const int32_t*>(list.shifts), list.distances,
