@@ -25,6 +25,10 @@ def test_reference_arm_prints_the_contract_line():
     assert line["cpu_baseline"]["kind"] in ("reference", "port") and line["cpu_baseline"]["cores"] >= 1
     assert line["e2e"]["h2d_bytes_per_step"] == 0 and line["e2e"]["d2h_bytes_per_step"] == 0
     assert line["e2e"]["value"] == line["value"]
+    # what was not the reference says so
+    restated = line["cpu_baseline"]["kind"] == "port"
+    assert ("unavailable" in line) == restated
+    assert ("not the reference" in line["cpu_baseline"]["sample"]) == restated
 
 
 def test_our_arm_refuses_to_run_without_a_gpu():
