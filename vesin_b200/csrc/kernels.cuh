@@ -29,9 +29,13 @@ struct DeviceHeader {
     double box[9];                   // copy of the caller's box
     unsigned char periodic[8];       // copy of the caller's periodic flags
     unsigned long long halo_count[2]; // slab decomposition: records in the two halo messages of this build
-    unsigned int finished;            // CTAs of the pair kernel that are done (the last one clears it)
+    unsigned long long finished;      // CTAs of the pair kernel that are done and the elements they claimed (see FINISHED_CTA)
     unsigned int exported;            // pinned mirror: written by a kernel (see export_header)
+    unsigned int reserved;
 };
+
+/// A CTA of the pair kernel that is done adds this and its claims to DeviceHeader::finished.
+constexpr unsigned long long FINISHED_CTA = 1ull << 48;
 
 constexpr unsigned int STATUS_MASK_OVERFLOW = 1u;
 constexpr unsigned int STATUS_BAD_POINT = 2u;  // a point has a non-finite coordinate
@@ -95,11 +99,16 @@ inline int paired_stores_fit(const PairOutput& out) {
 #ifdef __CUDACC__
 /// What the host wants to know of a pass, written into pinned memory by the pass itself, one warp:
 /// a copy behind the kernel costs its own launch and 3 us on the device, a few per cent of a small
-/// build. The host looks after it has waited for the stream, so the stores need no order.
-__device__ __forceinline__ void export_header(const DeviceHeader* header, DeviceHeader* mirror, int lane) {
+/// build. The host looks after it has waited for the stream, so the stores need no order. `pairs`
+/// (unless ~0) stands for the pair cursor, which CTAs of the same kernel have added to.
+__device__ __forceinline__ void export_header(const DeviceHeader* header, DeviceHeader* mirror, int lane, unsigned long long pairs = ~0ull) {
     static_assert(sizeof(DeviceHeader) % 8 == 0 && sizeof(DeviceHeader) <= 8 * 32, "a 64-bit word per lane");
     if (lane < static_cast<int>(sizeof(DeviceHeader) / 8)) {
-        reinterpret_cast<volatile unsigned long long*>(mirror)[lane] = __ldcg(reinterpret_cast<const unsigned long long*>(header) + lane);
+        unsigned long long word = __ldcg(reinterpret_cast<const unsigned long long*>(header) + lane);
+        if (pairs != ~0ull && lane == static_cast<int>(offsetof(DeviceHeader, pair_cursor) / 8)) {
+            word = pairs;
+        }
+        reinterpret_cast<volatile unsigned long long*>(mirror)[lane] = word;
     }
     __syncwarp();
     if (lane == 0) {
