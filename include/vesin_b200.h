@@ -68,9 +68,11 @@ VESIN_API int vesin_b200_neighbors_f32(
  * vesin/src/cuda/sort_pairs.cu:3-12): this entry point returns THE canonical
  * list, sorted by (i, j, Sx, Sy, Sz), so that two lists of the same system can
  * be compared element by element without sorting them on the host.
- * `options.sorted` is taken as set. Rows are sorted on the device after the
- * build, into a second set of output arrays (the list then owns twice the
- * memory of an unsorted one). Everything else as vesin_neighbors.
+ * `options.sorted` is taken as set. Rows are written in their final order by the
+ * build, but for systems with a lattice vector shorter than twice the cutoff or
+ * more than 2048 points around a cell: those are sorted on the device behind it,
+ * from a second set of output arrays (the list then owns twice the memory of an
+ * unsorted one). Everything else as vesin_neighbors.
  */
 VESIN_API int vesin_b200_neighbors_canonical(
     const double (*points)[3],

@@ -512,7 +512,8 @@ __global__ void __launch_bounds__(CTA_THREADS) bin_kernel(
     // warp-aggregated histogram: one atomic per distinct cell in the warp. Finding the lanes of a
     // cell costs a step per distinct cell, which points in random order (no two neighbours in the
     // same cell) do not gain anything by: they take an atomic each. 2.1 M points of a liquid in
-    // random order: 53 -> 28 us; 512k atoms in lattice order pay for the look at their neighbours, 8.7 -> 9.7.
+    // random order: 53 -> 28 us; 512k atoms in lattice order pay for the look at their neighbours, 8.7
+    // -> 9.7 (and the scatter behind it, which does not read their cells any more, takes 5 less).
     const int lane = threadIdx.x & 31;
     const int before = __shfl_up_sync(FULL_MASK, linear, 1);
     const bool scattered = __all_sync(FULL_MASK, lane == 0 || before != linear) != 0;
@@ -2371,12 +2372,15 @@ using CanonicalRows = RowShape<true, 896, 4>;
 using CanonicalRowsWide = RowShape<true, 2048, 2>;
 
 /// Ranks the candidates of a unit by their indices (images of one point, which a row never has
-/// two of, in any order): sh.ordering.key[0 ... n) -> sh.rank and sh.order. Buckets of equal width between the smallest and the largest index, counted
-/// and scanned; a candidate's rank is the start of its bucket plus the smaller ones inside it. The
-/// indices around a unit are either scattered (a bucket holds one or two) or come in runs (crystals
-/// in lattice order: about a dozen), so this takes a third of the instructions of a bitonic sort of
-/// the same keys, and no more when all fall into one bucket. Starts behind a barrier that follows
-/// the writes of the keys, least and most, and ends with one.
+/// two of, in any order): sh.ordering.key[0 ... n) -> sh.rank and sh.order. Buckets of equal width
+/// between the smallest and the largest index, counted and scanned; a candidate's rank is the start
+/// of its bucket plus the smaller ones inside it. The indices around a unit are either scattered (a
+/// bucket holds one or two) or come in runs (crystals in lattice order: about a dozen), and this then
+/// takes a third of the instructions of a bitonic sort of the same keys. Comparisons grow with the
+/// square of what a bucket holds: neighbouring indices with a few far away ones share few buckets.
+/// 512k crystal in blocks of 14 A, row kernel 1247 us, with one atom in 20 at the end of the order
+/// 1410; sorting the rows behind the kernel took 2018. Starts behind a barrier that follows the writes
+/// of the keys, least and most, and ends with one.
 template <class Shape>
 __device__ __forceinline__ void rank_candidates(typename Shape::Shared& sh, int n) {
     auto& o = sh.ordering;

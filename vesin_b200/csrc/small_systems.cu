@@ -13,7 +13,7 @@
 // at a time through the coalesced stores of the large-system kernels. Walking
 // the (i, j) of the flattened triangle instead, a square root and a few
 // corrections per candidate, the 16 384 molecules of 16 to 64 atoms (float, 5.3 M
-// pairs) took 64 us to count and 120 us to write; now 23 and 64 (the 230 MB of the
+// pairs) took 64 us to count and 120 us to write; now 21 and 63 (the 230 MB of the
 // list take 35 us at the copy bandwidth: half the time is the chain of a warp,
 // points -> decisions -> list -> stores).
 //
@@ -516,8 +516,8 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
 // (box, points, scan, stage) for the few thousand tiles that a batch of
 // hundreds of cells has; the work itself is the emission of the hits.
 // Several CTAs share the tiles of a system when the systems alone would not
-// fill the GPU. 512 cells of 4 to 200 atoms (5 A cutoff, 2.7 M pairs): 56 us to
-// count and 107 us to write; exact arithmetic on every image of every pair, a CTA
+// fill the GPU. 512 cells of 4 to 200 atoms (5 A cutoff, 2.7 M pairs): 49 us to
+// count and 101 us to write; exact arithmetic on every image of every pair, a CTA
 // per system, took 640 and 954.
 
 constexpr int SMALL_CHUNK = SMALL_THREADS; // points whose images are listed at a time
