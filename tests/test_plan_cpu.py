@@ -184,3 +184,49 @@ def test_slab_window(planner):
         planner(box, periodic, [0, 0, 0], [40, 50, 120], 1000, 6.0, slab=(2, 0.0, 0.04), n_owned=10)
     with pytest.raises(RuntimeError, match="longer than the box"):
         planner(np.diag([40.0, 50.0, 20.0]), periodic, [0, 0, 0], [40, 50, 20], 1000, 6.0, slab=(2, 0.0, 0.5), n_owned=10)
+
+
+def _screen_value(home, candidate):
+    """The squared distance as the pair passes evaluate it in fp32: coordinates relative to the unit
+    centre, |c|^2 + |i|^2 - 2 c.i term by term (the kernels fuse products and sums, one rounding less each)."""
+    f = np.float32
+    h, c = home.astype(f), candidate.astype(f)
+    norm = lambda v: f(f(v[:, 0] * v[:, 0]) + f(v[:, 1] * v[:, 1])) + f(v[:, 2] * v[:, 2])
+    total = norm(c) + norm(h)
+    for k in (2, 1, 0):
+        total = total + c[:, k] * (f(-2.0) * h[:, k])
+    return total.astype(np.float64)
+
+
+@pytest.mark.parametrize("n_points,length", [(1000, 18.0), (30000, 60.0), (40, 40.0), (8, 200.0), (500, 4.0)])
+def test_screen_band_covers_the_rounding(planner, n_points, length):
+    """What the fp32 screen decides must be what fp64 decides: candidates near the cutoff are off by
+    less than half the band, candidates anywhere else are on the right side of its middle."""
+    rng = np.random.default_rng(n_points)
+    for _ in range(20):
+        box = _random_box(rng, length)
+        cutoff = float(rng.uniform(3.0, 7.0))
+        try:
+            plan = planner(box, np.array([True, True, True]), np.zeros(3), np.zeros(3), n_points, cutoff)
+        except RuntimeError:
+            continue
+        cells = np.array(plan.cell_vec).reshape(3, 3)
+        unit = cells * np.array([plan.pencil, 1, 1])[:, None]
+        n = 4000
+        corners = rng.integers(0, 2, (n, 3)) - 0.5
+        inside = np.where(rng.random((n, 1)) < 0.5, corners, rng.random((n, 3)) - 0.5)
+        home = inside @ unit
+        direction = rng.normal(size=(n, 3))
+        direction /= np.linalg.norm(direction, axis=1)[:, None]
+        middle = 0.5 * (plan.cutoff2_lo + plan.cutoff2_hi)
+        half = 0.5 * (plan.cutoff2_hi - plan.cutoff2_lo)
+        if plan.cutoff2_lo <= 0.0:
+            continue  # nothing is decided in fp32
+        for distance in (cutoff, cutoff * rng.uniform(0.9, 1.1, n), cutoff * rng.uniform(1.1, 6.0, n), cutoff * rng.uniform(0.0, 0.9, n)):
+            candidate = home + direction * np.reshape(distance, (-1, 1))
+            exact = ((candidate - home) ** 2).sum(axis=1)
+            screened = _screen_value(home, candidate)
+            near = np.abs(exact - plan.cutoff2) < 0.21 * plan.cutoff2
+            assert np.all(np.abs(screened - exact)[near] < 0.5 * half)
+            decided = np.abs(screened - middle) > half
+            assert np.array_equal(screened[decided] < middle, exact[decided] < plan.cutoff2)
