@@ -1527,7 +1527,6 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
     }
     const int run = (splits > 1) ? claimed / splits : claimed;
     const int share = (splits > 1) ? claimed - run * splits : 0;
-    int batch_counter = 0;
     const int run_first = (run < n_runs0) ? ranges.begin0 + run * UNIT_RUN : ranges.begin1 + (run - n_runs0) * UNIT_RUN;
     const int run_end = min((run < n_runs0) ? ranges.end0 : ranges.end1, run_first + UNIT_RUN);
     Unit unit = unit_of(plan, cell_start, run_first);
@@ -1583,6 +1582,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
         }
 
         PHASE_MARK(0); // unit setup
+        int batches_before = 0; // of the earlier groups of segments
         for (int g = 0; g < n_groups; g++) {
             int home_row_slots;
             const int group_total = setup_half_segments<SLAB>(plan, cell_start, unit, g, sh, home_row_slots);
@@ -1599,17 +1599,13 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                 }
                 // visible after the barrier that ends the staging of the first batch
             }
-            for (int batch0 = 0; batch0 < group_total; batch0 += Shape::BATCH) {
+            // (the CTAs that share a unit take its batches in turn: looking at every batch for whose it is
+            // took a 64-atom cell with 63 batches 6 us of 31)
+            const int first_batch = (splits > 1) ? (share + splits - batches_before % splits) % splits : 0;
+            batches_before += (group_total + Shape::BATCH - 1) / Shape::BATCH;
+            for (int batch0 = first_batch * Shape::BATCH; batch0 < group_total; batch0 += splits * Shape::BATCH) {
                 const int batch_slots = min(Shape::BATCH, group_total - batch0);
                 const int batch_words = (batch_slots + 31) >> 5;
-                if (splits > 1) {
-                    // the same decision in every thread of the CTA
-                    const bool mine = (batch_counter % splits) == share;
-                    batch_counter++;
-                    if (!mine) {
-                        continue;
-                    }
-                }
 
                 if (SLAB && FULL) {
                     // which slots of the batch hold owned points: every owned segment marks its range
