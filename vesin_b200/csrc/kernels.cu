@@ -2049,7 +2049,10 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
 /// Shared memory of the deciding pass. It writes no pairs, so it holds what the screen reads and
 /// little else; the few candidates that the screen can not decide are fetched again from the
 /// cell-sorted records. 1024 candidates at a time: the 600 or so of a unit of a dense crystal are
-/// one batch.
+/// one batch. What bounds the pass is the latency of the chain of a unit (segments, staging,
+/// decisions, words, counts) and its barriers, so 8 CTAs of 4 warps share an SM instead of 4 of 8,
+/// and the claim of storage is on its way while the candidates are staged: 216k crystal 156 -> 127
+/// us, 262k liquid 146 -> 118, its half list 250 -> 193.
 struct RowCountShared {
     static constexpr int BATCH = 1024;
     static constexpr int WORDS = BATCH / 32;
@@ -2096,8 +2099,12 @@ __device__ __forceinline__ int row_words_of_unit(
     return words;
 }
 
+constexpr int ROW_COUNT_THREADS = 128;
+constexpr int ROW_COUNT_WARPS = ROW_COUNT_THREADS / 32;
+constexpr int ROW_COUNT_CTAS = 8; // per SM
+
 template <bool FULL>
-__global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
+__global__ void __launch_bounds__(ROW_COUNT_THREADS, ROW_COUNT_CTAS) row_count_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, uint32_t* __restrict__ masks,
     unsigned long long mask_capacity, unsigned long long* __restrict__ unit_mask_base, uint32_t* __restrict__ unit_words,
     uint32_t* __restrict__ row_count, DeviceHeader* header
@@ -2132,25 +2139,14 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
         int group_total = 0;
         const int words = row_words_of_unit(plan, cell_start, unit, n_groups, sh.table, group_total);
         most_candidates = max(most_candidates, (n_groups == 1) ? static_cast<unsigned>(group_total) : 0xffffffffu);
-        // claim the storage of the hit words: n_tiles blocks of `words` x 32 lanes
+        // claim the storage of the hit words: n_tiles blocks of `words` x 32 lanes. The answer is not
+        // looked at before the first candidates have been staged
+        const unsigned long long need = static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS;
+        unsigned long long base = 0;
         if (threadIdx.x == 0) {
-            const unsigned long long need = static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS;
-            unsigned long long base = atomicAdd(&header->mask_cursor, need);
-            if (base + need > mask_capacity) {
-                atomicOr(&header->status, STATUS_MASK_OVERFLOW);
-                base = ~0ull;
-            } else {
-                unit_mask_base[u] = base;
-                unit_words[u] = static_cast<uint32_t>(words);
-            }
-            sh.mask_base = base;
+            base = atomicAdd(&header->mask_cursor, need);
         }
-        __syncthreads();
-        const unsigned long long base = sh.mask_base;
-        if (base == ~0ull) {
-            __syncthreads();
-            continue; // the host grows the storage and runs the pass again
-        }
+        bool base_known = false;
 
         // the unit's own cells open the entries own_entry ... of the stencil: the slot of a home
         // point among the candidates is the slot of its first cell plus its number in the unit
@@ -2176,7 +2172,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                     unpack_segment_image(sh.table.image[t], r0, r1, r2);
                     return make_int4(r0 - record.s0, r1 - record.s1, r2 - record.s2, record.index);
                 };
-                for (int s = threadIdx.x; s < 32 * batch_words; s += CTA_THREADS) {
+                for (int s = threadIdx.x; s < 32 * batch_words; s += ROW_COUNT_THREADS) {
                     float fx = 0.0f, fy = 0.0f, fz = 0.0f;
                     float norm = __int_as_float(0x7f800000); // past the end: never a hit
                     if (s < batch_slots) {
@@ -2204,6 +2200,19 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                     sh.near_n[s] = norm;
                 }
 
+                if (!base_known) {
+                    if (threadIdx.x == 0) {
+                        if (base + need > mask_capacity) {
+                            // the host grows the storage and runs the pass again
+                            atomicOr(&header->status, STATUS_MASK_OVERFLOW);
+                            base = ~0ull;
+                        } else {
+                            unit_mask_base[u] = base;
+                            unit_words[u] = static_cast<uint32_t>(words);
+                        }
+                        sh.mask_base = base;
+                    }
+                }
                 for (int tile = 0; tile < n_tiles; tile++) {
                     __syncthreads(); // staging done; previous tile done with the hit words and the home points
                     const int il = tile * TILE_POINTS + lane;
@@ -2240,14 +2249,14 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                                plan.cutoff2;
                     };
                     // (no half shell here: home_row_slots = 0 keeps every candidate)
-                    if (batch_words <= CTA_WARPS) {
+                    if (batch_words <= ROW_COUNT_WARPS) {
                         if (warp < batch_words) {
                             sh.mask[warp * TILE_POINTS + lane] =
                                 decide_piece<32>(sh, warp, 0, batch0, 0, il, ax2, ay2, az2, an2, screen.half, exact);
                         }
                     } else {
                         unsigned short* halves = reinterpret_cast<unsigned short*>(sh.mask);
-                        for (int piece = warp; piece < 2 * batch_words; piece += CTA_WARPS) {
+                        for (int piece = warp; piece < 2 * batch_words; piece += ROW_COUNT_WARPS) {
                             const int half = (piece >= batch_words) ? 1 : 0;
                             const int w = piece - half * batch_words;
                             halves[2 * (w * TILE_POINTS + lane) + half] = static_cast<unsigned short>(
@@ -2259,12 +2268,15 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                     // ---- indices and shifts have their say on the hits; the words go to global
                     //      memory as [tile][word][lane], the counts to the rows. A thread meets the
                     //      same home point in all of its tasks (256 is a multiple of 32). ----
+                    base_known = true;
+                    base = sh.mask_base;
+                    const bool fits = base != ~0ull;
                     uint32_t* mask_tile = masks + base + (static_cast<unsigned long long>(tile) * words + word_base + (batch0 >> 5)) * TILE_POINTS;
                     const int4 home = sh.home_sj[lane];
                     // full lists: the only candidate to drop is the point itself, whose slot is known
                     const int self_bit = (g == own_group) ? own_slot0 + tile * TILE_POINTS + lane - batch0 : -1;
                     int my_hits = 0;
-                    for (int task = threadIdx.x; task < batch_words * TILE_POINTS; task += CTA_THREADS) {
+                    for (int task = threadIdx.x; task < batch_words * TILE_POINTS; task += ROW_COUNT_THREADS) {
                         unsigned word = sh.mask[task];
                         unsigned kept = word;
                         const int slot0 = (task >> 5) << 5;
@@ -2289,7 +2301,9 @@ __global__ void __launch_bounds__(CTA_THREADS, 4) row_count_kernel(
                                 }
                             }
                         }
-                        mask_tile[task] = kept;
+                        if (fits) {
+                            mask_tile[task] = kept;
+                        }
                         my_hits += __popc(kept);
                     }
                     if (my_hits != 0) {
@@ -3101,13 +3115,13 @@ void launch_count(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, uint32_t* masks, unsigned long long mask_capacity,
     unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, cudaStream_t stream
 ) {
-    const int grid = pair_grid(plan.n_units, 4);
+    const int grid = pair_grid(plan.n_units, ROW_COUNT_CTAS);
     if (plan.full) {
-        row_count_kernel<true><<<grid, CTA_THREADS, 0, stream>>>(
+        row_count_kernel<true><<<grid, ROW_COUNT_THREADS, 0, stream>>>(
             plan, cell_start, sorted, masks, mask_capacity, unit_mask_base, unit_words, row_count, header
         );
     } else {
-        row_count_kernel<false><<<grid, CTA_THREADS, 0, stream>>>(
+        row_count_kernel<false><<<grid, ROW_COUNT_THREADS, 0, stream>>>(
             plan, cell_start, sorted, masks, mask_capacity, unit_mask_base, unit_words, row_count, header
         );
     }
