@@ -138,6 +138,7 @@ struct Workspace {
         double cutoff = 0.0;
         bool full = false;
         bool sorted = false;
+        int ranked_batch = -1; // canonical lists: room pass 1 needs to rank the candidates of a unit, 0 if it can not, -1 if not known
         GridPlan plan{};
     } cache;
 
@@ -815,6 +816,7 @@ void neighbors(
         cache.cutoff = options.cutoff;
         cache.full = options.full;
         cache.sorted = options.sorted;
+        cache.ranked_batch = -1;
         cache.valid = true;
     };
 
@@ -996,14 +998,28 @@ void neighbors(
         ws.unit_words.reserve(n_units * sizeof(uint32_t));
         ws.row_start.reserve((n_points + 1) * sizeof(unsigned long long));
         ws.row_fill.reserve(n_points * sizeof(uint32_t));
+        // a second index can come twice in a row only with two images of the same point
+        // within the cutoff of the first: a lattice vector shorter than twice the cutoff
+        bool duplicates_possible = false;
+        for (int k = 0; k < 3; k++) {
+            duplicates_possible = duplicates_possible || (plan.periodic[k] && plan.face_dist[k] < 2.0 * options.cutoff * (1.0 + 1e-9));
+        }
+        const double per_cell = static_cast<double>(n_points) / static_cast<double>(n_cells);
+        const double stencil_cells = (plan.pencil + 2.0 * plan.n_search[0]) * (2.0 * plan.n_search[1] + 1.0) * (2.0 * plan.n_search[2] + 1.0);
+        // Canonical lists: the deciding pass ranks the candidates of a unit by their indices when it can
+        // hold all of them, and the rows then come out in their final order. Whether it can is seen when
+        // it has run (the first time: a fifth more than the average unit has); the next builds know.
+        int& ranked_batch = ws.cache.ranked_batch;
+        if (ranked_batch < 0) {
+            ranked_batch = ranked_count_batch(1.2 * per_cell * stencil_cells);
+        }
+        int ranked = (canonical && !duplicates_possible) ? ranked_batch : 0;
         if (ws.masks.bytes == 0) {
             // first guess for the hit-mask storage: uniform density. Every unit
             // stores (tiles of 32 lanes) x (words per home point).
-            double per_cell = static_cast<double>(n_points) / static_cast<double>(n_cells);
-            double stencil_cells = (plan.pencil + 2.0 * plan.n_search[0]) * (2.0 * plan.n_search[1] + 1.0) * (2.0 * plan.n_search[2] + 1.0);
             double words = per_cell * stencil_cells / 32.0 + 1.5;
             double lanes = static_cast<double>(n_units) * 32.0 * std::ceil(per_cell * plan.pencil / 32.0 + 0.35);
-            double guess = std::min(1.2 * words * lanes * sizeof(uint32_t), 2.0e9);
+            double guess = std::min((ranked != 0 ? 1.8 : 1.2) * words * lanes * sizeof(uint32_t), 2.0e9);
             ws.masks.reserve(static_cast<size_t>(guess) + 1024);
         }
 
@@ -1015,7 +1031,7 @@ void neighbors(
             }
             launch_count(
                 plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.masks.bytes / sizeof(uint32_t),
-                ws.unit_mask_base.as<unsigned long long>(), ws.unit_words.as<uint32_t>(), ws.row_count.as<uint32_t>(), ws.d_header, stream
+                ws.unit_mask_base.as<unsigned long long>(), ws.unit_words.as<uint32_t>(), ws.row_count.as<uint32_t>(), ws.d_header, ranked, stream
             );
             timer.end(VesinB200StageCount);
             timer.begin(VesinB200StageScanRows);
@@ -1035,13 +1051,17 @@ void neighbors(
             }
             timer.collect(VesinB200StageCount);
             timer.collect(VesinB200StageScanRows);
-            if ((header.status & STATUS_MASK_OVERFLOW) == 0) {
+            const bool refused_ranks = ranked != 0 && header.max_candidates > static_cast<unsigned>(ranked);
+            if ((header.status & STATUS_MASK_OVERFLOW) == 0 && !refused_ranks) {
                 break;
             }
-            if (attempt >= 2) {
+            if (attempt >= 4) {
                 throw std::runtime_error("internal error: hit-mask storage kept overflowing");
             }
-            // the cursor holds the exact requirement: grow and decide again
+            if (refused_ranks) {
+                ranked = ranked_batch = ranked_count_batch(static_cast<double>(header.max_candidates));
+            }
+            // the cursor holds the exact requirement (of the units that were decided): grow and decide again
             size_t wanted = static_cast<size_t>(header.mask_cursor) * sizeof(uint32_t);
             ws.masks.reserve(wanted + wanted / 16 + 1024);
             size_t offset = offsetof(DeviceHeader, total_pairs);
@@ -1061,16 +1081,9 @@ void neighbors(
         }
         if (total > 0) {
             const PairOutput out = target.view();
-            // a second index can come twice in a row only with two images of the same point
-            // within the cutoff of the first: a lattice vector shorter than twice the cutoff
-            bool duplicates_possible = false;
-            for (int k = 0; k < 3; k++) {
-                duplicates_possible = duplicates_possible || (plan.periodic[k] && plan.face_dist[k] < 2.0 * options.cutoff * (1.0 + 1e-9));
-            }
-            const int canonical_batch = canonical ? canonical_emit_batch(header.max_candidates, duplicates_possible) : 0;
             // a canonical list whose rows can not be written in their final order: they go to a second set
             // of arrays first, from where they are sorted into the list's
-            const bool sort_behind = canonical && canonical_batch == 0;
+            const bool sort_behind = canonical && ranked == 0;
             PairOutput rows = out;
             if (sort_behind) {
                 ws.alt_pairs.reserve(total * 2 * sizeof(size_t));
@@ -1092,12 +1105,12 @@ void neighbors(
                 }
             }
             timer.begin(VesinB200StageEmit);
-            if (header.max_candidates > static_cast<unsigned>(row_batch(canonical_batch))) {
+            if (header.max_candidates > static_cast<unsigned>(row_batch(header.max_candidates))) {
                 VB200_CUDA(cudaMemsetAsync(ws.row_fill.ptr, 0, n_points * sizeof(uint32_t), stream));
             }
             launch_emit(
                 plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.unit_mask_base.as<unsigned long long>(),
-                ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), rows, canonical_batch, stream
+                ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), rows, header.max_candidates, ranked != 0, stream
             );
             if (sort_behind) {
                 launch_sort_rows(ws.row_start.as<unsigned long long>(), n_points, rows, out, duplicates_possible, stream);

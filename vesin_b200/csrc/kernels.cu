@@ -97,15 +97,26 @@ struct LoadedRecord {
 
 /// The whole record in one 256-bit load. (volatile: not moved above the wait for the kernel
 /// that wrote the records)
-__device__ __forceinline__ LoadedRecord load_record(const SortedPoints& sorted, size_t p) {
+__device__ __forceinline__ PointRecord load_packed_record(const SortedPoints& sorted, size_t p) {
     long long a, b, c, d;
     asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(sorted.records + p));
-    LoadedRecord record;
+    PointRecord record;
     record.x = __longlong_as_double(a);
     record.y = __longlong_as_double(b);
     record.z = __longlong_as_double(c);
     record.index = static_cast<int>(d & 0xffffffffll);
-    const uint32_t packed = static_cast<uint32_t>(static_cast<unsigned long long>(d) >> 32);
+    record.shift = static_cast<uint32_t>(static_cast<unsigned long long>(d) >> 32);
+    return record;
+}
+
+__device__ __forceinline__ LoadedRecord load_record(const SortedPoints& sorted, size_t p) {
+    const PointRecord loaded = load_packed_record(sorted, p);
+    LoadedRecord record;
+    record.x = loaded.x;
+    record.y = loaded.y;
+    record.z = loaded.z;
+    record.index = loaded.index;
+    const uint32_t packed = loaded.shift;
     record.s0 = static_cast<int>(packed & 1023u) - WRAP_BIAS;
     record.s1 = static_cast<int>((packed >> 10) & 1023u) - WRAP_BIAS;
     record.s2 = static_cast<int>((packed >> 20) & 1023u) - WRAP_BIAS;
@@ -2046,6 +2057,110 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
 // in the order the candidates were staged.
 // ---------------------------------------------------------------------------
 
+constexpr int RANK_BUCKETS = 2048; // see rank_candidates (216k crystal, ranking kernel of 8 warps: 1024 527 us, 2048 513, 4096 534)
+constexpr int RANKED_HOME = 256;   // home points of a unit whose candidates are ranked, at most
+
+/// What ranking the candidates of a unit needs, before they are staged.
+template <int BATCH>
+struct Ordering {
+    unsigned key[BATCH];          // index of the candidate in a slot
+    unsigned gathered[BATCH];     // the same, bucket by bucket
+    int first[RANK_BUCKETS + 1];  // candidates in a bucket, then where the bucket starts
+    unsigned least, most;
+};
+
+/// Ranks the candidates of a unit by their indices (images of one point, which a row never has
+/// two of, in any order): o.key[0 ... n) -> order, the slots in the order of the indices. Buckets of equal width
+/// between the smallest and the largest index, counted and scanned; a candidate's rank is the start
+/// of its bucket plus the smaller ones inside it. The indices around a unit are either scattered (a
+/// bucket holds one or two) or come in runs (crystals in lattice order: about a dozen), and this then
+/// takes a third of the instructions of a bitonic sort of the same keys. Comparisons grow with the
+/// square of what a bucket holds: neighbouring indices with a few far away ones share few buckets.
+/// 512k crystal in blocks of 14 A, when the row kernel ranked 1247 us, with one atom in 20 at the end of the order
+/// 1410; sorting the rows behind the kernel took 2018. Starts behind a barrier that follows the writes
+/// of the keys, least and most, and ends with one.
+template <int THREADS, int BATCH>
+__device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tmp, unsigned short* order, int n) {
+    constexpr int WARPS = THREADS / 32;
+    constexpr int PER_THREAD = (BATCH + THREADS - 1) / THREADS;
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    // (rounding is monotonic: a larger index never falls into an earlier bucket)
+    const float scale = static_cast<float>(RANK_BUCKETS) / (static_cast<float>(o.most - o.least) + 1.0f);
+    const unsigned least = o.least;
+    const auto bucket_of = [&](unsigned key) { return min(static_cast<int>(static_cast<float>(key - least) * scale), RANK_BUCKETS - 1); };
+    int arrival[PER_THREAD];
+#pragma unroll
+    for (int e = 0; e < PER_THREAD; e++) {
+        const int s = threadIdx.x + e * THREADS;
+        if (s < n) {
+            arrival[e] = atomicAdd(&o.first[bucket_of(o.key[s])], 1);
+        }
+    }
+    __syncthreads();
+    constexpr int SCAN = RANK_BUCKETS / THREADS;
+    int counts[SCAN];
+    int mine = 0;
+#pragma unroll
+    for (int e = 0; e < SCAN; e++) {
+        counts[e] = o.first[threadIdx.x * SCAN + e];
+        mine += counts[e];
+    }
+    int inclusive = mine;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+        const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
+        if (lane >= offset) {
+            inclusive += up;
+        }
+    }
+    if (lane == 31) {
+        scan_tmp[warp] = inclusive;
+    }
+    __syncthreads();
+    int start = inclusive - mine;
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) {
+        start += (w < warp) ? scan_tmp[w] : 0;
+    }
+#pragma unroll
+    for (int e = 0; e < SCAN; e++) {
+        o.first[threadIdx.x * SCAN + e] = start;
+        start += counts[e];
+    }
+    if (threadIdx.x == 0) {
+        o.first[RANK_BUCKETS] = n;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < PER_THREAD; e++) {
+        const int s = threadIdx.x + e * THREADS;
+        if (s < n) {
+            const unsigned key = o.key[s];
+            o.gathered[o.first[bucket_of(key)] + arrival[e]] = key;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < PER_THREAD; e++) {
+        const int s = threadIdx.x + e * THREADS;
+        if (s < n) {
+            const unsigned key = o.key[s];
+            const int bucket = bucket_of(key);
+            const int first = o.first[bucket];
+            const int last = o.first[bucket + 1];
+            const int mine = first + arrival[e];
+            int place = first;
+            for (int k = first; k < last; k++) {
+                const unsigned other = o.gathered[k];
+                place += (other < key || (other == key && k < mine)) ? 1 : 0;
+            }
+            order[place] = static_cast<unsigned short>(s);
+        }
+    }
+    __syncthreads();
+}
+
 /// Shared memory of the deciding pass. It writes no pairs, so it holds what the screen reads and
 /// little else; the few candidates that the screen can not decide are fetched again from the
 /// cell-sorted records. 1024 candidates at a time: the 600 or so of a unit of a dense crystal are
@@ -2053,20 +2168,36 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
 /// decisions, words, counts) and its barriers, so 8 CTAs of 4 warps share an SM instead of 4 of 8,
 /// and the claim of storage is on its way while the candidates are staged: 216k crystal 156 -> 127
 /// us, 262k liquid 146 -> 118, its half list 250 -> 193.
-struct RowCountShared {
-    static constexpr int BATCH = 1024;
-    static constexpr int WORDS = BATCH / 32;
-    SegmentTable table;
-    alignas(16) float near_x[BATCH]; // relative to the unit centre, read as 16-byte vectors
-    alignas(16) float near_y[BATCH];
-    alignas(16) float near_z[BATCH];
-    alignas(16) float near_n[BATCH];
-    int index[BATCH];                   // half lists: indices of the candidates
-    int4 home_sj[TILE_POINTS];          // x, y, z: wrap shift of the home point; w: its index
-    unsigned mask[WORDS * TILE_POINTS]; // [word][lane]
-    double centre[3];                   // centre of the unit: origin of the fp32 local frame
-    int tile_hits[TILE_POINTS];         // hits of the home points of the tile in the current batch
-    unsigned long long mask_base;
+/// RANKED: the candidates of a unit, which all fit a batch, are staged in the order of their indices.
+template <bool FULL_, bool RANKED_, int BATCH_, int CTAS_PER_SM_>
+struct RowCountShape {
+    static constexpr bool FULL = FULL_;
+    static constexpr bool RANKED = RANKED_;
+    static constexpr int BATCH = BATCH_;
+    static constexpr int WORDS = BATCH_ / 32;
+    static constexpr int CTAS_PER_SM = CTAS_PER_SM_;
+    struct Nothing {};
+    struct Shared {
+        union {
+            struct {
+                alignas(16) float near_x[BATCH_]; // relative to the unit centre, read as 16-byte vectors
+                alignas(16) float near_y[BATCH_];
+                alignas(16) float near_z[BATCH_];
+                alignas(16) float near_n[BATCH_];
+            };
+            typename std::conditional<RANKED_, Ordering<BATCH_>, Nothing>::type ordering;
+        };
+        SegmentTable table;
+        int index[FULL_ ? 1 : BATCH_];                    // half lists: indices of the candidates
+        int4 home_sj[TILE_POINTS];                        // x, y, z: wrap shift of the home point; w: its index
+        unsigned mask[WORDS * TILE_POINTS];               // [word][lane]
+        double centre[3];                                 // centre of the unit: origin of the fp32 local frame
+        int tile_hits[TILE_POINTS];                       // hits of the home points of the tile in the current batch
+        unsigned long long mask_base;
+        alignas(4) unsigned short order[RANKED_ ? BATCH_ : 2]; // place -> slot
+        unsigned short own_place[RANKED_ ? RANKED_HOME : 2]; // places of the home points among the candidates
+    };
+    static_assert((sizeof(Shared) + 1024) * CTAS_PER_SM_ <= 228 * 1024, "CTAS_PER_SM CTAs fit on an SM");
 };
 
 /// Does the pair (home point, candidate) belong to the list, as far as indices
@@ -2101,16 +2232,19 @@ __device__ __forceinline__ int row_words_of_unit(
 
 constexpr int ROW_COUNT_THREADS = 128;
 constexpr int ROW_COUNT_WARPS = ROW_COUNT_THREADS / 32;
-constexpr int ROW_COUNT_CTAS = 8; // per SM
 
-template <bool FULL>
-__global__ void __launch_bounds__(ROW_COUNT_THREADS, ROW_COUNT_CTAS) row_count_kernel(
+template <class Shape>
+__global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_count_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, uint32_t* __restrict__ masks,
     unsigned long long mask_capacity, unsigned long long* __restrict__ unit_mask_base, uint32_t* __restrict__ unit_words,
     uint32_t* __restrict__ row_count, DeviceHeader* header
 ) {
-    __shared__ RowCountShared sh;
-    constexpr int BATCH = RowCountShared::BATCH;
+    using Shared = typename Shape::Shared;
+    constexpr int BATCH = Shape::BATCH;
+    constexpr bool FULL = Shape::FULL;
+    constexpr bool RANKED = Shape::RANKED;
+    extern __shared__ __align__(16) unsigned char row_count_smem[];
+    Shared& sh = *reinterpret_cast<Shared*>(row_count_smem);
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -2138,10 +2272,20 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, ROW_COUNT_CTAS) row_count_k
 
         int group_total = 0;
         const int words = row_words_of_unit(plan, cell_start, unit, n_groups, sh.table, group_total);
-        most_candidates = max(most_candidates, (n_groups == 1) ? static_cast<unsigned>(group_total) : 0xffffffffu);
-        // claim the storage of the hit words: n_tiles blocks of `words` x 32 lanes. The answer is not
+        if (RANKED) {
+            const bool rankable = n_groups == 1 && unit.n_home <= RANKED_HOME;
+            most_candidates = max(most_candidates, rankable ? static_cast<unsigned>(group_total) : 0xffffffffu);
+            if (!rankable || group_total > BATCH) {
+                __syncthreads(); // (the table has been read)
+                continue; // the host runs the pass again without ranks, or with room for more candidates
+            }
+        } else {
+            most_candidates = max(most_candidates, (n_groups == 1) ? static_cast<unsigned>(group_total) : 0xffffffffu);
+        }
+        // claim the storage of the hit words: n_tiles blocks of `words` x 32 lanes, and behind them the
+        // slots of ranked candidates in their order, two to a word. The answer is not
         // looked at before the first candidates have been staged
-        const unsigned long long need = static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS;
+        const unsigned long long need = static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS + (RANKED ? words * 16 : 0);
         unsigned long long base = 0;
         if (threadIdx.x == 0) {
             base = atomicAdd(&header->mask_cursor, need);
@@ -2164,14 +2308,46 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, ROW_COUNT_CTAS) row_count_k
                 const int batch_words = (batch_slots + 31) >> 5;
                 // candidate in a slot of the batch, as it lies in the cell-sorted records: image
                 // minus wrap shift and index
+                const auto position_of = [&](int slot, int& t) {
+                    t = (unit.n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
+                    return static_cast<size_t>(sh.table.start[t]) + (slot - sh.table.slot0[t]);
+                };
                 const auto fetch = [&](int s, LoadedRecord& record) {
-                    const int slot = batch0 + s;
-                    const int t = (unit.n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
-                    record = load_record(sorted, static_cast<size_t>(sh.table.start[t]) + (slot - sh.table.slot0[t]));
+                    int t;
+                    record = load_record(sorted, position_of(RANKED ? static_cast<int>(sh.order[s]) : batch0 + s, t));
                     int r0, r1, r2;
                     unpack_segment_image(sh.table.image[t], r0, r1, r2);
                     return make_int4(r0 - record.s0, r1 - record.s1, r2 - record.s2, record.index);
                 };
+                if constexpr (RANKED) {
+                    // (the only batch of the unit)
+                    for (int k = threadIdx.x; k < RANK_BUCKETS; k += ROW_COUNT_THREADS) {
+                        sh.ordering.first[k] = 0;
+                    }
+                    if (threadIdx.x == 0) {
+                        sh.ordering.least = 0xffffffffu;
+                        sh.ordering.most = 0u;
+                    }
+                    __syncthreads();
+                    unsigned least = 0xffffffffu;
+                    unsigned most = 0u;
+#pragma unroll 4
+                    for (int s = threadIdx.x; s < batch_slots; s += ROW_COUNT_THREADS) {
+                        int t;
+                        const unsigned key = static_cast<unsigned>(sorted.records[position_of(s, t)].index);
+                        sh.ordering.key[s] = key;
+                        least = min(least, key);
+                        most = max(most, key);
+                    }
+                    least = __reduce_min_sync(FULL_MASK, least);
+                    most = __reduce_max_sync(FULL_MASK, most);
+                    if (lane == 0 && least <= most) {
+                        atomicMin(&sh.ordering.least, least);
+                        atomicMax(&sh.ordering.most, most);
+                    }
+                    __syncthreads();
+                    rank_candidates<ROW_COUNT_THREADS>(sh.ordering, sh.table.scan_tmp, sh.order, batch_slots);
+                }
                 for (int s = threadIdx.x; s < 32 * batch_words; s += ROW_COUNT_THREADS) {
                     float fx = 0.0f, fy = 0.0f, fz = 0.0f;
                     float norm = __int_as_float(0x7f800000); // past the end: never a hit
@@ -2192,6 +2368,12 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, ROW_COUNT_CTAS) row_count_k
                         norm = fx * fx + fy * fy + fz * fz;
                         if (!FULL) {
                             sh.index[s] = cand.w;
+                        }
+                        if (RANKED) {
+                            const int own = static_cast<int>(sh.order[s]) - own_slot0;
+                            if (own >= 0 && own < unit.n_home) {
+                                sh.own_place[own] = static_cast<unsigned short>(s);
+                            }
                         }
                     }
                     sh.near_x[s] = fx;
@@ -2274,7 +2456,17 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, ROW_COUNT_CTAS) row_count_k
                     uint32_t* mask_tile = masks + base + (static_cast<unsigned long long>(tile) * words + word_base + (batch0 >> 5)) * TILE_POINTS;
                     const int4 home = sh.home_sj[lane];
                     // full lists: the only candidate to drop is the point itself, whose slot is known
-                    const int self_bit = (g == own_group) ? own_slot0 + tile * TILE_POINTS + lane - batch0 : -1;
+                    int self_bit = (g == own_group) ? own_slot0 + tile * TILE_POINTS + lane - batch0 : -1;
+                    if (RANKED) {
+                        self_bit = sh.own_place[min(tile * TILE_POINTS + lane, unit.n_home - 1)];
+                    }
+                    if (RANKED && tile == 0 && fits) {
+                        // where the writing pass finds the candidates: two slots to a word
+                        uint32_t* order = masks + base + static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS;
+                        for (int k = threadIdx.x; k < 16 * words; k += ROW_COUNT_THREADS) {
+                            order[k] = reinterpret_cast<const uint32_t*>(sh.order)[k];
+                        }
+                    }
                     int my_hits = 0;
                     for (int task = threadIdx.x; task < batch_words * TILE_POINTS; task += ROW_COUNT_THREADS) {
                         unsigned word = sh.mask[task];
@@ -2332,144 +2524,38 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, ROW_COUNT_CTAS) row_count_k
 // warp, so that every store covers one contiguous span of it)
 
 constexpr int ROW_WINDOW = 128;    // hits of a row a warp lists at a time
-constexpr int RANK_BUCKETS = 2048; // see rank_candidates (216k crystal, row kernel: 1024 527 us, 2048 513, 4096 534)
 
-/// Shape of the CTAs of the row-writing kernel: BATCH candidates are staged at a time.
-/// CANONICAL: all candidates of a unit fit one batch and are staged in the order of their indices.
-template <bool CANONICAL_, int BATCH_, int CTAS_PER_SM_>
+constexpr int ROW_EMIT_THREADS = 128;
+constexpr int ROW_EMIT_WARPS = ROW_EMIT_THREADS / 32;
+
+/// Shape of the CTAs of the row-writing kernel: BATCH candidates are looked at at a time. The
+/// candidates themselves stay in L1, where a lane fetches the record of its hit: staging all of them
+/// first (40 bytes each, which left room for 4 CTAs of 8 warps) was a third of the kernel. 216k
+/// crystal 316 -> 302 us, 262k liquid 250 -> 231, its half list 208 -> 185.
+template <int BATCH_, int CTAS_PER_SM_>
 struct RowShape {
-    static constexpr bool CANONICAL = CANONICAL_;
     static constexpr int BATCH = BATCH_;
     static constexpr int WORDS = BATCH_ / 32;
     static constexpr int LANE_WORDS = (WORDS + 31) / 32; // consecutive words of a row that a lane looks after
     static constexpr int CTAS_PER_SM = CTAS_PER_SM_;
     static_assert(BATCH_ % 32 == 0 && BATCH_ <= 65536, "whole words, slots of 16 bits");
+    static_assert(SEG_MAX <= 256, "segments of 8 bits");
 
-    struct Staged {
-        double x[BATCH_]; // original positions of the candidates
-        double y[BATCH_];
-        double z[BATCH_];
-        int4 sj[BATCH_];  // x, y, z: q - wrap shift of the candidate; w: its index
-    };
-    struct Ordering { // what ranking the candidates needs, before they are staged
-        unsigned key[BATCH_];                 // index of the candidate in a slot
-        unsigned gathered[BATCH_];            // the same, bucket by bucket
-        int first[RANK_BUCKETS + 1];          // candidates in a bucket, then where the bucket starts
-        unsigned least, most;
-    };
     struct Shared {
-        union {
-            Staged staged;
-            Ordering ordering;
-        };
-        union {
-            unsigned mask[TILE_POINTS * (WORDS + 1)]; // [home point][word], padded against bank conflicts
-            unsigned short order[BATCH_];             // place -> slot, until the candidates are staged
-        };
-        alignas(16) double transpose[CTA_WARPS][TRANSPOSE_DOUBLES / 2]; // per warp: on the way to coalesced stores
+        alignas(16) double transpose[ROW_EMIT_WARPS][TRANSPOSE_DOUBLES / 2]; // per warp: on the way to coalesced stores
+        unsigned mask[TILE_POINTS * (WORDS + 1)]; // [home point][word], padded against bank conflicts
+        unsigned short list[ROW_EMIT_WARPS][ROW_WINDOW];
+        int position[BATCH_];           // of the candidate among the cell-sorted points
+        unsigned char segment[BATCH_];  // the segment it comes from
         SegmentTable table;
         double home_pos[3][TILE_POINTS];
         int4 home_sj[TILE_POINTS];                // x, y, z: wrap shift of the home point; w: its index
         unsigned long long home_row[TILE_POINTS]; // where the row of a home point continues
-        unsigned short list[CTA_WARPS][ROW_WINDOW];
-        unsigned short rank[CANONICAL_ ? BATCH_ : 1];                              // slot -> place in the order of the indices
-        unsigned bitmap[CANONICAL_ ? CTA_WARPS : 1][CANONICAL_ ? 32 * LANE_WORDS : 1]; // hits of a row in that order
     };
     static_assert((sizeof(Shared) + 1024) * CTAS_PER_SM_ <= 228 * 1024, "CTAS_PER_SM CTAs fit on an SM");
 };
-using SortedRows = RowShape<false, 1024, 4>;
-using CanonicalRows = RowShape<true, 896, 4>;
-using CanonicalRowsWide = RowShape<true, 2048, 2>;
-
-/// Ranks the candidates of a unit by their indices (images of one point, which a row never has
-/// two of, in any order): sh.ordering.key[0 ... n) -> sh.rank and sh.order. Buckets of equal width
-/// between the smallest and the largest index, counted and scanned; a candidate's rank is the start
-/// of its bucket plus the smaller ones inside it. The indices around a unit are either scattered (a
-/// bucket holds one or two) or come in runs (crystals in lattice order: about a dozen), and this then
-/// takes a third of the instructions of a bitonic sort of the same keys. Comparisons grow with the
-/// square of what a bucket holds: neighbouring indices with a few far away ones share few buckets.
-/// 512k crystal in blocks of 14 A, row kernel 1247 us, with one atom in 20 at the end of the order
-/// 1410; sorting the rows behind the kernel took 2018. Starts behind a barrier that follows the writes
-/// of the keys, least and most, and ends with one.
-template <class Shape>
-__device__ __forceinline__ void rank_candidates(typename Shape::Shared& sh, int n) {
-    auto& o = sh.ordering;
-    constexpr int PER_THREAD = (Shape::BATCH + CTA_THREADS - 1) / CTA_THREADS;
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    // (rounding is monotonic: a larger index never falls into an earlier bucket)
-    const float scale = static_cast<float>(RANK_BUCKETS) / (static_cast<float>(o.most - o.least) + 1.0f);
-    int bucket[PER_THREAD], arrival[PER_THREAD];
-#pragma unroll
-    for (int e = 0; e < PER_THREAD; e++) {
-        const int s = threadIdx.x + e * CTA_THREADS;
-        if (s < n) {
-            bucket[e] = min(static_cast<int>(static_cast<float>(o.key[s] - o.least) * scale), RANK_BUCKETS - 1);
-            arrival[e] = atomicAdd(&o.first[bucket[e]], 1);
-        }
-    }
-    __syncthreads();
-    constexpr int SCAN = RANK_BUCKETS / CTA_THREADS;
-    int counts[SCAN];
-    int mine = 0;
-#pragma unroll
-    for (int e = 0; e < SCAN; e++) {
-        counts[e] = o.first[threadIdx.x * SCAN + e];
-        mine += counts[e];
-    }
-    int inclusive = mine;
-#pragma unroll
-    for (int offset = 1; offset < 32; offset <<= 1) {
-        const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
-        if (lane >= offset) {
-            inclusive += up;
-        }
-    }
-    if (lane == 31) {
-        sh.table.scan_tmp[warp] = inclusive;
-    }
-    __syncthreads();
-    int start = inclusive - mine;
-#pragma unroll
-    for (int w = 0; w < CTA_WARPS; w++) {
-        start += (w < warp) ? sh.table.scan_tmp[w] : 0;
-    }
-#pragma unroll
-    for (int e = 0; e < SCAN; e++) {
-        o.first[threadIdx.x * SCAN + e] = start;
-        start += counts[e];
-    }
-    if (threadIdx.x == 0) {
-        o.first[RANK_BUCKETS] = n;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < PER_THREAD; e++) {
-        const int s = threadIdx.x + e * CTA_THREADS;
-        if (s < n) {
-            o.gathered[o.first[bucket[e]] + arrival[e]] = o.key[s];
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < PER_THREAD; e++) {
-        const int s = threadIdx.x + e * CTA_THREADS;
-        if (s < n) {
-            const unsigned key = o.key[s];
-            const int first = o.first[bucket[e]];
-            const int last = o.first[bucket[e] + 1];
-            const int mine = first + arrival[e];
-            int place = first;
-            for (int k = first; k < last; k++) {
-                const unsigned other = o.gathered[k];
-                place += (other < key || (other == key && k < mine)) ? 1 : 0;
-            }
-            sh.rank[s] = static_cast<unsigned short>(place);
-            sh.order[place] = static_cast<unsigned short>(s);
-        }
-    }
-    __syncthreads();
-}
+using SortedRows = RowShape<1024, 8>;
+using SortedRowsWide = RowShape<2048, 8>;
 
 /// Hits [from, to) of a row whose words lie in shared memory, lane l being the one that counted the
 /// LANE_WORDS words from l * LANE_WORDS on (`begin`: hits before them): use(number, slot) for each,
@@ -2535,10 +2621,10 @@ __device__ __forceinline__ int count_row_hits(const unsigned* words, int n_words
 }
 
 template <class Shape>
-__global__ void __launch_bounds__(CTA_THREADS, Shape::CTAS_PER_SM) row_emit_kernel(
+__global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, const uint32_t* __restrict__ masks,
     const unsigned long long* __restrict__ unit_mask_base, const uint32_t* __restrict__ unit_words,
-    const unsigned long long* __restrict__ row_start, uint32_t* __restrict__ row_fill, PairOutput out
+    const unsigned long long* __restrict__ row_start, uint32_t* __restrict__ row_fill, PairOutput out, const int ranked
 ) {
     using Shared = typename Shape::Shared;
     constexpr int BATCH = Shape::BATCH;
@@ -2572,47 +2658,14 @@ __global__ void __launch_bounds__(CTA_THREADS, Shape::CTAS_PER_SM) row_emit_kern
             for (int batch0 = 0; batch0 < group_total; batch0 += BATCH) {
                 const int batch_slots = min(BATCH, group_total - batch0);
                 const int batch_words = (batch_slots + 31) >> 5;
-                if (Shape::CANONICAL) {
-                    // (the only batch of the unit; the caller made sure of that)
-                    for (int k = threadIdx.x; k < RANK_BUCKETS; k += CTA_THREADS) {
-                        sh.ordering.first[k] = 0;
-                    }
-                    if (threadIdx.x == 0) {
-                        sh.ordering.least = 0xffffffffu;
-                        sh.ordering.most = 0u;
-                    }
-                    __syncthreads();
-                    unsigned least = 0xffffffffu;
-                    unsigned most = 0u;
-#pragma unroll 4
-                    for (int s = threadIdx.x; s < batch_slots; s += CTA_THREADS) {
-                        int t;
-                        const unsigned key = static_cast<unsigned>(sorted.records[record_of(s, t)].index);
-                        sh.ordering.key[s] = key;
-                        least = min(least, key);
-                        most = max(most, key);
-                    }
-                    least = __reduce_min_sync(FULL_MASK, least);
-                    most = __reduce_max_sync(FULL_MASK, most);
-                    if (lane == 0 && least <= most) {
-                        atomicMin(&sh.ordering.least, least);
-                        atomicMax(&sh.ordering.most, most);
-                    }
-                    __syncthreads();
-                    rank_candidates<Shape>(sh, batch_slots);
-                }
-                // ---- stage the candidates: in the order of their slots, or of their indices ----
-#pragma unroll 2
-                for (int s = threadIdx.x; s < batch_slots; s += CTA_THREADS) {
-                    const int slot = Shape::CANONICAL ? static_cast<int>(sh.order[s]) : batch0 + s;
+                // ---- where the candidates are, in the order of their slots or of their indices ----
+                // (ranked: the only batch of the unit)
+                const auto* order = reinterpret_cast<const unsigned short*>(masks + base + static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS);
+                for (int s = threadIdx.x; s < batch_slots; s += ROW_EMIT_THREADS) {
+                    const int slot = ranked ? static_cast<int>(order[s]) : batch0 + s;
                     int t;
-                    const LoadedRecord record = load_record(sorted, record_of(slot, t));
-                    int r0, r1, r2;
-                    unpack_segment_image(sh.table.image[t], r0, r1, r2);
-                    sh.staged.x[s] = record.x;
-                    sh.staged.y[s] = record.y;
-                    sh.staged.z[s] = record.z;
-                    sh.staged.sj[s] = make_int4(r0 - record.s0, r1 - record.s1, r2 - record.s2, record.index);
+                    sh.position[s] = static_cast<int>(record_of(slot, t));
+                    sh.segment[s] = static_cast<unsigned char>(t);
                 }
 
                 for (int tile = 0; tile < n_tiles; tile++) {
@@ -2629,36 +2682,18 @@ __global__ void __launch_bounds__(CTA_THREADS, Shape::CTAS_PER_SM) row_emit_kern
                     }
                     // hit words of the tile, from [word][home point] to [home point][word]
                     const uint32_t* mask_tile = masks + base + (static_cast<unsigned long long>(tile) * words + word_base + (batch0 >> 5)) * TILE_POINTS;
-                    for (int k = threadIdx.x; k < batch_words * TILE_POINTS; k += CTA_THREADS) {
+                    for (int k = threadIdx.x; k < batch_words * TILE_POINTS; k += ROW_EMIT_THREADS) {
                         sh.mask[(k & 31) * (WORDS + 1) + (k >> 5)] = mask_tile[k];
                     }
                     __syncthreads();
 
-                    for (int h = warp; h < n_in_tile; h += CTA_WARPS) {
+                    for (int h = warp; h < n_in_tile; h += ROW_EMIT_WARPS) {
                         const unsigned* row_words = sh.mask + h * (WORDS + 1);
                         int total;
-                        int begin = count_row_hits<LANE_WORDS>(row_words, batch_words, lane, total);
+                        const int begin = count_row_hits<LANE_WORDS>(row_words, batch_words, lane, total);
                         if (total == 0) {
                             continue;
                         }
-                        if (Shape::CANONICAL) {
-                            // hits by slot -> hits by place in the order of the indices
-                            unsigned* bitmap = sh.bitmap[warp];
-                            __syncwarp();
-#pragma unroll
-                            for (int k = 0; k < LANE_WORDS; k++) {
-                                bitmap[lane + 32 * k] = 0;
-                            }
-                            __syncwarp();
-                            for_row_hits<LANE_WORDS>(row_words, begin, 0, total, lane, [&](int, int slot) {
-                                const unsigned place = sh.rank[slot];
-                                atomicOr(&bitmap[place >> 5], 1u << (place & 31));
-                            });
-                            __syncwarp();
-                            row_words = bitmap;
-                            begin = count_row_hits<LANE_WORDS>(row_words, 32 * LANE_WORDS, lane, total);
-                        }
-
                         const int4 home = sh.home_sj[h];
                         const double hx = sh.home_pos[0][h];
                         const double hy = sh.home_pos[1][h];
@@ -2674,25 +2709,27 @@ __global__ void __launch_bounds__(CTA_THREADS, Shape::CTAS_PER_SM) row_emit_kern
                             for (int c0 = 0; c0 < in_window; c0 += 32) {
                                 const int n_valid = min(32, in_window - c0);
                                 const int s = (lane < n_valid) ? sh.list[warp][c0 + lane] : sh.list[warp][c0];
-                                const int4 cand = sh.staged.sj[s];
-                                const int s0 = cand.x + home.x;
-                                const int s1 = cand.y + home.y;
-                                const int s2 = cand.z + home.z;
+                                const LoadedRecord cand = load_record(sorted, static_cast<size_t>(sh.position[s]));
+                                int s0, s1, s2;
+                                unpack_segment_image(sh.table.image[sh.segment[s]], s0, s1, s2);
+                                s0 += home.x - cand.s0;
+                                s1 += home.y - cand.s1;
+                                s2 += home.z - cand.s2;
                                 double vx, vy, vz, d2;
                                 const bool shifted = __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0;
                                 if (shifted) {
-                                    d2 = exact_pair(plan, hx, hy, hz, sh.staged.x[s], sh.staged.y[s], sh.staged.z[s], s0, s1, s2, vx, vy, vz);
+                                    d2 = exact_pair(plan, hx, hy, hz, cand.x, cand.y, cand.z, s0, s1, s2, vx, vy, vz);
                                 } else {
                                     // (the signed zeros that the products with S = 0 give)
-                                    vx = __dadd_rn(__dsub_rn(sh.staged.x[s], hx), plan.zero_shift[0]);
-                                    vy = __dadd_rn(__dsub_rn(sh.staged.y[s], hy), plan.zero_shift[1]);
-                                    vz = __dadd_rn(__dsub_rn(sh.staged.z[s], hz), plan.zero_shift[2]);
+                                    vx = __dadd_rn(__dsub_rn(cand.x, hx), plan.zero_shift[0]);
+                                    vy = __dadd_rn(__dsub_rn(cand.y, hy), plan.zero_shift[1]);
+                                    vz = __dadd_rn(__dsub_rn(cand.z, hz), plan.zero_shift[2]);
                                     d2 = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
                                 }
                                 store_pairs(
                                     sh.transpose[warp], out, lane, row + static_cast<unsigned long long>(window + c0), n_valid,
-                                    static_cast<unsigned long long>(home.w), static_cast<unsigned long long>(cand.w), s0, s1, s2, __dsqrt_rn(d2), vx, vy,
-                                    vz, shifted
+                                    static_cast<unsigned long long>(home.w), static_cast<unsigned long long>(cand.index), s0, s1, s2, __dsqrt_rn(d2), vx,
+                                    vy, vz, shifted
                                 );
                             }
                         }
@@ -2975,10 +3012,25 @@ int pair_grid(int n_units, int per_sm) {
 // launch wrappers
 // ---------------------------------------------------------------------------
 
+namespace {
+template <bool FULL>
+using RowCount = RowCountShape<FULL, false, 1024, 8>;
+template <bool FULL>
+using RankedCount = RowCountShape<FULL, true, 1024, FULL ? 8 : 7>;
+template <bool FULL>
+using RankedCountWide = RowCountShape<FULL, true, 2048, 4>;
+} // namespace
+
 void configure_kernels() {
-    cudaFuncSetAttribute(row_emit_kernel<SortedRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SortedRows::Shared)));
-    cudaFuncSetAttribute(row_emit_kernel<CanonicalRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(CanonicalRows::Shared)));
-    cudaFuncSetAttribute(row_emit_kernel<CanonicalRowsWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(CanonicalRowsWide::Shared)));
+    const auto allow = [](auto kernel, size_t bytes) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)); };
+    allow(row_emit_kernel<SortedRows>, sizeof(SortedRows::Shared));
+    allow(row_emit_kernel<SortedRowsWide>, sizeof(SortedRowsWide::Shared));
+    allow(row_count_kernel<RowCount<true>>, sizeof(RowCount<true>::Shared));
+    allow(row_count_kernel<RowCount<false>>, sizeof(RowCount<false>::Shared));
+    allow(row_count_kernel<RankedCount<true>>, sizeof(RankedCount<true>::Shared));
+    allow(row_count_kernel<RankedCount<false>>, sizeof(RankedCount<false>::Shared));
+    allow(row_count_kernel<RankedCountWide<true>>, sizeof(RankedCountWide<true>::Shared));
+    allow(row_count_kernel<RankedCountWide<false>>, sizeof(RankedCountWide<false>::Shared));
     cudaFuncSetAttribute(pairs_kernel<false, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<true, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<false, false, TinyCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(TinyCta::Shared)));
@@ -3113,50 +3165,50 @@ void launch_scatter(
 
 void launch_count(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, uint32_t* masks, unsigned long long mask_capacity,
-    unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, cudaStream_t stream
+    unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, int ranked_batch, cudaStream_t stream
 ) {
-    const int grid = pair_grid(plan.n_units, ROW_COUNT_CTAS);
-    if (plan.full) {
-        row_count_kernel<true><<<grid, ROW_COUNT_THREADS, 0, stream>>>(
+    const auto launch = [&](auto shape, auto kernel) {
+        using Shape = decltype(shape);
+        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_COUNT_THREADS, sizeof(typename Shape::Shared), stream>>>(
             plan, cell_start, sorted, masks, mask_capacity, unit_mask_base, unit_words, row_count, header
         );
+    };
+    if (ranked_batch == 0) {
+        plan.full ? launch(RowCount<true>{}, row_count_kernel<RowCount<true>>) : launch(RowCount<false>{}, row_count_kernel<RowCount<false>>);
+    } else if (ranked_batch == RankedCount<true>::BATCH) {
+        plan.full ? launch(RankedCount<true>{}, row_count_kernel<RankedCount<true>>) : launch(RankedCount<false>{}, row_count_kernel<RankedCount<false>>);
     } else {
-        row_count_kernel<false><<<grid, ROW_COUNT_THREADS, 0, stream>>>(
-            plan, cell_start, sorted, masks, mask_capacity, unit_mask_base, unit_words, row_count, header
-        );
+        plan.full ? launch(RankedCountWide<true>{}, row_count_kernel<RankedCountWide<true>>)
+                  : launch(RankedCountWide<false>{}, row_count_kernel<RankedCountWide<false>>);
     }
 }
 
-int canonical_emit_batch(unsigned max_candidates, bool duplicates_possible) {
-    if (duplicates_possible) {
-        return 0;
+int ranked_count_batch(double candidates) {
+    if (candidates <= RankedCount<true>::BATCH) {
+        return RankedCount<true>::BATCH;
     }
-    if (max_candidates <= CanonicalRows::BATCH) {
-        return CanonicalRows::BATCH;
-    }
-    return (max_candidates <= CanonicalRowsWide::BATCH) ? CanonicalRowsWide::BATCH : 0;
+    return (candidates <= RankedCountWide<true>::BATCH) ? RankedCountWide<true>::BATCH : 0;
 }
 
-int row_batch(int canonical_batch) {
-    return (canonical_batch != 0) ? canonical_batch : SortedRows::BATCH;
+int row_batch(unsigned max_candidates) {
+    return (max_candidates > SortedRows::BATCH && max_candidates <= SortedRowsWide::BATCH) ? SortedRowsWide::BATCH : SortedRows::BATCH;
 }
 
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
-    const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, int canonical_batch, cudaStream_t stream
+    const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, unsigned max_candidates, bool ranked,
+    cudaStream_t stream
 ) {
     const auto launch = [&](auto shape, auto kernel) {
         using Shape = decltype(shape);
-        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), CTA_THREADS, sizeof(typename Shape::Shared), stream>>>(
-            plan, cell_start, sorted, masks, unit_mask_base, unit_words, row_start, row_fill, out
+        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_EMIT_THREADS, sizeof(typename Shape::Shared), stream>>>(
+            plan, cell_start, sorted, masks, unit_mask_base, unit_words, row_start, row_fill, out, ranked ? 1 : 0
         );
     };
-    if (canonical_batch == CanonicalRows::BATCH) {
-        launch(CanonicalRows{}, row_emit_kernel<CanonicalRows>);
-    } else if (canonical_batch == CanonicalRowsWide::BATCH) {
-        launch(CanonicalRowsWide{}, row_emit_kernel<CanonicalRowsWide>);
-    } else {
+    if (row_batch(max_candidates) == SortedRows::BATCH) {
         launch(SortedRows{}, row_emit_kernel<SortedRows>);
+    } else {
+        launch(SortedRowsWide{}, row_emit_kernel<SortedRowsWide>);
     }
 }
 

@@ -227,25 +227,26 @@ void launch_scan_units(
 /// Sorted lists, pass 1: fp32 screen + fp64 decision for every (point,
 /// candidate) of the full stencil; writes one hit bit per candidate and adds
 /// the pairs of every point to row_count (which must start at zero).
+/// `ranked_batch`: 0, or what ranked_count_batch() said: the candidates of a unit are then numbered in
+/// the order of their indices, and the order left behind the unit's words. Units with more
+/// candidates than that are left out; header->max_candidates tells, and the pass has to be run again.
 void launch_count(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, uint32_t* masks, unsigned long long mask_capacity,
-    unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, cudaStream_t stream
+    unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, int ranked_batch, cudaStream_t stream
 );
+/// Room for the candidates of a unit in pass 1 when it ranks them (0: it can not hold as many).
+int ranked_count_batch(double candidates);
 
 /// Sorted lists, pass 2: walks the hit bits and writes i, j, S, d, D, one row
 /// per point in index order (row_start from the scan of row_count; row_fill
 /// must start at zero when a unit has more than row_batch() candidates, and is not looked at
-/// otherwise). `canonical_batch`: 0, or what canonical_emit_batch()
-/// said: the rows then come out sorted by the second index.
+/// otherwise). `ranked`: pass 1 ranked the candidates, and the rows come out sorted by the second index.
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
-    const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, int canonical_batch, cudaStream_t stream
+    const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, unsigned max_candidates, bool ranked,
+    cudaStream_t stream
 );
-int row_batch(int canonical_batch);
-/// Can pass 2 write the rows of a canonical list in their final order? It can when a CTA holds all
-/// candidates of a unit at once and no second index comes twice in a row. 0: it can not, the rows
-/// have to be sorted behind it (launch_sort_rows).
-int canonical_emit_batch(unsigned max_candidates, bool duplicates_possible);
+int row_batch(unsigned max_candidates);
 
 /// Sorts the pairs inside every row by (second index, shift): `in` holds rows
 /// [row_start[r], row_start[r + 1]), `out` receives the sorted rows.
