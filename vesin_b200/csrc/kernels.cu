@@ -109,6 +109,18 @@ __device__ __forceinline__ PointRecord load_packed_record(const SortedPoints& so
     return record;
 }
 
+/// The wrap shift of the record at p, whose packed form is `packed`.
+__device__ __forceinline__ void unpack_wrap(const SortedPoints& sorted, size_t p, uint32_t packed, int& s0, int& s1, int& s2) {
+    s0 = static_cast<int>(packed & 1023u) - WRAP_BIAS;
+    s1 = static_cast<int>((packed >> 10) & 1023u) - WRAP_BIAS;
+    s2 = static_cast<int>((packed >> 20) & 1023u) - WRAP_BIAS;
+    if (packed & WRAP_WIDE) {
+        s0 = sorted.wide_shift[3 * p + 0];
+        s1 = sorted.wide_shift[3 * p + 1];
+        s2 = sorted.wide_shift[3 * p + 2];
+    }
+}
+
 __device__ __forceinline__ LoadedRecord load_record(const SortedPoints& sorted, size_t p) {
     const PointRecord loaded = load_packed_record(sorted, p);
     LoadedRecord record;
@@ -116,15 +128,7 @@ __device__ __forceinline__ LoadedRecord load_record(const SortedPoints& sorted, 
     record.y = loaded.y;
     record.z = loaded.z;
     record.index = loaded.index;
-    const uint32_t packed = loaded.shift;
-    record.s0 = static_cast<int>(packed & 1023u) - WRAP_BIAS;
-    record.s1 = static_cast<int>((packed >> 10) & 1023u) - WRAP_BIAS;
-    record.s2 = static_cast<int>((packed >> 20) & 1023u) - WRAP_BIAS;
-    if (packed & WRAP_WIDE) {
-        record.s0 = sorted.wide_shift[3 * p + 0];
-        record.s1 = sorted.wide_shift[3 * p + 1];
-        record.s2 = sorted.wide_shift[3 * p + 2];
-    }
+    unpack_wrap(sorted, p, loaded.shift, record.s0, record.s1, record.s2);
     return record;
 }
 
@@ -2526,6 +2530,7 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
 constexpr int ROW_WINDOW = 128;    // hits of a row a warp lists at a time
 
 constexpr int ROW_EMIT_THREADS = 128;
+constexpr int IS_IMAGE = static_cast<int>(0x80000000u); // (31 bits index the points)
 constexpr int ROW_EMIT_WARPS = ROW_EMIT_THREADS / 32;
 
 /// Shape of the CTAs of the row-writing kernel: BATCH candidates are looked at at a time. The
@@ -2545,7 +2550,7 @@ struct RowShape {
         alignas(16) double transpose[ROW_EMIT_WARPS][TRANSPOSE_DOUBLES / 2]; // per warp: on the way to coalesced stores
         unsigned mask[TILE_POINTS * (WORDS + 1)]; // [home point][word], padded against bank conflicts
         unsigned short list[ROW_EMIT_WARPS][ROW_WINDOW];
-        int position[BATCH_];           // of the candidate among the cell-sorted points
+        int position[BATCH_];           // of the candidate among the cell-sorted points; IS_IMAGE: in a shifted cell
         unsigned char segment[BATCH_];  // the segment it comes from
         SegmentTable table;
         double home_pos[3][TILE_POINTS];
@@ -2664,7 +2669,9 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
                 for (int s = threadIdx.x; s < batch_slots; s += ROW_EMIT_THREADS) {
                     const int slot = ranked ? static_cast<int>(order[s]) : batch0 + s;
                     int t;
-                    sh.position[s] = static_cast<int>(record_of(slot, t));
+                    const int position = static_cast<int>(record_of(slot, t));
+                    const bool image = (sh.table.image[t] << 1) != 0; // (the top bit is a flag)
+                    sh.position[s] = position | (image ? IS_IMAGE : 0);
                     sh.segment[s] = static_cast<unsigned char>(t);
                 }
 
@@ -2699,6 +2706,7 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
                         const double hy = sh.home_pos[1][h];
                         const double hz = sh.home_pos[2][h];
                         const unsigned long long row = sh.home_row[h];
+                        const bool home_wrapped = (home.x | home.y | home.z) != 0;
                         for (int window = 0; window < total; window += ROW_WINDOW) {
                             __syncwarp();
                             for_row_hits<LANE_WORDS>(row_words, begin, window, min(window + ROW_WINDOW, total), lane, [&](int number, int slot) {
@@ -2709,14 +2717,21 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
                             for (int c0 = 0; c0 < in_window; c0 += 32) {
                                 const int n_valid = min(32, in_window - c0);
                                 const int s = (lane < n_valid) ? sh.list[warp][c0 + lane] : sh.list[warp][c0];
-                                const LoadedRecord cand = load_record(sorted, static_cast<size_t>(sh.position[s]));
-                                int s0, s1, s2;
-                                unpack_segment_image(sh.table.image[sh.segment[s]], s0, s1, s2);
-                                s0 += home.x - cand.s0;
-                                s1 += home.y - cand.s1;
-                                s2 += home.z - cand.s2;
+                                const int position = sh.position[s];
+                                const PointRecord cand = load_packed_record(sorted, static_cast<size_t>(position & ~IS_IMAGE));
+                                int s0 = 0, s1 = 0, s2 = 0;
                                 double vx, vy, vz, d2;
-                                const bool shifted = __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0;
+                                // (most groups of a large box: no image, no wrapped point, nothing to unpack)
+                                bool shifted = __any_sync(FULL_MASK, home_wrapped || position < 0 || cand.shift != NO_WRAP) != 0;
+                                if (shifted) {
+                                    int w0, w1, w2;
+                                    unpack_wrap(sorted, static_cast<size_t>(position & ~IS_IMAGE), cand.shift, w0, w1, w2);
+                                    unpack_segment_image(sh.table.image[sh.segment[s]], s0, s1, s2);
+                                    s0 += home.x - w0;
+                                    s1 += home.y - w1;
+                                    s2 += home.z - w2;
+                                    shifted = __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0;
+                                }
                                 if (shifted) {
                                     d2 = exact_pair(plan, hx, hy, hz, cand.x, cand.y, cand.z, s0, s1, s2, vx, vy, vz);
                                 } else {

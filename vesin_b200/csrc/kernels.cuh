@@ -59,6 +59,7 @@ struct alignas(32) PointRecord {
 };
 constexpr int WRAP_BIAS = 512;
 constexpr uint32_t WRAP_WIDE = 0x80000000u;
+constexpr uint32_t NO_WRAP = WRAP_BIAS | (WRAP_BIAS << 10) | (WRAP_BIAS << 20); // PointRecord::shift of a point in the box
 
 struct SortedPoints {
     PointRecord* records; // [n]
