@@ -36,6 +36,19 @@ def split_batch(system_offsets, world_size):
     return [(bounds[r], bounds[r + 1]) for r in range(world_size)]
 
 
+def _offsets_array(system_offsets):
+    """The offsets as the C ABI reads them. (64-bit integers are read where they are)"""
+    if (
+        isinstance(system_offsets, np.ndarray)
+        and system_offsets.dtype == np.int64
+        and system_offsets.ndim == 1
+        and system_offsets.flags.c_contiguous
+        and system_offsets.flags.aligned
+    ):
+        return system_offsets.view(np.uint64)
+    return np.ascontiguousarray(system_offsets, dtype=np.uint64)
+
+
 class BatchNeighborList:
     """Neighbor lists of many small systems at once (CUDA engine)."""
 
@@ -45,6 +58,7 @@ class BatchNeighborList:
         self.full_list = bool(full_list)
         self._neighbors = VesinNeighborList()
         self._last = (0, 0)  # pairs and points of the last list: what the next one will roughly need
+        self._options_made = (None, None)  # of the last call: what they were made from, and the structure
 
     def __del__(self):
         try:
@@ -66,14 +80,14 @@ class BatchNeighborList:
         # float32 data goes through the fp32 entry point (float d and D come out, decisions stay fp64)
         float_io = points.dtype == torch.float32
         work_dtype = torch.float32 if float_io else torch.float64
-        points = points.to(work_dtype).contiguous()
+        points = (points if points.dtype == work_dtype else points.to(work_dtype)).contiguous()
         n_systems = len(system_offsets) - 1
         if (boxes is None) != (periodic is None):
             raise ValueError("`boxes` and `periodic` must be given together")
         if boxes is not None:
             boxes = torch.as_tensor(boxes, device=device).to(work_dtype).contiguous()
             periodic = torch.as_tensor(periodic, device=device).to(torch.bool).contiguous()
-            if tuple(boxes.shape) != (n_systems, 3, 3) or tuple(periodic.shape) != (n_systems, 3):
+            if boxes.shape != (n_systems, 3, 3) or periodic.shape != (n_systems, 3):
                 raise ValueError("`boxes` must be (n_systems, 3, 3) and `periodic` (n_systems, 3)")
         if copy:
             return self._build_into(points, system_offsets, boxes, periodic, quantities, global_indices)
@@ -116,14 +130,14 @@ class BatchNeighborList:
         complete. The result stays in the list; returns the device address of
         the n_systems + 1 pair offsets."""
         float_io = points.dtype == torch.float32
-        offsets = np.ascontiguousarray(system_offsets, dtype=np.uint64)
+        offsets = _offsets_array(system_offsets)
         options = self._options(quantities)
         error = ctypes.c_char_p()
         pair_offsets = ctypes.c_void_p()
         entry_point = self._lib.vesin_b200_neighbors_batch_f32 if float_io else self._lib.vesin_b200_neighbors_batch
         status = entry_point(
             points.data_ptr(),
-            offsets.ctypes.data,
+            offsets.__array_interface__["data"][0],
             len(offsets) - 1,
             boxes.data_ptr() if boxes is not None else None,
             periodic.data_ptr() if periodic is not None else None,
@@ -140,19 +154,23 @@ class BatchNeighborList:
         return pair_offsets.value
 
     def _options(self, quantities):
+        made_from = (quantities, self.cutoff, self.full_list)
+        if self._options_made[0] == made_from:
+            return self._options_made[1]
         options = VesinOptions()
         options.cutoff = self.cutoff
         options.full = self.full_list
         options.return_shifts = "S" in quantities
         options.return_distances = "d" in quantities
         options.return_vectors = "D" in quantities
+        self._options_made = (made_from, options)
         return options
 
     def _build_into(self, points, system_offsets, boxes, periodic, quantities, global_indices):
         """``compute`` with tensors of their own for the outputs, which the
         engine writes directly (``vesin_b200_neighbors_batch_into``)."""
         float_io = points.dtype == torch.float32
-        offsets = np.ascontiguousarray(system_offsets, dtype=np.uint64)
+        offsets = _offsets_array(system_offsets)
         outputs = OutputTensors(quantities, points.device, torch.int64, points.dtype)
         outputs.allocate_guess(self._last, points.shape[0])
         pair_offsets = torch.empty(len(offsets), dtype=torch.int64, device=points.device)
@@ -162,7 +180,7 @@ class BatchNeighborList:
         with outputs:
             status = self._lib.vesin_b200_neighbors_batch_into(
                 points.data_ptr(),
-                offsets.ctypes.data,
+                offsets.__array_interface__["data"][0],
                 len(offsets) - 1,
                 boxes.data_ptr() if boxes is not None else None,
                 periodic.data_ptr() if periodic is not None else None,

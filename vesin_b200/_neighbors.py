@@ -52,6 +52,7 @@ def _view(ptr, shape, typestr, device, owner):
     return torch.as_tensor(_DeviceArray(ptr, shape, typestr, owner), device=device)
 
 
+_FLAG_TYPES = {bool, np.bool_}
 _PERIODIC = {}  # device copies of the (at most eight) constant flag triples, per device
 
 
@@ -59,7 +60,7 @@ def _periodic_flags(periodic, device):
     """`periodic` as three bools in device memory. Flags that come from the host
     are uploaded once per device: an upload from pageable memory makes the host
     wait for it, 15-20 us on every call."""
-    if isinstance(periodic, (list, tuple)) and len(periodic) == 3 and all(isinstance(flag, (bool, np.bool_)) for flag in periodic):
+    if isinstance(periodic, (list, tuple)) and len(periodic) == 3 and {type(flag) for flag in periodic} <= _FLAG_TYPES:
         key = (device, bool(periodic[0]), bool(periodic[1]), bool(periodic[2]))
         flags = _PERIODIC.get(key)
         if flags is None:
@@ -86,6 +87,8 @@ class NeighborList:
             raise ValueError("n_threads must be zero or a positive integer")
         self._neighbors = VesinNeighborList()
         self._last = (0, 0)  # pairs and points of the last list: what the next one will roughly need
+        self._device = None  # of the last call, with its number
+        self._options = (None, None)  # of the last call: what they were made from, and the structure
 
     def __del__(self):
         try:
@@ -116,14 +119,15 @@ class NeighborList:
         ``periodic``) and return the requested ``quantities``: any of ``i``,
         ``j``, ``P`` (both indices), ``S`` (periodic shifts), ``d`` (distances)
         and ``D`` (vectors), as a tuple in the order given."""
-        if not torch.cuda.is_available():
-            raise RuntimeError("vesin_b200 needs a CUDA device: there is no CPU engine in this package")
-
+        # (a call on a small system is bound by the host: what is looked up or converted here is
+        # done once and kept where it can be)
         from_torch = isinstance(points, torch.Tensor)
+        if not (from_torch and points.is_cuda) and not torch.cuda.is_available():
+            raise RuntimeError("vesin_b200 needs a CUDA device: there is no CPU engine in this package")
         if from_torch:
-            if points.device.type != "cuda":
-                raise RuntimeError("torch inputs must live on a CUDA device (there is no CPU engine in this package)")
             device = points.device
+            if device.type != "cuda":
+                raise RuntimeError("torch inputs must live on a CUDA device (there is no CPU engine in this package)")
             if points.requires_grad or (isinstance(box, torch.Tensor) and box.requires_grad):
                 raise RuntimeError("NeighborList.compute does not support autograd for torch tensors")
             box = torch.as_tensor(box, device=device)
@@ -141,10 +145,12 @@ class NeighborList:
         if isinstance(periodic, (bool, np.bool_)):
             periodic = [bool(periodic)] * 3
 
-        if tuple(box.shape) != (3, 3):
+        if box.shape != (3, 3):
             raise ValueError("`box` must be a 3x3 matrix")
-        if len(points.shape) != 2 or points.shape[1] != 3:
+        shape = points.shape
+        if len(shape) != 2 or shape[1] != 3:
             raise ValueError("`points` must be a nx3 array")
+        n_points = shape[0]
 
         # float32 data goes through the fp32 entry point: no upcast pass before
         # the call, no downcast pass after it (the decisions are fp64 either way)
@@ -154,8 +160,8 @@ class NeighborList:
             # (the canonical entry point for arrays of the library is fp64)
             float_io = initial_dtype == torch.float32 and (copy or not self.canonical)
             work_dtype = torch.float32 if float_io else torch.float64
-            d_points = points.to(work_dtype).contiguous()
-            d_box = box.to(work_dtype).contiguous()
+            d_points = (points if initial_dtype == work_dtype else points.to(work_dtype)).contiguous()
+            d_box = (box if initial_dtype == work_dtype else box.to(work_dtype)).contiguous()
             d_periodic = _periodic_flags(periodic, device)
         else:
             floating = np.issubdtype(initial_dtype, np.floating)
@@ -166,41 +172,39 @@ class NeighborList:
             d_box = torch.from_numpy(np.ascontiguousarray(box, dtype=work_dtype)).to(device)
             # (numpy makes flags of anything with a truth value)
             d_periodic = _periodic_flags(np.ascontiguousarray(periodic, dtype=np.bool_).tolist(), device)
-        if tuple(d_periodic.shape) != (3,):
+        if d_periodic.shape != (3,):
             raise ValueError(
                 "`periodic` must be a single boolean or a sequence of three "
                 f"booleans, got {periodic} of type {type(periodic)}"
             )
 
-        options = VesinOptions()
-        options.cutoff = self.cutoff
-        options.full = self.full_list
-        options.sorted = self.sorted
-        options.return_shifts = "S" in quantities
-        options.return_distances = "d" in quantities
-        options.return_vectors = "D" in quantities
-        options.algorithm = self._c_algorithm
-        options.skin = self.skin
-        options.n_threads = self.n_threads
+        made_from = (quantities, self.cutoff, self.full_list, self.sorted, self._c_algorithm, self.skin, self.n_threads)
+        if self._options[0] != made_from:
+            self._options = (made_from, self._make_options(quantities))
+        options = self._options[1]
 
-        c_device = VesinDevice(VesinCUDA, device.index or 0)
-        if self._neighbors.device.type != VesinUnknownDevice and (
-            self._neighbors.device.type != c_device.type or self._neighbors.device.device_id != c_device.device_id
-        ):
-            self._lib.vesin_free(ctypes.byref(self._neighbors))
-            ctypes.memset(ctypes.byref(self._neighbors), 0, ctypes.sizeof(self._neighbors))
+        number = device.index or 0
+        if self._device is None or self._device.device_id != number:
+            c_device = VesinDevice(VesinCUDA, number)
+            if self._neighbors.device.type != VesinUnknownDevice and (
+                self._neighbors.device.type != c_device.type or self._neighbors.device.device_id != c_device.device_id
+            ):
+                self._lib.vesin_free(ctypes.byref(self._neighbors))
+                ctypes.memset(ctypes.byref(self._neighbors), 0, ctypes.sizeof(self._neighbors))
+            self._device = c_device
+        c_device = self._device
 
         error_message = ctypes.c_char_p()
 
         if from_torch and copy:
             outputs = OutputTensors(quantities, device, torch.uint64, work_dtype)
-            outputs.allocate_guess(self._last, d_points.shape[0])
+            outputs.allocate_guess(self._last, n_points)
             wait_for_caller(device)
             n_pairs = ctypes.c_size_t()
             with outputs:
                 status = self._lib.vesin_b200_neighbors_into(
                     d_points.data_ptr(),
-                    d_points.shape[0],
+                    n_points,
                     d_box.data_ptr(),
                     d_periodic.data_ptr(),
                     c_device,
@@ -215,8 +219,10 @@ class NeighborList:
                 )
             if status != 0:
                 raise outputs.error or RuntimeError(error_message.value.decode("utf8"))
-            self._last = (n_pairs.value, d_points.shape[0])
+            self._last = (n_pairs.value, n_points)
             values = outputs.take(n_pairs.value)
+            if out_dtype is work_dtype:
+                return tuple(values)
             return tuple(value.to(out_dtype) if value.dtype == work_dtype else value for value in values)
 
         wait_for_caller(device)
@@ -225,7 +231,7 @@ class NeighborList:
             entry_point = self._lib.vesin_b200_neighbors_canonical
         status = entry_point(
             d_points.data_ptr(),
-            d_points.shape[0],
+            n_points,
             d_box.data_ptr(),
             d_periodic.data_ptr(),
             c_device,
@@ -247,12 +253,13 @@ class NeighborList:
             owner = self  # a view keeps the calculator, and with it the arrays, alive
             pairs = _view(self._neighbors.pairs, (n_pairs, 2), "<u8", device, owner)
             shifts = distances = vectors = None
+            value = "<f4" if float_io else "<f8"
             if "S" in quantities:
                 shifts = _view(self._neighbors.shifts, (n_pairs, 3), "<i4", device, owner)
             if "d" in quantities:
-                distances = _view(self._neighbors.distances, (n_pairs,), "<f4" if float_io else "<f8", device, owner).to(torch_float)
+                distances = _view(self._neighbors.distances, (n_pairs,), value, device, owner).to(torch_float)
             if "D" in quantities:
-                vectors = _view(self._neighbors.vectors, (n_pairs, 3), "<f4" if float_io else "<f8", device, owner).to(torch_float)
+                vectors = _view(self._neighbors.vectors, (n_pairs, 3), value, device, owner).to(torch_float)
 
         def finish(tensor):
             return tensor if from_torch else tensor.cpu().numpy()
@@ -272,6 +279,19 @@ class NeighborList:
             elif quantity == "D":
                 data.append(finish(vectors))
         return tuple(data)
+
+    def _make_options(self, quantities):
+        options = VesinOptions()
+        options.cutoff = self.cutoff
+        options.full = self.full_list
+        options.sorted = self.sorted
+        options.return_shifts = "S" in quantities
+        options.return_distances = "d" in quantities
+        options.return_vectors = "D" in quantities
+        options.algorithm = self._c_algorithm
+        options.skin = self.skin
+        options.n_threads = self.n_threads
+        return options
 
     def stage_times(self):
         """Device milliseconds per stage of the last build (needs

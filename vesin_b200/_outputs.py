@@ -13,11 +13,17 @@ from ._c_api import VesinB200Allocate, VesinB200Arrays
 _active = threading.local()
 
 
+# the address of the current stream without the object that torch wraps it in (a few us)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def wait_for_caller(device):
     """The engine works on a stream of its own, which only the legacy default
     stream is ordered with: on any other stream, what the caller has queued
     (inputs being made, memory that a stream-ordered allocator has handed out)
     must be done before the engine touches it."""
+    if _raw_stream is not None and device.index is not None and _raw_stream(device.index) == 0:
+        return
     stream = torch.cuda.current_stream(device)
     if stream.cuda_stream != 0:
         stream.synchronize()
@@ -78,7 +84,8 @@ class OutputTensors:
 
     def allocate(self, n_pairs):
         quantities, device, arrays = self.quantities, self.device, self.arrays
-        self.release()  # what there is too little of goes back to the allocator first
+        if arrays.capacity != 0:
+            self.release()  # what there is too little of goes back to the allocator first
         if "P" in quantities:
             self.pairs = torch.empty((n_pairs, 2), dtype=self.index_dtype, device=device)
             arrays.pairs = self.pairs.data_ptr()
@@ -109,19 +116,29 @@ class OutputTensors:
         # eighth and 128 rows more than its own at most, or it is copied
         wasteful = capacity > n_pairs + n_pairs // 8 + 128
 
-        def rows(tensor):
-            if capacity == n_pairs:
-                return tensor
-            tensor = tensor[:n_pairs]
-            return tensor.clone() if wasteful else tensor
-
-        columns = {"P": self.pairs, "i": self.i, "j": self.j, "S": self.shifts, "d": self.distances, "D": self.vectors}
         result = []
         for k, quantity in enumerate(self.quantities):
-            if quantity in "ij" and self.pairs is not None:
+            if quantity == "i":
+                tensor = self.i
+            elif quantity == "j":
+                tensor = self.j
+            elif quantity == "S":
+                tensor = self.shifts
+            elif quantity == "d":
+                tensor = self.distances
+            elif quantity == "D":
+                tensor = self.vectors
+            elif quantity == "P":
+                tensor = self.pairs
+            else:
+                continue
+            if tensor is None:  # an index beside the pairs
                 result.append(self.pairs[:n_pairs, "ij".index(quantity)].clone())
-            elif quantity in columns:
-                tensor = rows(columns[quantity])
-                # a quantity asked for twice comes back as two tensors
-                result.append(tensor.clone() if quantity in self.quantities[:k] else tensor)
+                continue
+            if capacity != n_pairs:
+                tensor = tensor[:n_pairs]
+                if wasteful:
+                    tensor = tensor.clone()
+            # a quantity asked for twice comes back as two tensors
+            result.append(tensor.clone() if quantity in self.quantities[:k] else tensor)
         return result
