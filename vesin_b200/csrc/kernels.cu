@@ -1211,8 +1211,9 @@ struct FusedSharedT {
     int slab_mode;    // slab decomposition: bit 0 = the unit's points are owned, bit 1 = so are all candidates of the group
 };
 
-/// Shape of the CTAs of the pair kernel of unsorted lists.
-template <int THREADS_, int BATCH_, int LIST_, int CTAS_PER_SM_>
+/// Shape of the CTAs of the pair kernel of unsorted lists. SHARES: several CTAs may share a unit
+/// (launches of few units; what it takes to know one's share costs large launches 2 % otherwise).
+template <int THREADS_, int BATCH_, int LIST_, int CTAS_PER_SM_, bool SHARES_>
 struct PairShape {
     using Shared = FusedSharedT<THREADS_, BATCH_, LIST_>;
     static constexpr int THREADS = THREADS_;
@@ -1222,6 +1223,7 @@ struct PairShape {
     static constexpr int LIST = LIST_;
     static constexpr int TASKS = Shared::TASKS;
     static constexpr int CTAS_PER_SM = CTAS_PER_SM_;
+    static constexpr bool SHARES = SHARES_;
     static_assert(THREADS_ >= SEG_MAX, "one thread per stencil segment of a group");
     // 228 KB of shared memory per SM, 1 KB of it reserved per resident CTA
     static_assert((sizeof(Shared) + 1024) * CTAS_PER_SM_ <= 228 * 1024, "CTAS_PER_SM CTAs fit on an SM");
@@ -1235,14 +1237,15 @@ struct PairShape {
 /// Ordinary units: CTAs of 4 warps with 256 candidates per batch, 8 of them per SM. A barrier
 /// holds up 4 warps instead of 8 and twice as many CTAs are there to issue meanwhile: sparse
 /// systems (a unit of 30 points with 400 hits) gain 17 %, dense ones 4 %.
-using SmallCta = PairShape<128, 256, 1024, 8>;
+using SmallCta = PairShape<128, 256, 1024, 8, false>;
+using SmallSharedCta = PairShape<128, 256, 1024, 8, true>;
 /// Launches that do not fill the GPU (one small system): 64 candidates per batch, so that the
 /// batches of a unit go to four times as many CTAs (see launch_pairs). What bounds such a launch
 /// is the chain of one CTA, and most of that is writing its hits.
-using TinyCta = PairShape<128, 64, 1024, 8>;
+using TinyCta = PairShape<128, 64, 1024, 8, true>;
 /// Units next to the halo of a slab (they sort their hits into owned and halo candidates and go
 /// over every batch twice): CTAs of 8 warps with 512 candidates per batch, 4 per SM.
-using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4>;
+using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4, true>;
 /// Offset (in cells, relative to the first cell of the unit) of entry `index`
 /// of the half-shell stencil of a unit of `cells` cells.
 __device__ __forceinline__ void half_stencil_offset(const GridPlan& plan, int cells, int index, int& ox, int& oy, int& oz) {
@@ -1477,8 +1480,10 @@ __device__ __forceinline__ unsigned decide_piece(
 struct UnitRanges {
     int begin0, end0, begin1, end1;
     /// Launches with far fewer units than CTAs (one small box whose stencil holds many
-    /// images): every unit is handed to `splits` CTAs, which share out its candidate batches.
+    /// images): every unit is handed to `splits` CTAs, which share out its candidate batches and, in
+    /// `tile_splits` of them for each share of the batches, its tiles of home points.
     int splits = 1;
+    int tile_splits = 1;
 };
 
 template <bool FULL, bool SLAB, class Shape>
@@ -1531,7 +1536,8 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
     // the current one is fetched while the current one is processed.
     // (the launch covers one or two ranges of units; a run lies inside one range)
     // (with splits > 1 a run is one unit, taken `splits` times: once per share of its batches)
-    const int splits = ranges.splits;
+    const int splits = Shape::SHARES ? ranges.splits : 1;
+    const int tile_splits = Shape::SHARES ? ranges.tile_splits : 1;
     const int n_runs0 = (ranges.end0 - ranges.begin0 + UNIT_RUN - 1) / UNIT_RUN;
     const int n_runs = (n_runs0 + (ranges.end1 - ranges.begin1 + UNIT_RUN - 1) / UNIT_RUN) * splits;
     int claimed = blockIdx.x;
@@ -1542,6 +1548,9 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
     }
     const int run = (splits > 1) ? claimed / splits : claimed;
     const int share = (splits > 1) ? claimed - run * splits : 0;
+    const int batch_splits = splits / tile_splits;
+    const int batch_share = share / tile_splits;
+    const int first_tile = share - batch_share * tile_splits;
     const int run_first = (run < n_runs0) ? ranges.begin0 + run * UNIT_RUN : ranges.begin1 + (run - n_runs0) * UNIT_RUN;
     const int run_end = min((run < n_runs0) ? ranges.end0 : ranges.end1, run_first + UNIT_RUN);
     Unit unit = unit_of(plan, cell_start, run_first);
@@ -1560,6 +1569,9 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
         }
         const int n_groups = (unit.n_stencil + SEG_MAX - 1) / SEG_MAX;
         const int n_tiles = (unit.n_home + TILE_POINTS - 1) / TILE_POINTS;
+        if (Shape::SHARES && first_tile >= n_tiles) {
+            continue;
+        }
 
         // Slab decomposition: a unit lies in one layer along the cut direction.
         // Full lists: this rank writes (i, j) for its own i. A unit of owned
@@ -1616,9 +1628,9 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
             }
             // (the CTAs that share a unit take its batches in turn: looking at every batch for whose it is
             // took a 64-atom cell with 63 batches 6 us of 31)
-            const int first_batch = (splits > 1) ? (share + splits - batches_before % splits) % splits : 0;
+            const int first_batch = (batch_splits > 1) ? (batch_share + batch_splits - batches_before % batch_splits) % batch_splits : 0;
             batches_before += (group_total + Shape::BATCH - 1) / Shape::BATCH;
-            for (int batch0 = first_batch * Shape::BATCH; batch0 < group_total; batch0 += splits * Shape::BATCH) {
+            for (int batch0 = first_batch * Shape::BATCH; batch0 < group_total; batch0 += batch_splits * Shape::BATCH) {
                 const int batch_slots = min(Shape::BATCH, group_total - batch0);
                 const int batch_words = (batch_slots + 31) >> 5;
 
@@ -1680,7 +1692,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                     sh.near_n[s] = __int_as_float(0x7f800000); // never a hit
                 }
 
-                for (int tile = 0; tile < n_tiles; tile++) {
+                for (int tile = first_tile; tile < n_tiles; tile += tile_splits) {
                     PHASE_MARK(2); // staging (first tile) or the end of the previous tile
                     __syncthreads(); // staging done; previous tile done with mask / list / home
                     PHASE_MARK(3); // wait
@@ -3048,6 +3060,8 @@ void configure_kernels() {
     allow(row_count_kernel<RankedCountWide<false>>, sizeof(RankedCountWide<false>::Shared));
     cudaFuncSetAttribute(pairs_kernel<false, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<true, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
+    cudaFuncSetAttribute(pairs_kernel<false, false, SmallSharedCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallSharedCta::Shared)));
+    cudaFuncSetAttribute(pairs_kernel<true, false, SmallSharedCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallSharedCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<false, false, TinyCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(TinyCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<true, false, TinyCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(TinyCta::Shared)));
     cudaFuncSetAttribute(pairs_kernel<false, true, LargeCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(LargeCta::Shared)));
@@ -3269,7 +3283,7 @@ void launch_pairs(
         unit_candidates = stencil_cells * static_cast<double>(n_records) / static_cast<double>(plan.n_cells_total);
     }
 
-    const auto launch = [&](auto shape, auto kernel, UnitRanges ranges, unsigned long long* run_cursor, bool follows = false) {
+    const auto launch_shape = [&](auto shape, auto kernel, UnitRanges ranges, unsigned long long* run_cursor, bool follows = false) {
         using Shape = decltype(shape);
         const int per_sm = Shape::CTAS_PER_SM;
         const size_t smem = sizeof(typename Shape::Shared);
@@ -3282,9 +3296,14 @@ void launch_pairs(
         int runs = (ranges.end0 - ranges.begin0 + unit_run - 1) / unit_run + (ranges.end1 - ranges.begin1 + unit_run - 1) / unit_run;
         // A handful of units whose stencils hold many batches of candidates (a small box with
         // many images): several CTAs share the batches of a unit.
-        if (unit_run == 1 && runs * 2 <= sms * per_sm) {
+        if (Shape::SHARES && unit_run == 1 && runs * 2 <= sms * per_sm) {
+            // (and, where they do not fill the GPU either, its tiles: 64 atoms with 4000 images 19.8 -> 15.9 us,
+            // 1000 atoms 15.6 -> 13.4)
             const int wanted = std::min(MAX_UNIT_SPLITS, (sms * per_sm) / runs);
             ranges.splits = std::max(1, static_cast<int>(std::min<double>(wanted, std::ceil(unit_candidates / Shape::BATCH))));
+            const double unit_tiles = static_cast<double>(n_records) / n_units / TILE_POINTS;
+            ranges.tile_splits = std::max(1, std::min(static_cast<int>(std::ceil(unit_tiles)), (sms * per_sm) / (runs * ranges.splits)));
+            ranges.splits *= ranges.tile_splits;
             runs *= ranges.splits;
         }
         const int grid = pair_grid(runs, per_sm);
@@ -3293,21 +3312,30 @@ void launch_pairs(
             (plan.window_axis < 0) ? mirror : nullptr
         );
     };
+    const auto launch = [&](auto full, UnitRanges ranges, unsigned long long* run_cursor) {
+        constexpr bool FULL = decltype(full)::value;
+        const int n_units = (ranges.end0 - ranges.begin0) + (ranges.end1 - ranges.begin1);
+        if (n_units * 2 <= sms * SmallCta::CTAS_PER_SM) {
+            launch_shape(SmallSharedCta{}, pairs_kernel<FULL, false, SmallSharedCta>, ranges, run_cursor);
+        } else {
+            launch_shape(SmallCta{}, pairs_kernel<FULL, false, SmallCta>, ranges, run_cursor);
+        }
+    };
     const UnitRanges all{0, plan.n_units, 0, 0};
     if (plan.window_axis < 0 && unit_candidates > 0.0 && plan.n_units * std::ceil(unit_candidates / SmallCta::BATCH) <= sms) {
         // Less than a CTA per SM even when every batch of 256 candidates gets its own: batches of
         // 64 (1000 atoms: 20.6 -> 13.7 us, 64 atoms with 4000 images: 29.5 -> 25.7 us; from two CTAs per
         // SM on the smaller batches cost more than they spread).
         if (plan.full) {
-            launch(TinyCta{}, pairs_kernel<true, false, TinyCta>, all, &header->run_cursor);
+            launch_shape(TinyCta{}, pairs_kernel<true, false, TinyCta>, all, &header->run_cursor);
         } else {
-            launch(TinyCta{}, pairs_kernel<false, false, TinyCta>, all, &header->run_cursor);
+            launch_shape(TinyCta{}, pairs_kernel<false, false, TinyCta>, all, &header->run_cursor);
         }
     } else if (plan.window_axis < 0) {
         if (plan.full) {
-            launch(SmallCta{}, pairs_kernel<true, false, SmallCta>, all, &header->run_cursor);
+            launch(std::true_type{}, all, &header->run_cursor);
         } else {
-            launch(SmallCta{}, pairs_kernel<false, false, SmallCta>, all, &header->run_cursor);
+            launch(std::false_type{}, all, &header->run_cursor);
         }
     } else if (plan.window_axis == 2) {
         // Slab cut along the last direction: a layer of cells is a contiguous range of units.
@@ -3328,18 +3356,18 @@ void launch_pairs(
         const int interior_end = per_layer * (owned_layers - 1);
         if (!plan.full) {
             if (part == PAIR_PART_ALL) {
-                launch(SmallCta{}, pairs_kernel<false, false, SmallCta>, UnitRanges{0, per_layer * owned_layers, 0, 0}, &header->run_cursor);
+                launch(std::false_type{}, UnitRanges{0, per_layer * owned_layers, 0, 0}, &header->run_cursor);
             } else if (part == PAIR_PART_INTERIOR) {
-                launch(SmallCta{}, pairs_kernel<false, false, SmallCta>, UnitRanges{0, interior_end, 0, 0}, &header->run_cursor);
+                launch(std::false_type{}, UnitRanges{0, interior_end, 0, 0}, &header->run_cursor);
             } else {
-                launch(SmallCta{}, pairs_kernel<false, false, SmallCta>, UnitRanges{interior_end, per_layer * owned_layers, 0, 0}, &header->mask_cursor);
+                launch(std::false_type{}, UnitRanges{interior_end, per_layer * owned_layers, 0, 0}, &header->mask_cursor);
             }
         } else {
             if (part != PAIR_PART_BOUNDARY) {
-                launch(SmallCta{}, pairs_kernel<true, false, SmallCta>, UnitRanges{0, interior_end, 0, 0}, &header->run_cursor);
+                launch(std::true_type{}, UnitRanges{0, interior_end, 0, 0}, &header->run_cursor);
             }
             if (part != PAIR_PART_INTERIOR) {
-                launch(
+                launch_shape(
                     LargeCta{}, pairs_kernel<true, true, LargeCta>,
                     UnitRanges{interior_end, per_layer * owned_layers, per_layer * (owned_layers + 1), per_layer * (owned_layers + 2)},
                     &header->mask_cursor, /*follows=*/part == PAIR_PART_ALL && owned_layers > 1
@@ -3347,9 +3375,9 @@ void launch_pairs(
             }
         }
     } else if (plan.full) {
-        launch(LargeCta{}, pairs_kernel<true, true, LargeCta>, all, &header->run_cursor);
+        launch_shape(LargeCta{}, pairs_kernel<true, true, LargeCta>, all, &header->run_cursor);
     } else {
-        launch(LargeCta{}, pairs_kernel<false, true, LargeCta>, all, &header->run_cursor);
+        launch_shape(LargeCta{}, pairs_kernel<false, true, LargeCta>, all, &header->run_cursor);
     }
 }
 
