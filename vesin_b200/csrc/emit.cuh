@@ -33,15 +33,18 @@ __device__ __forceinline__ void store_indices(const PairOutput& out, unsigned lo
 /// lane l holds pair l. 12- and 24-byte elements are transposed through
 /// shared memory so that every store instruction covers one contiguous span.
 /// `shifted` (the same in every lane): does any of the pairs have a shift? Most
-/// groups of 32 pairs of a large box have none, and zeros need no transposing.
+/// groups of 32 pairs of a large box have none, and zeros need no transposing. VALUES: are distances and
+/// vectors float (1) or double (0), or does `out` tell (-1)?
+template <int VALUES = -1>
 __device__ __forceinline__ void store_pairs(
     double* transpose, const PairOutput& out, int lane, unsigned long long first, int n_valid, unsigned long long a,
     unsigned long long b, int s0, int s1, int s2, double d, double vx, double vy, double vz, bool shifted
 ) {
+    const bool values_float = (VALUES < 0) ? out.values_float != 0 : VALUES != 0;
     if (lane < n_valid) {
         store_indices(out, first + lane, a, b);
         if (out.distances != nullptr) {
-            if (out.values_float) {
+            if (values_float) {
                 __stcs(reinterpret_cast<float*>(out.distances) + first + lane, static_cast<float>(d));
             } else {
                 __stcs(out.distances + first + lane, d);
@@ -73,7 +76,7 @@ __device__ __forceinline__ void store_pairs(
         }
         __syncwarp();
     }
-    if (out.vectors != nullptr && out.values_float) {
+    if (out.vectors != nullptr && values_float) {
         // fp32 output: rounded once from the fp64 result
         float* buffer = reinterpret_cast<float*>(transpose);
         buffer[3 * lane + 0] = static_cast<float>(vx);
@@ -119,11 +122,13 @@ __device__ __forceinline__ void store_pairs(
 /// is even again; the reversed pair of its LAST hit then does not fit behind
 /// the block and goes to the block's first element instead. `tail_lane` is the
 /// lane that holds that hit in this chunk (-1: none), `tail_to` the element.
+template <int VALUES = -1>
 __device__ __forceinline__ void store_both(
     double* transpose, const PairOutput& out, int lane, unsigned long long first, int n_valid, unsigned long long a,
     unsigned long long b, int s0, int s1, int s2, double d, double vx, double vy, double vz, bool shifted, int tail_lane = -1,
     unsigned long long tail_to = 0
 ) {
+    const bool values_float = (VALUES < 0) ? out.values_float != 0 : VALUES != 0;
     const unsigned long long mine = first + 2 * lane;
     const bool is_tail = lane == tail_lane;
     if (lane < n_valid && !is_tail) {
@@ -139,7 +144,7 @@ __device__ __forceinline__ void store_both(
             }
         }
         if (out.distances != nullptr) {
-            if (out.values_float) {
+            if (values_float) {
                 const float df = static_cast<float>(d);
                 __stcs(reinterpret_cast<float2*>(reinterpret_cast<float*>(out.distances) + mine), make_float2(df, df));
             } else {
@@ -152,7 +157,7 @@ __device__ __forceinline__ void store_both(
         store_indices(out, mine, a, b);
         store_indices(out, tail_to, b, a);
         if (out.distances != nullptr) {
-            if (out.values_float) {
+            if (values_float) {
                 reinterpret_cast<float*>(out.distances)[mine] = static_cast<float>(d);
                 reinterpret_cast<float*>(out.distances)[tail_to] = static_cast<float>(d);
             } else {
@@ -166,7 +171,7 @@ __device__ __forceinline__ void store_both(
             out.shifts[3 * tail_to + 2] = -s2;
         }
         if (out.vectors != nullptr) {
-            if (out.values_float) {
+            if (values_float) {
                 float* vectors = reinterpret_cast<float*>(out.vectors);
                 vectors[3 * tail_to + 0] = -static_cast<float>(vx);
                 vectors[3 * tail_to + 1] = -static_cast<float>(vy);
@@ -212,7 +217,7 @@ __device__ __forceinline__ void store_both(
         }
         __syncwarp();
     }
-    if (out.vectors != nullptr && out.values_float) {
+    if (out.vectors != nullptr && values_float) {
         const float fx = static_cast<float>(vx);
         const float fy = static_cast<float>(vy);
         const float fz = static_cast<float>(vz);

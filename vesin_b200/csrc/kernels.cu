@@ -1212,8 +1212,11 @@ struct FusedSharedT {
 };
 
 /// Shape of the CTAs of the pair kernel of unsorted lists. SHARES: several CTAs may share a unit
-/// (launches of few units; what it takes to know one's share costs large launches 2 % otherwise).
-template <int THREADS_, int BATCH_, int LIST_, int CTAS_PER_SM_, bool SHARES_>
+/// (launches of few units). ANY: handles slab windows, two ranges of units and arrays that are not
+/// aligned for paired stores, with the type of the values known at run time only. The kernel is at its
+/// limit of registers, and ordinary launches have none of this: without it 512k crystal atoms take 498 us instead of
+/// 523 (float: 110k atoms 119, 123), 2.1 M liquid 783 instead of 809.
+template <int THREADS_, int BATCH_, int LIST_, int CTAS_PER_SM_, bool SHARES_, bool ANY_>
 struct PairShape {
     using Shared = FusedSharedT<THREADS_, BATCH_, LIST_>;
     static constexpr int THREADS = THREADS_;
@@ -1224,6 +1227,7 @@ struct PairShape {
     static constexpr int TASKS = Shared::TASKS;
     static constexpr int CTAS_PER_SM = CTAS_PER_SM_;
     static constexpr bool SHARES = SHARES_;
+    static constexpr bool ANY = ANY_;
     static_assert(THREADS_ >= SEG_MAX, "one thread per stencil segment of a group");
     // 228 KB of shared memory per SM, 1 KB of it reserved per resident CTA
     static_assert((sizeof(Shared) + 1024) * CTAS_PER_SM_ <= 228 * 1024, "CTAS_PER_SM CTAs fit on an SM");
@@ -1237,15 +1241,15 @@ struct PairShape {
 /// Ordinary units: CTAs of 4 warps with 256 candidates per batch, 8 of them per SM. A barrier
 /// holds up 4 warps instead of 8 and twice as many CTAs are there to issue meanwhile: sparse
 /// systems (a unit of 30 points with 400 hits) gain 17 %, dense ones 4 %.
-using SmallCta = PairShape<128, 256, 1024, 8, false>;
-using SmallSharedCta = PairShape<128, 256, 1024, 8, true>;
+using SmallCta = PairShape<128, 256, 1024, 8, false, false>;
+using SmallAnyCta = PairShape<128, 256, 1024, 8, true, true>;
 /// Launches that do not fill the GPU (one small system): 64 candidates per batch, so that the
 /// batches of a unit go to four times as many CTAs (see launch_pairs). What bounds such a launch
 /// is the chain of one CTA, and most of that is writing its hits.
-using TinyCta = PairShape<128, 64, 1024, 8, true>;
+using TinyCta = PairShape<128, 64, 1024, 8, true, true>;
 /// Units next to the halo of a slab (they sort their hits into owned and halo candidates and go
 /// over every batch twice): CTAs of 8 warps with 512 candidates per batch, 4 per SM.
-using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4, true>;
+using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4, true, true>;
 /// Offset (in cells, relative to the first cell of the unit) of entry `index`
 /// of the half-shell stencil of a unit of `cells` cells.
 __device__ __forceinline__ void half_stencil_offset(const GridPlan& plan, int cells, int index, int& ox, int& oy, int& oz) {
@@ -1278,7 +1282,7 @@ __device__ __forceinline__ void half_stencil_offset(const GridPlan& plan, int ce
 /// A stencil of at most 32 cells is the work of one warp, whose scan needs no barrier: the others
 /// wait once, not twice (SLAB reads the table beyond 32 entries). 512k crystal, 14 cells: pair kernel 527 -> 523 us; 2.1 M
 /// liquid, 29 cells: 851 -> 841.
-template <bool SLAB, class Shared>
+template <bool SLAB, bool WINDOW, class Shared>
 __device__ __forceinline__ int setup_half_segments(
     const GridPlan& plan, const int32_t* __restrict__ cell_start, const Unit& unit, int group, Shared& sh, int& home_row_slots
 ) {
@@ -1306,7 +1310,7 @@ __device__ __forceinline__ int setup_half_segments(
             int nb[3] = {unit.c0 + ox, unit.c1 + oy, unit.c2 + oz};
             int q[3] = {0, 0, 0};
             bool valid = true;
-            if (plan.window_axis >= 0) {
+            if (WINDOW && plan.window_axis >= 0) {
                 // the offset counts layers in space
                 const int k = plan.window_axis;
                 const int offset = (k == 0) ? ox : ((k == 1) ? oy : oz);
@@ -1316,7 +1320,7 @@ __device__ __forceinline__ int setup_half_segments(
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 const bool outside = nb[k] < 0 || nb[k] >= plan.n_cells[k];
-                if (plan.periodic[k] && k != plan.window_axis) {
+                if (plan.periodic[k] && (!WINDOW || k != plan.window_axis)) {
                     if (outside) {
                         q[k] = floor_div(nb[k], plan.n_cells[k]);
                         nb[k] -= q[k] * plan.n_cells[k];
@@ -1326,7 +1330,7 @@ __device__ __forceinline__ int setup_half_segments(
                 }
             }
             if (valid) {
-                if (plan.window_axis >= 0) {
+                if (WINDOW && plan.window_axis >= 0) {
                     const int k = plan.window_axis;
                     owned = (nb[k] >= 1 && nb[k] <= plan.n_cells[k] - 2) ? 1 : 0;
                     nb[k] = window_storage_layer(nb[k], plan.n_cells[k]);
@@ -1486,7 +1490,7 @@ struct UnitRanges {
     int tile_splits = 1;
 };
 
-template <bool FULL, bool SLAB, class Shape>
+template <bool FULL, bool SLAB, int VALUES, class Shape>
 __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, PairOutput out, unsigned long long capacity,
     DeviceHeader* header, const int UNIT_RUN, const UnitRanges ranges, unsigned long long* run_cursor, const int follows_pair_kernel,
@@ -1539,7 +1543,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
     const int splits = Shape::SHARES ? ranges.splits : 1;
     const int tile_splits = Shape::SHARES ? ranges.tile_splits : 1;
     const int n_runs0 = (ranges.end0 - ranges.begin0 + UNIT_RUN - 1) / UNIT_RUN;
-    const int n_runs = (n_runs0 + (ranges.end1 - ranges.begin1 + UNIT_RUN - 1) / UNIT_RUN) * splits;
+    const int n_runs = (n_runs0 + (Shape::ANY ? (ranges.end1 - ranges.begin1 + UNIT_RUN - 1) / UNIT_RUN : 0)) * splits;
     int claimed = blockIdx.x;
     int run_parity = 0;
     while (claimed < n_runs) {
@@ -1551,8 +1555,9 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
     const int batch_splits = splits / tile_splits;
     const int batch_share = share / tile_splits;
     const int first_tile = share - batch_share * tile_splits;
-    const int run_first = (run < n_runs0) ? ranges.begin0 + run * UNIT_RUN : ranges.begin1 + (run - n_runs0) * UNIT_RUN;
-    const int run_end = min((run < n_runs0) ? ranges.end0 : ranges.end1, run_first + UNIT_RUN);
+    const bool in_first = !Shape::ANY || run < n_runs0;
+    const int run_first = in_first ? ranges.begin0 + run * UNIT_RUN : ranges.begin1 + (run - n_runs0) * UNIT_RUN;
+    const int run_end = min(in_first ? ranges.end0 : ranges.end1, run_first + UNIT_RUN);
     Unit unit = unit_of(plan, cell_start, run_first);
     for (int u = run_first; u < run_end; u++) {
         if (u != run_first) {
@@ -1601,9 +1606,9 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
         if (threadIdx.x >= 32 && threadIdx.x < 35) { // (the first warp is busy with the segments)
             const int c = threadIdx.x - 32;
             // (along the cut direction of a slab the geometry follows the layer in space)
-            const int g0 = (plan.window_axis == 0) ? window_space_layer(unit.c0, plan.n_cells[0]) : unit.c0;
-            const int g1 = (plan.window_axis == 1) ? window_space_layer(unit.c1, plan.n_cells[1]) : unit.c1;
-            const int g2 = (plan.window_axis == 2) ? window_space_layer(unit.c2, plan.n_cells[2]) : unit.c2;
+            const int g0 = (Shape::ANY && plan.window_axis == 0) ? window_space_layer(unit.c0, plan.n_cells[0]) : unit.c0;
+            const int g1 = (Shape::ANY && plan.window_axis == 1) ? window_space_layer(unit.c1, plan.n_cells[1]) : unit.c1;
+            const int g2 = (Shape::ANY && plan.window_axis == 2) ? window_space_layer(unit.c2, plan.n_cells[2]) : unit.c2;
             sh.centre[c] = plan.origin[c] + (g0 + 0.5 * unit.cells) * plan.cell_vec[0][c] + (g1 + 0.5) * plan.cell_vec[1][c] +
                            (g2 + 0.5) * plan.cell_vec[2][c];
         }
@@ -1612,7 +1617,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
         int batches_before = 0; // of the earlier groups of segments
         for (int g = 0; g < n_groups; g++) {
             int home_row_slots;
-            const int group_total = setup_half_segments<SLAB>(plan, cell_start, unit, g, sh, home_row_slots);
+            const int group_total = setup_half_segments<SLAB, Shape::ANY>(plan, cell_start, unit, g, sh, home_row_slots);
             PHASE_MARK(1); // segments
             if (SLAB) {
                 int segment_ok = 1;
@@ -1951,7 +1956,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                             // both orientations side by side when the claim and the arrays allow it
                             // (a claim on an odd element is moved on by one, see store_both; plain full
                             // lists only ever claim even blocks)
-                            const bool interleave = FULL && write_forward && write_reverse && out.interleave_ok && (SLAB || (claim & 1ull) == 0);
+                            const bool interleave = FULL && (!Shape::ANY || (write_forward && write_reverse && out.interleave_ok && (SLAB || (claim & 1ull) == 0)));
                             const unsigned long long moved_on = SLAB ? (claim & 1ull) : 0ull;
                             for (int chunk0 = warp * 32; chunk0 < in_round; chunk0 += Shape::WARPS * 32) {
                                 const int n_valid = min(32, in_round - chunk0);
@@ -1990,24 +1995,24 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                                     if (SLAB && moved_on != 0 && round0 + chunk0 + n_valid == total_hits) {
                                         tail_lane = n_valid - 1; // the last hit of the block is in this chunk
                                     }
-                                    store_both(
+                                    store_both<VALUES>(
                                         sh.transpose[warp], out, lane, claim + moved_on + 2ull * (round0 + chunk0), n_valid, index_i, index_j, s0, s1, s2, d,
                                         vx, vy, vz, shifted, tail_lane, claim
                                     );
                                     continue;
                                 }
                                 const unsigned long long first = claim + round0 + chunk0;
-                                if (FULL) {
+                                if (FULL && Shape::ANY) {
                                     if (write_forward) {
-                                        store_pairs(sh.transpose[warp], out, lane, first, n_valid, index_i, index_j, s0, s1, s2, d, vx, vy, vz, shifted);
+                                        store_pairs<VALUES>(sh.transpose[warp], out, lane, first, n_valid, index_i, index_j, s0, s1, s2, d, vx, vy, vz, shifted);
                                     }
                                     if (write_reverse) {
-                                        store_pairs(
+                                        store_pairs<VALUES>(
                                             sh.transpose[warp], out, lane, first + (write_forward ? total_hits : 0), n_valid, index_j, index_i, -s0, -s1, -s2,
                                             d, -vx, -vy, -vz, shifted
                                         );
                                     }
-                                } else {
+                                } else if (!FULL) {
                                     // the orientation the reference's half list keeps
                                     const bool forward = (index_i < index_j) || (index_i == index_j && half_rule(s0, s1, s2));
                                     if (!forward) {
@@ -2021,7 +2026,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                                         vy = -vy;
                                         vz = -vz;
                                     }
-                                    store_pairs(sh.transpose[warp], out, lane, first, n_valid, index_i, index_j, s0, s1, s2, d, vx, vy, vz, shifted);
+                                    store_pairs<VALUES>(sh.transpose[warp], out, lane, first, n_valid, index_i, index_j, s0, s1, s2, d, vx, vy, vz, shifted);
                                 }
                             }
                             PHASE_MARK(8); // emission
@@ -3058,14 +3063,16 @@ void configure_kernels() {
     allow(row_count_kernel<RankedCount<false>>, sizeof(RankedCount<false>::Shared));
     allow(row_count_kernel<RankedCountWide<true>>, sizeof(RankedCountWide<true>::Shared));
     allow(row_count_kernel<RankedCountWide<false>>, sizeof(RankedCountWide<false>::Shared));
-    cudaFuncSetAttribute(pairs_kernel<false, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
-    cudaFuncSetAttribute(pairs_kernel<true, false, SmallCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallCta::Shared)));
-    cudaFuncSetAttribute(pairs_kernel<false, false, SmallSharedCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallSharedCta::Shared)));
-    cudaFuncSetAttribute(pairs_kernel<true, false, SmallSharedCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallSharedCta::Shared)));
-    cudaFuncSetAttribute(pairs_kernel<false, false, TinyCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(TinyCta::Shared)));
-    cudaFuncSetAttribute(pairs_kernel<true, false, TinyCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(TinyCta::Shared)));
-    cudaFuncSetAttribute(pairs_kernel<false, true, LargeCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(LargeCta::Shared)));
-    cudaFuncSetAttribute(pairs_kernel<true, true, LargeCta>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(LargeCta::Shared)));
+    allow(pairs_kernel<false, false, 0, SmallCta>, sizeof(SmallCta::Shared));
+    allow(pairs_kernel<true, false, 0, SmallCta>, sizeof(SmallCta::Shared));
+    allow(pairs_kernel<false, false, 1, SmallCta>, sizeof(SmallCta::Shared));
+    allow(pairs_kernel<true, false, 1, SmallCta>, sizeof(SmallCta::Shared));
+    allow(pairs_kernel<false, false, -1, SmallAnyCta>, sizeof(SmallAnyCta::Shared));
+    allow(pairs_kernel<true, false, -1, SmallAnyCta>, sizeof(SmallAnyCta::Shared));
+    allow(pairs_kernel<false, false, -1, TinyCta>, sizeof(TinyCta::Shared));
+    allow(pairs_kernel<true, false, -1, TinyCta>, sizeof(TinyCta::Shared));
+    allow(pairs_kernel<false, true, -1, LargeCta>, sizeof(LargeCta::Shared));
+    allow(pairs_kernel<true, true, -1, LargeCta>, sizeof(LargeCta::Shared));
 }
 
 static ExpectedInputs expected_inputs(const double box[9], const bool periodic[3]) {
@@ -3315,10 +3322,12 @@ void launch_pairs(
     const auto launch = [&](auto full, UnitRanges ranges, unsigned long long* run_cursor) {
         constexpr bool FULL = decltype(full)::value;
         const int n_units = (ranges.end0 - ranges.begin0) + (ranges.end1 - ranges.begin1);
-        if (n_units * 2 <= sms * SmallCta::CTAS_PER_SM) {
-            launch_shape(SmallSharedCta{}, pairs_kernel<FULL, false, SmallSharedCta>, ranges, run_cursor);
+        if (plan.window_axis >= 0 || n_units * 2 <= sms * SmallCta::CTAS_PER_SM || (FULL && !out.interleave_ok)) {
+            launch_shape(SmallAnyCta{}, pairs_kernel<FULL, false, -1, SmallAnyCta>, ranges, run_cursor);
+        } else if (out.values_float) {
+            launch_shape(SmallCta{}, pairs_kernel<FULL, false, 1, SmallCta>, ranges, run_cursor);
         } else {
-            launch_shape(SmallCta{}, pairs_kernel<FULL, false, SmallCta>, ranges, run_cursor);
+            launch_shape(SmallCta{}, pairs_kernel<FULL, false, 0, SmallCta>, ranges, run_cursor);
         }
     };
     const UnitRanges all{0, plan.n_units, 0, 0};
@@ -3327,9 +3336,9 @@ void launch_pairs(
         // 64 (1000 atoms: 20.6 -> 13.7 us, 64 atoms with 4000 images: 29.5 -> 25.7 us; from two CTAs per
         // SM on the smaller batches cost more than they spread).
         if (plan.full) {
-            launch_shape(TinyCta{}, pairs_kernel<true, false, TinyCta>, all, &header->run_cursor);
+            launch_shape(TinyCta{}, pairs_kernel<true, false, -1, TinyCta>, all, &header->run_cursor);
         } else {
-            launch_shape(TinyCta{}, pairs_kernel<false, false, TinyCta>, all, &header->run_cursor);
+            launch_shape(TinyCta{}, pairs_kernel<false, false, -1, TinyCta>, all, &header->run_cursor);
         }
     } else if (plan.window_axis < 0) {
         if (plan.full) {
@@ -3368,16 +3377,16 @@ void launch_pairs(
             }
             if (part != PAIR_PART_INTERIOR) {
                 launch_shape(
-                    LargeCta{}, pairs_kernel<true, true, LargeCta>,
+                    LargeCta{}, pairs_kernel<true, true, -1, LargeCta>,
                     UnitRanges{interior_end, per_layer * owned_layers, per_layer * (owned_layers + 1), per_layer * (owned_layers + 2)},
                     &header->mask_cursor, /*follows=*/part == PAIR_PART_ALL && owned_layers > 1
                 );
             }
         }
     } else if (plan.full) {
-        launch_shape(LargeCta{}, pairs_kernel<true, true, LargeCta>, all, &header->run_cursor);
+        launch_shape(LargeCta{}, pairs_kernel<true, true, -1, LargeCta>, all, &header->run_cursor);
     } else {
-        launch_shape(LargeCta{}, pairs_kernel<false, true, LargeCta>, all, &header->run_cursor);
+        launch_shape(LargeCta{}, pairs_kernel<false, true, -1, LargeCta>, all, &header->run_cursor);
     }
 }
 
