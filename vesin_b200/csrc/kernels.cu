@@ -1213,10 +1213,13 @@ struct FusedSharedT {
 
 /// Shape of the CTAs of the pair kernel of unsorted lists. SHARES: several CTAs may share a unit
 /// (launches of few units). ANY: handles slab windows, two ranges of units and arrays that are not
-/// aligned for paired stores, with the type of the values known at run time only. The kernel is at its
+/// aligned for paired stores, with the type of the values known at run time only, and stencils of any
+/// size. The kernel is at its
 /// limit of registers, and ordinary launches have none of this: without it 512k crystal atoms take 498 us instead of
-/// 523 (float: 110k atoms 119, 123), 2.1 M liquid 783 instead of 809.
-template <int THREADS_, int BATCH_, int LIST_, int CTAS_PER_SM_, bool SHARES_, bool ANY_>
+/// 523 (float: 110k atoms 119, 123), 2.1 M liquid 783 instead of 809. SEGMENTS: where not ANY, the
+/// half stencil of a unit has at most 32 or 64 cells, one group of segments that one warp looks up (512k
+/// crystal 498 -> 490, 2.1 M liquid 783 -> 758).
+template <int THREADS_, int BATCH_, int LIST_, int CTAS_PER_SM_, bool SHARES_, bool ANY_, int SEGMENTS_>
 struct PairShape {
     using Shared = FusedSharedT<THREADS_, BATCH_, LIST_>;
     static constexpr int THREADS = THREADS_;
@@ -1228,6 +1231,8 @@ struct PairShape {
     static constexpr int CTAS_PER_SM = CTAS_PER_SM_;
     static constexpr bool SHARES = SHARES_;
     static constexpr bool ANY = ANY_;
+    static constexpr int SEGMENTS = SEGMENTS_;
+    static_assert(ANY_ || SEGMENTS_ == 32 || SEGMENTS_ == 64, "entries of one warp");
     static_assert(THREADS_ >= SEG_MAX, "one thread per stencil segment of a group");
     // 228 KB of shared memory per SM, 1 KB of it reserved per resident CTA
     static_assert((sizeof(Shared) + 1024) * CTAS_PER_SM_ <= 228 * 1024, "CTAS_PER_SM CTAs fit on an SM");
@@ -1241,15 +1246,16 @@ struct PairShape {
 /// Ordinary units: CTAs of 4 warps with 256 candidates per batch, 8 of them per SM. A barrier
 /// holds up 4 warps instead of 8 and twice as many CTAs are there to issue meanwhile: sparse
 /// systems (a unit of 30 points with 400 hits) gain 17 %, dense ones 4 %.
-using SmallCta = PairShape<128, 256, 1024, 8, false, false>;
-using SmallAnyCta = PairShape<128, 256, 1024, 8, true, true>;
+template <int SEGMENTS>
+using SmallCta = PairShape<128, 256, 1024, 8, false, false, SEGMENTS>;
+using SmallAnyCta = PairShape<128, 256, 1024, 8, true, true, SEG_MAX>;
 /// Launches that do not fill the GPU (one small system): 64 candidates per batch, so that the
 /// batches of a unit go to four times as many CTAs (see launch_pairs). What bounds such a launch
 /// is the chain of one CTA, and most of that is writing its hits.
-using TinyCta = PairShape<128, 64, 1024, 8, true, true>;
+using TinyCta = PairShape<128, 64, 1024, 8, true, true, SEG_MAX>;
 /// Units next to the halo of a slab (they sort their hits into owned and halo candidates and go
 /// over every batch twice): CTAs of 8 warps with 512 candidates per batch, 4 per SM.
-using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4, true, true>;
+using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4, true, true, SEG_MAX>;
 /// Offset (in cells, relative to the first cell of the unit) of entry `index`
 /// of the half-shell stencil of a unit of `cells` cells.
 __device__ __forceinline__ void half_stencil_offset(const GridPlan& plan, int cells, int index, int& ox, int& oy, int& oz) {
@@ -1282,25 +1288,25 @@ __device__ __forceinline__ void half_stencil_offset(const GridPlan& plan, int ce
 /// A stencil of at most 32 cells is the work of one warp, whose scan needs no barrier: the others
 /// wait once, not twice (SLAB reads the table beyond 32 entries). 512k crystal, 14 cells: pair kernel 527 -> 523 us; 2.1 M
 /// liquid, 29 cells: 851 -> 841.
-template <bool SLAB, bool WINDOW, class Shared>
+template <bool SLAB, bool ANY, int SEGMENTS, class Shared>
 __device__ __forceinline__ int setup_half_segments(
     const GridPlan& plan, const int32_t* __restrict__ cell_start, const Unit& unit, int group, Shared& sh, int& home_row_slots
 ) {
     SegmentTable& table = sh.table;
     const int t = threadIdx.x;
     const int own_row = unit.cells + plan.n_search[0];
-    int length = 0;
-    const bool one_warp = !SLAB && unit.n_stencil <= 32;
-    if (t < (one_warp ? 32 : SEG_MAX)) {
-        const int global_t = group * SEG_MAX + t;
+    const bool one_warp = !ANY || (!SLAB && unit.n_stencil <= 32);
+    // entry `entry` of the table, of the whole stencil `global_t`; returns the length of the segment
+    const auto set_entry = [&](int entry, int global_t) -> int {
+        int length = 0;
         int start = 0;
         int q0 = 0, q1 = 0, q2 = 0;
         int owned = 1;
         if (global_t < unit.n_stencil) {
             int ox, oy, oz;
-            if (group == 0 && unit.cells == plan.pencil && sh.stencil_cached) {
+            if ((!ANY || (group == 0 && sh.stencil_cached)) && unit.cells == plan.pencil) {
                 // the usual unit: offsets decoded once per CTA
-                const int packed = sh.stencil_offset[t];
+                const int packed = sh.stencil_offset[entry];
                 ox = (packed & 1023) - 512;
                 oy = ((packed >> 10) & 1023) - 512;
                 oz = (packed >> 20) - 512;
@@ -1310,7 +1316,7 @@ __device__ __forceinline__ int setup_half_segments(
             int nb[3] = {unit.c0 + ox, unit.c1 + oy, unit.c2 + oz};
             int q[3] = {0, 0, 0};
             bool valid = true;
-            if (WINDOW && plan.window_axis >= 0) {
+            if (ANY && plan.window_axis >= 0) {
                 // the offset counts layers in space
                 const int k = plan.window_axis;
                 const int offset = (k == 0) ? ox : ((k == 1) ? oy : oz);
@@ -1320,7 +1326,7 @@ __device__ __forceinline__ int setup_half_segments(
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 const bool outside = nb[k] < 0 || nb[k] >= plan.n_cells[k];
-                if (plan.periodic[k] && (!WINDOW || k != plan.window_axis)) {
+                if (plan.periodic[k] && (!ANY || k != plan.window_axis)) {
                     if (outside) {
                         q[k] = floor_div(nb[k], plan.n_cells[k]);
                         nb[k] -= q[k] * plan.n_cells[k];
@@ -1330,7 +1336,7 @@ __device__ __forceinline__ int setup_half_segments(
                 }
             }
             if (valid) {
-                if (WINDOW && plan.window_axis >= 0) {
+                if (ANY && plan.window_axis >= 0) {
                     const int k = plan.window_axis;
                     owned = (nb[k] >= 1 && nb[k] <= plan.n_cells[k] - 2) ? 1 : 0;
                     nb[k] = window_storage_layer(nb[k], plan.n_cells[k]);
@@ -1343,28 +1349,41 @@ __device__ __forceinline__ int setup_half_segments(
                 q2 = q[2];
             }
         }
-        table.start[t] = start;
-        table.image[t] = pack_segment_image(q0, q1, q2, owned); // (flag: does the segment hold owned points?)
-    }
+        table.start[entry] = start;
+        table.image[entry] = pack_segment_image(q0, q1, q2, owned); // (flag: does the segment hold owned points?)
+        return length;
+    };
     if (one_warp) {
+        constexpr int ENTRIES = ANY ? 1 : SEGMENTS / 32; // per lane
         if (t < 32) {
-            int inclusive = length;
+            int length[ENTRIES];
 #pragma unroll
-            for (int offset = 1; offset < 32; offset <<= 1) {
-                const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
-                if (t >= offset) {
-                    inclusive += up;
-                }
+            for (int e = 0; e < ENTRIES; e++) {
+                length[e] = set_entry(t + 32 * e, group * SEG_MAX + t + 32 * e);
             }
-            table.slot0[t] = inclusive - length;
+            int before = 0;
+#pragma unroll
+            for (int e = 0; e < ENTRIES; e++) {
+                int inclusive = length[e];
+#pragma unroll
+                for (int offset = 1; offset < 32; offset <<= 1) {
+                    const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
+                    if (t >= offset) {
+                        inclusive += up;
+                    }
+                }
+                table.slot0[t + 32 * e] = before + inclusive - length[e];
+                before += __shfl_sync(FULL_MASK, inclusive, 31);
+            }
             if (t == 31) {
-                table.slot0[32] = inclusive;
+                table.slot0[32 * ENTRIES] = before;
             }
         }
         __syncthreads();
         home_row_slots = table.slot0[own_row]; // (own_row <= n_stencil)
-        return table.slot0[32];
+        return table.slot0[32 * ENTRIES];
     }
+    const int length = (t < SEG_MAX) ? set_entry(t, group * SEG_MAX + t) : 0;
     const int prefix = block_exclusive_scan<SEG_MAX / 32>(length, table.scan_tmp);
     if (t < SEG_MAX) {
         table.slot0[t] = prefix;
@@ -1572,7 +1591,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
             const int rows_above = plan.n_search[1] + plan.n_search[2] * (2 * plan.n_search[1] + 1);
             unit.n_stencil = own_row + row_width * rows_above;
         }
-        const int n_groups = (unit.n_stencil + SEG_MAX - 1) / SEG_MAX;
+        const int n_groups = Shape::ANY ? (unit.n_stencil + SEG_MAX - 1) / SEG_MAX : 1;
         const int n_tiles = (unit.n_home + TILE_POINTS - 1) / TILE_POINTS;
         if (Shape::SHARES && first_tile >= n_tiles) {
             continue;
@@ -1617,7 +1636,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
         int batches_before = 0; // of the earlier groups of segments
         for (int g = 0; g < n_groups; g++) {
             int home_row_slots;
-            const int group_total = setup_half_segments<SLAB, Shape::ANY>(plan, cell_start, unit, g, sh, home_row_slots);
+            const int group_total = setup_half_segments<SLAB, Shape::ANY, Shape::SEGMENTS>(plan, cell_start, unit, g, sh, home_row_slots);
             PHASE_MARK(1); // segments
             if (SLAB) {
                 int segment_ok = 1;
@@ -1661,7 +1680,12 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                 //      found by bisection), so all loads of a batch are in flight at once ----
                 for (int s = threadIdx.x; s < batch_slots; s += Shape::THREADS) {
                     const int slot = batch0 + s;
-                    const int t = (unit.n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
+                    int t;
+                    if constexpr (Shape::ANY) {
+                        t = (unit.n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
+                    } else {
+                        t = find_segment<(Shape::SEGMENTS == 32) ? 5 : 6>(sh.table, slot);
+                    }
                     const size_t p = static_cast<size_t>(sh.table.start[t]) + (slot - sh.table.slot0[t]);
                     const LoadedRecord record = load_record(sorted, p);
                     int r0, r1, r2;
@@ -3063,10 +3087,15 @@ void configure_kernels() {
     allow(row_count_kernel<RankedCount<false>>, sizeof(RankedCount<false>::Shared));
     allow(row_count_kernel<RankedCountWide<true>>, sizeof(RankedCountWide<true>::Shared));
     allow(row_count_kernel<RankedCountWide<false>>, sizeof(RankedCountWide<false>::Shared));
-    allow(pairs_kernel<false, false, 0, SmallCta>, sizeof(SmallCta::Shared));
-    allow(pairs_kernel<true, false, 0, SmallCta>, sizeof(SmallCta::Shared));
-    allow(pairs_kernel<false, false, 1, SmallCta>, sizeof(SmallCta::Shared));
-    allow(pairs_kernel<true, false, 1, SmallCta>, sizeof(SmallCta::Shared));
+    const auto allow_plain = [&](auto shape) {
+        using Shape = decltype(shape);
+        allow(pairs_kernel<false, false, 0, Shape>, sizeof(typename Shape::Shared));
+        allow(pairs_kernel<true, false, 0, Shape>, sizeof(typename Shape::Shared));
+        allow(pairs_kernel<false, false, 1, Shape>, sizeof(typename Shape::Shared));
+        allow(pairs_kernel<true, false, 1, Shape>, sizeof(typename Shape::Shared));
+    };
+    allow_plain(SmallCta<32>{});
+    allow_plain(SmallCta<64>{});
     allow(pairs_kernel<false, false, -1, SmallAnyCta>, sizeof(SmallAnyCta::Shared));
     allow(pairs_kernel<true, false, -1, SmallAnyCta>, sizeof(SmallAnyCta::Shared));
     allow(pairs_kernel<false, false, -1, TinyCta>, sizeof(TinyCta::Shared));
@@ -3322,16 +3351,26 @@ void launch_pairs(
     const auto launch = [&](auto full, UnitRanges ranges, unsigned long long* run_cursor) {
         constexpr bool FULL = decltype(full)::value;
         const int n_units = (ranges.end0 - ranges.begin0) + (ranges.end1 - ranges.begin1);
-        if (plan.window_axis >= 0 || n_units * 2 <= sms * SmallCta::CTAS_PER_SM || (FULL && !out.interleave_ok)) {
+        const long long above = static_cast<long long>(plan.n_search[1]) + static_cast<long long>(plan.n_search[2]) * (2 * plan.n_search[1] + 1);
+        const long long segments = plan.pencil + plan.n_search[0] + (plan.pencil + 2 * plan.n_search[0]) * above;
+        const auto launch_plain = [&](auto shape) {
+            using Shape = decltype(shape);
+            if (out.values_float) {
+                launch_shape(shape, pairs_kernel<FULL, false, 1, Shape>, ranges, run_cursor);
+            } else {
+                launch_shape(shape, pairs_kernel<FULL, false, 0, Shape>, ranges, run_cursor);
+            }
+        };
+        if (plan.window_axis >= 0 || segments > 64 || n_units * 2 <= sms * SmallAnyCta::CTAS_PER_SM || (FULL && !out.interleave_ok)) {
             launch_shape(SmallAnyCta{}, pairs_kernel<FULL, false, -1, SmallAnyCta>, ranges, run_cursor);
-        } else if (out.values_float) {
-            launch_shape(SmallCta{}, pairs_kernel<FULL, false, 1, SmallCta>, ranges, run_cursor);
+        } else if (segments > 32) {
+            launch_plain(SmallCta<64>{});
         } else {
-            launch_shape(SmallCta{}, pairs_kernel<FULL, false, 0, SmallCta>, ranges, run_cursor);
+            launch_plain(SmallCta<32>{});
         }
     };
     const UnitRanges all{0, plan.n_units, 0, 0};
-    if (plan.window_axis < 0 && unit_candidates > 0.0 && plan.n_units * std::ceil(unit_candidates / SmallCta::BATCH) <= sms) {
+    if (plan.window_axis < 0 && unit_candidates > 0.0 && plan.n_units * std::ceil(unit_candidates / SmallAnyCta::BATCH) <= sms) {
         // Less than a CTA per SM even when every batch of 256 candidates gets its own: batches of
         // 64 (1000 atoms: 20.6 -> 13.7 us, 64 atoms with 4000 images: 29.5 -> 25.7 us; from two CTAs per
         // SM on the smaller batches cost more than they spread).
