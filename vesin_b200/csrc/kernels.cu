@@ -928,15 +928,17 @@ __global__ void __launch_bounds__(SMALL_FRONT_THREADS) small_front_kernel(
 constexpr int SEG_MAX = 128;
 constexpr int TILE_POINTS = 32; // home points handled at once: one per lane
 
-struct SegmentTable {
+template <int ENTRIES>
+struct SegmentTableT {
     /// Image shift of the segment, 21 bits per direction (a stencil never reaches further:
     /// MAX_STENCIL_CELLS), and in the top bit a flag: may a point pair with its own image in
     /// this segment (sorted lists) / does the segment hold owned points (slab decomposition)?
-    unsigned long long image[SEG_MAX];
-    int start[SEG_MAX];     // first cell-sorted point of the segment
-    int slot0[SEG_MAX + 1]; // exclusive prefix of the segment lengths
+    unsigned long long image[ENTRIES];
+    int start[ENTRIES];     // first cell-sorted point of the segment
+    int slot0[ENTRIES + 1]; // exclusive prefix of the segment lengths
     int scan_tmp[CTA_WARPS + 1];
 };
+using SegmentTable = SegmentTableT<SEG_MAX>;
 static_assert(MAX_STENCIL_CELLS <= (1 << 20), "image shifts are stored in 21 bits");
 
 __device__ __forceinline__ unsigned long long pack_segment_image(int q0, int q1, int q2, int flag) {
@@ -1085,9 +1087,9 @@ __device__ __forceinline__ int setup_segments(const GridPlan& plan, const int32_
 /// Segment that holds `slot`: last t with slot0[t] <= slot, among the first
 /// 2^STEPS segments (entries past the stencil hold the total, so any power of
 /// two that covers the stencil will do).
-template <int STEPS = 7>
-__device__ __forceinline__ int find_segment(const SegmentTable& table, int slot) {
-    static_assert((1 << STEPS) <= SEG_MAX, "the table has SEG_MAX entries");
+template <int STEPS = 7, int ENTRIES>
+__device__ __forceinline__ int find_segment(const SegmentTableT<ENTRIES>& table, int slot) {
+    static_assert((1 << STEPS) <= ENTRIES, "entries of the table");
     int lo = 0;
     int hi = 1 << STEPS; // slot0[hi] > slot always holds for slot < total
 #pragma unroll
@@ -1171,7 +1173,7 @@ constexpr int FUSED_LIST = 2048;
 
 /// Shared memory of a CTA of THREADS_ threads that stages BATCH_ candidates at a time and
 /// lists up to LIST_ hits per round.
-template <int THREADS_, int BATCH_, int LIST_>
+template <int THREADS_, int BATCH_, int LIST_, int SEGMENTS_>
 struct FusedSharedT {
     static constexpr int THREADS = THREADS_;
     static constexpr int WARPS = THREADS_ / 32;
@@ -1180,11 +1182,11 @@ struct FusedSharedT {
     static constexpr int LIST = LIST_;
     /// (home point, word) tasks per thread when the hits of a tile are counted
     static constexpr int TASKS = (TILE_POINTS * WORDS + THREADS_ - 1) / THREADS_;
-    static_assert(BATCH_ % 32 == 0 && (WORDS & (WORDS - 1)) == 0, "whole words, a power of two of them");
+    static_assert(BATCH_ % 32 == 0, "whole words");
     static_assert(TILE_POINTS * BATCH_ < 65536, "hit counts of a tile are kept in 16 bits");
     static_assert(BATCH_ <= 512 && TILE_POINTS <= 32, "a list entry packs (lane, slot) into 14 bits");
 
-    SegmentTable table;
+    SegmentTableT<SEGMENTS_> table;
     // fp32 coordinates of the candidates relative to the unit centre and their squared norm,
     // one array per component so that two candidates fill one packed fp32x2 operand
     alignas(16) float near_x[BATCH]; // read as 16-byte vectors
@@ -1206,7 +1208,7 @@ struct FusedSharedT {
     unsigned long long claimed; // output elements this CTA has claimed (thread 0)
     double centre[3]; // centre of the unit: origin of the fp32 local frame
     int stencil_cached;          // are the packed offsets below usable?
-    int stencil_offset[SEG_MAX]; // first SEG_MAX entries of the stencil of a full-length unit, 10 bits per direction
+    int stencil_offset[SEGMENTS_]; // first entries of the stencil of a full-length unit, 10 bits per direction
     int next_run[2];  // run of units this CTA takes next (two slots: one is read while the other is written)
     int slab_mode;    // slab decomposition: bit 0 = the unit's points are owned, bit 1 = so are all candidates of the group
 };
@@ -1221,7 +1223,7 @@ struct FusedSharedT {
 /// crystal 498 -> 490, 2.1 M liquid 783 -> 758).
 template <int THREADS_, int BATCH_, int LIST_, int CTAS_PER_SM_, bool SHARES_, bool ANY_, int SEGMENTS_>
 struct PairShape {
-    using Shared = FusedSharedT<THREADS_, BATCH_, LIST_>;
+    using Shared = FusedSharedT<THREADS_, BATCH_, LIST_, SEGMENTS_>;
     static constexpr int THREADS = THREADS_;
     static constexpr int WARPS = THREADS_ / 32;
     static constexpr int BATCH = BATCH_;
@@ -1246,8 +1248,9 @@ struct PairShape {
 /// Ordinary units: CTAs of 4 warps with 256 candidates per batch, 8 of them per SM. A barrier
 /// holds up 4 warps instead of 8 and twice as many CTAs are there to issue meanwhile: sparse
 /// systems (a unit of 30 points with 400 hits) gain 17 %, dense ones 4 %.
-template <int SEGMENTS>
-using SmallCta = PairShape<128, 256, 1024, 8, false, false, SEGMENTS>;
+/// Of 256 candidates per batch, 8 of them per SM, or of 224 and 9 (56 registers; see launch_pairs).
+template <int SEGMENTS, int BATCH>
+using SmallCta = PairShape<128, BATCH, 1024, (BATCH == 256) ? 8 : 9, false, false, SEGMENTS>;
 using SmallAnyCta = PairShape<128, 256, 1024, 8, true, true, SEG_MAX>;
 /// Launches that do not fill the GPU (one small system): 64 candidates per batch, so that the
 /// batches of a unit go to four times as many CTAs (see launch_pairs). What bounds such a launch
@@ -1292,7 +1295,7 @@ template <bool SLAB, bool ANY, int SEGMENTS, class Shared>
 __device__ __forceinline__ int setup_half_segments(
     const GridPlan& plan, const int32_t* __restrict__ cell_start, const Unit& unit, int group, Shared& sh, int& home_row_slots
 ) {
-    SegmentTable& table = sh.table;
+    auto& table = sh.table;
     const int t = threadIdx.x;
     const int own_row = unit.cells + plan.n_search[0];
     const bool one_warp = !ANY || (!SLAB && unit.n_stencil <= 32);
@@ -1383,19 +1386,22 @@ __device__ __forceinline__ int setup_half_segments(
         home_row_slots = table.slot0[own_row]; // (own_row <= n_stencil)
         return table.slot0[32 * ENTRIES];
     }
-    const int length = (t < SEG_MAX) ? set_entry(t, group * SEG_MAX + t) : 0;
-    const int prefix = block_exclusive_scan<SEG_MAX / 32>(length, table.scan_tmp);
-    if (t < SEG_MAX) {
-        table.slot0[t] = prefix;
+    if constexpr (ANY) {
+        const int length = (t < SEG_MAX) ? set_entry(t, group * SEG_MAX + t) : 0;
+        const int prefix = block_exclusive_scan<SEG_MAX / 32>(length, table.scan_tmp);
+        if (t < SEG_MAX) {
+            table.slot0[t] = prefix;
+        }
+        const int total = table.scan_tmp[CTA_WARPS]; // where block_exclusive_scan leaves the total
+        if (t == 0) {
+            table.slot0[SEG_MAX] = total;
+        }
+        __syncthreads();
+        // slots of this group that belong to the unit's own row
+        home_row_slots = (group == 0) ? table.slot0[min(own_row, SEG_MAX)] : 0;
+        return total;
     }
-    const int total = table.scan_tmp[CTA_WARPS]; // where block_exclusive_scan leaves the total
-    if (t == 0) {
-        table.slot0[SEG_MAX] = total;
-    }
-    __syncthreads();
-    // slots of this group that belong to the unit's own row
-    home_row_slots = (group == 0) ? table.slot0[min(own_row, SEG_MAX)] : 0;
-    return total;
+    return 0; // (not reached)
 }
 
 /// The fp32 screen of the pair passes as its inner loop wants it: a squared distance is compared
@@ -1545,7 +1551,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
         // 10 bits per direction hold the offsets unless the stencil reaches very far
         sh.stencil_cached = (plan.pencil + plan.n_search[0] < 500 && plan.n_search[1] < 500 && plan.n_search[2] < 500) ? 1 : 0;
     }
-    if (threadIdx.x < SEG_MAX) {
+    if (threadIdx.x < Shape::SEGMENTS) {
         // entries beyond the stencil are never read
         int ox, oy, oz;
         half_stencil_offset(plan, plan.pencil, threadIdx.x, ox, oy, oz);
@@ -1803,7 +1809,7 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
                             const unsigned of_home = __shfl_sync(FULL_MASK, word, (lane & 7) * 4);
                             sh.mask[w * TILE_POINTS + lane] = (lane < TILE_POINTS / 4) ? of_home : 0u;
                         }
-                    } else if (batch_words <= Shape::WARPS && 2 * batch_words > Shape::WARPS) {
+                    } else if (Shape::ANY && batch_words <= Shape::WARPS && 2 * batch_words > Shape::WARPS) {
                         // a word of 32 candidates per warp
                         if (warp < batch_words) {
                             sh.mask[warp * TILE_POINTS + lane] =
@@ -3094,8 +3100,10 @@ void configure_kernels() {
         allow(pairs_kernel<false, false, 1, Shape>, sizeof(typename Shape::Shared));
         allow(pairs_kernel<true, false, 1, Shape>, sizeof(typename Shape::Shared));
     };
-    allow_plain(SmallCta<32>{});
-    allow_plain(SmallCta<64>{});
+    allow_plain(SmallCta<32, 224>{});
+    allow_plain(SmallCta<32, 256>{});
+    allow_plain(SmallCta<64, 224>{});
+    allow_plain(SmallCta<64, 256>{});
     allow(pairs_kernel<false, false, -1, SmallAnyCta>, sizeof(SmallAnyCta::Shared));
     allow(pairs_kernel<true, false, -1, SmallAnyCta>, sizeof(SmallAnyCta::Shared));
     allow(pairs_kernel<false, false, -1, TinyCta>, sizeof(TinyCta::Shared));
@@ -3363,10 +3371,17 @@ void launch_pairs(
         };
         if (plan.window_axis >= 0 || segments > 64 || n_units * 2 <= sms * SmallAnyCta::CTAS_PER_SM || (FULL && !out.interleave_ok)) {
             launch_shape(SmallAnyCta{}, pairs_kernel<FULL, false, -1, SmallAnyCta>, ranges, run_cursor);
-        } else if (segments > 32) {
-            launch_plain(SmallCta<64>{});
+            return;
+        }
+        // A ninth CTA per SM is worth 1 to 4 % (110k crystal in float 115 -> 111 us, 512k 490 -> 486; 326
+        // candidates) unless its smaller batches make for more of them, in the average unit or in one of the fuller
+        // ones (2.1 M liquid, 203 candidates: 755 -> 772).
+        const double fuller = unit_candidates + 2.0 * std::sqrt(unit_candidates);
+        const auto as_many = [](double candidates) { return std::ceil(candidates / 224.0) <= std::ceil(candidates / 256.0); };
+        if (as_many(unit_candidates) && as_many(fuller)) {
+            (segments > 32) ? launch_plain(SmallCta<64, 224>{}) : launch_plain(SmallCta<32, 224>{});
         } else {
-            launch_plain(SmallCta<32>{});
+            (segments > 32) ? launch_plain(SmallCta<64, 256>{}) : launch_plain(SmallCta<32, 256>{});
         }
     };
     const UnitRanges all{0, plan.n_units, 0, 0};
