@@ -1,7 +1,7 @@
 // Batches of independent small systems. Two passes (count, emit) so that every
 // system owns one contiguous, exactly sized block of the output. Two kernels:
 //   * molecules (no periodic direction, at most 96 points): a WARP per system,
-//     eight systems per CTA;
+//     two systems per CTA;
 //   * everything else (periodic systems, up to 2048 points): one or more CTAs
 //     per system, which list the periodic images that can reach a tile of home
 //     points and stage them a batch at a time.
@@ -13,7 +13,7 @@
 // at a time through the coalesced stores of the large-system kernels. Walking
 // the (i, j) of the flattened triangle instead, a square root and a few
 // corrections per candidate, the 16 384 molecules of 16 to 64 atoms (float, 5.3 M
-// pairs) took 64 us to count and 120 us to write; now 21 and 63 (the 230 MB of the
+// pairs) took 64 us to count and 120 us to write; now 18 and 54 (the 230 MB of the
 // list take 35 us at the copy bandwidth: half the time is the chain of a warp,
 // points -> decisions -> list -> stores).
 //
@@ -28,6 +28,7 @@
 #include "plan.hpp"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace vb200 {
 
@@ -35,6 +36,7 @@ namespace {
 
 constexpr int SMALL_THREADS = 128;
 constexpr int SMALL_WARPS = SMALL_THREADS / 32;
+constexpr int SMALL_CTAS = 7; // per SM (72 registers; 512 cells, both passes: 6 132 us, 7 131, 8 132 with spills)
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
 struct SystemFrame {
@@ -166,11 +168,14 @@ __device__ __forceinline__ bool half_rule_small(int s0, int s1, int s2) {
 }
 
 constexpr int MOLECULE_MAX_POINTS = 96;  // largest system the warp-per-system kernel takes
-constexpr int MOLECULE_WARPS = 8;
+// A CTA is done when its largest system is: 16 384 molecules of 16 to 64 atoms, both passes, with 8
+// systems per CTA 79 us, 4 75, 2 72 (1, where 32 CTAs fill an SM: 70, but 16 000 of 4 to 10 atoms 26 instead of 23)
+constexpr int MOLECULE_WARPS = 2;
 
+template <class Kind>
 __device__ __forceinline__ double batch_coordinate(const BatchInput& in, size_t k) {
     // float -> double is exact: fp32 inputs are decided with the same fp64 arithmetic
-    return in.is_float ? static_cast<double>(static_cast<const float*>(in.points)[k]) : static_cast<const double*>(in.points)[k];
+    return Kind::FLOAT ? static_cast<double>(static_cast<const float*>(in.points)[k]) : static_cast<const double*>(in.points)[k];
 }
 
 /// Systems without a periodic direction and with few points go to the
@@ -352,20 +357,34 @@ __device__ __forceinline__ double molecule_pair(const MoleculeShared& sh, int wa
     return __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
 }
 
+/// What a launch of the batch kernels does is compiled in: counts or writes, full or half lists, points
+/// and values in float or double, arrays that are aligned for paired stores. Looked at while the
+/// kernels ran it took registers, which decide how many CTAs share an SM: both passes over 16 384
+/// molecules 83 -> 79 us, over 512 cells 149 -> 131.
+template <bool EMIT_, bool FULL_, bool FLOAT_, bool PAIRED_>
+struct BatchKind {
+    static constexpr bool EMIT = EMIT_;
+    static constexpr bool FULL = FULL_;
+    static constexpr bool FLOAT = FLOAT_;
+    static constexpr int VALUES = FLOAT_ ? 1 : 0;
+    static constexpr bool PAIRED = PAIRED_;
+};
+
 /// Writes the hits of up to 32 lanes from element `first` of the output on, both orientations
 /// side by side for full lists.
+template <class Kind>
 __device__ __forceinline__ void write_hits(
-    double* transpose, const BatchInput& in, const PairOutput& out, int lane, unsigned long long first, int n_valid, unsigned long long gi,
+    double* transpose, const PairOutput& out, int lane, unsigned long long first, int n_valid, unsigned long long gi,
     unsigned long long gj, int s0, int s1, int s2, double d, double vx, double vy, double vz, bool shifted
 ) {
-    if (!in.full) {
+    if (!Kind::FULL) {
         // half lists keep i <= j: the forward pair
-        store_pairs(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
-    } else if (out.interleave_ok) {
-        store_both(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
+        store_pairs<Kind::VALUES>(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
+    } else if (Kind::PAIRED) {
+        store_both<Kind::VALUES>(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
     } else {
-        store_pairs(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
-        store_pairs(transpose, out, lane, first + n_valid, n_valid, gj, gi, -s0, -s1, -s2, d, -vx, -vy, -vz, shifted);
+        store_pairs<Kind::VALUES>(transpose, out, lane, first, n_valid, gi, gj, s0, s1, s2, d, vx, vy, vz, shifted);
+        store_pairs<Kind::VALUES>(transpose, out, lane, first + n_valid, n_valid, gj, gi, -s0, -s1, -s2, d, -vx, -vy, -vz, shifted);
     }
 }
 
@@ -381,11 +400,12 @@ __global__ void batch_header_kernel(DeviceHeader* header) {
     }
 }
 
-template <bool EMIT>
-__global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
+template <class Kind>
+__global__ void __launch_bounds__(MOLECULE_WARPS * 32, Kind::EMIT ? 16 : 20) molecules_kernel(
     const BatchInput in, unsigned long long* __restrict__ system_count, const unsigned long long* __restrict__ system_start, PairOutput out,
     DeviceHeader* header, const unsigned long long capacity, DeviceHeader* mirror
 ) {
+    constexpr bool EMIT = Kind::EMIT;
     extern __shared__ __align__(16) unsigned char molecule_smem[];
     MoleculeShared& sh = *reinterpret_cast<MoleculeShared*>(molecule_smem);
     const int lane = threadIdx.x & 31;
@@ -410,17 +430,17 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
         __syncwarp();
         // ---- the system's points: originals for the exact arithmetic, fp32 copies relative to the
         //      first point for the screen ----
-        const double ox = (n > 0) ? batch_coordinate(in, 3 * begin + 0) : 0.0;
-        const double oy = (n > 0) ? batch_coordinate(in, 3 * begin + 1) : 0.0;
-        const double oz = (n > 0) ? batch_coordinate(in, 3 * begin + 2) : 0.0;
+        const double ox = (n > 0) ? batch_coordinate<Kind>(in, 3 * begin + 0) : 0.0;
+        const double oy = (n > 0) ? batch_coordinate<Kind>(in, 3 * begin + 1) : 0.0;
+        const double oz = (n > 0) ? batch_coordinate<Kind>(in, 3 * begin + 2) : 0.0;
         float reach = 0.0f;
         bool finite = true;
         for (int k = lane; k < ((n + 3) & ~3); k += 32) {
             double x = ox, y = oy, z = oz;
             if (k < n) {
-                x = batch_coordinate(in, 3 * (begin + k) + 0);
-                y = batch_coordinate(in, 3 * (begin + k) + 1);
-                z = batch_coordinate(in, 3 * (begin + k) + 2);
+                x = batch_coordinate<Kind>(in, 3 * (begin + k) + 0);
+                y = batch_coordinate<Kind>(in, 3 * (begin + k) + 1);
+                z = batch_coordinate<Kind>(in, 3 * (begin + k) + 2);
             }
             sh.x[warp][k] = x;
             sh.y[warp][k] = y;
@@ -451,7 +471,7 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
         const ScreenBand band = screen_band(reach * 1.7320508f, in.cutoff, in.cutoff2);
 
         const unsigned long long index_offset = in.global_indices ? begin : 0ull;
-        const unsigned per_hit = in.full ? 2u : 1u;
+        constexpr unsigned per_hit = Kind::FULL ? 2u : 1u;
         unsigned long long next = EMIT ? system_start[system] : 0ull; // where the next hits go
         int listed = 0;                                               // hits waiting in the list (the same value in every lane)
         int hits = 0;
@@ -466,7 +486,7 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32) molecules_kernel(
                 }
                 double vx, vy, vz;
                 const double d = __dsqrt_rn(molecule_pair(sh, warp, i, j, vx, vy, vz));
-                write_hits(sh.transpose[warp], in, out, lane, next, n_valid, index_offset + i, index_offset + j, 0, 0, 0, d, vx, vy, vz, false);
+                write_hits<Kind>(sh.transpose[warp], out, lane, next, n_valid, index_offset + i, index_offset + j, 0, 0, 0, d, vx, vy, vz, false);
                 next += static_cast<unsigned long long>(n_valid) * per_hit;
             }
         };
@@ -563,15 +583,16 @@ __device__ __forceinline__ double small_pair(
     return __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
 }
 
-template <bool EMIT>
-__global__ void __launch_bounds__(SMALL_THREADS, 6) small_systems_kernel(
+template <class Kind>
+__global__ void __launch_bounds__(SMALL_THREADS, SMALL_CTAS) small_systems_kernel(
     const BatchInput in, const unsigned splits, unsigned long long* __restrict__ system_count, unsigned long long* __restrict__ share_count,
     const unsigned long long* __restrict__ system_start, PairOutput out, DeviceHeader* header, const unsigned long long capacity
 ) {
+    constexpr bool EMIT = Kind::EMIT;
     __shared__ SmallShared sh;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const unsigned per_hit = in.full ? 2u : 1u;
+    constexpr unsigned per_hit = Kind::FULL ? 2u : 1u;
 
     const unsigned long long n_items = static_cast<unsigned long long>(in.n_systems) * splits;
     for (unsigned long long item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -612,8 +633,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 6) small_systems_kernel(
         const bool usable = frame.singular == 0;
         if (!EMIT && share == 0) {
             for (int k = threadIdx.x; k < n; k += SMALL_THREADS) {
-                const bool finite = isfinite(batch_coordinate(in, 3 * (begin + k) + 0)) && isfinite(batch_coordinate(in, 3 * (begin + k) + 1)) &&
-                                    isfinite(batch_coordinate(in, 3 * (begin + k) + 2));
+                const bool finite = isfinite(batch_coordinate<Kind>(in, 3 * (begin + k) + 0)) && isfinite(batch_coordinate<Kind>(in, 3 * (begin + k) + 1)) &&
+                                    isfinite(batch_coordinate<Kind>(in, 3 * (begin + k) + 2));
                 if (!finite) {
                     atomicOr(&header->status, STATUS_BAD_POINT);
                     atomicMin(&header->first_bad, begin + k);
@@ -627,9 +648,9 @@ __global__ void __launch_bounds__(SMALL_THREADS, 6) small_systems_kernel(
             const int n_home = min(SMALL_TILE, n - i0);
             // everything is seen from the first home point: fractional coordinates, wrap shifts
             // (what they have in common cancels in the shift of a pair) and fp32 positions
-            const double ox = batch_coordinate(in, 3 * (begin + i0) + 0);
-            const double oy = batch_coordinate(in, 3 * (begin + i0) + 1);
-            const double oz = batch_coordinate(in, 3 * (begin + i0) + 2);
+            const double ox = batch_coordinate<Kind>(in, 3 * (begin + i0) + 0);
+            const double oy = batch_coordinate<Kind>(in, 3 * (begin + i0) + 1);
+            const double oz = batch_coordinate<Kind>(in, 3 * (begin + i0) + 2);
             float hx = 0, hy = 0, hz = 0; // the lane's home point, negated
             bool exact_only = false;
             for (int chunk0 = i0; chunk0 < n; chunk0 += SMALL_CHUNK) {
@@ -637,9 +658,9 @@ __global__ void __launch_bounds__(SMALL_THREADS, 6) small_systems_kernel(
                 bool have = j < n;
                 double rx = ox, ry = oy, rz = oz;
                 if (have) {
-                    rx = batch_coordinate(in, 3 * (begin + j) + 0);
-                    ry = batch_coordinate(in, 3 * (begin + j) + 1);
-                    rz = batch_coordinate(in, 3 * (begin + j) + 2);
+                    rx = batch_coordinate<Kind>(in, 3 * (begin + j) + 0);
+                    ry = batch_coordinate<Kind>(in, 3 * (begin + j) + 1);
+                    rz = batch_coordinate<Kind>(in, 3 * (begin + j) + 2);
                     have = isfinite(rx) && isfinite(ry) && isfinite(rz); // others are reported by the counting pass
                 }
                 const double dx = rx - ox, dy = ry - oy, dz = rz - oz;
@@ -836,8 +857,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 6) small_systems_kernel(
                             const double d = __dsqrt_rn(small_pair(
                                 frame, sh.home[0][h], sh.home[1][h], sh.home[2][h], sh.x[image.w], sh.y[image.w], sh.z[image.w], s0, s1, s2, vx, vy, vz
                             ));
-                            write_hits(
-                                sh.transpose[warp], in, out, lane, first + static_cast<unsigned long long>(c0) * per_hit, n_valid, index_offset + i0 + h,
+                            write_hits<Kind>(
+                                sh.transpose[warp], out, lane, first + static_cast<unsigned long long>(c0) * per_hit, n_valid, index_offset + i0 + h,
                                 index_offset + chunk0 + image.w, s0, s1, s2, d, vx, vy, vz,
                                 __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0
                             );
@@ -901,10 +922,38 @@ size_t small_systems_max_points() {
     return 2048;
 }
 
+/// Calls use(kind) with the kind of the launch.
+template <bool EMIT, class Use>
+static void with_kind(const BatchInput& in, bool paired, Use use) {
+    const auto with_type = [&](auto full, auto aligned) {
+        if (in.is_float) {
+            use(BatchKind<EMIT, decltype(full)::value, true, decltype(aligned)::value>{});
+        } else {
+            use(BatchKind<EMIT, decltype(full)::value, false, decltype(aligned)::value>{});
+        }
+    };
+    // (half lists and counts store no pairs side by side)
+    if (!in.full) {
+        with_type(std::false_type{}, std::false_type{});
+    } else if (!EMIT || !paired) {
+        with_type(std::true_type{}, std::false_type{});
+    } else {
+        with_type(std::true_type{}, std::true_type{});
+    }
+}
+
 void configure_small_systems() {
-    const int bytes = static_cast<int>(sizeof(MoleculeShared));
-    cudaFuncSetAttribute(molecules_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(molecules_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    BatchInput in{};
+    for (int k = 0; k < 8; k++) {
+        in.is_float = k & 1;
+        in.full = (k >> 1) & 1;
+        const bool paired = (k >> 2) & 1;
+        const auto allow = [](auto kind) {
+            cudaFuncSetAttribute(molecules_kernel<decltype(kind)>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(MoleculeShared)));
+        };
+        with_kind<false>(in, paired, allow);
+        with_kind<true>(in, paired, allow);
+    }
 }
 
 static unsigned multiprocessors() {
@@ -918,7 +967,7 @@ static unsigned multiprocessors() {
 unsigned small_splits(unsigned n_systems, size_t max_points) {
     // about four waves of CTAs, so that systems of different sizes even out; never more than tiles
     const unsigned tiles = static_cast<unsigned>((max_points + SMALL_TILE - 1) / SMALL_TILE);
-    const unsigned wanted = 4 * 6 * multiprocessors() / std::max(n_systems, 1u);
+    const unsigned wanted = 4 * SMALL_CTAS * multiprocessors() / std::max(n_systems, 1u);
     return std::max(1u, std::min(wanted, tiles));
 }
 
@@ -928,8 +977,7 @@ static unsigned small_grid(unsigned n_systems, unsigned splits) {
 
 static unsigned molecules_grid(unsigned n_systems) {
     const unsigned wanted = (n_systems + MOLECULE_WARPS - 1) / MOLECULE_WARPS;
-    const unsigned cap = multiprocessors() * 8;
-    return wanted < cap ? (wanted ? wanted : 1) : cap;
+    return std::max(1u, std::min(wanted, 1u << 20));
 }
 
 void launch_batch_reset(DeviceHeader* header, cudaStream_t stream) {
@@ -942,15 +990,18 @@ void launch_small_count(
     DeviceHeader* header, cudaStream_t stream
 ) {
     const PairOutput nothing{};
-    molecules_kernel<false><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
-        in, system_count, nullptr, nothing, header, 0ull, nullptr
-    );
-    if (any_for_cta_kernel) {
-        const unsigned splits = small_splits(in.n_systems, max_points);
-        small_systems_kernel<false><<<small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream>>>(
-            in, splits, system_count, share_count, nullptr, nothing, header, 0ull
+    with_kind<false>(in, false, [&](auto kind) {
+        using Kind = decltype(kind);
+        molecules_kernel<Kind><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
+            in, system_count, nullptr, nothing, header, 0ull, nullptr
         );
-    }
+        if (any_for_cta_kernel) {
+            const unsigned splits = small_splits(in.n_systems, max_points);
+            small_systems_kernel<Kind><<<small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream>>>(
+                in, splits, system_count, share_count, nullptr, nothing, header, 0ull
+            );
+        }
+    });
 }
 
 void launch_small_emit(
@@ -959,16 +1010,18 @@ void launch_small_emit(
     DeviceHeader* mirror
 ) {
     // paired stores of full lists need aligned arrays (every system of a full list starts on an even element)
-    out.interleave_ok = paired_stores_fit(out);
-    molecules_kernel<true><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
-        in, nullptr, system_start, out, header, capacity, mirror
-    );
-    if (any_for_cta_kernel) {
-        const unsigned splits = small_splits(in.n_systems, max_points);
-        small_systems_kernel<true><<<small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream>>>(
-            in, splits, nullptr, share_count, system_start, out, header, capacity
+    with_kind<true>(in, paired_stores_fit(out) != 0, [&](auto kind) {
+        using Kind = decltype(kind);
+        molecules_kernel<Kind><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
+            in, nullptr, system_start, out, header, capacity, mirror
         );
-    }
+        if (any_for_cta_kernel) {
+            const unsigned splits = small_splits(in.n_systems, max_points);
+            small_systems_kernel<Kind><<<small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream>>>(
+                in, splits, nullptr, share_count, system_start, out, header, capacity
+            );
+        }
+    });
 }
 
 size_t molecules_max_points() {
