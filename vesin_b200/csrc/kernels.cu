@@ -15,6 +15,7 @@
 #include "emit.cuh"
 
 #include <algorithm>
+#include <type_traits>
 #include <cfloat>
 
 namespace vb200 {
@@ -1008,38 +1009,69 @@ __device__ __forceinline__ bool half_rule(int s0, int s1, int s2) {
     return true;
 }
 
+/// Offset (in cells, relative to the first cell of the unit) of entry `index` of the stencil of a
+/// unit of `cells` cells.
+__device__ __forceinline__ void stencil_offset(const GridPlan& plan, int cells, int index, int& ox, int& oy, int& oz) {
+    const int w0 = cells + 2 * plan.n_search[0];
+    const int w1 = 2 * plan.n_search[1] + 1;
+    ox = index % w0 - plan.n_search[0];
+    oy = (index / w0) % w1 - plan.n_search[1];
+    oz = index / (w0 * w1) - plan.n_search[2];
+}
+
+/// SEGMENTS entries of the stencil of a full-length unit, 10 bits per direction, decoded once per CTA
+/// (where the whole stencil has no more entries). Followed by a barrier of the caller.
+template <int SEGMENTS>
+__device__ __forceinline__ void cache_stencil(const GridPlan& plan, int* offsets) {
+    if (threadIdx.x < SEGMENTS) {
+        int ox, oy, oz;
+        stencil_offset(plan, plan.pencil, threadIdx.x, ox, oy, oz);
+        offsets[threadIdx.x] = ((ox + 512) & 1023) | (((oy + 512) & 1023) << 10) | (((oz + 512) & 1023) << 20);
+    }
+}
+
 /// Fill the table for segment group `group` of a unit. Returns the number of
-/// slots of the group. Ends with a __syncthreads().
-__device__ __forceinline__ int setup_segments(const GridPlan& plan, const int32_t* __restrict__ cell_start, const Unit& unit, int group, SegmentTable& table) {
-    int t = threadIdx.x;
-    int length = 0;
-    const bool one_warp = unit.n_stencil <= 32; // (see setup_half_segments)
-    if (t < (one_warp ? 32 : SEG_MAX)) {
-        int global_t = group * SEG_MAX + t;
+/// slots of the group. Ends with a __syncthreads(). SEGMENTS: 32 or 64 where the launch knows that the
+/// stencil has no more cells (one group, the work of one warp, `offsets` from cache_stencil), else SEG_MAX.
+template <int SEGMENTS>
+__device__ __forceinline__ int setup_segments(
+    const GridPlan& plan, const int32_t* __restrict__ cell_start, const Unit& unit, int group, SegmentTableT<SEGMENTS>& table, const int* offsets
+) {
+    constexpr bool ANY = SEGMENTS == SEG_MAX;
+    const int t = threadIdx.x;
+    const bool one_warp = !ANY || unit.n_stencil <= 32; // (see setup_half_segments)
+    const auto set_entry = [&](int entry, int global_t) -> int {
+        int length = 0;
         int start = 0;
         int q0 = 0, q1 = 0, q2 = 0;
         int self_ok = 0;
         if (global_t < unit.n_stencil) {
-            int w0 = unit.cells + 2 * plan.n_search[0];
-            int w1 = 2 * plan.n_search[1] + 1;
-            int nb[3] = {
-                unit.c0 + (global_t % w0) - plan.n_search[0],
-                unit.c1 + ((global_t / w0) % w1) - plan.n_search[1],
-                unit.c2 + (global_t / (w0 * w1)) - plan.n_search[2],
-            };
+            int ox, oy, oz;
+            if (!ANY && unit.cells == plan.pencil) {
+                const int packed = offsets[entry];
+                ox = (packed & 1023) - 512;
+                oy = ((packed >> 10) & 1023) - 512;
+                oz = (packed >> 20) - 512;
+            } else {
+                stencil_offset(plan, unit.cells, global_t, ox, oy, oz);
+            }
+            int nb[3] = {unit.c0 + ox, unit.c1 + oy, unit.c2 + oz};
             int q[3] = {0, 0, 0};
             bool valid = true;
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                if (plan.periodic[k] && k != plan.window_axis) {
-                    q[k] = floor_div(nb[k], plan.n_cells[k]);
-                    nb[k] -= q[k] * plan.n_cells[k];
-                } else if (nb[k] < 0 || nb[k] >= plan.n_cells[k]) {
+                const bool outside = nb[k] < 0 || nb[k] >= plan.n_cells[k];
+                if (plan.periodic[k] && (!ANY || k != plan.window_axis)) {
+                    if (outside) {
+                        q[k] = floor_div(nb[k], plan.n_cells[k]);
+                        nb[k] -= q[k] * plan.n_cells[k];
+                    }
+                } else if (outside) {
                     valid = false;
                 }
             }
             if (valid) {
-                int linear = (nb[2] * plan.n_cells[1] + nb[1]) * plan.n_cells[0] + nb[0];
+                const int linear = (nb[2] * plan.n_cells[1] + nb[1]) * plan.n_cells[0] + nb[0];
                 start = cell_start[linear];
                 length = cell_start[linear + 1] - start;
                 q0 = q[0];
@@ -1047,41 +1079,57 @@ __device__ __forceinline__ int setup_segments(const GridPlan& plan, const int32_
                 q2 = q[2];
                 // only consulted for a point meeting itself, i.e. in an image
                 // of its own cell: the un-shifted copy is the point itself
-                bool nonzero = (q0 | q1 | q2) != 0;
+                const bool nonzero = (q0 | q1 | q2) != 0;
                 self_ok = nonzero && (plan.full || half_rule(q0, q1, q2));
             }
         }
-        table.start[t] = start;
-        table.image[t] = pack_segment_image(q0, q1, q2, self_ok);
-    }
+        table.start[entry] = start;
+        table.image[entry] = pack_segment_image(q0, q1, q2, self_ok);
+        return length;
+    };
     if (one_warp) {
+        constexpr int ENTRIES = ANY ? 1 : SEGMENTS / 32; // per lane
         if (t < 32) {
-            int inclusive = length;
+            int length[ENTRIES];
 #pragma unroll
-            for (int offset = 1; offset < 32; offset <<= 1) {
-                const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
-                if (t >= offset) {
-                    inclusive += up;
-                }
+            for (int e = 0; e < ENTRIES; e++) {
+                length[e] = set_entry(t + 32 * e, group * SEG_MAX + t + 32 * e);
             }
-            table.slot0[t] = inclusive - length;
+            int before = 0;
+#pragma unroll
+            for (int e = 0; e < ENTRIES; e++) {
+                int inclusive = length[e];
+#pragma unroll
+                for (int offset = 1; offset < 32; offset <<= 1) {
+                    const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
+                    if (t >= offset) {
+                        inclusive += up;
+                    }
+                }
+                table.slot0[t + 32 * e] = before + inclusive - length[e];
+                before += __shfl_sync(FULL_MASK, inclusive, 31);
+            }
             if (t == 31) {
-                table.slot0[32] = inclusive;
+                table.slot0[32 * ENTRIES] = before;
             }
         }
         __syncthreads();
-        return table.slot0[32];
+        return table.slot0[32 * ENTRIES];
     }
-    int prefix = block_exclusive_scan<SEG_MAX / 32>(length, table.scan_tmp);
-    if (t < SEG_MAX) {
-        table.slot0[t] = prefix;
+    if constexpr (ANY) {
+        const int length = (t < SEG_MAX) ? set_entry(t, group * SEG_MAX + t) : 0;
+        const int prefix = block_exclusive_scan<SEG_MAX / 32>(length, table.scan_tmp);
+        if (t < SEG_MAX) {
+            table.slot0[t] = prefix;
+        }
+        const int total = table.scan_tmp[CTA_WARPS];
+        if (t == 0) {
+            table.slot0[SEG_MAX] = total;
+        }
+        __syncthreads();
+        return total;
     }
-    int total = table.scan_tmp[CTA_WARPS];
-    if (t == 0) {
-        table.slot0[SEG_MAX] = total;
-    }
-    __syncthreads();
-    return total;
+    return 0; // (not reached)
 }
 
 /// Segment that holds `slot`: last t with slot0[t] <= slot, among the first
@@ -1102,6 +1150,16 @@ __device__ __forceinline__ int find_segment(const SegmentTableT<ENTRIES>& table,
         }
     }
     return lo;
+}
+
+/// The same for a unit whose launch knows the size of stencils, or not (SEG_MAX).
+template <int SEGMENTS>
+__device__ __forceinline__ int segment_of(const SegmentTableT<SEGMENTS>& table, const Unit& unit, int slot) {
+    if constexpr (SEGMENTS == SEG_MAX) {
+        return (unit.n_stencil <= 32) ? find_segment<5>(table, slot) : find_segment<7>(table, slot);
+    } else {
+        return find_segment<(SEGMENTS == 32) ? 5 : 6>(table, slot);
+    }
 }
 
 /// The reference's pair vector and squared distance, operation for operation:
@@ -2220,8 +2278,10 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
 /// and the claim of storage is on its way while the candidates are staged: 216k crystal 156 -> 127
 /// us, 262k liquid 146 -> 118, its half list 250 -> 193.
 /// RANKED: the candidates of a unit, which all fit a batch, are staged in the order of their indices.
-template <bool FULL_, bool RANKED_, int BATCH_, int CTAS_PER_SM_>
+/// SEGMENTS: see setup_segments.
+template <bool FULL_, bool RANKED_, int BATCH_, int CTAS_PER_SM_, int SEGMENTS_>
 struct RowCountShape {
+    static constexpr int SEGMENTS = SEGMENTS_;
     static constexpr bool FULL = FULL_;
     static constexpr bool RANKED = RANKED_;
     static constexpr int BATCH = BATCH_;
@@ -2238,7 +2298,8 @@ struct RowCountShape {
             };
             typename std::conditional<RANKED_, Ordering<BATCH_>, Nothing>::type ordering;
         };
-        SegmentTable table;
+        SegmentTableT<SEGMENTS_> table;
+        int offsets[SEGMENTS_]; // of the stencil of a full-length unit
         int index[FULL_ ? 1 : BATCH_];                    // half lists: indices of the candidates
         int4 home_sj[TILE_POINTS];                        // x, y, z: wrap shift of the home point; w: its index
         unsigned mask[WORDS * TILE_POINTS];               // [word][lane]
@@ -2270,12 +2331,14 @@ __device__ __forceinline__ bool row_keeps(const int4& home, const int4& candidat
 
 /// Words of hit bits one home point of the unit needs: every segment group
 /// starts on a fresh word. Leaves the table of the LAST group in place.
+template <int SEGMENTS>
 __device__ __forceinline__ int row_words_of_unit(
-    const GridPlan& plan, const int32_t* __restrict__ cell_start, const Unit& unit, int n_groups, SegmentTable& table, int& last_total
+    const GridPlan& plan, const int32_t* __restrict__ cell_start, const Unit& unit, int n_groups, SegmentTableT<SEGMENTS>& table,
+    const int* offsets, int& last_total
 ) {
     int words = 0;
     for (int g = 0; g < n_groups; g++) {
-        last_total = setup_segments(plan, cell_start, unit, g, table);
+        last_total = setup_segments(plan, cell_start, unit, g, table, offsets);
         words += (last_total + 31) >> 5;
     }
     return words;
@@ -2306,6 +2369,10 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
     if (threadIdx.x < TILE_POINTS) {
         sh.tile_hits[threadIdx.x] = 0;
     }
+    if (Shape::SEGMENTS != SEG_MAX) {
+        cache_stencil<Shape::SEGMENTS>(plan, sh.offsets);
+        __syncthreads();
+    }
     unsigned most_candidates = 0; // of the units of this CTA
 
     for (int u = blockIdx.x; u < plan.n_units; u += gridDim.x) {
@@ -2313,7 +2380,7 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
         if (unit.n_home == 0) {
             continue;
         }
-        const int n_groups = (unit.n_stencil + SEG_MAX - 1) / SEG_MAX;
+        const int n_groups = (Shape::SEGMENTS == SEG_MAX) ? (unit.n_stencil + SEG_MAX - 1) / SEG_MAX : 1;
         const int n_tiles = (unit.n_home + TILE_POINTS - 1) / TILE_POINTS;
         if (threadIdx.x < 3) {
             const int c = threadIdx.x;
@@ -2322,7 +2389,7 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
         }
 
         int group_total = 0;
-        const int words = row_words_of_unit(plan, cell_start, unit, n_groups, sh.table, group_total);
+        const int words = row_words_of_unit(plan, cell_start, unit, n_groups, sh.table, sh.offsets, group_total);
         if (RANKED) {
             const bool rankable = n_groups == 1 && unit.n_home <= RANKED_HOME;
             most_candidates = max(most_candidates, rankable ? static_cast<unsigned>(group_total) : 0xffffffffu);
@@ -2351,7 +2418,7 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
         int word_base = 0;
         for (int g = 0; g < n_groups; g++) {
             if (n_groups > 1) {
-                group_total = setup_segments(plan, cell_start, unit, g, sh.table);
+                group_total = setup_segments(plan, cell_start, unit, g, sh.table, sh.offsets);
             }
             const int own_slot0 = (g == own_group) ? sh.table.slot0[own_entry % SEG_MAX] : 0;
             for (int batch0 = 0; batch0 < group_total; batch0 += BATCH) {
@@ -2360,7 +2427,7 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
                 // candidate in a slot of the batch, as it lies in the cell-sorted records: image
                 // minus wrap shift and index
                 const auto position_of = [&](int slot, int& t) {
-                    t = (unit.n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
+                    t = segment_of(sh.table, unit, slot);
                     return static_cast<size_t>(sh.table.start[t]) + (slot - sh.table.slot0[t]);
                 };
                 const auto fetch = [&](int s, LoadedRecord& record) {
@@ -2584,8 +2651,11 @@ constexpr int ROW_EMIT_WARPS = ROW_EMIT_THREADS / 32;
 /// candidates themselves stay in L1, where a lane fetches the record of its hit: staging all of them
 /// first (40 bytes each, which left room for 4 CTAs of 8 warps) was a third of the kernel. 216k
 /// crystal 316 -> 302 us, 262k liquid 250 -> 231, its half list 208 -> 185.
-template <int BATCH_, int CTAS_PER_SM_>
+/// SEGMENTS: see setup_segments. VALUES: see store_pairs.
+template <int BATCH_, int CTAS_PER_SM_, int SEGMENTS_, int VALUES_>
 struct RowShape {
+    static constexpr int SEGMENTS = SEGMENTS_;
+    static constexpr int VALUES = VALUES_;
     static constexpr int BATCH = BATCH_;
     static constexpr int WORDS = BATCH_ / 32;
     static constexpr int LANE_WORDS = (WORDS + 31) / 32; // consecutive words of a row that a lane looks after
@@ -2599,15 +2669,17 @@ struct RowShape {
         unsigned short list[ROW_EMIT_WARPS][ROW_WINDOW];
         int position[BATCH_];           // of the candidate among the cell-sorted points; IS_IMAGE: in a shifted cell
         unsigned char segment[BATCH_];  // the segment it comes from
-        SegmentTable table;
+        SegmentTableT<SEGMENTS_> table;
+        int offsets[SEGMENTS_];         // of the stencil of a full-length unit
         double home_pos[3][TILE_POINTS];
         int4 home_sj[TILE_POINTS];                // x, y, z: wrap shift of the home point; w: its index
         unsigned long long home_row[TILE_POINTS]; // where the row of a home point continues
     };
     static_assert((sizeof(Shared) + 1024) * CTAS_PER_SM_ <= 228 * 1024, "CTAS_PER_SM CTAs fit on an SM");
 };
-using SortedRows = RowShape<1024, 8>;
-using SortedRowsWide = RowShape<2048, 8>;
+template <int SEGMENTS, int VALUES>
+using SortedRows = RowShape<1024, 8, SEGMENTS, VALUES>;
+using SortedRowsWide = RowShape<2048, 8, SEG_MAX, -1>;
 
 /// Hits [from, to) of a row whose words lie in shared memory, lane l being the one that counted the
 /// LANE_WORDS words from l * LANE_WORDS on (`begin`: hits before them): use(number, slot) for each,
@@ -2687,24 +2759,28 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
+    if (Shape::SEGMENTS != SEG_MAX) {
+        cache_stencil<Shape::SEGMENTS>(plan, sh.offsets);
+        __syncthreads();
+    }
 
     for (int u = blockIdx.x; u < plan.n_units; u += gridDim.x) {
         const Unit unit = unit_of(plan, cell_start, u);
         if (unit.n_home == 0) {
             continue;
         }
-        const int n_groups = (unit.n_stencil + SEG_MAX - 1) / SEG_MAX;
+        const int n_groups = (Shape::SEGMENTS == SEG_MAX) ? (unit.n_stencil + SEG_MAX - 1) / SEG_MAX : 1;
         const int n_tiles = (unit.n_home + TILE_POINTS - 1) / TILE_POINTS;
         const unsigned long long base = unit_mask_base[u];
         const int words = static_cast<int>(unit_words[u]);
 
         int word_base = 0;
         for (int g = 0; g < n_groups; g++) {
-            const int group_total = setup_segments(plan, cell_start, unit, g, sh.table);
+            const int group_total = setup_segments(plan, cell_start, unit, g, sh.table, sh.offsets);
             // (a row whose candidates come in several batches is continued from batch to batch)
             const bool continued = n_groups > 1 || group_total > BATCH;
             const auto record_of = [&](int slot, int& t) {
-                t = (unit.n_stencil <= 32) ? find_segment<5>(sh.table, slot) : find_segment<7>(sh.table, slot);
+                t = segment_of(sh.table, unit, slot);
                 return static_cast<size_t>(sh.table.start[t]) + (slot - sh.table.slot0[t]);
             };
             for (int batch0 = 0; batch0 < group_total; batch0 += BATCH) {
@@ -2788,7 +2864,7 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
                                     vz = __dadd_rn(__dsub_rn(cand.z, hz), plan.zero_shift[2]);
                                     d2 = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
                                 }
-                                store_pairs(
+                                store_pairs<Shape::VALUES>(
                                     sh.transpose[warp], out, lane, row + static_cast<unsigned long long>(window + c0), n_valid,
                                     static_cast<unsigned long long>(home.w), static_cast<unsigned long long>(cand.index), s0, s1, s2, __dsqrt_rn(d2), vx,
                                     vy, vz, shifted
@@ -3075,24 +3151,50 @@ int pair_grid(int n_units, int per_sm) {
 // ---------------------------------------------------------------------------
 
 namespace {
-template <bool FULL>
-using RowCount = RowCountShape<FULL, false, 1024, 8>;
-template <bool FULL>
-using RankedCount = RowCountShape<FULL, true, 1024, FULL ? 8 : 7>;
-template <bool FULL>
-using RankedCountWide = RowCountShape<FULL, true, 2048, 4>;
+template <bool FULL, int SEGMENTS>
+using RowCount = RowCountShape<FULL, false, 1024, 8, SEGMENTS>;
+template <bool FULL, int SEGMENTS>
+using RankedCount = RowCountShape<FULL, true, 1024, FULL ? 8 : 7, SEGMENTS>;
+template <bool FULL, int SEGMENTS>
+using RankedCountWide = RowCountShape<FULL, true, 2048, 4, SEGMENTS>;
+constexpr int RANKED_BATCH = 1024;
+constexpr int RANKED_BATCH_WIDE = 2048;
+constexpr int ROW_BATCH = 1024;
+constexpr int ROW_BATCH_WIDE = 2048;
+
+/// Calls use(entries) with the room that the stencil of every unit fits: 32, 64 or any (SEG_MAX).
+template <class Use>
+void with_segments(const GridPlan& plan, Use use) {
+    const long long cells = static_cast<long long>(plan.pencil + 2 * plan.n_search[0]) * (2 * plan.n_search[1] + 1) * (2 * plan.n_search[2] + 1);
+    if (cells <= 32) {
+        use(std::integral_constant<int, 32>{});
+    } else if (cells <= 64) {
+        use(std::integral_constant<int, 64>{});
+    } else {
+        use(std::integral_constant<int, SEG_MAX>{});
+    }
+}
 } // namespace
 
 void configure_kernels() {
     const auto allow = [](auto kernel, size_t bytes) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)); };
-    allow(row_emit_kernel<SortedRows>, sizeof(SortedRows::Shared));
     allow(row_emit_kernel<SortedRowsWide>, sizeof(SortedRowsWide::Shared));
-    allow(row_count_kernel<RowCount<true>>, sizeof(RowCount<true>::Shared));
-    allow(row_count_kernel<RowCount<false>>, sizeof(RowCount<false>::Shared));
-    allow(row_count_kernel<RankedCount<true>>, sizeof(RankedCount<true>::Shared));
-    allow(row_count_kernel<RankedCount<false>>, sizeof(RankedCount<false>::Shared));
-    allow(row_count_kernel<RankedCountWide<true>>, sizeof(RankedCountWide<true>::Shared));
-    allow(row_count_kernel<RankedCountWide<false>>, sizeof(RankedCountWide<false>::Shared));
+    const auto allow_rows = [&](auto segments) {
+        constexpr int SEGMENTS = decltype(segments)::value;
+        const auto allow_count = [&](auto shape) { allow(row_count_kernel<decltype(shape)>, sizeof(typename decltype(shape)::Shared)); };
+        const auto allow_emit = [&](auto shape) { allow(row_emit_kernel<decltype(shape)>, sizeof(typename decltype(shape)::Shared)); };
+        allow_count(RowCount<true, SEGMENTS>{});
+        allow_count(RowCount<false, SEGMENTS>{});
+        allow_count(RankedCount<true, SEGMENTS>{});
+        allow_count(RankedCount<false, SEGMENTS>{});
+        allow_count(RankedCountWide<true, SEGMENTS>{});
+        allow_count(RankedCountWide<false, SEGMENTS>{});
+        allow_emit(SortedRows<SEGMENTS, 0>{});
+        allow_emit(SortedRows<SEGMENTS, 1>{});
+    };
+    allow_rows(std::integral_constant<int, 32>{});
+    allow_rows(std::integral_constant<int, 64>{});
+    allow_rows(std::integral_constant<int, SEG_MAX>{});
     const auto allow_plain = [&](auto shape) {
         using Shape = decltype(shape);
         allow(pairs_kernel<false, false, 0, Shape>, sizeof(typename Shape::Shared));
@@ -3246,25 +3348,31 @@ void launch_count(
             plan, cell_start, sorted, masks, mask_capacity, unit_mask_base, unit_words, row_count, header
         );
     };
-    if (ranked_batch == 0) {
-        plan.full ? launch(RowCount<true>{}, row_count_kernel<RowCount<true>>) : launch(RowCount<false>{}, row_count_kernel<RowCount<false>>);
-    } else if (ranked_batch == RankedCount<true>::BATCH) {
-        plan.full ? launch(RankedCount<true>{}, row_count_kernel<RankedCount<true>>) : launch(RankedCount<false>{}, row_count_kernel<RankedCount<false>>);
-    } else {
-        plan.full ? launch(RankedCountWide<true>{}, row_count_kernel<RankedCountWide<true>>)
-                  : launch(RankedCountWide<false>{}, row_count_kernel<RankedCountWide<false>>);
-    }
+    const auto launch_kind = [&](auto full) {
+        constexpr bool FULL = decltype(full)::value;
+        with_segments(plan, [&](auto segments) {
+            constexpr int SEGMENTS = decltype(segments)::value;
+            if (ranked_batch == 0) {
+                launch(RowCount<FULL, SEGMENTS>{}, row_count_kernel<RowCount<FULL, SEGMENTS>>);
+            } else if (ranked_batch == RANKED_BATCH) {
+                launch(RankedCount<FULL, SEGMENTS>{}, row_count_kernel<RankedCount<FULL, SEGMENTS>>);
+            } else {
+                launch(RankedCountWide<FULL, SEGMENTS>{}, row_count_kernel<RankedCountWide<FULL, SEGMENTS>>);
+            }
+        });
+    };
+    plan.full ? launch_kind(std::true_type{}) : launch_kind(std::false_type{});
 }
 
 int ranked_count_batch(double candidates) {
-    if (candidates <= RankedCount<true>::BATCH) {
-        return RankedCount<true>::BATCH;
+    if (candidates <= RANKED_BATCH) {
+        return RANKED_BATCH;
     }
-    return (candidates <= RankedCountWide<true>::BATCH) ? RankedCountWide<true>::BATCH : 0;
+    return (candidates <= RANKED_BATCH_WIDE) ? RANKED_BATCH_WIDE : 0;
 }
 
 int row_batch(unsigned max_candidates) {
-    return (max_candidates > SortedRows::BATCH && max_candidates <= SortedRowsWide::BATCH) ? SortedRowsWide::BATCH : SortedRows::BATCH;
+    return (max_candidates > ROW_BATCH && max_candidates <= ROW_BATCH_WIDE) ? ROW_BATCH_WIDE : ROW_BATCH;
 }
 
 void launch_emit(
@@ -3278,11 +3386,18 @@ void launch_emit(
             plan, cell_start, sorted, masks, unit_mask_base, unit_words, row_start, row_fill, out, ranked ? 1 : 0
         );
     };
-    if (row_batch(max_candidates) == SortedRows::BATCH) {
-        launch(SortedRows{}, row_emit_kernel<SortedRows>);
-    } else {
+    if (row_batch(max_candidates) == ROW_BATCH_WIDE) {
         launch(SortedRowsWide{}, row_emit_kernel<SortedRowsWide>);
+        return;
     }
+    with_segments(plan, [&](auto segments) {
+        constexpr int SEGMENTS = decltype(segments)::value;
+        if (out.values_float) {
+            launch(SortedRows<SEGMENTS, 1>{}, row_emit_kernel<SortedRows<SEGMENTS, 1>>);
+        } else {
+            launch(SortedRows<SEGMENTS, 0>{}, row_emit_kernel<SortedRows<SEGMENTS, 0>>);
+        }
+    });
 }
 
 void launch_sort_rows(
