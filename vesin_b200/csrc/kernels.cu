@@ -2363,15 +2363,17 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const Screen screen = screen_of(plan);
-    if (header->status & STATUS_ABORT_MASK) {
-        return;
-    }
     if (threadIdx.x < TILE_POINTS) {
         sh.tile_hits[threadIdx.x] = 0;
     }
     if (Shape::SEGMENTS != SEG_MAX) {
         cache_stencil<Shape::SEGMENTS>(plan, sh.offsets);
         __syncthreads();
+    }
+    let_next_kernel_start();
+    wait_for_previous_kernel();
+    if (header->status & STATUS_ABORT_MASK) {
+        return;
     }
     unsigned most_candidates = 0; // of the units of this CTA
 
@@ -2748,7 +2750,7 @@ template <class Shape>
 __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, const uint32_t* __restrict__ masks,
     const unsigned long long* __restrict__ unit_mask_base, const uint32_t* __restrict__ unit_words,
-    const unsigned long long* __restrict__ row_start, uint32_t* __restrict__ row_fill, PairOutput out, const int ranked
+    const unsigned long long* __restrict__ row_start, uint32_t* __restrict__ row_fill, PairOutput out, const int ranked, const RowLimits limits
 ) {
     using Shared = typename Shape::Shared;
     constexpr int BATCH = Shape::BATCH;
@@ -2762,6 +2764,12 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
     if (Shape::SEGMENTS != SEG_MAX) {
         cache_stencil<Shape::SEGMENTS>(plan, sh.offsets);
         __syncthreads();
+    }
+    wait_for_previous_kernel();
+    if (limits.header != nullptr &&
+        ((limits.header->status & (STATUS_ABORT_MASK | STATUS_MASK_OVERFLOW)) != 0 || limits.header->total_pairs > limits.capacity ||
+         limits.header->max_candidates > limits.candidates)) {
+        return; // (launched before the host knew: it decides or writes again)
     }
 
     for (int u = blockIdx.x; u < plan.n_units; u += gridDim.x) {
@@ -3344,8 +3352,9 @@ void launch_count(
 ) {
     const auto launch = [&](auto shape, auto kernel) {
         using Shape = decltype(shape);
-        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_COUNT_THREADS, sizeof(typename Shape::Shared), stream>>>(
-            plan, cell_start, sorted, masks, mask_capacity, unit_mask_base, unit_words, row_count, header
+        launch_chained(
+            kernel, pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_COUNT_THREADS, sizeof(typename Shape::Shared), stream, plan, cell_start, sorted, masks,
+            mask_capacity, unit_mask_base, unit_words, row_count, header
         );
     };
     const auto launch_kind = [&](auto full) {
@@ -3378,12 +3387,13 @@ int row_batch(unsigned max_candidates) {
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
     const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, unsigned max_candidates, bool ranked,
-    cudaStream_t stream
+    cudaStream_t stream, RowLimits limits
 ) {
     const auto launch = [&](auto shape, auto kernel) {
         using Shape = decltype(shape);
-        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_EMIT_THREADS, sizeof(typename Shape::Shared), stream>>>(
-            plan, cell_start, sorted, masks, unit_mask_base, unit_words, row_start, row_fill, out, ranked ? 1 : 0
+        launch_chained(
+            kernel, pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_EMIT_THREADS, sizeof(typename Shape::Shared), stream, plan, cell_start, sorted, masks,
+            unit_mask_base, unit_words, row_start, row_fill, out, ranked ? 1 : 0, limits
         );
     };
     if (row_batch(max_candidates) == ROW_BATCH_WIDE) {

@@ -242,10 +242,17 @@ int ranked_count_batch(double candidates);
 /// per point in index order (row_start from the scan of row_count; row_fill
 /// must start at zero when a unit has more than row_batch() candidates, and is not looked at
 /// otherwise). `ranked`: pass 1 ranked the candidates, and the rows come out sorted by the second index.
+/// `limits` with a header: the pass is launched before the host has seen what pass 1 found, and does
+/// nothing if that is beyond them.
+struct RowLimits {
+    const DeviceHeader* header = nullptr;
+    unsigned long long capacity = 0; // pairs the arrays hold
+    unsigned candidates = 0;         // candidates of a unit that this launch was made for
+};
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
     const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, unsigned max_candidates, bool ranked,
-    cudaStream_t stream
+    cudaStream_t stream, RowLimits limits = {}
 );
 int row_batch(unsigned max_candidates);
 
