@@ -98,3 +98,36 @@ def test_diamond_512k_canonical():
     assert torch.equal(S, cS[order])
     assert torch.equal(d, torch.from_numpy(cpu["d"]).to(device)[order])
     assert torch.equal(D, torch.from_numpy(cpu["D"]).to(device)[order])
+
+
+@pytest.mark.parametrize("full", [True, False])
+@pytest.mark.parametrize("ratio", [2.05, 2.5, 2.95, 3.1, 4.5])
+def test_points_that_are_candidates_twice(ratio, full, monkeypatch):
+    """Two cells per direction: a point is among the candidates of a unit with several images."""
+    monkeypatch.setenv("VESIN_CUDA_MAX_PAIRS_PER_POINT", "100000")
+    rng = np.random.default_rng(int(100 * ratio))
+    cutoff = 3.0
+    box = ratio * cutoff * np.eye(3)
+    points = rng.uniform(0.0, ratio * cutoff, (120, 3))
+    _check_order(points, box, cutoff, full)
+
+
+@pytest.mark.parametrize("cells,shuffled", [(19, False), (20, False), (20, True)])
+def test_ranges_of_indices(cells, shuffled):
+    """Units whose indices lie within what has a bit each (61 440), and beyond."""
+    points, box, _ = W.diamond(cells, seed=cells)
+    if shuffled:
+        points = points[np.random.default_rng(0).permutation(len(points))]
+    _check_order(points, box, 3.0, True)
+
+
+def _check_order(points, box, cutoff, full):
+    import torch
+    import vesin_b200
+
+    calculator = vesin_b200.NeighborList(cutoff, full, canonical=True)
+    expected = O.canonical(O.restated_neighbors(points, box, [True] * 3, cutoff, full, "ijSdD"))
+    for _ in range(2):
+        values = calculator.compute(torch.tensor(points, device="cuda"), torch.tensor(box, device="cuda"), True, "ijSdD")
+        for key, value in zip("ijSdD", values):
+            assert np.array_equal(value.cpu().numpy().astype(expected[key].dtype), expected[key]), key

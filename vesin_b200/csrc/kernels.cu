@@ -2166,7 +2166,9 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
 // in the order the candidates were staged.
 // ---------------------------------------------------------------------------
 
-constexpr int RANK_BUCKETS = 2048; // see rank_candidates (216k crystal, ranking kernel of 8 warps: 1024 527 us, 2048 513, 4096 534)
+// see rank_candidates: 15 consecutive buckets per thread, an odd number, which keeps the threads of a
+// scan out of each other's banks
+constexpr int RANK_BUCKETS = 1920;
 constexpr int RANKED_HOME = 256;   // home points of a unit whose candidates are ranked, at most
 
 /// What ranking the candidates of a unit needs, before they are staged.
@@ -2194,6 +2196,85 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
     constexpr int PER_THREAD = (BATCH + THREADS - 1) / THREADS;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
+    const unsigned least_index = o.least;
+    const unsigned range = o.most - least_index;
+    if (range < 32u * RANK_BUCKETS) {
+        // Indices close enough together that a bucket can have a bit for each: the rank of a candidate is the
+        // start of its bucket plus the bits below its own. (Units of up to 64k points, and of larger crystals in lattice
+        // order, whose runs of indices make for long comparisons below: 216k crystal, deciding pass 211 -> 171 us.)
+        static_assert(offsetof(Ordering<BATCH>, gathered) == BATCH * sizeof(unsigned) && 2 * BATCH >= RANK_BUCKETS, "the keys make room for the bits");
+        static_assert(RANK_BUCKETS % THREADS == 0 && (RANK_BUCKETS / THREADS) % 2 == 1, "an odd number of buckets per thread");
+        unsigned* bits = o.key;
+        unsigned key[PER_THREAD];
+#pragma unroll
+        for (int e = 0; e < PER_THREAD; e++) {
+            const int s = threadIdx.x + e * THREADS;
+            key[e] = (s < n) ? o.key[s] - least_index : 0u;
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < RANK_BUCKETS; k += THREADS) {
+            bits[k] = 0;
+        }
+        __syncthreads();
+        bool twice = false; // images of one point: no bit for each
+#pragma unroll
+        for (int e = 0; e < PER_THREAD; e++) {
+            const int s = threadIdx.x + e * THREADS;
+            if (s < n) {
+                const unsigned bit = 1u << (key[e] & 31u);
+                twice = twice || (atomicOr(&bits[key[e] >> 5], bit) & bit) != 0;
+            }
+        }
+        if (!__syncthreads_or(twice ? 1 : 0)) {
+            constexpr int SCAN = RANK_BUCKETS / THREADS;
+            int mine = 0;
+#pragma unroll
+            for (int e = 0; e < SCAN; e++) {
+                mine += __popc(bits[threadIdx.x * SCAN + e]);
+            }
+            int inclusive = mine;
+#pragma unroll
+            for (int offset = 1; offset < 32; offset <<= 1) {
+                const int up = __shfl_up_sync(FULL_MASK, inclusive, offset);
+                if (lane >= offset) {
+                    inclusive += up;
+                }
+            }
+            if (lane == 31) {
+                scan_tmp[warp] = inclusive;
+            }
+            __syncthreads();
+            int start = inclusive - mine;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) {
+                start += (w < warp) ? scan_tmp[w] : 0;
+            }
+#pragma unroll
+            for (int e = 0; e < SCAN; e++) {
+                o.first[threadIdx.x * SCAN + e] = start;
+                start += __popc(bits[threadIdx.x * SCAN + e]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int e = 0; e < PER_THREAD; e++) {
+                const int s = threadIdx.x + e * THREADS;
+                if (s < n) {
+                    const unsigned below = bits[key[e] >> 5] & ((1u << (key[e] & 31u)) - 1u);
+                    order[o.first[key[e] >> 5] + __popc(below)] = static_cast<unsigned short>(s);
+                }
+            }
+            __syncthreads();
+            return;
+        }
+#pragma unroll
+        for (int e = 0; e < PER_THREAD; e++) {
+            const int s = threadIdx.x + e * THREADS;
+            if (s < n) {
+                o.key[s] = key[e] + least_index;
+            }
+        }
+        __syncthreads();
+    }
     // (rounding is monotonic: a larger index never falls into an earlier bucket)
     const float scale = static_cast<float>(RANK_BUCKETS) / (static_cast<float>(o.most - o.least) + 1.0f);
     const unsigned least = o.least;
