@@ -110,6 +110,7 @@ struct Workspace {
     DeviceBuffer masks, unit_mask_base, unit_words, unit_count, unit_start;
     DeviceBuffer row_count, row_start, row_fill, scan_tmp;
     DeviceBuffer batch_offsets; // batches: where each system starts in the points array
+    DeviceBuffer batch_frames;  // ... and the box, its inverse and the reach of each
     DeviceBuffer batch_shares;  // ... and the pairs each of the CTAs that share a system has
     DeviceBuffer checksum;      // 4 words of vesin_b200_list_checksum
     bool values_float = false;  // element type of `distances` / `vectors` of the last build
@@ -177,7 +178,7 @@ struct Workspace {
     ~Workspace() {
         for (DeviceBuffer* buffer :
              {&rank, &cell_count, &cell_start, &sorted_records, &sorted_wide_shift, &masks, &unit_mask_base,
-              &unit_words, &unit_count, &unit_start, &row_count, &row_start, &row_fill, &scan_tmp, &batch_offsets, &batch_shares, &checksum, &out_pairs,
+              &unit_words, &unit_count, &unit_start, &row_count, &row_start, &row_fill, &scan_tmp, &batch_offsets, &batch_frames, &batch_shares, &checksum, &out_pairs,
               &out_shifts, &out_distances, &out_vectors, &alt_pairs, &alt_shifts, &alt_distances, &alt_vectors}) {
             buffer->release();
         }
@@ -1240,8 +1241,6 @@ void neighbors_batch(
             ws.batch_offsets.ptr, ws.batch_offsets_host.data(), (n_systems + 1) * sizeof(size_t), cudaMemcpyHostToDevice, stream
         ));
     }
-    launch_batch_reset(ws.d_header, stream);
-
     BatchInput in{};
     in.points = points;
     in.is_float = float_io ? 1 : 0;
@@ -1258,7 +1257,10 @@ void neighbors_batch(
     const bool any_for_cta_kernel = periodic != nullptr || largest > molecules_max_points();
     if (any_for_cta_kernel && n_systems > 0) {
         ws.batch_shares.reserve(n_systems * small_splits(in.n_systems, largest) * sizeof(unsigned long long));
+        ws.batch_frames.reserve(n_systems * small_frame_bytes());
+        in.frames = ws.batch_frames.ptr;
     }
+    launch_batch_front(in, any_for_cta_kernel && n_systems > 0, ws.d_header, stream);
     auto* share_count = ws.batch_shares.as<unsigned long long>();
     Target target(list, ws, options, float_io, caller);
     // A list that was filled before writes into the arrays it has, right behind the counting pass

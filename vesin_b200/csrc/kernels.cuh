@@ -292,6 +292,7 @@ struct BatchInput {
     const unsigned long long* offsets; // [n_systems + 1], device memory
     const void* boxes;                 // [n_systems][9], double or float, or null (then nothing is periodic)
     const bool* periodic;              // [n_systems][3] or null (then nothing is periodic)
+    void* frames;                      // small_frame_bytes() per system: what launch_batch_front makes of the boxes
     unsigned n_systems;
     double cutoff;
     double cutoff2;
@@ -304,7 +305,8 @@ struct BatchInput {
 size_t small_systems_max_points();
 void configure_small_systems();
 /// Header of a batch: nothing found yet (first_bad, mask_cursor: the largest values).
-void launch_batch_reset(DeviceHeader* header, cudaStream_t stream);
+void launch_batch_front(const BatchInput& in, bool any_for_cta_kernel, DeviceHeader* header, cudaStream_t stream);
+size_t small_frame_bytes();
 /// Pass 1: pairs of every system -> system_count; the first non-finite point
 /// and the first singular box are reported through the header.
 /// (`any_for_cta_kernel`: some system is periodic or has more points than

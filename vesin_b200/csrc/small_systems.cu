@@ -388,15 +388,37 @@ __device__ __forceinline__ void write_hits(
     }
 }
 
-/// Header of a batch: nothing found yet.
-__global__ void batch_header_kernel(DeviceHeader* header) {
-    if (threadIdx.x < sizeof(DeviceHeader) / 4) {
-        reinterpret_cast<unsigned*>(header)[threadIdx.x] = 0;
+constexpr int FRONT_THREADS = 256;
+
+/// Header of a batch: nothing found yet. And the frames of the systems of the CTA kernel, a warp each:
+/// the box, its inverse and the reach are a chain of divisions and roots that every CTA of both
+/// passes went through before it did anything else (512 cells, both passes: 108.5 -> 98.4 us, and 1.8 here).
+__global__ void __launch_bounds__(FRONT_THREADS) batch_front_kernel(const BatchInput in, SystemFrame* __restrict__ frames, DeviceHeader* header) {
+    __shared__ SystemFrame sh_frames[FRONT_THREADS / 32];
+    if (blockIdx.x == 0) {
+        if (threadIdx.x < sizeof(DeviceHeader) / 4) {
+            reinterpret_cast<unsigned*>(header)[threadIdx.x] = 0;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            header->first_bad = NO_BAD_POINT;
+            header->mask_cursor = ~0ull; // first singular system
+        }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        header->first_bad = NO_BAD_POINT;
-        header->mask_cursor = ~0ull; // first singular system
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const unsigned warps_in_grid = gridDim.x * (FRONT_THREADS / 32);
+    for (unsigned system = blockIdx.x * (FRONT_THREADS / 32) + warp; frames != nullptr && system < in.n_systems; system += warps_in_grid) {
+        const int n = static_cast<int>(in.offsets[system + 1] - in.offsets[system]);
+        if (taken_by_warp_kernel(in, system, n)) {
+            continue;
+        }
+        SystemFrame& frame = sh_frames[warp];
+        make_frame(frame, in, system, lane);
+        for (int k = lane; k < static_cast<int>(sizeof(SystemFrame) / 4); k += 32) {
+            reinterpret_cast<unsigned*>(frames + system)[k] = reinterpret_cast<const unsigned*>(&frame)[k];
+        }
+        __syncwarp();
     }
 }
 
@@ -536,8 +558,8 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32, Kind::EMIT ? 16 : 20) mol
 // (box, points, scan, stage) for the few thousand tiles that a batch of
 // hundreds of cells has; the work itself is the emission of the hits.
 // Several CTAs share the tiles of a system when the systems alone would not
-// fill the GPU. 512 cells of 4 to 200 atoms (5 A cutoff, 2.8 M pairs): 36 us to
-// count and 75 us to write; exact arithmetic on every image of every pair, a CTA
+// fill the GPU. 512 cells of 4 to 200 atoms (5 A cutoff, 2.8 M pairs): 31 us to
+// count and 67 us to write; exact arithmetic on every image of every pair, a CTA
 // per system, took 640 and 954.
 
 constexpr int SMALL_CHUNK = SMALL_THREADS; // points whose images are listed at a time
@@ -613,8 +635,10 @@ __global__ void __launch_bounds__(SMALL_THREADS, SMALL_CTAS) small_systems_kerne
             continue; // as in the warp kernel
         }
         __syncthreads(); // previous item done with shared memory
+        if (threadIdx.x >= 32 && threadIdx.x < 32 + sizeof(SystemFrame) / 4) {
+            reinterpret_cast<unsigned*>(&sh.frame)[threadIdx.x - 32] = reinterpret_cast<const unsigned*>(static_cast<const SystemFrame*>(in.frames) + system)[threadIdx.x - 32];
+        }
         if (warp == 0) {
-            make_frame(sh.frame, in, system, lane);
             unsigned long long before = 0;
             if (EMIT) {
                 before = system_start[system];
@@ -624,15 +648,15 @@ __global__ void __launch_bounds__(SMALL_THREADS, SMALL_CTAS) small_systems_kerne
             }
             if (lane == 0) {
                 sh.counter = before;
-                if (sh.frame.singular && !EMIT) {
-                    atomicOr(&header->status, sh.frame.singular == 2 ? STATUS_STENCIL_TOO_LARGE : STATUS_SINGULAR_BOX);
-                    atomicMin(&header->mask_cursor, static_cast<unsigned long long>(system)); // first offending system
-                }
             }
         }
         __syncthreads();
         const SystemFrame& frame = sh.frame;
         const bool usable = frame.singular == 0;
+        if (!EMIT && !usable && threadIdx.x == 0) {
+            atomicOr(&header->status, frame.singular == 2 ? STATUS_STENCIL_TOO_LARGE : STATUS_SINGULAR_BOX);
+            atomicMin(&header->mask_cursor, static_cast<unsigned long long>(system)); // first offending system
+        }
         if (!EMIT && share == 0) {
             for (int k = threadIdx.x; k < n; k += SMALL_THREADS) {
                 const bool finite = isfinite(batch_coordinate<Kind>(in, 3 * (begin + k) + 0)) && isfinite(batch_coordinate<Kind>(in, 3 * (begin + k) + 1)) &&
@@ -982,9 +1006,16 @@ static unsigned molecules_grid(unsigned n_systems) {
     return std::max(1u, std::min(wanted, 1u << 20));
 }
 
-void launch_batch_reset(DeviceHeader* header, cudaStream_t stream) {
-    static_assert(sizeof(DeviceHeader) % 4 == 0 && sizeof(DeviceHeader) <= 4 * 256, "a thread per word");
-    batch_header_kernel<<<1, 256, 0, stream>>>(header);
+size_t small_frame_bytes() {
+    return sizeof(SystemFrame);
+}
+
+void launch_batch_front(const BatchInput& in, bool any_for_cta_kernel, DeviceHeader* header, cudaStream_t stream) {
+    static_assert(sizeof(DeviceHeader) % 4 == 0 && sizeof(DeviceHeader) <= 4 * FRONT_THREADS, "a thread per word");
+    static_assert(sizeof(SystemFrame) % 4 == 0 && sizeof(SystemFrame) <= 4 * (SMALL_THREADS - 32), "copied word by word");
+    constexpr unsigned per_block = FRONT_THREADS / 32;
+    const unsigned blocks = any_for_cta_kernel ? std::min((in.n_systems + per_block - 1) / per_block, 1u << 16) : 1u;
+    batch_front_kernel<<<std::max(blocks, 1u), FRONT_THREADS, 0, stream>>>(in, any_for_cta_kernel ? static_cast<SystemFrame*>(in.frames) : nullptr, header);
 }
 
 void launch_small_count(
