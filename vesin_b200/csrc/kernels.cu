@@ -154,19 +154,6 @@ __device__ __forceinline__ void store_record(const SortedPoints& sorted, size_t 
                  : "memory");
 }
 
-// Programmatic dependent launch: the kernels of a build form a chain on one
-// stream, each reading what the one before wrote. A kernel lets the next one
-// be scheduled as soon as all of its own blocks are running, and waits for the
-// one before it (complete, memory visible) before it touches anything. Launch
-// latency and block scheduling of the short kernels then overlap with the tail
-// of their predecessor. Both instructions do nothing in a plain launch.
-__device__ __forceinline__ void let_next_kernel_start() {
-    asm volatile("griddepcontrol.launch_dependents;");
-}
-__device__ __forceinline__ void wait_for_previous_kernel() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned mask;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(mask));
@@ -3207,22 +3194,6 @@ extern "C" __attribute__((visibility("default"))) void vesin_b200_debug_phase_cl
 }
 #endif
 namespace {
-/// Launch as a link of the chain of a build (see let_next_kernel_start).
-template <typename... KernelArgs, typename... Args>
-void launch_chained(void (*kernel)(KernelArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args&&... args) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(grid);
-    config.blockDim = dim3(block);
-    config.dynamicSmemBytes = smem;
-    config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[0].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attribute;
-    config.numAttrs = 1;
-    cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
-}
-
 int pair_grid(int n_units, int per_sm) {
     int device = 0;
     int sms = 148;

@@ -98,6 +98,35 @@ inline int paired_stores_fit(const PairOutput& out) {
 }
 
 #ifdef __CUDACC__
+// Programmatic dependent launch: the kernels of a build form a chain on one
+// stream, each reading what the one before wrote. A kernel lets the next one
+// be scheduled as soon as all of its own blocks are running, and waits for the
+// one before it (complete, memory visible) before it touches anything. Launch
+// latency and block scheduling of the short kernels then overlap with the tail
+// of their predecessor. Both instructions do nothing in a plain launch.
+__device__ __forceinline__ void let_next_kernel_start() {
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+__device__ __forceinline__ void wait_for_previous_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+/// Launch as a link of the chain of a build (see let_next_kernel_start).
+template <typename... KernelArgs, typename... Args>
+void launch_chained(void (*kernel)(KernelArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(block);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attribute;
+    config.numAttrs = 1;
+    cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
+}
+
 /// What the host wants to know of a pass, written into pinned memory by the pass itself, one warp:
 /// a copy behind the kernel costs its own launch and 3 us on the device, a few per cent of a small
 /// build. The host looks after it has waited for the stream, so the stores need no order. `pairs`

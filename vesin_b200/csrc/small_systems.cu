@@ -395,6 +395,7 @@ constexpr int FRONT_THREADS = 256;
 /// passes went through before it did anything else (512 cells, both passes: 108.5 -> 98.4 us, and 1.8 here).
 __global__ void __launch_bounds__(FRONT_THREADS) batch_front_kernel(const BatchInput in, SystemFrame* __restrict__ frames, DeviceHeader* header) {
     __shared__ SystemFrame sh_frames[FRONT_THREADS / 32];
+    let_next_kernel_start();
     if (blockIdx.x == 0) {
         if (threadIdx.x < sizeof(DeviceHeader) / 4) {
             reinterpret_cast<unsigned*>(header)[threadIdx.x] = 0;
@@ -428,6 +429,8 @@ __global__ void __launch_bounds__(MOLECULE_WARPS * 32, Kind::EMIT ? 16 : 20) mol
     DeviceHeader* header, const unsigned long long capacity, DeviceHeader* mirror
 ) {
     constexpr bool EMIT = Kind::EMIT;
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     extern __shared__ __align__(16) unsigned char molecule_smem[];
     MoleculeShared& sh = *reinterpret_cast<MoleculeShared*>(molecule_smem);
     const int lane = threadIdx.x & 31;
@@ -611,6 +614,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, SMALL_CTAS) small_systems_kerne
     const unsigned long long* __restrict__ system_start, PairOutput out, DeviceHeader* header, const unsigned long long capacity
 ) {
     constexpr bool EMIT = Kind::EMIT;
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     __shared__ SmallShared sh;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -1025,13 +1030,15 @@ void launch_small_count(
     const PairOutput nothing{};
     with_kind<false>(in, false, [&](auto kind) {
         using Kind = decltype(kind);
-        molecules_kernel<Kind><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
-            in, system_count, nullptr, nothing, header, 0ull, nullptr
+        launch_chained(
+            molecules_kernel<Kind>, molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream, in, system_count, nullptr, nothing,
+            header, 0ull, nullptr
         );
         if (any_for_cta_kernel) {
             const unsigned splits = small_splits(in.n_systems, max_points);
-            small_systems_kernel<Kind><<<small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream>>>(
-                in, splits, system_count, share_count, nullptr, nothing, header, 0ull
+            launch_chained(
+                small_systems_kernel<Kind>, small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream, in, splits, system_count, share_count, nullptr,
+                nothing, header, 0ull
             );
         }
     });
@@ -1045,13 +1052,15 @@ void launch_small_emit(
     // paired stores of full lists need aligned arrays (every system of a full list starts on an even element)
     with_kind<true>(in, paired_stores_fit(out) != 0, [&](auto kind) {
         using Kind = decltype(kind);
-        molecules_kernel<Kind><<<molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream>>>(
-            in, nullptr, system_start, out, header, capacity, mirror
+        launch_chained(
+            molecules_kernel<Kind>, molecules_grid(in.n_systems), MOLECULE_WARPS * 32, sizeof(MoleculeShared), stream, in, nullptr, system_start, out, header,
+            capacity, mirror
         );
         if (any_for_cta_kernel) {
             const unsigned splits = small_splits(in.n_systems, max_points);
-            small_systems_kernel<Kind><<<small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream>>>(
-                in, splits, nullptr, share_count, system_start, out, header, capacity
+            launch_chained(
+                small_systems_kernel<Kind>, small_grid(in.n_systems, splits), SMALL_THREADS, 0, stream, in, splits, nullptr, share_count, system_start, out,
+                header, capacity
             );
         }
     });
