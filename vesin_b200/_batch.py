@@ -58,7 +58,6 @@ class BatchNeighborList:
         self.full_list = bool(full_list)
         self._neighbors = VesinNeighborList()
         self._last = (0, 0)  # pairs and points of the last list: what the next one will roughly need
-        self._options_made = (None, None)  # of the last call: what they were made from, and the structure
 
     def __del__(self):
         try:
@@ -154,16 +153,13 @@ class BatchNeighborList:
         return pair_offsets.value
 
     def _options(self, quantities):
-        made_from = (quantities, self.cutoff, self.full_list)
-        if self._options_made[0] == made_from:
-            return self._options_made[1]
+        # (made for every call: see NeighborList)
         options = VesinOptions()
         options.cutoff = self.cutoff
         options.full = self.full_list
         options.return_shifts = "S" in quantities
         options.return_distances = "d" in quantities
         options.return_vectors = "D" in quantities
-        self._options_made = (made_from, options)
         return options
 
     def _build_into(self, points, system_offsets, boxes, periodic, quantities, global_indices):

@@ -88,7 +88,6 @@ class NeighborList:
         self._neighbors = VesinNeighborList()
         self._last = (0, 0)  # pairs and points of the last list: what the next one will roughly need
         self._device = None  # of the last call, with its number
-        self._options = (None, None)  # of the last call: what they were made from, and the structure
 
     def __del__(self):
         try:
@@ -178,10 +177,7 @@ class NeighborList:
                 f"booleans, got {periodic} of type {type(periodic)}"
             )
 
-        made_from = (quantities, self.cutoff, self.full_list, self.sorted, self._c_algorithm, self.skin, self.n_threads)
-        if self._options[0] != made_from:
-            self._options = (made_from, self._make_options(quantities))
-        options = self._options[1]
+        options = self._options(quantities)
 
         number = device.index or 0
         if self._device is None or self._device.device_id != number:
@@ -280,7 +276,8 @@ class NeighborList:
                 data.append(finish(vectors))
         return tuple(data)
 
-    def _make_options(self, quantities):
+    def _options(self, quantities):
+        # (made for every call, half a microsecond: `quantities` may be a list that has changed since the last one)
         options = VesinOptions()
         options.cutoff = self.cutoff
         options.full = self.full_list
