@@ -228,7 +228,6 @@ Workspace& workspace_of(VesinNeighborList& list) {
         VB200_CUDA(cudaMalloc(reinterpret_cast<void**>(&ws->d_header), sizeof(DeviceHeader)));
         VB200_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ws->h_header), sizeof(DeviceHeader), cudaHostAllocDefault));
         configure_kernels();
-        configure_small_systems();
     }
     return *static_cast<Workspace*>(list.opaque);
 }

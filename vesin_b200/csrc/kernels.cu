@@ -3236,42 +3236,71 @@ void with_segments(const GridPlan& plan, Use use) {
 }
 } // namespace
 
-void configure_kernels() {
-    const auto allow = [](auto kernel, size_t bytes) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)); };
-    allow(row_emit_kernel<SortedRowsWide>, sizeof(SortedRowsWide::Shared));
-    const auto allow_rows = [&](auto segments) {
-        constexpr int SEGMENTS = decltype(segments)::value;
-        const auto allow_count = [&](auto shape) { allow(row_count_kernel<decltype(shape)>, sizeof(typename decltype(shape)::Shared)); };
-        const auto allow_emit = [&](auto shape) { allow(row_emit_kernel<decltype(shape)>, sizeof(typename decltype(shape)::Shared)); };
-        allow_count(RowCount<true, SEGMENTS>{});
-        allow_count(RowCount<false, SEGMENTS>{});
-        allow_count(RankedCount<true, SEGMENTS>{});
-        allow_count(RankedCount<false, SEGMENTS>{});
-        allow_count(RankedCountWide<true, SEGMENTS>{});
-        allow_count(RankedCountWide<false, SEGMENTS>{});
-        allow_emit(SortedRows<SEGMENTS, 0>{});
-        allow_emit(SortedRows<SEGMENTS, 1>{});
-    };
-    allow_rows(std::integral_constant<int, 32>{});
-    allow_rows(std::integral_constant<int, 64>{});
-    allow_rows(std::integral_constant<int, SEG_MAX>{});
-    const auto allow_plain = [&](auto shape) {
+namespace {
+/// use(shape, kernel) for every pair kernel of unsorted lists.
+template <class Use>
+void each_pair_kernel(Use use) {
+    const auto plain = [&](auto shape) {
         using Shape = decltype(shape);
-        allow(pairs_kernel<false, false, 0, Shape>, sizeof(typename Shape::Shared));
-        allow(pairs_kernel<true, false, 0, Shape>, sizeof(typename Shape::Shared));
-        allow(pairs_kernel<false, false, 1, Shape>, sizeof(typename Shape::Shared));
-        allow(pairs_kernel<true, false, 1, Shape>, sizeof(typename Shape::Shared));
+        use(shape, pairs_kernel<false, false, 0, Shape>);
+        use(shape, pairs_kernel<true, false, 0, Shape>);
+        use(shape, pairs_kernel<false, false, 1, Shape>);
+        use(shape, pairs_kernel<true, false, 1, Shape>);
     };
-    allow_plain(SmallCta<32, 224>{});
-    allow_plain(SmallCta<32, 256>{});
-    allow_plain(SmallCta<64, 224>{});
-    allow_plain(SmallCta<64, 256>{});
-    allow(pairs_kernel<false, false, -1, SmallAnyCta>, sizeof(SmallAnyCta::Shared));
-    allow(pairs_kernel<true, false, -1, SmallAnyCta>, sizeof(SmallAnyCta::Shared));
-    allow(pairs_kernel<false, false, -1, TinyCta>, sizeof(TinyCta::Shared));
-    allow(pairs_kernel<true, false, -1, TinyCta>, sizeof(TinyCta::Shared));
-    allow(pairs_kernel<false, true, -1, LargeCta>, sizeof(LargeCta::Shared));
-    allow(pairs_kernel<true, true, -1, LargeCta>, sizeof(LargeCta::Shared));
+    plain(SmallCta<32, 224>{});
+    plain(SmallCta<32, 256>{});
+    plain(SmallCta<64, 224>{});
+    plain(SmallCta<64, 256>{});
+    use(SmallAnyCta{}, pairs_kernel<false, false, -1, SmallAnyCta>);
+    use(SmallAnyCta{}, pairs_kernel<true, false, -1, SmallAnyCta>);
+    use(TinyCta{}, pairs_kernel<false, false, -1, TinyCta>);
+    use(TinyCta{}, pairs_kernel<true, false, -1, TinyCta>);
+    use(LargeCta{}, pairs_kernel<false, true, -1, LargeCta>);
+    use(LargeCta{}, pairs_kernel<true, true, -1, LargeCta>);
+}
+
+/// use(shape, kernel) for every kernel of sorted lists.
+template <class Use>
+void each_row_kernel(Use use) {
+    const auto of_stencil = [&](auto segments) {
+        constexpr int SEGMENTS = decltype(segments)::value;
+        const auto count = [&](auto shape) { use(shape, row_count_kernel<decltype(shape)>); };
+        const auto emit = [&](auto shape) { use(shape, row_emit_kernel<decltype(shape)>); };
+        count(RowCount<true, SEGMENTS>{});
+        count(RowCount<false, SEGMENTS>{});
+        count(RankedCount<true, SEGMENTS>{});
+        count(RankedCount<false, SEGMENTS>{});
+        count(RankedCountWide<true, SEGMENTS>{});
+        count(RankedCountWide<false, SEGMENTS>{});
+        emit(SortedRows<SEGMENTS, 0>{});
+        emit(SortedRows<SEGMENTS, 1>{});
+    };
+    of_stencil(std::integral_constant<int, 32>{});
+    of_stencil(std::integral_constant<int, 64>{});
+    of_stencil(std::integral_constant<int, SEG_MAX>{});
+    use(SortedRowsWide{}, row_emit_kernel<SortedRowsWide>);
+}
+} // namespace
+
+void configure_kernels() {
+    // Only what takes more shared memory than any kernel may has to ask for it: 5 kernels of 47. Asking for
+    // all of them, for every new list, had all of them loaded by the first one (first call of a
+    // process 21.0 ms, now 16.6).
+    const auto allow = [](auto shape, auto kernel) {
+        constexpr size_t bytes = sizeof(typename decltype(shape)::Shared);
+        if constexpr (bytes > SHARED_WITHOUT_ASKING) {
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+        }
+    };
+    each_pair_kernel(allow);
+    each_row_kernel(allow);
+}
+
+void load_pair_kernels() {
+    each_pair_kernel([](auto, auto kernel) {
+        cudaFuncAttributes attributes;
+        cudaFuncGetAttributes(&attributes, kernel);
+    });
 }
 
 static ExpectedInputs expected_inputs(const double box[9], const bool periodic[3]) {

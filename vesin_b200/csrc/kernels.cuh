@@ -332,7 +332,6 @@ struct BatchInput {
 
 /// Largest system the batch kernels accept (its points live in shared memory).
 size_t small_systems_max_points();
-void configure_small_systems();
 /// Header of a batch: nothing found yet (first_bad, mask_cursor: the largest values).
 void launch_batch_front(const BatchInput& in, bool any_for_cta_kernel, DeviceHeader* header, cudaStream_t stream);
 size_t small_frame_bytes();
@@ -406,8 +405,12 @@ void launch_verlet_filter(
     PairOutput out, unsigned long long capacity, VerletState* state, int call, cudaStream_t stream
 );
 
-/// One-time per-device kernel attribute setup (shared-memory opt-in).
+/// Dynamic shared memory that a kernel gets without asking for it.
+constexpr size_t SHARED_WITHOUT_ASKING = 48 * 1024;
+/// Asks for the shared memory of the kernels that take more (per device, before their first launch).
 void configure_kernels();
+/// Loads the pair kernels of unsorted lists, which otherwise happens at the first launch of each.
+void load_pair_kernels();
 
 } // namespace vb200
 

@@ -28,8 +28,8 @@
 //     run on the legacy default stream, so that can only happen across
 //     processes that share nothing anyway (each process has its own array).
 //   * the first call on a device looks up the device address of the array
-//     (cudaGetSymbolAddress) and opts the kernels into large shared memory;
-//     make that first call before any stream capture begins.
+//     (cudaGetSymbolAddress) and loads the pair kernels; make that first call
+//     before any stream capture begins.
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -142,7 +142,7 @@ size_t build(
         // once per device, with that device current
         void* address = nullptr;
         check(cudaGetSymbolAddress(&address, NO_ALLOC_SCRATCH), "cudaGetSymbolAddress(NO_ALLOC_SCRATCH)");
-        configure_kernels();
+        load_pair_kernels(); // (a kernel that is loaded at its first launch may allocate)
         state.scratch = static_cast<unsigned char*>(address);
     }
     unsigned char* base = state.scratch;

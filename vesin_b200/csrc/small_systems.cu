@@ -347,6 +347,7 @@ struct MoleculeShared {
     unsigned short list[MOLECULE_WARPS][HIT_LIST]; // hits waiting to be written: (i << 8) | j
 };
 static_assert(MOLECULE_MAX_POINTS % 32 == 0 && MOLECULE_MAX_POINTS <= 256, "whole words of candidates, indices of 8 bits");
+static_assert(sizeof(MoleculeShared) <= SHARED_WITHOUT_ASKING, "no launch has to ask for its shared memory");
 
 /// The reference's arithmetic for S = 0 (vesin/src/cpu_cell_list.cpp:135-138), operation for
 /// operation: the shift term is an exact zero.
@@ -970,20 +971,6 @@ static void with_kind(const BatchInput& in, bool paired, Use use) {
         with_type(std::true_type{}, std::false_type{});
     } else {
         with_type(std::true_type{}, std::true_type{});
-    }
-}
-
-void configure_small_systems() {
-    BatchInput in{};
-    for (int k = 0; k < 8; k++) {
-        in.is_float = k & 1;
-        in.full = (k >> 1) & 1;
-        const bool paired = (k >> 2) & 1;
-        const auto allow = [](auto kind) {
-            cudaFuncSetAttribute(molecules_kernel<decltype(kind)>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(MoleculeShared)));
-        };
-        with_kind<false>(in, paired, allow);
-        with_kind<true>(in, paired, allow);
     }
 }
 
