@@ -1296,14 +1296,16 @@ struct PairShape {
 /// Of 256 candidates per batch, 8 of them per SM, or of 224 and 9 (56 registers; see launch_pairs).
 template <int SEGMENTS, int BATCH>
 using SmallCta = PairShape<128, BATCH, 1024, (BATCH == 256) ? 8 : 9, false, false, SEGMENTS>;
-using SmallAnyCta = PairShape<128, 256, 1024, 8, true, true, SEG_MAX>;
+template <bool SHARES>
+using SmallAnyCta = PairShape<128, 256, 1024, 8, SHARES, true, SEG_MAX>;
 /// Launches that do not fill the GPU (one small system): 64 candidates per batch, so that the
 /// batches of a unit go to four times as many CTAs (see launch_pairs). What bounds such a launch
 /// is the chain of one CTA, and most of that is writing its hits.
 using TinyCta = PairShape<128, 64, 1024, 8, true, true, SEG_MAX>;
 /// Units next to the halo of a slab (they sort their hits into owned and halo candidates and go
 /// over every batch twice): CTAs of 8 warps with 512 candidates per batch, 4 per SM.
-using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4, true, true, SEG_MAX>;
+template <bool SHARES>
+using LargeCta = PairShape<CTA_THREADS, FUSED_BATCH, FUSED_LIST, 4, SHARES, true, SEG_MAX>;
 /// Offset (in cells, relative to the first cell of the unit) of entry `index`
 /// of the half-shell stencil of a unit of `cells` cells.
 __device__ __forceinline__ void half_stencil_offset(const GridPlan& plan, int cells, int index, int& ox, int& oy, int& oz) {
@@ -3251,12 +3253,18 @@ void each_pair_kernel(Use use) {
     plain(SmallCta<32, 256>{});
     plain(SmallCta<64, 224>{});
     plain(SmallCta<64, 256>{});
-    use(SmallAnyCta{}, pairs_kernel<false, false, -1, SmallAnyCta>);
-    use(SmallAnyCta{}, pairs_kernel<true, false, -1, SmallAnyCta>);
     use(TinyCta{}, pairs_kernel<false, false, -1, TinyCta>);
     use(TinyCta{}, pairs_kernel<true, false, -1, TinyCta>);
-    use(LargeCta{}, pairs_kernel<false, true, -1, LargeCta>);
-    use(LargeCta{}, pairs_kernel<true, true, -1, LargeCta>);
+    const auto any = [&](auto shares) {
+        using Small = SmallAnyCta<decltype(shares)::value>;
+        using Large = LargeCta<decltype(shares)::value>;
+        use(Small{}, pairs_kernel<false, false, -1, Small>);
+        use(Small{}, pairs_kernel<true, false, -1, Small>);
+        use(Large{}, pairs_kernel<false, true, -1, Large>);
+        use(Large{}, pairs_kernel<true, true, -1, Large>);
+    };
+    any(std::false_type{});
+    any(std::true_type{});
 }
 
 /// use(shape, kernel) for every kernel of sorted lists.
@@ -3283,7 +3291,7 @@ void each_row_kernel(Use use) {
 } // namespace
 
 void configure_kernels() {
-    // Only what takes more shared memory than any kernel may has to ask for it: 5 kernels of 47. Asking for
+    // Only what takes more shared memory than any kernel may has to ask for it: 7 kernels of 51. Asking for
     // all of them, for every new list, had all of them loaded by the first one (first call of a
     // process 21.0 ms, now 16.6).
     const auto allow = [](auto shape, auto kernel) {
@@ -3533,6 +3541,12 @@ void launch_pairs(
         unit_candidates = stencil_cells * static_cast<double>(n_records) / static_cast<double>(plan.n_cells_total);
     }
 
+    // Several CTAs share a unit where the units take half of the places or less. Knowing one's share costs registers
+    // that launches of more units have better uses for: a call on a slab of 1 M points, full list 674 us with it, 653
+    // without, half list 582 and 566; a full list of 512k crystal atoms into unaligned arrays 658 and 641.
+    const auto few_units = [&](auto shape, const UnitRanges& ranges) {
+        return ((ranges.end0 - ranges.begin0) + (ranges.end1 - ranges.begin1)) * 2 <= sms * decltype(shape)::CTAS_PER_SM;
+    };
     const auto launch_shape = [&](auto shape, auto kernel, UnitRanges ranges, unsigned long long* run_cursor, bool follows = false) {
         using Shape = decltype(shape);
         const int per_sm = Shape::CTAS_PER_SM;
@@ -3562,9 +3576,17 @@ void launch_pairs(
             (plan.window_axis < 0) ? mirror : nullptr
         );
     };
+    // Units next to the halo of a slab.
+    const auto launch_slab = [&](auto full, UnitRanges ranges, unsigned long long* run_cursor, bool follows = false) {
+        constexpr bool FULL = decltype(full)::value;
+        if (few_units(LargeCta<true>{}, ranges)) {
+            launch_shape(LargeCta<true>{}, pairs_kernel<FULL, true, -1, LargeCta<true>>, ranges, run_cursor, follows);
+        } else {
+            launch_shape(LargeCta<false>{}, pairs_kernel<FULL, true, -1, LargeCta<false>>, ranges, run_cursor, follows);
+        }
+    };
     const auto launch = [&](auto full, UnitRanges ranges, unsigned long long* run_cursor) {
         constexpr bool FULL = decltype(full)::value;
-        const int n_units = (ranges.end0 - ranges.begin0) + (ranges.end1 - ranges.begin1);
         const long long above = static_cast<long long>(plan.n_search[1]) + static_cast<long long>(plan.n_search[2]) * (2 * plan.n_search[1] + 1);
         const long long segments = plan.pencil + plan.n_search[0] + (plan.pencil + 2 * plan.n_search[0]) * above;
         const auto launch_plain = [&](auto shape) {
@@ -3575,8 +3597,12 @@ void launch_pairs(
                 launch_shape(shape, pairs_kernel<FULL, false, 0, Shape>, ranges, run_cursor);
             }
         };
-        if (plan.window_axis >= 0 || segments > 64 || n_units * 2 <= sms * SmallAnyCta::CTAS_PER_SM || (FULL && !out.interleave_ok)) {
-            launch_shape(SmallAnyCta{}, pairs_kernel<FULL, false, -1, SmallAnyCta>, ranges, run_cursor);
+        if (few_units(SmallAnyCta<true>{}, ranges)) {
+            launch_shape(SmallAnyCta<true>{}, pairs_kernel<FULL, false, -1, SmallAnyCta<true>>, ranges, run_cursor);
+            return;
+        }
+        if (plan.window_axis >= 0 || segments > 64 || (FULL && !out.interleave_ok)) {
+            launch_shape(SmallAnyCta<false>{}, pairs_kernel<FULL, false, -1, SmallAnyCta<false>>, ranges, run_cursor);
             return;
         }
         // A ninth CTA per SM is worth 1 to 4 % (110k crystal in float 115 -> 111 us, 512k 490 -> 486; 326
@@ -3591,7 +3617,7 @@ void launch_pairs(
         }
     };
     const UnitRanges all{0, plan.n_units, 0, 0};
-    if (plan.window_axis < 0 && unit_candidates > 0.0 && plan.n_units * std::ceil(unit_candidates / SmallAnyCta::BATCH) <= sms) {
+    if (plan.window_axis < 0 && unit_candidates > 0.0 && plan.n_units * std::ceil(unit_candidates / SmallAnyCta<true>::BATCH) <= sms) {
         // Less than a CTA per SM even when every batch of 256 candidates gets its own: batches of
         // 64 (1000 atoms: 20.6 -> 13.7 us, 64 atoms with 4000 images: 29.5 -> 25.7 us; from two CTAs per
         // SM on the smaller batches cost more than they spread).
@@ -3636,17 +3662,17 @@ void launch_pairs(
                 launch(std::true_type{}, UnitRanges{0, interior_end, 0, 0}, &header->run_cursor);
             }
             if (part != PAIR_PART_INTERIOR) {
-                launch_shape(
-                    LargeCta{}, pairs_kernel<true, true, -1, LargeCta>,
+                launch_slab(
+                    std::true_type{},
                     UnitRanges{interior_end, per_layer * owned_layers, per_layer * (owned_layers + 1), per_layer * (owned_layers + 2)},
                     &header->mask_cursor, /*follows=*/part == PAIR_PART_ALL && owned_layers > 1
                 );
             }
         }
     } else if (plan.full) {
-        launch_shape(LargeCta{}, pairs_kernel<true, true, -1, LargeCta>, all, &header->run_cursor);
+        launch_slab(std::true_type{}, all, &header->run_cursor);
     } else {
-        launch_shape(LargeCta{}, pairs_kernel<false, true, -1, LargeCta>, all, &header->run_cursor);
+        launch_slab(std::false_type{}, all, &header->run_cursor);
     }
 }
 
