@@ -926,7 +926,6 @@ struct SegmentTableT {
     int slot0[ENTRIES + 1]; // exclusive prefix of the segment lengths
     int scan_tmp[CTA_WARPS + 1];
 };
-using SegmentTable = SegmentTableT<SEG_MAX>;
 static_assert(MAX_STENCIL_CELLS <= (1 << 20), "image shifts are stored in 21 bits");
 
 __device__ __forceinline__ unsigned long long pack_segment_image(int q0, int q1, int q2, int flag) {

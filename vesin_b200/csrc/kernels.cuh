@@ -332,7 +332,8 @@ struct BatchInput {
 
 /// Largest system the batch kernels accept (its points live in shared memory).
 size_t small_systems_max_points();
-/// Header of a batch: nothing found yet (first_bad, mask_cursor: the largest values).
+/// Header of a batch: nothing found yet (first_bad, mask_cursor: the largest values). With systems for
+/// the CTA kernel, also their frames: box, inverse and reach of the images -> in.frames.
 void launch_batch_front(const BatchInput& in, bool any_for_cta_kernel, DeviceHeader* header, cudaStream_t stream);
 size_t small_frame_bytes();
 /// Pass 1: pairs of every system -> system_count; the first non-finite point

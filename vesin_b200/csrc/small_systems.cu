@@ -965,13 +965,13 @@ static void with_kind(const BatchInput& in, bool paired, Use use) {
         }
     };
     // (half lists and counts store no pairs side by side)
-    if (!in.full) {
-        with_type(std::false_type{}, std::false_type{});
-    } else if (!EMIT || !paired) {
-        with_type(std::true_type{}, std::false_type{});
-    } else {
-        with_type(std::true_type{}, std::true_type{});
+    if constexpr (EMIT) {
+        if (in.full && paired) {
+            with_type(std::true_type{}, std::true_type{});
+            return;
+        }
     }
+    in.full ? with_type(std::true_type{}, std::false_type{}) : with_type(std::false_type{}, std::false_type{});
 }
 
 static unsigned multiprocessors() {
