@@ -131,3 +131,15 @@ def _check_order(points, box, cutoff, full):
         values = calculator.compute(torch.tensor(points, device="cuda"), torch.tensor(box, device="cuda"), True, "ijSdD")
         for key, value in zip("ijSdD", values):
             assert np.array_equal(value.cpu().numpy().astype(expected[key].dtype), expected[key]), key
+
+
+@pytest.mark.parametrize("full", [True, False])
+@pytest.mark.parametrize("span", [61438, 61439, 61440, 61441])
+def test_span_of_indices_of_a_unit(span, full):
+    """A cluster on its own whose indices lie exactly as far apart as has a bit each, or one further."""
+    rng = np.random.default_rng(span)
+    length, n = 220.0, 61500
+    points = rng.uniform(20.0, length - 20.0, (n, 3))  # (nothing within a cell of the corner)
+    cluster = np.concatenate([[0, 30, 31, 32, 33, span - 33, span - 32, span - 1, span], rng.choice(np.arange(40, span - 40), 31, replace=False)])
+    points[cluster] = rng.uniform(-2.0, 2.0, (len(cluster), 3))
+    _check_order(points, length * np.eye(3), 3.0, full)

@@ -2162,10 +2162,16 @@ constexpr int RANKED_HOME = 256;   // home points of a unit whose candidates are
 /// What ranking the candidates of a unit needs, before they are staged.
 template <int BATCH>
 struct Ordering {
-    unsigned key[BATCH];          // index of the candidate in a slot
-    unsigned gathered[BATCH];     // the same, bucket by bucket
-    int first[RANK_BUCKETS + 1];  // candidates in a bucket, then where the bucket starts
+    union {
+        struct {
+            unsigned key[BATCH];      // index of the candidate in a slot
+            unsigned gathered[BATCH]; // the same, bucket by bucket
+        };
+        unsigned bits[RANK_BUCKETS];  // instead of both: a bit for every index from the least on
+    };
+    int first[RANK_BUCKETS + 1]; // candidates in a bucket, then where the bucket starts
     unsigned least, most;
+    static_assert(2 * BATCH >= RANK_BUCKETS, "the bits take no more room than the keys");
 };
 
 /// Ranks the candidates of a unit by their indices (images of one point, which a row never has
@@ -2190,10 +2196,8 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
         // Indices close enough together that a bucket can have a bit for each: the rank of a candidate is the
         // start of its bucket plus the bits below its own. (Units of up to 64k points, and of larger crystals in lattice
         // order, whose runs of indices make for long comparisons below: 216k crystal, deciding pass 211 -> 171 us.)
-        static_assert(offsetof(Ordering<BATCH>, gathered) == BATCH * sizeof(unsigned) && 2 * BATCH >= RANK_BUCKETS, "the keys make room for the bits");
         static_assert(RANK_BUCKETS % THREADS == 0 && (RANK_BUCKETS / THREADS) % 2 == 1, "an odd number of buckets per thread");
-        unsigned* bits = o.key;
-        unsigned key[PER_THREAD];
+        unsigned key[PER_THREAD]; // (the bits take the place of the keys)
 #pragma unroll
         for (int e = 0; e < PER_THREAD; e++) {
             const int s = threadIdx.x + e * THREADS;
@@ -2201,7 +2205,7 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
         }
         __syncthreads();
         for (int k = threadIdx.x; k < RANK_BUCKETS; k += THREADS) {
-            bits[k] = 0;
+            o.bits[k] = 0;
         }
         __syncthreads();
         bool twice = false; // images of one point: no bit for each
@@ -2210,7 +2214,7 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
             const int s = threadIdx.x + e * THREADS;
             if (s < n) {
                 const unsigned bit = 1u << (key[e] & 31u);
-                twice = twice || (atomicOr(&bits[key[e] >> 5], bit) & bit) != 0;
+                twice = twice || (atomicOr(&o.bits[key[e] >> 5], bit) & bit) != 0;
             }
         }
         if (!__syncthreads_or(twice ? 1 : 0)) {
@@ -2218,7 +2222,7 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
             int mine = 0;
 #pragma unroll
             for (int e = 0; e < SCAN; e++) {
-                mine += __popc(bits[threadIdx.x * SCAN + e]);
+                mine += __popc(o.bits[threadIdx.x * SCAN + e]);
             }
             int inclusive = mine;
 #pragma unroll
@@ -2240,14 +2244,14 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
 #pragma unroll
             for (int e = 0; e < SCAN; e++) {
                 o.first[threadIdx.x * SCAN + e] = start;
-                start += __popc(bits[threadIdx.x * SCAN + e]);
+                start += __popc(o.bits[threadIdx.x * SCAN + e]);
             }
             __syncthreads();
 #pragma unroll
             for (int e = 0; e < PER_THREAD; e++) {
                 const int s = threadIdx.x + e * THREADS;
                 if (s < n) {
-                    const unsigned below = bits[key[e] >> 5] & ((1u << (key[e] & 31u)) - 1u);
+                    const unsigned below = o.bits[key[e] >> 5] & ((1u << (key[e] & 31u)) - 1u);
                     order[o.first[key[e] >> 5] + __popc(below)] = static_cast<unsigned short>(s);
                 }
             }
