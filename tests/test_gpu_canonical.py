@@ -143,3 +143,12 @@ def test_span_of_indices_of_a_unit(span, full):
     cluster = np.concatenate([[0, 30, 31, 32, 33, span - 33, span - 32, span - 1, span], rng.choice(np.arange(40, span - 40), 31, replace=False)])
     points[cluster] = rng.uniform(-2.0, 2.0, (len(cluster), 3))
     _check_order(points, length * np.eye(3), 3.0, full)
+
+
+@pytest.mark.parametrize("full", [True, False])
+@pytest.mark.parametrize("cells,cutoff", [(9, 6.3), (8, 7.0), (10, 7.0), (11, 7.7)])
+def test_units_as_full_as_ranks_have_room_for(cells, cutoff, full, monkeypatch):
+    """Units of a crystal with 1260 to 2300 candidates: what the first build tries to rank fits, or does not."""
+    monkeypatch.setenv("VESIN_CUDA_MAX_PAIRS_PER_POINT", "100000")
+    points, box, _ = W.diamond(cells, seed=cells)
+    _check_order(points, box, cutoff, full)
