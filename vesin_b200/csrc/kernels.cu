@@ -2838,7 +2838,6 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
         cache_stencil<Shape::SEGMENTS>(plan, sh.offsets);
         __syncthreads();
     }
-    wait_for_previous_kernel();
     if (limits.header != nullptr &&
         ((limits.header->status & (STATUS_ABORT_MASK | STATUS_MASK_OVERFLOW)) != 0 || limits.header->total_pairs > limits.capacity ||
          limits.header->max_candidates > limits.candidates)) {
@@ -3483,9 +3482,11 @@ void launch_emit(
 ) {
     const auto launch = [&](auto shape, auto kernel) {
         using Shape = decltype(shape);
-        launch_chained(
-            kernel, pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_EMIT_THREADS, sizeof(typename Shape::Shared), stream, plan, cell_start, sorted, masks,
-            unit_mask_base, unit_words, row_start, row_fill, out, ranked ? 1 : 0, limits
+        // (not a link of the chain: CTAs that are scheduled while the pass before still runs crowd on the SMs that are
+        // done first, and on shared memory that was divided for the other kernel. 110k crystal at 7 A, a call 787
+        // us chained, 709 behind the scan; 20k liquid at 10 A 228, 200; 27k crystal at 5 A 139, 140)
+        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_EMIT_THREADS, sizeof(typename Shape::Shared), stream>>>(
+            plan, cell_start, sorted, masks, unit_mask_base, unit_words, row_start, row_fill, out, ranked ? 1 : 0, limits
         );
     };
     if (row_batch(max_candidates) == ROW_BATCH_WIDE) {
