@@ -1036,6 +1036,7 @@ void neighbors(
         Target target(list, ws, options, float_io, caller);
         const size_t existing = target.capacity();
         const unsigned expected_candidates = ws.cache.row_candidates;
+        const bool few = rows_of_few_units(plan, n_points, expected_candidates);
         bool written = false;
 
         bool refused = false;
@@ -1046,7 +1047,7 @@ void neighbors(
             }
             launch_count(
                 plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.masks.bytes / sizeof(uint32_t),
-                ws.unit_mask_base.as<unsigned long long>(), ws.unit_words.as<uint32_t>(), ws.row_count.as<uint32_t>(), ws.d_header, ranked, stream
+                ws.unit_mask_base.as<unsigned long long>(), ws.unit_words.as<uint32_t>(), ws.row_count.as<uint32_t>(), ws.d_header, ranked, few, stream
             );
             timer.end(VesinB200StageCount);
             timer.begin(VesinB200StageScanRows);
@@ -1062,7 +1063,7 @@ void neighbors(
                 launch_emit(
                     plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.unit_mask_base.as<unsigned long long>(),
                     ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), target.view(), expected_candidates,
-                    ranked != 0, stream, RowLimits{ws.d_header, existing, (ranked != 0) ? std::min(room, static_cast<unsigned>(ranked)) : room}
+                    ranked != 0, few, stream, RowLimits{ws.d_header, existing, (ranked != 0) ? std::min(room, static_cast<unsigned>(ranked)) : room}
                 );
                 timer.end(VesinB200StageEmit);
             }
@@ -1140,7 +1141,8 @@ void neighbors(
             }
             launch_emit(
                 plan, ws.cell_start.as<int32_t>(), sorted, ws.masks.as<uint32_t>(), ws.unit_mask_base.as<unsigned long long>(),
-                ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), rows, header.max_candidates, ranked != 0, stream
+                ws.unit_words.as<uint32_t>(), ws.row_start.as<unsigned long long>(), ws.row_fill.as<uint32_t>(), rows, header.max_candidates, ranked != 0,
+                rows_of_few_units(plan, n_points, header.max_candidates), stream
             );
             if (sort_behind) {
                 launch_sort_rows(ws.row_start.as<unsigned long long>(), n_points, rows, out, duplicates_possible, stream);

@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <type_traits>
 #include <cfloat>
+#include <cmath>
 
 namespace vb200 {
 
@@ -2154,24 +2155,24 @@ __global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) pairs_kern
 // in the order the candidates were staged.
 // ---------------------------------------------------------------------------
 
-// see rank_candidates: 15 consecutive buckets per thread, an odd number, which keeps the threads of a
+// see rank_candidates: consecutive buckets per thread, an odd number, which keeps the threads of a
 // scan out of each other's banks
-constexpr int RANK_BUCKETS = 1920;
+constexpr int RANK_BUCKETS_PER_THREAD = 15;
 constexpr int RANKED_HOME = 256;   // home points of a unit whose candidates are ranked, at most
 
 /// What ranking the candidates of a unit needs, before they are staged.
-template <int BATCH>
+template <int THREADS, int BATCH>
 struct Ordering {
+    static constexpr int BUCKETS = THREADS * RANK_BUCKETS_PER_THREAD;
     union {
         struct {
             unsigned key[BATCH];      // index of the candidate in a slot
             unsigned gathered[BATCH]; // the same, bucket by bucket
         };
-        unsigned bits[RANK_BUCKETS];  // instead of both: a bit for every index from the least on
+        unsigned bits[BUCKETS];       // instead of both: a bit for every index from the least on
     };
-    int first[RANK_BUCKETS + 1]; // candidates in a bucket, then where the bucket starts
+    int first[BUCKETS + 1]; // candidates in a bucket, then where the bucket starts
     unsigned least, most;
-    static_assert(2 * BATCH >= RANK_BUCKETS, "the bits take no more room than the keys");
 };
 
 /// Ranks the candidates of a unit by their indices (images of one point, which a row never has
@@ -2185,18 +2186,18 @@ struct Ordering {
 /// 1410; sorting the rows behind the kernel took 2018. Starts behind a barrier that follows the writes
 /// of the keys, least and most, and ends with one.
 template <int THREADS, int BATCH>
-__device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tmp, unsigned short* order, int n) {
+__device__ __forceinline__ void rank_candidates(Ordering<THREADS, BATCH>& o, int* scan_tmp, unsigned short* order, int n) {
     constexpr int WARPS = THREADS / 32;
+    constexpr int BUCKETS = Ordering<THREADS, BATCH>::BUCKETS;
     constexpr int PER_THREAD = (BATCH + THREADS - 1) / THREADS;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const unsigned least_index = o.least;
     const unsigned range = o.most - least_index;
-    if (range < 32u * RANK_BUCKETS) {
+    if (range < 32u * BUCKETS) {
         // Indices close enough together that a bucket can have a bit for each: the rank of a candidate is the
-        // start of its bucket plus the bits below its own. (Units of up to 64k points, and of larger crystals in lattice
+        // start of its bucket plus the bits below its own. (Systems of up to 61 440 points, and larger crystals in lattice
         // order, whose runs of indices make for long comparisons below: 216k crystal, deciding pass 211 -> 171 us.)
-        static_assert(RANK_BUCKETS % THREADS == 0 && (RANK_BUCKETS / THREADS) % 2 == 1, "an odd number of buckets per thread");
         unsigned key[PER_THREAD]; // (the bits take the place of the keys)
 #pragma unroll
         for (int e = 0; e < PER_THREAD; e++) {
@@ -2204,7 +2205,7 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
             key[e] = (s < n) ? o.key[s] - least_index : 0u;
         }
         __syncthreads();
-        for (int k = threadIdx.x; k < RANK_BUCKETS; k += THREADS) {
+        for (int k = threadIdx.x; k < BUCKETS; k += THREADS) {
             o.bits[k] = 0;
         }
         __syncthreads();
@@ -2218,7 +2219,7 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
             }
         }
         if (!__syncthreads_or(twice ? 1 : 0)) {
-            constexpr int SCAN = RANK_BUCKETS / THREADS;
+            constexpr int SCAN = RANK_BUCKETS_PER_THREAD;
             int mine = 0;
 #pragma unroll
             for (int e = 0; e < SCAN; e++) {
@@ -2268,9 +2269,9 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
         __syncthreads();
     }
     // (rounding is monotonic: a larger index never falls into an earlier bucket)
-    const float scale = static_cast<float>(RANK_BUCKETS) / (static_cast<float>(o.most - o.least) + 1.0f);
+    const float scale = static_cast<float>(BUCKETS) / (static_cast<float>(o.most - o.least) + 1.0f);
     const unsigned least = o.least;
-    const auto bucket_of = [&](unsigned key) { return min(static_cast<int>(static_cast<float>(key - least) * scale), RANK_BUCKETS - 1); };
+    const auto bucket_of = [&](unsigned key) { return min(static_cast<int>(static_cast<float>(key - least) * scale), BUCKETS - 1); };
     int arrival[PER_THREAD];
 #pragma unroll
     for (int e = 0; e < PER_THREAD; e++) {
@@ -2280,7 +2281,7 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
         }
     }
     __syncthreads();
-    constexpr int SCAN = RANK_BUCKETS / THREADS;
+    constexpr int SCAN = RANK_BUCKETS_PER_THREAD;
     int counts[SCAN];
     int mine = 0;
 #pragma unroll
@@ -2311,7 +2312,7 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
         start += counts[e];
     }
     if (threadIdx.x == 0) {
-        o.first[RANK_BUCKETS] = n;
+        o.first[BUCKETS] = n;
     }
     __syncthreads();
 #pragma unroll
@@ -2350,11 +2351,14 @@ __device__ __forceinline__ void rank_candidates(Ordering<BATCH>& o, int* scan_tm
 /// decisions, words, counts) and its barriers, so 8 CTAs of 4 warps share an SM instead of 4 of 8,
 /// and the claim of storage is on its way while the candidates are staged: 216k crystal 156 -> 127
 /// us, 262k liquid 146 -> 118, its half list 250 -> 193.
+/// (CTAs of 8 warps again where units are few, see rows_of_few_units, or ranked 2048 candidates at a time.)
 /// RANKED: the candidates of a unit, which all fit a batch, are staged in the order of their indices.
 /// SEGMENTS: see setup_segments.
-template <bool FULL_, bool RANKED_, int BATCH_, int CTAS_PER_SM_, int SEGMENTS_>
+template <bool FULL_, bool RANKED_, int BATCH_, int THREADS_, int CTAS_PER_SM_, int SEGMENTS_>
 struct RowCountShape {
     static constexpr int SEGMENTS = SEGMENTS_;
+    static constexpr int THREADS = THREADS_;
+    static constexpr int WARPS = THREADS_ / 32;
     static constexpr bool FULL = FULL_;
     static constexpr bool RANKED = RANKED_;
     static constexpr int BATCH = BATCH_;
@@ -2369,7 +2373,7 @@ struct RowCountShape {
                 alignas(16) float near_z[BATCH_];
                 alignas(16) float near_n[BATCH_];
             };
-            typename std::conditional<RANKED_, Ordering<BATCH_>, Nothing>::type ordering;
+            typename std::conditional<RANKED_, Ordering<THREADS_, BATCH_>, Nothing>::type ordering;
         };
         SegmentTableT<SEGMENTS_> table;
         int offsets[SEGMENTS_]; // of the stencil of a full-length unit
@@ -2417,11 +2421,8 @@ __device__ __forceinline__ int row_words_of_unit(
     return words;
 }
 
-constexpr int ROW_COUNT_THREADS = 128;
-constexpr int ROW_COUNT_WARPS = ROW_COUNT_THREADS / 32;
-
 template <class Shape>
-__global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_count_kernel(
+__global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) row_count_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, uint32_t* __restrict__ masks,
     unsigned long long mask_capacity, unsigned long long* __restrict__ unit_mask_base, uint32_t* __restrict__ unit_words,
     uint32_t* __restrict__ row_count, DeviceHeader* header
@@ -2514,7 +2515,7 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
                 };
                 if constexpr (RANKED) {
                     // (the only batch of the unit)
-                    for (int k = threadIdx.x; k < RANK_BUCKETS; k += ROW_COUNT_THREADS) {
+                    for (int k = threadIdx.x; k < Ordering<Shape::THREADS, BATCH>::BUCKETS; k += Shape::THREADS) {
                         sh.ordering.first[k] = 0;
                     }
                     if (threadIdx.x == 0) {
@@ -2525,7 +2526,7 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
                     unsigned least = 0xffffffffu;
                     unsigned most = 0u;
 #pragma unroll 4
-                    for (int s = threadIdx.x; s < batch_slots; s += ROW_COUNT_THREADS) {
+                    for (int s = threadIdx.x; s < batch_slots; s += Shape::THREADS) {
                         int t;
                         const unsigned key = static_cast<unsigned>(sorted.records[position_of(s, t)].index);
                         sh.ordering.key[s] = key;
@@ -2539,9 +2540,9 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
                         atomicMax(&sh.ordering.most, most);
                     }
                     __syncthreads();
-                    rank_candidates<ROW_COUNT_THREADS>(sh.ordering, sh.table.scan_tmp, sh.order, batch_slots);
+                    rank_candidates<Shape::THREADS>(sh.ordering, sh.table.scan_tmp, sh.order, batch_slots);
                 }
-                for (int s = threadIdx.x; s < 32 * batch_words; s += ROW_COUNT_THREADS) {
+                for (int s = threadIdx.x; s < 32 * batch_words; s += Shape::THREADS) {
                     float fx = 0.0f, fy = 0.0f, fz = 0.0f;
                     float norm = __int_as_float(0x7f800000); // past the end: never a hit
                     if (s < batch_slots) {
@@ -2624,14 +2625,14 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
                                plan.cutoff2;
                     };
                     // (no half shell here: home_row_slots = 0 keeps every candidate)
-                    if (batch_words <= ROW_COUNT_WARPS) {
+                    if (batch_words <= Shape::WARPS) {
                         if (warp < batch_words) {
                             sh.mask[warp * TILE_POINTS + lane] =
                                 decide_piece<32>(sh, warp, 0, batch0, 0, il, ax2, ay2, az2, an2, screen.half, exact);
                         }
                     } else {
                         unsigned short* halves = reinterpret_cast<unsigned short*>(sh.mask);
-                        for (int piece = warp; piece < 2 * batch_words; piece += ROW_COUNT_WARPS) {
+                        for (int piece = warp; piece < 2 * batch_words; piece += Shape::WARPS) {
                             const int half = (piece >= batch_words) ? 1 : 0;
                             const int w = piece - half * batch_words;
                             halves[2 * (w * TILE_POINTS + lane) + half] = static_cast<unsigned short>(
@@ -2642,7 +2643,7 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
                     __syncthreads();
                     // ---- indices and shifts have their say on the hits; the words go to global
                     //      memory as [tile][word][lane], the counts to the rows. A thread meets the
-                    //      same home point in all of its tasks (256 is a multiple of 32). ----
+                    //      same home point in all of its tasks (THREADS is a multiple of 32). ----
                     base_known = true;
                     base = sh.mask_base;
                     const bool fits = base != ~0ull;
@@ -2656,12 +2657,12 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
                     if (RANKED && tile == 0 && fits) {
                         // where the writing pass finds the candidates: two slots to a word
                         uint32_t* order = masks + base + static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS;
-                        for (int k = threadIdx.x; k < 16 * words; k += ROW_COUNT_THREADS) {
+                        for (int k = threadIdx.x; k < 16 * words; k += Shape::THREADS) {
                             order[k] = reinterpret_cast<const uint32_t*>(sh.order)[k];
                         }
                     }
                     int my_hits = 0;
-                    for (int task = threadIdx.x; task < batch_words * TILE_POINTS; task += ROW_COUNT_THREADS) {
+                    for (int task = threadIdx.x; task < batch_words * TILE_POINTS; task += Shape::THREADS) {
                         unsigned word = sh.mask[task];
                         unsigned kept = word;
                         const int slot0 = (task >> 5) << 5;
@@ -2718,34 +2719,43 @@ __global__ void __launch_bounds__(ROW_COUNT_THREADS, Shape::CTAS_PER_SM) row_cou
 
 constexpr int ROW_WINDOW = 128;    // hits of a row a warp lists at a time
 
-constexpr int ROW_EMIT_THREADS = 128;
 constexpr int IS_IMAGE = static_cast<int>(0x80000000u); // (31 bits index the points)
-constexpr int ROW_EMIT_WARPS = ROW_EMIT_THREADS / 32;
 
 /// Shape of the CTAs of the row-writing kernel: BATCH candidates are looked at at a time. The
 /// candidates themselves stay in L1, where a lane fetches the record of its hit: staging all of them
 /// first (40 bytes each, which left room for 4 CTAs of 8 warps) was a third of the kernel. 216k
 /// crystal 316 -> 302 us, 262k liquid 250 -> 231, its half list 208 -> 185.
+/// STAGED: they are copied to shared memory all the same, with their images worked out (see SortedRowsStaged).
 /// SEGMENTS: see setup_segments. VALUES: see store_pairs.
-template <int BATCH_, int CTAS_PER_SM_, int SEGMENTS_, int VALUES_>
+template <int BATCH_, int THREADS_, int CTAS_PER_SM_, int SEGMENTS_, int VALUES_, bool STAGED_>
 struct RowShape {
     static constexpr int SEGMENTS = SEGMENTS_;
     static constexpr int VALUES = VALUES_;
     static constexpr int BATCH = BATCH_;
+    static constexpr int THREADS = THREADS_;
+    static constexpr int WARPS = THREADS_ / 32;
     static constexpr int WORDS = BATCH_ / 32;
     static constexpr int LANE_WORDS = (WORDS + 31) / 32; // consecutive words of a row that a lane looks after
     static constexpr int CTAS_PER_SM = CTAS_PER_SM_;
+    static constexpr bool STAGED = STAGED_;
     static_assert(BATCH_ % 32 == 0 && BATCH_ <= 65536, "whole words, slots of 16 bits");
     static_assert(SEG_MAX <= 256, "segments of 8 bits");
 
+    struct InCache {
+        int position[BATCH_];          // of the candidate among the cell-sorted points; IS_IMAGE: in a shifted cell
+        unsigned char segment[BATCH_]; // the segment it comes from
+    };
+    struct InShared {
+        int4 sj[BATCH_]; // x, y, z: image minus wrap shift of the candidate; w: its index
+        double x[BATCH_], y[BATCH_], z[BATCH_];
+    };
     struct Shared {
-        alignas(16) double transpose[ROW_EMIT_WARPS][TRANSPOSE_DOUBLES / 2]; // per warp: on the way to coalesced stores
+        alignas(16) double transpose[WARPS][TRANSPOSE_DOUBLES / 2]; // per warp: on the way to coalesced stores
+        typename std::conditional<STAGED_, InShared, InCache>::type candidates;
         unsigned mask[TILE_POINTS * (WORDS + 1)]; // [home point][word], padded against bank conflicts
-        unsigned short list[ROW_EMIT_WARPS][ROW_WINDOW];
-        int position[BATCH_];           // of the candidate among the cell-sorted points; IS_IMAGE: in a shifted cell
-        unsigned char segment[BATCH_];  // the segment it comes from
+        unsigned short list[WARPS][ROW_WINDOW];
         SegmentTableT<SEGMENTS_> table;
-        int offsets[SEGMENTS_];         // of the stencil of a full-length unit
+        int offsets[(SEGMENTS_ == SEG_MAX) ? 1 : SEGMENTS_]; // of the stencil of a full-length unit
         double home_pos[3][TILE_POINTS];
         int4 home_sj[TILE_POINTS];                // x, y, z: wrap shift of the home point; w: its index
         unsigned long long home_row[TILE_POINTS]; // where the row of a home point continues
@@ -2753,8 +2763,15 @@ struct RowShape {
     static_assert((sizeof(Shared) + 1024) * CTAS_PER_SM_ <= 228 * 1024, "CTAS_PER_SM CTAs fit on an SM");
 };
 template <int SEGMENTS, int VALUES>
-using SortedRows = RowShape<1024, 8, SEGMENTS, VALUES>;
-using SortedRowsWide = RowShape<2048, 8, SEG_MAX, -1>;
+using SortedRows = RowShape<1024, 128, 8, SEGMENTS, VALUES, false>;
+/// Launches of few units (see rows_of_few_units), and units with more than 1024 candidates: 110k crystal at 7 A, writing
+/// pass with 4 warps in 8 CTAs, which leave little of the L1, 522 us, with 8 in 4 467.
+using SortedRowsWide = RowShape<2048, 256, 4, SEG_MAX, -1, false>;
+/// Few units with more candidates still, whose rows are continued from batch to batch: mostly periodic images of
+/// few points, where working out the image of a candidate for every hit costs more than a copy of all.
+/// Writing pass from the records and from copies: 64 points with 9 A 226 and 205 us, 500 with 63 000 candidates 12.7
+/// and 10.5 ms, 14k crystal at 9 A (3375 candidates) 720 and 620 us.
+using SortedRowsStaged = RowShape<1024, 256, 4, SEG_MAX, -1, true>;
 
 /// Hits [from, to) of a row whose words lie in shared memory, lane l being the one that counted the
 /// LANE_WORDS words from l * LANE_WORDS on (`begin`: hits before them): use(number, slot) for each,
@@ -2820,7 +2837,7 @@ __device__ __forceinline__ int count_row_hits(const unsigned* words, int n_words
 }
 
 template <class Shape>
-__global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit_kernel(
+__global__ void __launch_bounds__(Shape::THREADS, Shape::CTAS_PER_SM) row_emit_kernel(
     const GridPlan plan, const int32_t* __restrict__ cell_start, SortedPoints sorted, const uint32_t* __restrict__ masks,
     const unsigned long long* __restrict__ unit_mask_base, const uint32_t* __restrict__ unit_words,
     const unsigned long long* __restrict__ row_start, uint32_t* __restrict__ row_fill, PairOutput out, const int ranked, const RowLimits limits
@@ -2869,13 +2886,23 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
                 // ---- where the candidates are, in the order of their slots or of their indices ----
                 // (ranked: the only batch of the unit)
                 const auto* order = reinterpret_cast<const unsigned short*>(masks + base + static_cast<unsigned long long>(n_tiles) * words * TILE_POINTS);
-                for (int s = threadIdx.x; s < batch_slots; s += ROW_EMIT_THREADS) {
+                for (int s = threadIdx.x; s < batch_slots; s += Shape::THREADS) {
                     const int slot = ranked ? static_cast<int>(order[s]) : batch0 + s;
                     int t;
-                    const int position = static_cast<int>(record_of(slot, t));
-                    const bool image = (sh.table.image[t] << 1) != 0; // (the top bit is a flag)
-                    sh.position[s] = position | (image ? IS_IMAGE : 0);
-                    sh.segment[s] = static_cast<unsigned char>(t);
+                    const size_t position = record_of(slot, t);
+                    if constexpr (Shape::STAGED) {
+                        const LoadedRecord record = load_record(sorted, position);
+                        int r0, r1, r2;
+                        unpack_segment_image(sh.table.image[t], r0, r1, r2);
+                        sh.candidates.sj[s] = make_int4(r0 - record.s0, r1 - record.s1, r2 - record.s2, record.index);
+                        sh.candidates.x[s] = record.x;
+                        sh.candidates.y[s] = record.y;
+                        sh.candidates.z[s] = record.z;
+                    } else {
+                        const bool image = (sh.table.image[t] << 1) != 0; // (the top bit is a flag)
+                        sh.candidates.position[s] = static_cast<int>(position) | (image ? IS_IMAGE : 0);
+                        sh.candidates.segment[s] = static_cast<unsigned char>(t);
+                    }
                 }
 
                 for (int tile = 0; tile < n_tiles; tile++) {
@@ -2892,12 +2919,12 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
                     }
                     // hit words of the tile, from [word][home point] to [home point][word]
                     const uint32_t* mask_tile = masks + base + (static_cast<unsigned long long>(tile) * words + word_base + (batch0 >> 5)) * TILE_POINTS;
-                    for (int k = threadIdx.x; k < batch_words * TILE_POINTS; k += ROW_EMIT_THREADS) {
+                    for (int k = threadIdx.x; k < batch_words * TILE_POINTS; k += Shape::THREADS) {
                         sh.mask[(k & 31) * (WORDS + 1) + (k >> 5)] = mask_tile[k];
                     }
                     __syncthreads();
 
-                    for (int h = warp; h < n_in_tile; h += ROW_EMIT_WARPS) {
+                    for (int h = warp; h < n_in_tile; h += Shape::WARPS) {
                         const unsigned* row_words = sh.mask + h * (WORDS + 1);
                         int total;
                         const int begin = count_row_hits<LANE_WORDS>(row_words, batch_words, lane, total);
@@ -2920,21 +2947,35 @@ __global__ void __launch_bounds__(ROW_EMIT_THREADS, Shape::CTAS_PER_SM) row_emit
                             for (int c0 = 0; c0 < in_window; c0 += 32) {
                                 const int n_valid = min(32, in_window - c0);
                                 const int s = (lane < n_valid) ? sh.list[warp][c0 + lane] : sh.list[warp][c0];
-                                const int position = sh.position[s];
-                                const PointRecord cand = load_packed_record(sorted, static_cast<size_t>(position & ~IS_IMAGE));
+                                PointRecord cand;
                                 int s0 = 0, s1 = 0, s2 = 0;
-                                double vx, vy, vz, d2;
-                                // (most groups of a large box: no image, no wrapped point, nothing to unpack)
-                                bool shifted = __any_sync(FULL_MASK, home_wrapped || position < 0 || cand.shift != NO_WRAP) != 0;
-                                if (shifted) {
-                                    int w0, w1, w2;
-                                    unpack_wrap(sorted, static_cast<size_t>(position & ~IS_IMAGE), cand.shift, w0, w1, w2);
-                                    unpack_segment_image(sh.table.image[sh.segment[s]], s0, s1, s2);
-                                    s0 += home.x - w0;
-                                    s1 += home.y - w1;
-                                    s2 += home.z - w2;
+                                bool shifted;
+                                if constexpr (Shape::STAGED) {
+                                    const int4 sj = sh.candidates.sj[s];
+                                    cand.x = sh.candidates.x[s];
+                                    cand.y = sh.candidates.y[s];
+                                    cand.z = sh.candidates.z[s];
+                                    cand.index = sj.w;
+                                    s0 = sj.x + home.x;
+                                    s1 = sj.y + home.y;
+                                    s2 = sj.z + home.z;
                                     shifted = __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0;
+                                } else {
+                                    const int position = sh.candidates.position[s];
+                                    cand = load_packed_record(sorted, static_cast<size_t>(position & ~IS_IMAGE));
+                                    // (most groups of a large box: no image, no wrapped point, nothing to unpack)
+                                    shifted = __any_sync(FULL_MASK, home_wrapped || position < 0 || cand.shift != NO_WRAP) != 0;
+                                    if (shifted) {
+                                        int w0, w1, w2;
+                                        unpack_wrap(sorted, static_cast<size_t>(position & ~IS_IMAGE), cand.shift, w0, w1, w2);
+                                        unpack_segment_image(sh.table.image[sh.candidates.segment[s]], s0, s1, s2);
+                                        s0 += home.x - w0;
+                                        s1 += home.y - w1;
+                                        s2 += home.z - w2;
+                                        shifted = __any_sync(FULL_MASK, (s0 | s1 | s2) != 0) != 0;
+                                    }
                                 }
+                                double vx, vy, vz, d2;
                                 if (shifted) {
                                     d2 = exact_pair(plan, hx, hy, hz, cand.x, cand.y, cand.z, s0, s1, s2, vx, vy, vz);
                                 } else {
@@ -3216,11 +3257,13 @@ int pair_grid(int n_units, int per_sm) {
 
 namespace {
 template <bool FULL, int SEGMENTS>
-using RowCount = RowCountShape<FULL, false, 1024, 8, SEGMENTS>;
+using RowCount = RowCountShape<FULL, false, 1024, 128, 8, SEGMENTS>;
 template <bool FULL, int SEGMENTS>
-using RankedCount = RowCountShape<FULL, true, 1024, FULL ? 8 : 7, SEGMENTS>;
+using RankedCount = RowCountShape<FULL, true, 1024, 128, FULL ? 8 : 7, SEGMENTS>;
 template <bool FULL, int SEGMENTS>
-using RankedCountWide = RowCountShape<FULL, true, 2048, 4, SEGMENTS>;
+using RankedCountWide = RowCountShape<FULL, true, 2048, 256, 4, SEGMENTS>;
+template <bool FULL, bool RANKED>
+using RowCountFew = RowCountShape<FULL, RANKED, 1024, 256, 4, SEG_MAX>;
 constexpr int RANKED_BATCH = 1024;
 constexpr int RANKED_BATCH_WIDE = 2048;
 constexpr int ROW_BATCH = 1024;
@@ -3288,12 +3331,18 @@ void each_row_kernel(Use use) {
     of_stencil(std::integral_constant<int, 32>{});
     of_stencil(std::integral_constant<int, 64>{});
     of_stencil(std::integral_constant<int, SEG_MAX>{});
+    const auto count = [&](auto shape) { use(shape, row_count_kernel<decltype(shape)>); };
+    count(RowCountFew<true, true>{});
+    count(RowCountFew<true, false>{});
+    count(RowCountFew<false, true>{});
+    count(RowCountFew<false, false>{});
     use(SortedRowsWide{}, row_emit_kernel<SortedRowsWide>);
+    use(SortedRowsStaged{}, row_emit_kernel<SortedRowsStaged>);
 }
 } // namespace
 
 void configure_kernels() {
-    // Only what takes more shared memory than any kernel may has to ask for it: 7 kernels of 51. Asking for
+    // Only what takes more shared memory than any kernel may has to ask for it: 8 kernels of 56. Asking for
     // all of them, for every new list, had all of them loaded by the first one (first call of a
     // process 21.0 ms, now 16.6).
     const auto allow = [](auto shape, auto kernel) {
@@ -3439,17 +3488,26 @@ void launch_scatter(
 
 void launch_count(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, uint32_t* masks, unsigned long long mask_capacity,
-    unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, int ranked_batch, cudaStream_t stream
+    unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, int ranked_batch, bool few,
+    cudaStream_t stream
 ) {
     const auto launch = [&](auto shape, auto kernel) {
         using Shape = decltype(shape);
         launch_chained(
-            kernel, pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_COUNT_THREADS, sizeof(typename Shape::Shared), stream, plan, cell_start, sorted, masks,
+            kernel, pair_grid(plan.n_units, Shape::CTAS_PER_SM), Shape::THREADS, sizeof(typename Shape::Shared), stream, plan, cell_start, sorted, masks,
             mask_capacity, unit_mask_base, unit_words, row_count, header
         );
     };
     const auto launch_kind = [&](auto full) {
         constexpr bool FULL = decltype(full)::value;
+        if (few && ranked_batch <= RANKED_BATCH) {
+            if (ranked_batch == 0) {
+                launch(RowCountFew<FULL, false>{}, row_count_kernel<RowCountFew<FULL, false>>);
+            } else {
+                launch(RowCountFew<FULL, true>{}, row_count_kernel<RowCountFew<FULL, true>>);
+            }
+            return;
+        }
         with_segments(plan, [&](auto segments) {
             constexpr int SEGMENTS = decltype(segments)::value;
             if (ranked_batch == 0) {
@@ -3471,6 +3529,28 @@ int ranked_count_batch(double candidates) {
     return (candidates <= RANKED_BATCH_WIDE) ? RANKED_BATCH_WIDE : 0;
 }
 
+/// Do the units that hold the points take at most three and a half CTAs per SM? CTAs of 8 warps, 4 per SM, then have a
+/// unit each and run it in half the time of one of 4 warps; with more units, 8 CTAs of 4 warps hide more of each
+/// other's waits. With 4 and 8 warps, writing pass of crystals at 7 A (1728 candidates), 64 units 168 and 92 us, 512 203
+/// and 160, 729 222 and 248; at 5 A (330 candidates) 512 units 39 and 33, 4913 162 and 166; deciding pass at 5 A
+/// 512 units 20.5 and 19, 4913 66 and 80.
+/// A unit as full as the fullest of the last build (0: not known, 0xffffffff: not one group) has, but for three
+/// standard deviations of a random count, its share of the candidates as home points.
+bool rows_of_few_units(const GridPlan& plan, size_t n_points, unsigned max_candidates) {
+    double units = plan.n_units;
+    if (max_candidates != 0 && max_candidates != 0xffffffffu) {
+        const double stencil_cells = (plan.pencil + 2.0 * plan.n_search[0]) * (2.0 * plan.n_search[1] + 1.0) * (2.0 * plan.n_search[2] + 1.0);
+        const double candidates = std::max(1.0, max_candidates - 3.0 * std::sqrt(static_cast<double>(max_candidates)));
+        units = std::min(units, static_cast<double>(n_points) * stencil_cells / (candidates * plan.pencil));
+    }
+    int device = 0;
+    int sms = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) {
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    }
+    return units <= 3.5 * sms;
+}
+
 int row_batch(unsigned max_candidates) {
     return (max_candidates > ROW_BATCH && max_candidates <= ROW_BATCH_WIDE) ? ROW_BATCH_WIDE : ROW_BATCH;
 }
@@ -3478,19 +3558,23 @@ int row_batch(unsigned max_candidates) {
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
     const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, unsigned max_candidates, bool ranked,
-    cudaStream_t stream, RowLimits limits
+    bool few, cudaStream_t stream, RowLimits limits
 ) {
     const auto launch = [&](auto shape, auto kernel) {
         using Shape = decltype(shape);
         // (not a link of the chain: CTAs that are scheduled while the pass before still runs crowd on the SMs that are
         // done first, and on shared memory that was divided for the other kernel. 110k crystal at 7 A, a call 787
         // us chained, 709 behind the scan; 20k liquid at 10 A 228, 200; 27k crystal at 5 A 139, 140)
-        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), ROW_EMIT_THREADS, sizeof(typename Shape::Shared), stream>>>(
+        kernel<<<pair_grid(plan.n_units, Shape::CTAS_PER_SM), Shape::THREADS, sizeof(typename Shape::Shared), stream>>>(
             plan, cell_start, sorted, masks, unit_mask_base, unit_words, row_start, row_fill, out, ranked ? 1 : 0, limits
         );
     };
-    if (row_batch(max_candidates) == ROW_BATCH_WIDE) {
+    if (max_candidates <= ROW_BATCH_WIDE && (few || max_candidates > ROW_BATCH)) {
         launch(SortedRowsWide{}, row_emit_kernel<SortedRowsWide>);
+        return;
+    }
+    if (few) {
+        launch(SortedRowsStaged{}, row_emit_kernel<SortedRowsStaged>);
         return;
     }
     with_segments(plan, [&](auto segments) {

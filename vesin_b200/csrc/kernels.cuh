@@ -262,7 +262,8 @@ void launch_scan_units(
 /// candidates than that are left out; header->max_candidates tells, and the pass has to be run again.
 void launch_count(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, uint32_t* masks, unsigned long long mask_capacity,
-    unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, int ranked_batch, cudaStream_t stream
+    unsigned long long* unit_mask_base, uint32_t* unit_words, uint32_t* row_count, DeviceHeader* header, int ranked_batch, bool few,
+    cudaStream_t stream
 );
 /// Room for the candidates of a unit in pass 1 when it ranks them (0: it can not hold as many).
 int ranked_count_batch(double candidates);
@@ -281,9 +282,11 @@ struct RowLimits {
 void launch_emit(
     const GridPlan& plan, const int32_t* cell_start, SortedPoints sorted, const uint32_t* masks, const unsigned long long* unit_mask_base,
     const uint32_t* unit_words, const unsigned long long* row_start, uint32_t* row_fill, PairOutput out, unsigned max_candidates, bool ranked,
-    cudaStream_t stream, RowLimits limits = {}
+    bool few, cudaStream_t stream, RowLimits limits = {}
 );
 int row_batch(unsigned max_candidates);
+/// `few` of both passes: are there so few units that hold points that CTAs of 8 warps serve them better?
+bool rows_of_few_units(const GridPlan& plan, size_t n_points, unsigned max_candidates);
 
 /// Sorts the pairs inside every row by (second index, shift): `in` holds rows
 /// [row_start[r], row_start[r + 1]), `out` receives the sorted rows.
