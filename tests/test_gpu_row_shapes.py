@@ -22,14 +22,14 @@ def _by_pair(values, n):
     return {name: value[order] for name, value in [("key", key), ("S", values["S"]), ("d", values["d"]), ("D", values["D"])]}
 
 
-def _check(points, box, cutoff, full, canonical, dtype="float64"):
+def _check(points, box, cutoff, full, canonical, dtype="float64", calculator=None):
     """(no pair of points has two images within the cutoff)"""
     import torch
 
     kind = getattr(torch, dtype)
     p, b = torch.tensor(points, device="cuda", dtype=kind), torch.tensor(box, device="cuda", dtype=kind)
     expected = _by_pair(vesin_b200.NeighborList(cutoff, full).compute(p, b, True, "ijSdD"), len(p))
-    calculator = vesin_b200.NeighborList(cutoff, full, sorted=True, canonical=canonical)
+    calculator = calculator or vesin_b200.NeighborList(cutoff, full, sorted=True, canonical=canonical)
     for _ in range(2):  # the second build knows how full the units are, and writes ahead
         values = calculator.compute(p, b, True, "ijSdD")
         i, j = values[0].view(torch.int64), values[1].view(torch.int64)
@@ -68,7 +68,9 @@ def test_droplets(n, cutoff, canonical, monkeypatch):
     radius = (3.0 * n / 0.1 / 4.0 / np.pi) ** (1.0 / 3.0)
     points = rng.normal(size=(n, 3))
     points *= (radius * rng.random(n) ** (1.0 / 3.0) / np.linalg.norm(points, axis=1))[:, None]
-    _check(points + 3.0 * radius, 6.0 * radius * np.eye(3), cutoff, True, canonical)
+    calculator = vesin_b200.NeighborList(cutoff, True, sorted=True, canonical=canonical)
+    for scale in (1.0, 1.0, 1.01, 1.02, 0.9):  # (a new plan for every box)
+        _check(points + 3.0 * radius, scale * 6.0 * radius * np.eye(3), cutoff, True, canonical, calculator=calculator)
 
 
 @pytest.mark.parametrize("canonical", [False, True])
