@@ -1459,9 +1459,10 @@ struct Screen {
 __device__ __forceinline__ Screen screen_of(const GridPlan& plan) {
     Screen screen;
     if (plan.cutoff2_lo > 0.0f && plan.cutoff2_hi < 1.0e30f) {
-        // (5 % more than half the band of the plan: the rounding of both numbers. A candidate is
-        // within 700 cutoffs of the centre of its unit, or the band would be wider than the cutoff:
-        // no square overflows)
+        // (5 % more than half the band of the plan: the rounding of both numbers. Squares: where the band
+        // follows the unit, home points are within 100 cutoffs, 1e17, of its centre, and a candidate so far out that
+        // its square overflows comes out infinite or not a number, no hit either way; where it follows the stencil, it is
+        // wider than the cutoff from 700 cutoffs on)
         screen.mid = 0.5f * (plan.cutoff2_lo + plan.cutoff2_hi);
         screen.half = 0.525f * (plan.cutoff2_hi - plan.cutoff2_lo);
     } else {

@@ -36,7 +36,8 @@ namespace {
 
 constexpr int SMALL_THREADS = 128;
 constexpr int SMALL_WARPS = SMALL_THREADS / 32;
-constexpr int SMALL_CTAS = 7; // per SM (72 registers; 512 cells, both passes: 6 132 us, 7 131, 8 132 with spills)
+// per SM (72 registers, and 8 to 28 bytes of spills when pairs are written; 512 cells, both passes: 6 132 us, 7 131, 8 132)
+constexpr int SMALL_CTAS = 7;
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
 struct SystemFrame {
